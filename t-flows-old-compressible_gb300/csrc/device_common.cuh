@@ -94,88 +94,33 @@ __device__ __forceinline__ void raise_abort(DevCtl* c, int status, int where) {
     atomicExch(&c->abort, 1);
 }
 
-// ---- shared-memory staging with bulk async copies --------------------------------
-// The tiled IC sweeps stream each wavefront step's record (contiguous in its
-// step-major layout) into a ring of shared-memory slots with the bulk copy
-// engine (cp.async.bulk, global -> shared), one mbarrier per slot: the
-// issuing thread announces the byte count (arrive.expect_tx), the copy
-// completes the transaction, and the consumers wait on the slot's phase
-// parity.  Sizes are multiples of 16 bytes and both addresses 16-byte
-// aligned (the host sizes the layout so).
+// ---- asynchronous copies global -> shared (per thread, in commit groups) ----------
 __device__ __forceinline__ unsigned smem_u32(const void* p) {
     return (unsigned)__cvta_generic_to_shared(p);
 }
-__device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count)
-                 : "memory");
-}
-// Makes the initialised barriers visible to the async proxy (the bulk copies).
-__device__ __forceinline__ void mbar_init_fence() {
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-                 "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned parity) {
-    unsigned ok;
+// 16 bytes through L2 only; both addresses 16-byte aligned.  (The predicates
+// of these copies are part of the instruction: a branch around each of a few
+// copies costs more than the copies.)
+__device__ __forceinline__ void cp_async16(unsigned dst, const void* src, bool p = true) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// `bytes` from global `src` into this CTA's shared `dst`, completing on `bar`.
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes,
-                                         unsigned long long* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-            "r"(smem_u32(dst)),
-        "l"(src), "r"(bytes), "r"(smem_u32(bar))
+        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t"
+        "@q cp.async.cg.shared.global [%0], [%1], 16;\n\t}" ::"r"(dst), "l"(src), "r"((unsigned)p)
         : "memory");
 }
-// Explicit shared-memory accesses at 32-bit shared addresses (the tiled
-// sweeps' ring and neighbour exchange): ld.shared / st.shared rather than
-// generic accesses, which the compiler emits when the address space of a
-// pointer carried through structures is not known and which wait on the
-// long scoreboard.  Volatile, so they stay ordered after the barrier waits.
-template <typename T> __device__ __forceinline__ T lds(unsigned a);
-template <> __device__ __forceinline__ double lds<double>(unsigned a) {
-    double v;
-    asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a));
-    return v;
+// One value of 4 or 8 bytes, naturally aligned.
+template <int BYTES>
+__device__ __forceinline__ void cp_async(unsigned dst, const void* src, bool p) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\t"
+        "@q cp.async.ca.shared.global [%0], [%1], %2;\n\t}" ::"r"(dst), "l"(src), "n"(BYTES),
+        "r"((unsigned)p)
+        : "memory");
 }
-template <> __device__ __forceinline__ float lds<float>(unsigned a) {
-    float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
-    return v;
-}
-template <> __device__ __forceinline__ unsigned short lds<unsigned short>(unsigned a) {
-    unsigned short v;
-    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ void sts(unsigned a, double v) {
-    asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
-}
-__device__ __forceinline__ void sts(unsigned a, float v) {
-    asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
-}
-
-// Orders this thread's earlier generic-proxy accesses before its later
-// async-proxy accesses: in shared memory (the block's reads of a ring slot
-// before the bulk copy that refills it; cheap, issued every step) or in
-// global memory (words written before a barrier that bulk copies read after
-// it; once per sweep or tile, as it waits for this thread's global accesses).
-__device__ __forceinline__ void fence_proxy_async_smem() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ void fence_proxy_async_global() {
-    asm volatile("fence.proxy.async.global;" ::: "memory");
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// Waits until at most N of this thread's groups are in flight.
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
 // ---- value-as-flag cells ------------------------------------------------------
@@ -249,8 +194,8 @@ struct Grid {
     int tid;  // thread index within the group of blocks solving one system
     int nt;   // threads in the group
     int bid;  // block index within the group
-    unsigned ep_f;  // forward / backward level-sweep epochs (counter targets)
-    unsigned ep_b;
+    unsigned epoch;  // tiled IC sweeps: number of the current apply
+    int chunk0;      // and this block's chunks of all sweeps so far
     int stall;      // test hook: block 0 skips its first barrier arrival
 };
 
@@ -271,8 +216,8 @@ __device__ __forceinline__ void grid_init_group(Grid& g, DevCtl* ctl, double* pa
     g.nt = nb * blockDim.x;
     g.wg = g.tid >> 5;
     g.nw = g.nt >> 5;
-    g.ep_f = 0;
-    g.ep_b = 0;
+    g.epoch = 0;
+    g.chunk0 = 0;
     g.stall = 0;
 }
 

@@ -166,6 +166,11 @@ int planned_grid(const DeviceTopology& t, const SolveRequest& rq);
 // a launch needs for them, and their step records (allocated here, so call
 // before a stream capture).
 bool tiled_ic(const DeviceTopology& t, const SolveRequest& rq);
+// Threads per block of a request that names none: 512 with the tiled sweeps
+// (four patches a block: one apply at 256^3, FP32, takes 529 us in two blocks
+// of 512 threads per SM and 582 in four of 256), else 0, the kernels' own
+// default.  A batch takes the largest.
+int default_block(const DeviceTopology& t, const SolveRequest& rq);
 unsigned tile_smem_for(const DeviceTopology& t, const SolveRequest& rq);
 cudaError_t ensure_tiles(const DeviceTopology& t, Workspace& ws, const SolveRequest& rq);
 cudaError_t run_spmv(const DeviceTopology& t, Workspace& ws, const double* x, double* y, bool fp32,

@@ -70,44 +70,35 @@ __global__ void permute_kernel(int n, const int* __restrict__ rowptr, const int*
     }
 }
 
-// Coefficient fields of the tiled IC sweeps' step records from the SELL
-// values (the same numbers the level-ordered sweeps read: FP64, FP32, or
-// BF16 bit patterns).  For the row of thread t of tile k at step s, the
-// forward record (k, s) gets its lower coefficients by neighbour (z-1, y-1,
-// x-1) and the backward record its upper ones (x+1, y+1, z+1); absent
-// neighbours and idle slots hold 0.
-template <typename L>
-__global__ void tile_permute_kernel(int nx, int ny, int nz, int ty, int ntx, int steps,
-                                    long long total, const long long* __restrict__ soff,
-                                    const int* __restrict__ meta, const L* __restrict__ sval,
-                                    unsigned char* fwd, unsigned char* bwd, unsigned rec_f,
-                                    unsigned rec_b) {
-    const int B = kTileX * ty;
+// Factor entries of the tiled IC sweeps' records from the SELL values (the
+// same numbers the level-ordered sweeps read: FP64, FP32, or BF16 bit
+// patterns): per cell the lower entries by neighbour (z-1, y-1, x-1) in the
+// forward record, the upper ones (x+1, y+1, z+1) in the backward record;
+// absent neighbours and idle lanes hold 0.
+template <typename L, typename T>
+__global__ void tile_permute_kernel(Tiles<T> tl, long long total, const long long* __restrict__ soff,
+                                    const int* __restrict__ meta, const L* __restrict__ sval) {
+    const int sp = tl.chunks * kTileK;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
-        const int t = (int)(i % B);
-        const long long ks = i / B;
-        const int s = (int)(ks % steps), k = (int)(ks / steps);
-        const int lx = t % kTileX, ly = t / kTileX;
-        const int x = (k % ntx) * kTileX + lx, y = (k / ntx) * ty + ly, z = s - lx - ly;
-        L a[6] = {L(0), L(0), L(0), L(0), L(0), L(0)};
-        if (x < nx && y < ny && z >= 0 && z < nz) {
-            const int row = x + nx * (y + ny * z);
-            const long long base = soff[row >> 5] + (row & 31);
-            int q = 0;
-            if (z > 0) a[0] = sval[base + 32LL * q++];
-            if (y > 0) a[1] = sval[base + 32LL * q++];
-            if (x > 0) a[2] = sval[base + 32LL * q++];
-            q = (meta[row] >> 16) + 1;  // first entry after the diagonal
-            if (x < nx - 1) a[3] = sval[base + 32LL * q++];
-            if (y < ny - 1) a[4] = sval[base + 32LL * q++];
-            if (z < nz - 1) a[5] = sval[base + 32LL * q++];
-        }
-        L* rf = reinterpret_cast<L*>(fwd + ks * rec_f);
-        L* rb = reinterpret_cast<L*>(bwd + ks * rec_b);
-        for (int f = 0; f < 3; ++f) {
-            rf[f * B + t] = a[f];
-            rb[f * B + t] = a[3 + f];
+        const int lane = (int)(i & 31);
+        const long long ps = i >> 5;
+        const int s = (int)(ps % sp), pt = (int)(ps / sp);
+        int x0, y0, x, y, z;
+        patch_origin(tl, pt, x0, y0);
+        for (int dir = 0; dir < 2; ++dir) {
+            L a[3] = {L(0), L(0), L(0)};
+            if (patch_cell(tl, dir, x0, y0, s, lane, x, y, z)) {
+                const int row = x + tl.nx * (y + tl.ny * z);
+                const long long base = soff[row >> 5] + (row & 31);
+                int q = dir ? (meta[row] >> 16) + 1 : 0;  // upper entries follow the diagonal
+                const bool has[3] = {dir ? x < tl.nx - 1 : z > 0, dir ? y < tl.ny - 1 : y > 0,
+                                     dir ? z < tl.nz - 1 : x > 0};
+                for (int f = 0; f < 3; ++f)
+                    if (has[f]) a[f] = sval[base + 32LL * q++];
+            }
+            unsigned char* r = tl.rec[dir] + ps * tile_rec_bytes(sizeof(L), sizeof(T));
+            for (int f = 0; f < 3; ++f) *reinterpret_cast<L*>(r + TileRec<L, T>::at(f, lane)) = a[f];
         }
     }
 }
@@ -429,18 +420,30 @@ size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 // the update pass it saves).
 bool fuse_dir_fp64(const DeviceTopology& t) { return t.n <= (1 << 19); }
 
+// Patches per tile: as many as the block has warps for, up to four, whose
+// shared memory fits an SM twice (one apply at 128^3, FP32: 190 us with four,
+// 220 with two, 240 with one: every tile edge costs a hand-over through L2).
+int tile_patches(const SolveRequest& rq) {
+    const int block = rq.block > 0 ? rq.block : kMaxBlock;
+    int sw = 1;
+    while (2 * sw <= kMaxSweepWarps && 2 * sw * kWarpsPerPatch * 32 <= block) sw *= 2;
+    return sw;
+}
+
 struct TileGeom {
-    int ty = 0, ntx = 0, nty = 0, steps = 0;
-    long long slots = 0;
+    int sw = 0, ntx = 0, nty = 0, chunks = 0;
+    size_t patches = 0, lanes = 0;  // lanes: cells of all records
 };
 
-TileGeom tile_geom(const DeviceTopology& t, int block) {
+TileGeom tile_geom(const DeviceTopology& t, const SolveRequest& rq) {
     TileGeom g;
-    g.ty = block / kTileX;
-    g.ntx = (t.box_nx + kTileX - 1) / kTileX;
-    g.nty = (t.box_ny + g.ty - 1) / g.ty;
-    g.steps = kTileX + g.ty + t.box_nz - 2;
-    g.slots = (long long)g.ntx * g.nty * g.steps * block;
+    g.sw = tile_patches(rq);
+    const int px = g.sw > 1 ? 2 : 1, tx = px * kPatchX, ty = g.sw / px * kPatchY;
+    g.ntx = (t.box_nx + tx - 1) / tx;
+    g.nty = (t.box_ny + ty - 1) / ty;
+    g.chunks = (t.box_nz + kSkew + kTileK - 1) / kTileK;
+    g.patches = (size_t)g.ntx * g.nty * g.sw;
+    g.lanes = g.patches * g.chunks * kTileK * 32;
     return g;
 }
 
@@ -455,10 +458,10 @@ void tile_elem(const SolveRequest& rq, unsigned& ls, unsigned& sv) {
     }
 }
 
-// Forward and backward records (three coefficient and at most three value
-// fields each) plus the two cell arrays.
-size_t tile_buffer_bytes(long long slots, unsigned ls, unsigned sv) {
-    return 2 * align256((size_t)slots * (3 * ls + 3 * sv)) + 2 * align256((size_t)slots * sv);
+// Forward and backward records, the middle values, the edge words of both.
+size_t tile_buffer_bytes(const DeviceTopology& t, const TileGeom& g, unsigned ls, unsigned sv) {
+    return 2 * align256(g.lanes * (3 * ls + sv)) + align256(g.lanes * sv) +
+           2 * align256(g.patches * tile_edge_words(g.chunks) * tile_edge_bytes(sv));
 }
 
 }  // namespace
@@ -466,23 +469,27 @@ size_t tile_buffer_bytes(long long slots, unsigned ls, unsigned sv) {
 bool tiled_ic(const DeviceTopology& t, const SolveRequest& rq) {
     if (rq.prec != 2 || rq.ic_sweeps > 0 || t.box_nx <= 0 || rq.ic_tiled == 0) return false;
     if (rq.ic_tiled < 0 && !tiles_env_on()) return false;
-    const int B = rq.block > 0 ? rq.block : kBlock;
-    return B % 32 == 0 && B >= 64 && B <= kMaxBlock;
+    // (a patch takes four warps; smaller blocks run the level sweeps)
+    return rq.block == 0 || rq.block >= 32 * kWarpsPerPatch;
+}
+
+int default_block(const DeviceTopology& t, const SolveRequest& rq) {
+    return rq.block > 0 ? rq.block : (tiled_ic(t, rq) ? kMaxBlock : 0);
 }
 
 unsigned tile_smem_for(const DeviceTopology& t, const SolveRequest& rq) {
     if (!tiled_ic(t, rq)) return 0;
     unsigned ls, sv;
     tile_elem(rq, ls, sv);
-    return tile_smem_bytes(rq.block > 0 ? rq.block : kBlock, ls, sv);
+    return tile_smem_bytes(tile_patches(rq), ls, sv);
 }
 
 cudaError_t ensure_tiles(const DeviceTopology& t, Workspace& ws, const SolveRequest& rq) {
     if (!tiled_ic(t, rq)) return cudaSuccess;
-    const TileGeom tg = tile_geom(t, rq.block > 0 ? rq.block : kBlock);
+    const TileGeom tg = tile_geom(t, rq);
     const bool mixed = rq.precision == 1;
     // the FP32 buffer is sized for FP32 coefficients, which covers BF16 ones
-    const size_t need = mixed ? tile_buffer_bytes(tg.slots, 4, 4) : tile_buffer_bytes(tg.slots, 8, 8);
+    const size_t need = mixed ? tile_buffer_bytes(t, tg, 4, 4) : tile_buffer_bytes(t, tg, 8, 8);
     unsigned char*& buf = mixed ? ws.tile32 : ws.tile64;
     size_t& cap = mixed ? ws.tile_cap32 : ws.tile_cap64;
     if (need <= cap) return cudaSuccess;
@@ -506,34 +513,28 @@ cudaError_t fill_tiles(const DeviceTopology& t, Workspace& ws, const SolveReques
     if (!tiled_ic(t, rq)) return cudaSuccess;
     cudaError_t e = ensure_tiles(t, ws, rq);
     if (e != cudaSuccess) return e;
-    const int B = rq.block > 0 ? rq.block : kBlock;
-    const TileGeom tg = tile_geom(t, B);
+    const TileGeom tg = tile_geom(t, rq);
     unsigned char* p = sizeof(T) == 8 ? ws.tile64 : ws.tile32;
-    // the contracted FP64 build multiplies by 1/(D+TINY) in the middle step
-    const int recip = sizeof(T) == 8 && rq.precision == 2 ? 1 : 0;
-    const unsigned ls = sizeof(L), sv = sizeof(T);
-    const size_t recs = align256((size_t)tg.slots * (3 * ls + 3 * sv));
+    auto take = [&p](size_t bytes) {
+        unsigned char* q = p;
+        p += align256(bytes);
+        return q;
+    };
     tl.on = 1;
     tl.nx = t.box_nx;
     tl.ny = t.box_ny;
     tl.nz = t.box_nz;
-    tl.ty = tg.ty;
+    tl.sw = tg.sw;
     tl.ntx = tg.ntx;
     tl.nty = tg.nty;
-    tl.steps = tg.steps;
+    tl.chunks = tg.chunks;
     tl.lu_bf16 = sizeof(L) == 2 ? 1 : 0;
-    tl.recip = recip;
-    tl.half = tile_half(B, ls, sv);
-    tl.rec_f = B * (3 * ls + (recip ? 3 : 2) * sv);
-    tl.rec_b = B * (3 * ls + 3 * sv);
-    tl.fwd = p;
-    tl.bwd = p + recs;
-    tl.wt = reinterpret_cast<T*>(p + 2 * recs);
-    tl.zt = reinterpret_cast<T*>(p + 2 * recs + align256((size_t)tg.slots * sv));
-    const int nb = (int)std::min<long long>(std::max<long long>(1, (tg.slots + 255) / 256), sms() * 16LL);
-    tile_permute_kernel<L><<<nb, 256, 0, s>>>(t.box_nx, t.box_ny, t.box_nz, tg.ty, tg.ntx, tg.steps,
-                                              tg.slots, t.soff, t.meta, sval, tl.fwd, tl.bwd,
-                                              tl.rec_f, tl.rec_b);
+    for (int dir = 0; dir < 2; ++dir) tl.rec[dir] = take(tg.lanes * (3 * sizeof(L) + sizeof(T)));
+    tl.mid = reinterpret_cast<T*>(take(tg.lanes * sizeof(T)));
+    for (int dir = 0; dir < 2; ++dir)
+        tl.edge[dir] = take(tg.patches * tile_edge_words(tg.chunks) * tile_edge_bytes(sizeof(T)));
+    const int nb = (int)std::min<long long>(std::max<long long>(1, (long long)(tg.lanes / 256)), sms() * 16LL);
+    tile_permute_kernel<L, T><<<nb, 256, 0, s>>>(tl, (long long)tg.lanes, t.soff, t.meta, sval);
     return cudaGetLastError();
 }
 

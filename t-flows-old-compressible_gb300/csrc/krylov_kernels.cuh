@@ -28,6 +28,8 @@
 
 #include "device_common.cuh"
 
+#include <type_traits>
+
 namespace tflows {
 
 constexpr double kTiny = 1.0e-64;  // Library/allp_mod.f90:31
@@ -43,63 +45,64 @@ __device__ __forceinline__ T tiny_v() {
 enum : int { SLOT_A = 0, SLOT_B = 4, SLOT_C = 8, SLOT_D = 12, NUM_SLOTS = 16 };
 
 // Tiled IC(0) sweeps on a box-numbered pattern (row = x + nx (y + ny z),
-// 7-point stencil in TopolM order).  Each block owns tiles of 16 x ty
-// columns (ty = block size / 16) that run through all z; its threads walk
-// their columns along the wavefront step s = lx + ly + z.  Everything a step
-// reads sits in one contiguous record per (tile, step), fields of `block`
-// entries each, so one bulk copy stages it:
-//   forward record:  lower coefficients (z-1, y-1, x-1) | D | rhs | [1/(D+TINY)]
-//   backward record: upper coefficients (x+1, y+1, z+1) | D | mid | rhs
-// (mid = w / (D + TINY), written by the forward sweep; the reciprocal field
-// exists only where the forward sweep multiplies by it: the contracted FP64
-// build).  The cells of slot (k, s, t) = (k * steps + s) * block + t carry
-// the results a neighbouring tile reads.
-constexpr int kTileX = 16;     // tile width in x (columns per tile row)
-// The staged records form two halves of `half` steps each: one bulk copy
-// fills a half while the block works through the other.  The ring takes at
-// most kTileRingBytes of shared memory (so four 256-thread blocks still fit
-// on an SM) and a half at most kTileHalfMax steps.
-constexpr unsigned kTileRingBytes = 48u * 1024u;
-constexpr int kTileHalfMax = 4;
+// 7-point stencil in TopolM order).  A warp owns a patch of 8 x 4 columns of
+// the box over all z, one column per lane, and walks the wavefront: at step s
+// lane (mx, my) solves the cell z = s - mx - my of its column.  A tile is the
+// patches of one block, at most two of them side by side in x.
+// What a step reads -- the three factor entries and the pivot of 32 cells --
+// is one contiguous record of the patch, records in step order.  The backward
+// sweep runs the same code in mirrored coordinates (x, y, z and the lanes
+// counted from the far end), with its own records.  Each sweeping warp has
+// three more warps: one stages what it reads, one fetches its edges from
+// other blocks, one drains what it writes.
+constexpr int kPatchX = 8, kPatchY = 4;          // columns of a patch
+constexpr int kSkew = kPatchX + kPatchY - 2;     // steps a patch takes beyond nz
+constexpr int kTileK = 4;                        // steps per chunk (staging and hand-off unit)
+constexpr int kRing = 32;                        // steps of the per-warp ring (power of two)
+constexpr int kRowS = kPatchX + 1;               // elements of a ring slot: a column and
+constexpr int kSlot = kRowS * (kPatchY + 1);     // a row more than the patch
+constexpr int kWarpsPerPatch = 4;
+constexpr int kMaxSweepWarps = 4;
+
+// Chunks of records staged per patch, the one in use included.  Two more
+// cover an L2 miss at FP64 step times; the BF16 records are small enough for
+// a fourth within two blocks per SM.
+__host__ __device__ constexpr int tile_stages(unsigned coef_bytes) { return coef_bytes == 2 ? 4 : 3; }
 
 template <typename T>
 struct Tiles {
-    int on;                 // 1: IC applies of this solve run the tiled sweeps
-    int nx, ny, nz;         // box dimensions
-    int ty;                 // tile height in y (block size / 16)
-    int ntx, nty;           // tiles along x and y
-    int steps;              // wavefront steps per tile: 16 + ty + nz - 2
-    int lu_bf16;            // coefficients stored as BF16 bit patterns (FP32 solves)
-    int recip;              // forward: mid = w * (1/(D+TINY)) instead of w / (D+TINY)
-    int half;               // steps per ring half (tile_half)
-    unsigned rec_f, rec_b;  // bytes of one forward / backward record
-    unsigned char* fwd;     // [tile][step] forward records
-    unsigned char* bwd;     // [tile][step] backward records
-    T* wt;                  // forward results by slot (value-as-flag cells)
-    T* zt;                  // backward results by slot (value-as-flag cells)
+    int on;            // 1: IC applies of this solve run the tiled sweeps
+    int nx, ny, nz;    // box dimensions
+    int sw;            // sweeping warps per block = patches per tile (1, 2 or 4)
+    int ntx, nty;      // tiles along x and y
+    int chunks;        // ceil((nz + kSkew) / kTileK)
+    int lu_bf16;       // factor entries stored as BF16 bit patterns (FP32 solves)
+    unsigned char* rec[2];   // forward / backward records, [patch][step]
+    T* mid;                  // what the backward sweep starts from, [patch][step][lane]
+    unsigned char* edge[2];  // forward / backward edge words, [patch][tile_edge_words]
 };
 
-// Bytes of one ring slot (the larger record: three coefficients and three
-// value fields), rounded to 128; steps per ring half; and the whole dynamic
-// shared-memory block of a tiled solve (barriers and flags, the ring, the
-// neighbour exchange).
-__host__ __device__ constexpr unsigned tile_slot_bytes(unsigned block, unsigned coef_bytes,
-                                                       unsigned val_bytes) {
-    return (block * (3 * coef_bytes + 3 * val_bytes) + 127u) / 128u * 128u;
+// Edge words of a patch: per step of the reading patch its four edge cells
+// along x, then the eight along y.
+__host__ __device__ constexpr unsigned tile_edge_words(int chunks) {
+    return (unsigned)chunks * kTileK * (kPatchX + kPatchY);
 }
-__host__ __device__ constexpr int tile_half(unsigned block, unsigned coef_bytes, unsigned val_bytes) {
-    return kTileRingBytes / (2u * tile_slot_bytes(block, coef_bytes, val_bytes)) < 1u
-               ? 1
-               : (kTileRingBytes / (2u * tile_slot_bytes(block, coef_bytes, val_bytes)) >
-                          (unsigned)kTileHalfMax
-                      ? kTileHalfMax
-                      : (int)(kTileRingBytes / (2u * tile_slot_bytes(block, coef_bytes, val_bytes))));
+
+// Bytes of one record: three factor entries and the pivot of 32 cells.
+__host__ __device__ constexpr unsigned tile_rec_bytes(unsigned coef_bytes, unsigned val_bytes) {
+    return 32u * (3u * coef_bytes + val_bytes);
 }
-__host__ __device__ constexpr unsigned tile_smem_bytes(unsigned block, unsigned coef_bytes,
-                                                       unsigned val_bytes) {
-    return 128u + 2u * tile_half(block, coef_bytes, val_bytes) *
-                      tile_slot_bytes(block, coef_bytes, val_bytes) +
-           2u * block * val_bytes;
+// An edge word: the value and the epoch it belongs to, 8 bytes per 32 bits of value.
+__host__ __device__ constexpr unsigned tile_edge_bytes(unsigned val_bytes) { return 2u * val_bytes; }
+// Shared memory of one sweeping warp: the ring, the staged records, the
+// staged middle values.  Ring slot s holds what the lanes compute at step s,
+// and the column and the row of the patches before it that step s + 1 reads.
+__host__ __device__ constexpr unsigned tile_warp_smem(unsigned coef_bytes, unsigned val_bytes) {
+    return kRing * kSlot * val_bytes +
+           tile_stages(coef_bytes) * kTileK * (tile_rec_bytes(coef_bytes, val_bytes) + 32u * val_bytes);
+}
+__host__ __device__ constexpr unsigned tile_smem_bytes(int sw, unsigned coef_bytes, unsigned val_bytes) {
+    return 128u + sw * tile_warp_smem(coef_bytes, val_bytes);
 }
 
 template <typename T>
@@ -765,452 +768,565 @@ __device__ bool ic_jacobi_apply(Grid& g, const Mat<T>& m, const T* D, const T* r
 
 // ---- tiled IC(0) sweeps (box-numbered patterns) --------------------------------
 // Forward: row (x, y, z) needs (x, y, z-1), (x, y-1, z), (x-1, y, z), in the
-// stored order of its lower entries (columns ascending, CG.f90:135-142).
-// Thread (lx, ly) of a tile walks its column: at step s it computes the row
-// with z = s - lx - ly.  Its z-1 input is its own result of step s-1, its
-// y-1 and x-1 inputs are the results of threads (lx, ly-1) and (lx-1, ly)
-// at step s-1, exchanged through shared memory with one block barrier per
-// step -- or, on the tile's low edges, the cells of the neighbouring tiles,
-// which run the same steps ahead of this one (tiles are taken in increasing
-// index, each depending only on lower ones, all blocks resident, so the
-// sweep cannot deadlock).  Backward mirrors it (x+1, y+1, z+1; tiles and
-// steps in decreasing order).  Each row combines the same operands in the
-// same order as the sequential sweep (CG.f90:135-156), so in the
-// reference-arithmetic build the result is bit-identical to it and to the
-// level-ordered sweeps.
+// stored order of its lower entries (columns ascending, CG.f90:135-142).  The
+// first is the lane's own last result, the other two lie in the step before
+// of the patch's ring in shared memory, one lane or one row before; the
+// ring's edge column and row belong to the patches beside it.  Backward mirrors it (x+1, y+1,
+// z+1).  Each row combines the same operands in the same order as the
+// sequential sweep (CG.f90:135-156), so in the reference-arithmetic build the
+// result is bit-identical to it and to the level-ordered sweeps.
 //
-// The records are staged into a ring of two halves of `half` consecutive
-// steps each; one bulk async copy (one elected thread, one mbarrier per half)
-// fills a half while the block works through the other, so the issue cost is
-// paid once per `half` steps.  The right-hand side enters the forward records
-// through a gather each block runs for its own tiles before their first
-// step; the neighbour tiles' edge cells are loaded two steps ahead and
-// polled again only if they were not ready yet.
+// The sweep is a chain of nx + ny + nz - 2 dependent cells, so the time of a
+// step, not its bytes, bounds it.  Hence one warp per patch with no block
+// barrier inside the sweep, and nothing but the cells' own arithmetic in that
+// warp: per step it loads a record, the right-hand side and two neighbours
+// from shared memory, at constant offsets from one ring position per chunk,
+// and stores the result there, for its own next step and for the patches
+// after it; cells outside the box compute 0, and chunks inside it skip the
+// test.  Everything else is done by three more warps per patch: one stages
+// records, right-hand side and middle values with asynchronous copies
+// `tile_stages` chunks deep, one fetches the edges from other blocks, one
+// drains the results, in z slabs that all lanes touch at the same z
+// (coalesced), and publishes the edges for other blocks.  The warps hand over
+// once per chunk of kTileK steps through progress counters in shared memory.
+// Each of these loops is one warp's instruction latency, so they test with
+// predicates rather than branches, and patches and chunks inside the box take
+// paths without tests.  Edges between blocks are words in
+// global memory that carry value and epoch in one 8-byte store, so that no
+// fence and no reset is needed; a reader loads the words of the chunks ahead
+// and polls (bounded) only those that were not there yet.
+//
+// Tiles are taken in increasing index forward and decreasing backward, each
+// depending only on tiles before it, and all blocks are resident, so no
+// sweep can deadlock; the backward sweep of a tile needs the forward sweep of
+// that tile only, which the same warps ran, so no grid barrier separates the
+// two.
 
-struct TileSmem {
-    unsigned long long* bar;  // two barriers, one per ring half
-    volatile int* fail;       // set by a thread whose wait gave up
-    int* phase;               // the halves' phase parities between sweeps
-    unsigned char* ring;      // two halves of `half` records (at most tile_slot_bytes each)
-    unsigned slot;            // bytes of the largest record
+// Edge words: relaxed 8-byte stores and loads at gpu scope, predicated.
+__device__ __forceinline__ void st_word(unsigned char* p, unsigned long long w, bool on) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.relaxed.gpu.global.u64 [%0], %1;\n\t}" ::"l"(p),
+        "l"(w), "r"((unsigned)on)
+        : "memory");
+}
+__device__ __forceinline__ void ld_word(const unsigned char* p, unsigned long long& w, bool on) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.relaxed.gpu.global.u64 %0, [%1];\n\t}"
+        : "+l"(w)
+        : "l"(p), "r"((unsigned)on)
+        : "memory");
+}
+template <typename T> struct EdgeWord;
+template <> struct EdgeWord<float> {
+    unsigned long long w = 0;
+    __device__ static void store(unsigned char* p, float v, unsigned epoch, bool on) {
+        st_word(p, (unsigned long long)__float_as_uint(v) << 32 | epoch, on);
+    }
+    __device__ void load(const unsigned char* p, bool on) { ld_word(p, w, on); }
+    __device__ bool ready(unsigned epoch) const { return (unsigned)w == epoch; }
+    __device__ float value() const { return __uint_as_float((unsigned)(w >> 32)); }
+};
+template <> struct EdgeWord<double> {
+    unsigned long long h = 0, l = 0;
+    __device__ static void store(unsigned char* p, double v, unsigned epoch, bool on) {
+        const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+        st_word(p, (b & 0xffffffff00000000ull) | epoch, on);
+        st_word(p + 8, b << 32 | epoch, on);
+    }
+    __device__ void load(const unsigned char* p, bool on) {
+        ld_word(p, h, on);
+        ld_word(p + 8, l, on);
+    }
+    __device__ bool ready(unsigned epoch) const {
+        return (unsigned)h == epoch && (unsigned)l == epoch;
+    }
+    __device__ double value() const {
+        return __longlong_as_double((long long)((h & 0xffffffff00000000ull) | l >> 32));
+    }
 };
 
+// Record of one step for one lane: factor entries a[0..2] and the pivot d.
+template <typename L, typename T> struct TileRec {  // FP32 / FP64 entries
+    T a[3], d;
+    __device__ __forceinline__ void load(const unsigned char* r, int lane) {
+        if constexpr (sizeof(T) == 4) {
+            const float4 v = reinterpret_cast<const float4*>(r)[lane];
+            a[0] = v.x; a[1] = v.y; a[2] = v.z; d = v.w;
+        } else {
+            const double2 u = reinterpret_cast<const double2*>(r)[lane];
+            const double2 v = reinterpret_cast<const double2*>(r + 512)[lane];
+            a[0] = u.x; a[1] = u.y; a[2] = v.x; d = v.y;
+        }
+    }
+    // where entry f (3: the pivot) of lane's cell sits in a record
+    __host__ __device__ static constexpr unsigned at(int f, int lane) {
+        return sizeof(T) == 4 ? 16u * lane + 4u * f : (f & 2 ? 512u : 0u) + 16u * lane + 8u * (f & 1);
+    }
+};
+template <> struct TileRec<unsigned short, float> {  // BF16 entries, FP32 pivot
+    float a[3], d;
+    __device__ __forceinline__ void load(const unsigned char* r, int lane) {
+        const uint2 v = reinterpret_cast<const uint2*>(r)[lane];
+        const unsigned w = reinterpret_cast<const unsigned short*>(r + 256)[lane];
+        a[0] = __uint_as_float(v.x << 16);
+        a[1] = __uint_as_float(v.x & 0xffff0000u);
+        a[2] = __uint_as_float(w << 16);
+        d = __uint_as_float(v.y);
+    }
+    __host__ __device__ static constexpr unsigned at(int f, int lane) {
+        return f == 3 ? 8u * lane + 4u : f == 2 ? 256u + 2u * lane : 8u * lane + 2u * f;
+    }
+};
+
+// The contracted FP64 build scales the factor entries by the row's pivot, so
+// that a step's chain is two multiply-adds instead of three and a product
+// (an FP64 operation takes about 80 cycles here): forward w = D f - sum (D a)
+// w, backward z = w - sum (D a) z, w itself being D times the middle value.
+template <typename T> constexpr bool kScaledRec = sizeof(T) == 8 && kRecipDiag64;
+
+// Patch `pt` of the tile grid (patch order within a tile: x first).
 template <typename T>
-__device__ __forceinline__ TileSmem tile_smem(const Tiles<T>& tl) {
+__device__ __forceinline__ void patch_origin(const Tiles<T>& tl, int pt, int& x0, int& y0) {
+    const int k = pt / tl.sw, w = pt % tl.sw, px = tl.sw > 1 ? 2 : 1;
+    x0 = (px * (k % tl.ntx) + w % px) * kPatchX;
+    y0 = (tl.sw / px * (k / tl.ntx) + w / px) * kPatchY;
+}
+
+// The cell of lane `lane` of a patch at step s in direction `dir`; false
+// where there is none.
+template <typename T>
+__device__ __forceinline__ bool patch_cell(const Tiles<T>& tl, int dir, int x0, int y0, int s,
+                                           int lane, int& x, int& y, int& z) {
+    const int mx = lane % kPatchX, my = lane / kPatchX;
+    z = s - mx - my;
+    x = x0 + (dir ? kPatchX - 1 - mx : mx);
+    y = y0 + (dir ? kPatchY - 1 - my : my);
+    const bool in = x < tl.nx && y < tl.ny && z >= 0 && z < tl.nz;
+    if (dir) z = tl.nz - 1 - z;
+    return in;
+}
+
+// Once per solve, before the first apply (a grid barrier must follow): the
+// pivots into both record kinds, epoch 0 into every edge word, the block's
+// progress counters cleared.
+template <typename T>
+__device__ void tiles_init(Grid& g, const Mat<T>& m, const T* __restrict__ D) {
+    const Tiles<T>& tl = m.tile;
     extern __shared__ __align__(128) unsigned char tf_smem[];
-    TileSmem m;
-    m.bar = reinterpret_cast<unsigned long long*>(tf_smem);
-    m.fail = reinterpret_cast<volatile int*>(tf_smem + 64);
-    m.phase = reinterpret_cast<int*>(tf_smem + 68);
-    m.ring = tf_smem + 128;
-    m.slot = tile_slot_bytes(blockDim.x, tl.lu_bf16 ? 2u : (unsigned)sizeof(T), (unsigned)sizeof(T));
-    return m;
-}
-
-// Byte offset of value field v (0 = D, 1 = rhs / mid, 2 = 1/(D+TINY) / rhs)
-// in a record, after the three coefficient fields.
-template <typename T>
-__device__ __forceinline__ unsigned tile_vfield(const Tiles<T>& tl, int v) {
-    return blockDim.x * (3u * (tl.lu_bf16 ? 2u : (unsigned)sizeof(T)) + v * (unsigned)sizeof(T));
-}
-
-// Coefficient f of thread t in a staged record.
-template <typename T>
-__device__ __forceinline__ T tile_coef(const Tiles<T>& tl, const unsigned char* rec, int f, int t) {
-    if constexpr (sizeof(T) == 4) {
-        if (tl.lu_bf16) {
-            const unsigned short u =
-                reinterpret_cast<const unsigned short*>(rec + (size_t)f * blockDim.x * 2)[t];
-            return __uint_as_float((unsigned)u << 16);
+    const unsigned cb = tl.lu_bf16 ? 2u : (unsigned)sizeof(T);
+    const unsigned rec = tile_rec_bytes(cb, sizeof(T));
+    const int sp = tl.chunks * kTileK, patches = tl.ntx * tl.nty * tl.sw;
+    const long long total = (long long)patches * sp * 32;
+    for (long long i = g.tid; i < total; i += g.nt) {
+        const int lane = (int)(i & 31);
+        const long long ps = i >> 5;
+        const int s = (int)(ps % sp), pt = (int)(ps / sp);
+        int x0, y0, x, y, z;
+        patch_origin(tl, pt, x0, y0);
+        for (int dir = 0; dir < 2; ++dir) {
+            const bool in = patch_cell(tl, dir, x0, y0, s, lane, x, y, z);
+            const unsigned at = cb == sizeof(T) ? TileRec<T, T>::at(3, lane)
+                                                : TileRec<unsigned short, float>::at(3, lane);
+            const T d = in ? D[x + tl.nx * (y + tl.ny * z)] : T(0);
+            unsigned char* const r = tl.rec[dir] + ps * rec;
+            *reinterpret_cast<T*>(r + at) = d;
+            if constexpr (kScaledRec<T>)
+                for (int f = 0; f < 3; ++f) *reinterpret_cast<T*>(r + TileRec<T, T>::at(f, lane)) *= d;
         }
     }
-    return reinterpret_cast<const T*>(rec + (size_t)f * blockDim.x * sizeof(T))[t];
+    const long long words = (long long)patches * tile_edge_words(tl.chunks) * (sizeof(T) / 4);
+    for (int dir = 0; dir < 2; ++dir)
+        for (long long i = g.tid; i < words; i += g.nt)
+            reinterpret_cast<unsigned long long*>(tl.edge[dir])[i] = 0ull;
+    if (threadIdx.x < kWarpsPerPatch * kMaxSweepWarps) reinterpret_cast<int*>(tf_smem)[threadIdx.x] = 0;
+    g.epoch = 0;
+    g.chunk0 = 0;
+    __syncthreads();
 }
 
-// The same for a record staged in shared memory, at shared address `rec`.
-template <typename T>
-__device__ __forceinline__ T tile_coef_s(const Tiles<T>& tl, unsigned rec, int f, int t) {
-    if constexpr (sizeof(T) == 4) {
-        if (tl.lu_bf16)
-            return __uint_as_float((unsigned)lds<unsigned short>(rec + (f * blockDim.x + t) * 2u)
-                                   << 16);
-    }
-    return lds<T>(rec + (f * blockDim.x + t) * (unsigned)sizeof(T));
+// Progress counters in shared memory: chunks done, over all sweeps.
+__device__ __forceinline__ int progress_load(unsigned a) {
+    int v;
+    asm volatile("ld.acquire.cta.shared.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+// (by lane 0, after a __syncwarp that orders the other lanes' accesses)
+__device__ __forceinline__ void progress_store(unsigned a, int v, int lane) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.eq.s32 q, %2, 0;\n\t@q st.release.cta.shared.s32 [%0], %1;\n\t}" ::"r"(a),
+        "r"(v), "r"(lane)
+        : "memory");
 }
 
-template <typename T>
-__device__ __forceinline__ T& tile_val(const Tiles<T>& tl, unsigned char* rec, int v, int t) {
-    return reinterpret_cast<T*>(rec + tile_vfield(tl, v))[t];
-}
-
-// `count` consecutive records of `rec_bytes` each (a multiple of 128) into a
-// ring half, packed as they are in global memory: one copy, completing on
-// the half's barrier.
-__device__ __forceinline__ void tile_issue(unsigned char* dst, unsigned long long* bar,
-                                           const unsigned char* rec, unsigned rec_bytes,
-                                           int count) {
-    mbar_expect_tx(bar, rec_bytes * count);
-    bulk_g2s(dst, rec, rec_bytes * count, bar);
-}
-
-// A prefetched neighbour cell, polled again (bounded) while it still holds
-// the sentinel.  On giving up: abort raised, the block's fail flag set.
-// (`ctl` and the limit `tmo` come as values: the sweeps keep everything
-// they use per step in registers.)
-template <typename T>
-__device__ __forceinline__ T tile_cell(DevCtl* ctl, long long tmo, const TileSmem& sm, const T* p,
-                                       T v, int where) {
-    using C = Cell<T>;
-    if (C::bits(v) != C::kSentinel) return v;
-    const long long t0 = clock64();
-    unsigned spins = 0;
-    while (true) {
-        const auto b = C::load(p);
-        if (b != C::kSentinel) return C::value(b);
-        if ((++spins & 63u) == 0u) {
-            const bool quit = ld_relaxed_s32(&ctl->abort) != 0;
-            if (quit || clock64() - t0 > tmo) {
-                if (!quit) raise_abort(ctl, ST_TIMEOUT, where);
-                *sm.fail = 1;
-                return T(0);
+// The bounded wait of a warp: until ok() holds on every lane.  False: the
+// launch is aborted.
+template <typename Ok>
+__device__ __forceinline__ bool tile_wait(DevCtl* ctl, long long limit, int where, Ok ok) {
+    if (!__all_sync(0xffffffffu, ok())) {
+        const long long t0 = clock64();
+        unsigned spins = 0;
+        do {
+            if ((++spins & 63u) == 0u) {
+                bool quit = ld_relaxed_s32(&ctl->abort) != 0;
+                if (!quit && clock64() - t0 > limit) {
+                    raise_abort(ctl, ST_TIMEOUT, where);
+                    quit = true;
+                }
+                if (__any_sync(0xffffffffu, quit)) return false;
             }
-        }
+        } while (!__all_sync(0xffffffffu, ok()));
     }
+    __syncwarp();
+    return true;
 }
 
-// Waits for a ring half's copy (bounded).  False: abort raised, fail set.
-__device__ __forceinline__ bool tile_wait(DevCtl* ctl, long long tmo, const TileSmem& sm, int h,
-                                          unsigned parity, int where) {
-    if (mbar_try_wait(sm.bar + h, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_try_wait(sm.bar + h, parity)) {
-        if (clock64() - t0 > tmo) {
-            raise_abort(ctl, ST_TIMEOUT, where);
-            *sm.fail = 1;
-            return false;
+// One sweep over this block's tiles, forward (BWD = 0) or backward.  Forward
+// reads rhs and writes tl.mid; backward reads tl.mid and rhs and writes zout,
+// with epi(row, z_row, rhs_row) per row.  False: a wait gave up (the launch
+// is aborted).
+template <int BWD, typename L, typename T, typename Epi>
+__device__ __forceinline__ bool tile_sweep(Grid& g, const Mat<T>& m, const T* __restrict__ rhs,
+                                           T* __restrict__ zout, Epi epi) {
+    extern __shared__ __align__(128) unsigned char tf_smem[];
+    const Tiles<T>& tl = m.tile;
+    constexpr unsigned kRec = tile_rec_bytes(sizeof(L), sizeof(T));
+    constexpr unsigned kChunkRec = kTileK * kRec;
+    constexpr int kStages = tile_stages(sizeof(L));
+    constexpr unsigned kEdge = tile_edge_bytes(sizeof(T));
+    constexpr unsigned kWarpB = tile_warp_smem(sizeof(L), sizeof(T));
+    constexpr int kDn = BWD ? -1 : 1;  // towards the patches after
+    // A ring slot is filled again 32 steps on; staging runs ahead of its chunk
+    // by the skew, draining a slab lags by it, so the drained chunk may be
+    // this many behind the one filled.
+    constexpr int kDrainLag = (kRing - kSkew) / kTileK - 1;
+    constexpr int kNever = -(1 << 20);  // an offset that any progress meets
+    const int lane = g.lane, sw = tl.sw, px = sw > 1 ? 2 : 1, swy = sw / px;
+    // roles: 0 sweeps, 1 stages, 2 drains, 3 fetches edges
+    const int wid = threadIdx.x >> 5, role = wid / sw, w = wid % sw;
+    const int ntiles = tl.ntx * tl.nty, chunks = tl.chunks, nz = tl.nz;
+    const int mine = g.bid < ntiles ? (ntiles - 1 - g.bid) / g.nblocks + 1 : 0;
+    const int first = g.chunk0;
+    g.chunk0 += mine * chunks;
+    if (role >= kWarpsPerPatch) return true;
+    const unsigned prog = smem_u32(tf_smem) + 4 * w;  // chunks swept, staged, drained, fetched
+    const unsigned staged = prog + 4 * kMaxSweepWarps, drained = staged + 4 * kMaxSweepWarps,
+                   fetched = drained + 4 * kMaxSweepWarps;
+    T* const ring = reinterpret_cast<T*>(tf_smem + 128 + w * kWarpB);
+    unsigned char* const s_rec = tf_smem + 128 + w * kWarpB + kRing * kSlot * sizeof(T);
+    T* const s_mid = reinterpret_cast<T*>(s_rec + kStages * kChunkRec) + lane;
+    const int mx = lane % kPatchX, my = lane / kPatchX, skew = mx + my;
+    T* const own = ring + (my + 1) * kRowS + mx + 1;  // this lane's cell in slot 0
+    for (int q = 0; q < mine; ++q) {
+        const int base = first + q * chunks;
+        const int k = g.bid + (BWD ? mine - 1 - q : q) * g.nblocks;
+        const int tx = k % tl.ntx, ty = k / tl.ntx, wx = w % px, wy = w / px;
+        const int x0 = (px * tx + wx) * kPatchX, y0 = (swy * ty + wy) * kPatchY;
+        if (x0 >= tl.nx || y0 >= tl.ny) {  // no such patch: nothing to hand over
+            progress_store(prog + 4 * kMaxSweepWarps * role, base + chunks, lane);
+            continue;
+        }
+        // the patches before (up) and after (dn) this one along x and y:
+        // 0 none, 1 in this block, 2 in another block
+        const int hi_x = x0 + kPatchX < tl.nx ? (wx < px - 1 ? 1 : 2) : 0;
+        const int lo_x = wx > 0 ? 1 : (tx > 0 ? 2 : 0);
+        const int hi_y = y0 + kPatchY < tl.ny ? (wy < swy - 1 ? 1 : 2) : 0;
+        const int lo_y = wy > 0 ? 1 : (ty > 0 ? 2 : 0);
+        const int up_x = BWD ? hi_x : lo_x, up_y = BWD ? hi_y : lo_y;
+        const int dn_x = BWD ? lo_x : hi_x, dn_y = BWD ? lo_y : hi_y;
+        const bool far = up_x == 2 || up_y == 2;
+        const int x = x0 + (BWD ? kPatchX - 1 - mx : mx), y = y0 + (BWD ? kPatchY - 1 - my : my);
+        const bool whole = x0 + kPatchX <= tl.nx && y0 + kPatchY <= tl.ny;
+        const unsigned nzl = x < tl.nx && y < tl.ny ? nz : 0;  // this lane's cells: z in [0, nzl)
+        unsigned pos = (unsigned)base * kTileK & (kRing - 1);  // first slot of the chunk
+        int st = base % kStages;                               // its stage
+        if (role == 0) {
+            // ---- sweeping.  Lanes 0..3 watch the neighbours in this block,
+            // lanes 4 to 6 the warps that stage, drain and fetch.  At the same
+            // z the patch before runs kPatchX steps ahead along x and kPatchY
+            // along y; the patches after may lag by what their rings hold.
+            unsigned watch = prog;
+            int off = kNever;
+            if (lane == 0 && up_x == 1) { watch = prog - 4 * (unsigned)kDn; off = (kPatchX + 2 * kTileK - 2) / kTileK; }
+            if (lane == 1 && up_y == 1) { watch = prog - 4 * (unsigned)(px * kDn); off = (kPatchY + 2 * kTileK - 2) / kTileK; }
+            if (lane == 2 && dn_x == 1) { watch = prog + 4 * (unsigned)kDn; off = -(kRing / kTileK - 1); }
+            if (lane == 3 && dn_y == 1) { watch = prog + 4 * (unsigned)(px * kDn); off = -(kRing / kTileK - 1); }
+            if (lane == 4) { watch = staged; off = 1; }
+            if (lane == 5) { watch = drained; off = -kDrainLag; }
+            if (lane == 6 && far) { watch = fetched; off = 1; }
+            // edge cells go into the edge column / row of the patch after, 8 /
+            // 4 slots back; the other lanes store their own cell again
+            const bool give_x = dn_x == 1 && mx == kPatchX - 1, give_y = dn_y == 1 && my == kPatchY - 1;
+            T* const to_x = give_x ? own + kDn * (int)(kWarpB / sizeof(T)) - kPatchX : own;
+            T* const to_y = give_y ? own + px * kDn * (int)(kWarpB / sizeof(T)) - kPatchY * kRowS : own;
+            const unsigned back_x = give_x ? kPatchX : 0, back_y = give_y ? kPatchY : 0;
+            T prev = T(0);
+            for (int c = 0; c < chunks; ++c) {
+                const int target = base + min(c + off, chunks);
+                if (!tile_wait(g.ctl, g.timeout_cyc, BWD ? 28 : 26,
+                               [&] { return progress_load(watch) - target >= 0; }))
+                    return false;
+                const unsigned char* const rc = s_rec + st * kChunkRec;
+                const T* const mc = s_mid + st * (kTileK * 32);
+                T* const cur = own + pos * kSlot;
+                const T* const before = own + ((pos - 1) & (kRing - 1)) * kSlot;
+                T* const gx = to_x + ((pos - back_x) & (kRing - 1)) * kSlot;
+                T* const gy = to_y + ((pos - back_y) & (kRing - 1)) * kSlot;
+                auto steps = [&](auto all_inside) {
+                    TileRec<L, T> r[kTileK];
+                    T f[kTileK];
+#pragma unroll
+                    for (int u = 0; u < kTileK; ++u) {
+                        r[u].load(rc + u * kRec, lane);
+                        f[u] = BWD ? mc[u * 32] : cur[u * kSlot];
+                        if (!BWD && kScaledRec<T>) f[u] = f[u] * r[u].d;
+                    }
+#pragma unroll
+                    for (int u = 0; u < kTileK; ++u) {
+                        // absent neighbours have entry 0 and value 0
+                        const T* const nb = u == 0 ? before : cur + (u - 1) * kSlot;
+                        const T vx = nb[-1], vy = nb[-kRowS];
+                        T v;
+                        if (kScaledRec<T>) {
+                            v = f[u] - r[u].a[BWD ? 2 : 0] * prev;
+                            v = v - r[u].a[1] * vy;
+                            v = v - r[u].a[BWD ? 0 : 2] * vx;
+                        } else if (BWD && sizeof(T) == 4) {
+                            T a = r[u].a[2] * prev;  // the middle value is w, D times its own
+                            a = a + r[u].a[1] * vy;
+                            a = a + r[u].a[0] * vx;
+                            v = f[u] - a * r[u].d;
+                        } else {
+                            T a = f[u];
+                            a = a - r[u].a[0] * (BWD ? vx : prev);
+                            a = a - r[u].a[1] * vy;
+                            a = a - r[u].a[2] * (BWD ? prev : vx);
+                            v = a * r[u].d;
+                        }
+                        if (!decltype(all_inside)::value)
+                            v = (unsigned)(c * kTileK + u - skew) < nzl ? v : T(0);
+                        prev = v;
+                        cur[u * kSlot] = v;
+                        gx[u * kSlot] = v;
+                        gy[u * kSlot] = v;
+                        __syncwarp();
+                    }
+                };
+                if (whole && c * kTileK >= kSkew && (c + 1) * kTileK <= nz)
+                    steps(std::true_type{});
+                else
+                    steps(std::false_type{});
+                progress_store(prog, base + c + 1, lane);
+                pos = (pos + kTileK) & (kRing - 1);
+                st = st + 1 == kStages ? 0 : st + 1;
+            }
+            continue;
+        }
+        const int pt = k * sw + w;
+        const unsigned words = tile_edge_words(chunks), ywords = chunks * (kTileK * kPatchY);
+        const int nxy = tl.nx * tl.ny, zstep = BWD ? -nxy : nxy;
+        const int row0 = x + tl.nx * y + (BWD ? nxy * (nz - 1) : 0);  // z = 0 of the direction
+        T* const mid = tl.mid + (size_t)pt * chunks * kTileK * 32;
+        // Edge words: lane (xq, xe) of the first 16 has edge cell xe along x
+        // of step xq of the chunk, lane (my, mx) cell mx along y of step my.
+        const int xq = lane / kPatchY, xe = lane % kPatchY;
+        const bool row_in = lane < kTileK * kPatchY && y0 + (BWD ? kPatchY - 1 - xe : xe) < tl.ny;
+        if (role == 1) {
+            // ---- staging.  Chunk i: the records; forward four slabs of the
+            // right-hand side, each lane its own column, into the slots of
+            // their steps; backward the middle values of the steps.  kFlight
+            // chunks stay in flight behind the one handed over.
+            constexpr int kFlight = kStages - 2;
+            if (BWD && q == 0) {  // it starts from what the forward sweep drained
+                if (!tile_wait(g.ctl, g.timeout_cyc, 29, [&] { return progress_load(drained) - base >= 0; }))
+                    return false;
+            }
+            // lane 0: the stage is free; the others: the ring slots are
+            // drained (the reference's middle step also reads the pivots)
+            const unsigned watch = lane ? drained : prog;
+            const int off = !lane || (!BWD && sizeof(T) == 8 && !kRecipDiag64) ? -(kStages - 1) : -kDrainLag;
+            const unsigned char* rec_src = tl.rec[BWD] + (size_t)pt * chunks * kChunkRec + lane * 16;
+            const T* src = BWD ? mid + (nz + kSkew - 1) * 32 + (31 - lane) : rhs + row0;
+            const unsigned s_rec_a = smem_u32(s_rec) + lane * 16, s_mid_a = smem_u32(s_mid),
+                           own_a = smem_u32(own);
+            for (int i = 0; i < chunks + kFlight; ++i) {
+                if (i < chunks) {
+                    const int target = base + i + off;
+                    if (!tile_wait(g.ctl, g.timeout_cyc, BWD ? 29 : 27,
+                                   [&] { return progress_load(watch) - target >= 0; })) {
+                        cp_async_wait<0>();
+                        return false;
+                    }
+                    const unsigned d = s_rec_a + st * kChunkRec;
+#pragma unroll
+                    for (unsigned o = 0; o < kChunkRec; o += 512) {
+                        if (kChunkRec - o >= 512) cp_async16(d + o, rec_src + o);
+                        else cp_async16(d + o, rec_src + o, lane * 16 < kChunkRec - o);
+                    }
+                    rec_src += kChunkRec;
+                    if (!BWD) {
+#pragma unroll
+                        for (int u = 0; u < kTileK; ++u) {
+                            cp_async<sizeof(T)>(
+                                own_a + ((pos + u + skew) & (kRing - 1)) * (unsigned)(kSlot * sizeof(T)), src,
+                                (unsigned)(i * kTileK + u) < nzl);
+                            src += nxy;
+                        }
+                    } else {
+                        const unsigned md = s_mid_a + st * (unsigned)(kTileK * 32 * sizeof(T));
+#pragma unroll
+                        for (int u = 0; u < kTileK; ++u)
+                            cp_async<sizeof(T)>(md + u * (unsigned)(32 * sizeof(T)), src - u * 32,
+                                                (unsigned)(i * kTileK + u - skew) < nzl);
+                        src -= kTileK * 32;
+                    }
+                    // no patch before: its edge cells are 0 (step s reads slot s - 1)
+                    if (up_x == 0 && lane < kTileK * kPatchY)
+                        ring[((pos + xq - 1) & (kRing - 1)) * kSlot + (xe + 1) * kRowS] = T(0);
+                    if (up_y == 0) ring[((pos + my - 1) & (kRing - 1)) * kSlot + mx + 1] = T(0);
+                    pos = (pos + kTileK) & (kRing - 1);
+                    st = st + 1 == kStages ? 0 : st + 1;
+                }
+                cp_async_commit();
+                cp_async_wait<kFlight>();
+                __syncwarp();
+                if (i >= kFlight) progress_store(staged, base + i - kFlight + 1, lane);
+            }
+            continue;
+        }
+        if (role == 3) {
+            // ---- fetching edges from other blocks.  The words of two chunks
+            // ahead are on their way while a chunk waits for its own; two sets
+            // of registers take turns, as moving a word on would wait for it.
+            if (!far) {
+                progress_store(fetched, base + chunks, lane);
+                continue;
+            }
+            const unsigned epoch = g.epoch;
+            const bool want_x = up_x == 2 && row_in, want_y = up_y == 2 && x < tl.nx;
+            const unsigned char* const in_x =
+                tl.edge[BWD] + ((size_t)((k - kDn) * sw + w + (px - 1) * kDn) * words + lane) * kEdge;
+            const unsigned char* const in_y =
+                tl.edge[BWD] + ((size_t)((k - kDn * tl.ntx) * sw + (BWD ? wx : wx + px * (swy - 1))) * words +
+                                ywords + lane) * kEdge;
+            EdgeWord<T> ax, ay, bx, by;
+            auto has_x = [&](int c) { return want_x && (unsigned)(c * kTileK + xq - xe) < (unsigned)nz; };
+            auto has_y = [&](int c) { return want_y && (unsigned)(c * kTileK + my - mx) < (unsigned)nz; };
+            auto fetch = [&](int c, EdgeWord<T>& ex, EdgeWord<T>& ey) {
+                ex.load(in_x + c * (kTileK * kPatchY * kEdge), has_x(c));
+                ey.load(in_y + c * (kTileK * kPatchX * kEdge), has_y(c));
+            };
+            auto edges_in = [&](int c, EdgeWord<T>& ex, EdgeWord<T>& ey) {
+                const bool hx = has_x(c), hy = has_y(c);
+                const unsigned char* const cx = in_x + c * (kTileK * kPatchY * kEdge);
+                const unsigned char* const cy = in_y + c * (kTileK * kPatchX * kEdge);
+                // (the slots' last readers: the chunk before 32 steps ago)
+                const int room = base + c - (kRing / kTileK - 1);
+                bool again = false;
+                if (!tile_wait(g.ctl, g.timeout_cyc, BWD ? 29 : 27, [&] {
+                        const bool nx_ = hx && !ex.ready(epoch), ny_ = hy && !ey.ready(epoch);
+                        ex.load(cx, again && nx_);
+                        ey.load(cy, again && ny_);
+                        again = true;
+                        const bool here = (!hx || ex.ready(epoch)) && (!hy || ey.ready(epoch));
+                        return here & (progress_load(prog) - room >= 0);
+                    }))
+                    return false;
+                // step s reads its edges from slot s - 1
+                if (hx) ring[((pos + xq - 1) & (kRing - 1)) * kSlot + (xe + 1) * kRowS] = ex.value();
+                if (hy) ring[((pos + my - 1) & (kRing - 1)) * kSlot + mx + 1] = ey.value();
+                __syncwarp();
+                progress_store(fetched, base + c + 1, lane);
+                pos = (pos + kTileK) & (kRing - 1);
+                fetch(c + 2, ex, ey);
+                return true;
+            };
+            fetch(0, ax, ay);
+            fetch(1, bx, by);
+            for (int c = 0; c < chunks; ++c)
+                if (!(c & 1 ? edges_in(c, bx, by) : edges_in(c, ax, ay))) return false;
+            continue;
+        }
+        // ---- draining
+        const unsigned epoch = g.epoch;
+        unsigned char* const out_x = tl.edge[BWD] + ((size_t)pt * words + lane) * kEdge;
+        unsigned char* const out_y = out_x + (size_t)ywords * kEdge;
+        const bool far_x = dn_x == 2 && row_in, far_y = dn_y == 2 && x < tl.nx, publish_far = dn_x == 2 || dn_y == 2;
+        for (int c = 0; c < chunks; ++c) {
+            const int z0 = c * kTileK - kSkew;  // backward: first of the slabs whose last lane is done
+            const bool inside = whole && z0 >= 0 && z0 + kTileK <= nz;
+            T rpre[kTileK];  // their right-hand side
+            if (BWD) {
+                if (inside) {
+#pragma unroll
+                    for (int u = 0; u < kTileK; ++u) rpre[u] = rhs[row0 + (z0 + u) * zstep];
+                } else {
+#pragma unroll
+                    for (int u = 0; u < kTileK; ++u)
+                        rpre[u] = (unsigned)(z0 + u) < nzl ? rhs[row0 + (z0 + u) * zstep] : T(0);
+                }
+            }
+            const int target = base + c + 1;
+            if (!tile_wait(g.ctl, g.timeout_cyc, BWD ? 29 : 27,
+                           [&] { return progress_load(prog) - target >= 0; }))
+                return false;
+            if (publish_far) {
+                const int tx_ = c * kTileK + xq - (kPatchX - 1), ty_ = c * kTileK + my - (kPatchY - 1);  // the reader's steps
+                EdgeWord<T>::store(out_x + (c * kTileK - (kPatchX - 1)) * (int)(kPatchY * kEdge),
+                                   ring[(pos + (xq & (kTileK - 1))) * kSlot + (xe + 1) * kRowS + kPatchX], epoch,
+                                   far_x && (unsigned)(tx_ - xe) < (unsigned)nz);
+                EdgeWord<T>::store(out_y + (c * kTileK - (kPatchY - 1)) * (int)(kPatchX * kEdge),
+                                   ring[(pos + my) * kSlot + kPatchY * kRowS + mx + 1], epoch,
+                                   far_y && (unsigned)(ty_ - mx) < (unsigned)nz);
+            }
+            if (!BWD) {
+                // the middle step w / (D + TINY) of CG.f90:144-146 in the
+                // reference's arithmetic; the others go on from w itself
+                T* const mp = mid + c * (kTileK * 32) + lane;
+                const T* const vp = own + pos * kSlot;
+                const unsigned char* const rc = s_rec + st * kChunkRec;
+#pragma unroll
+                for (int u = 0; u < kTileK; ++u) {
+                    T v = vp[u * kSlot];
+                    if constexpr (sizeof(T) == 8 && !kRecipDiag64)
+                        v = v / (*reinterpret_cast<const T*>(rc + u * kRec + TileRec<L, T>::at(3, lane)) +
+                                 tiny_v<T>());
+                    mp[u * 32] = v;
+                }
+            } else {
+                auto flush = [&](int u) {
+                    const T v = own[((pos - kSkew + u + skew) & (kRing - 1)) * kSlot];
+                    const int row = row0 + (z0 + u) * zstep;
+                    zout[row] = v;
+                    epi(row, v, rpre[u]);
+                };
+                if (inside) {
+#pragma unroll
+                    for (int u = 0; u < kTileK; ++u) flush(u);
+                } else {
+#pragma unroll
+                    for (int u = 0; u < kTileK; ++u)
+                        if ((unsigned)(z0 + u) < nzl) flush(u);
+                }
+            }
+            __syncwarp();
+            progress_store(drained, base + c + 1, lane);
+            pos = (pos + kTileK) & (kRing - 1);
+            st = st + 1 == kStages ? 0 : st + 1;
         }
     }
     return true;
 }
 
-// After a failure: thread 0 waits (bounded) for the copies still in flight
-// into the ring (the halves issued and not yet waited for, bits of `pend`).
-__device__ __forceinline__ void tile_drain(long long tmo, const TileSmem& sm, unsigned pend,
-                                           unsigned phase) {
-    if (threadIdx.x != 0) return;
-    for (int h = 0; h < 2; ++h) {
-        if (!(pend & (1u << h))) continue;
-        const long long t0 = clock64();
-        while (!mbar_try_wait(sm.bar + h, (phase >> h) & 1u))
-            if (clock64() - t0 > tmo) break;
-    }
-}
-
-// Once per solve, before the first apply (a grid barrier must follow): the
-// pivots (and the reciprocals) into both record kinds, sentinels into both
-// cell arrays, the ring barriers initialised.
-template <typename T>
-__device__ void tiles_init(Grid& g, const Mat<T>& m, const T* __restrict__ D) {
-    const Tiles<T>& tl = m.tile;
-    const int B = blockDim.x;
-    const long long total = (long long)tl.ntx * tl.nty * tl.steps * B;
-    const T sen = Cell<T>::sentinel();
-    for (long long i = g.tid; i < total; i += g.nt) {
-        const int t = (int)(i % B);
-        const long long ks = i / B;
-        const int s = (int)(ks % tl.steps), k = (int)(ks / tl.steps);
-        const int lx = t % kTileX, ly = t / kTileX;
-        const int x = (k % tl.ntx) * kTileX + lx, y = (k / tl.ntx) * tl.ty + ly, z = s - lx - ly;
-        const bool act = x < tl.nx && y < tl.ny && z >= 0 && z < tl.nz;
-        const T d = act ? D[x + tl.nx * (y + tl.ny * z)] : T(0);
-        unsigned char* rf = tl.fwd + ks * tl.rec_f;
-        unsigned char* rb = tl.bwd + ks * tl.rec_b;
-        tile_val(tl, rf, 0, t) = d;
-        tile_val(tl, rb, 0, t) = d;
-        if (tl.recip) tile_val(tl, rf, 2, t) = act ? T(1) / (d + tiny_v<T>()) : T(0);
-        tl.wt[i] = sen;
-        tl.zt[i] = sen;
-    }
-    const TileSmem sm = tile_smem(tl);
-    if (threadIdx.x == 0) {
-        mbar_init(sm.bar, 1);
-        mbar_init(sm.bar + 1, 1);
-        *sm.fail = 0;
-        *sm.phase = 0;
-        mbar_init_fence();
-    }
-    __syncthreads();
-}
-
-template <typename T>
-__device__ bool tile_forward(Grid& g, const Mat<T>& m, const T* __restrict__ rhs) {
-    const Tiles<T> tl = m.tile;  // a copy: the per-step fields stay in registers
-    DevCtl* const ctl = g.ctl;
-    const long long tmo = g.timeout_cyc;
-    const TileSmem sm = tile_smem(tl);
-    const int B = blockDim.x, t = threadIdx.x, lx = t % kTileX, ly = t / kTileX;
-    const int S = tl.steps, ntiles = tl.ntx * tl.nty, H = tl.half;
-    const size_t plane = (size_t)S * B;
-    // shared addresses of the ring and of the neighbour exchange (two step
-    // parities of B values); this thread's own offsets within a record
-    const unsigned ring_a = smem_u32(sm.ring);
-    const unsigned nbv_a = ring_a + 2 * H * sm.slot;
-    const unsigned sz = (unsigned)sizeof(T);
-    const unsigned vf0 = tile_vfield(tl, 0) + t * sz, vf1 = tile_vfield(tl, 1) + t * sz,
-                   vf2 = tile_vfield(tl, 2) + t * sz;
-    __syncthreads();
-    unsigned phase = (unsigned)*sm.phase, pend = 0;
-    bool ok = true;
-    for (int k = g.bid; k < ntiles && ok; k += g.nblocks) {
-        const int x = (k % tl.ntx) * kTileX + lx, y = (k / tl.ntx) * tl.ty + ly;
-        const bool inb = x < tl.nx && y < tl.ny;
-        const size_t base = (size_t)k * plane;
-        unsigned char* recf = tl.fwd + (size_t)k * S * tl.rec_f;
-        unsigned char* recb = tl.bwd + (size_t)k * S * tl.rec_b;
-        // gather this tile's right-hand side into its forward records
-        // (eight independent loads in flight per thread)
-        for (int s0 = 0; s0 < S; s0 += 8) {
-            T v[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int z = s0 + q - lx - ly;
-                v[q] = inb && z >= 0 && z < tl.nz && s0 + q < S ? rhs[x + tl.nx * (y + tl.ny * z)]
-                                                                : T(0);
-            }
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-                if (s0 + q < S) *reinterpret_cast<T*>(recf + (size_t)(s0 + q) * tl.rec_f + vf1) = v[q];
-        }
-        __syncthreads();
-        // edge cells of the left (x-1) and lower (y-1) tiles at step s
-        // (used only where that tile exists: x > 0 resp. y > 0)
-        const long long sb = (long long)base, sp = (long long)plane;
-        const T* xcell = tl.wt + (sb - sp + (long long)(kTileX - 1) * B + ly * kTileX + (kTileX - 1));
-        const T* ycell =
-            tl.wt + (sb - tl.ntx * sp + (long long)(tl.ty - 1) * B + (tl.ty - 1) * kTileX + lx);
-        if (t == 0) {
-            // the gathered words (and the records written before the sweep)
-            // and the previous tile's reads of the ring before the bulk copies
-            fence_proxy_async_global();
-            fence_proxy_async_smem();
-            for (int h = 0; h < 2 && h * H < S; ++h) {
-                tile_issue(sm.ring + h * H * tl.rec_f, sm.bar + h, recf + (size_t)h * H * tl.rec_f,
-                           tl.rec_f, min(H, S - h * H));
-                pend |= 1u << h;
-            }
-        }
-        // neighbour cells two steps ahead, by step parity
-        T xp0 = T(0), xp1 = T(0), yp0 = T(0), yp1 = T(0);
-        auto prefetch = [&](int s) {
-            const int z = s - lx - ly;
-            if (inb && z >= 0 && z < tl.nz) {
-                T xv = T(0), yv = T(0);
-                if (lx == 0 && x > 0) xv = Cell<T>::value(Cell<T>::load(xcell + (size_t)s * B));
-                if (ly == 0 && y > 0) yv = Cell<T>::value(Cell<T>::load(ycell + (size_t)s * B));
-                if (s & 1) { xp1 = xv; yp1 = yv; } else { xp0 = xv; yp0 = yv; }
-            }
-        };
-        prefetch(0);
-        if (S > 1) prefetch(1);
-        T ycur = T(0);
-        // one ring half per outer pass (no index arithmetic by a runtime
-        // divisor per step); a failed wait ends the tile at the half's end
-        int hb = 0;
-        for (int s0 = 0; s0 < S; s0 += H, hb ^= 1) {
-            tile_wait(ctl, tmo, sm, hb, (phase >> hb) & 1u, 26);
-            phase ^= 1u << hb;
-            pend &= ~(1u << hb);
-            const int cnt = min(H, S - s0);
-            const unsigned half = ring_a + (unsigned)(hb * H) * tl.rec_f;
-            for (int q = 0; q < cnt; ++q) {
-                const int s = s0 + q;
-                const int z = s - lx - ly;
-                if (inb && z >= 0 && z < tl.nz) {
-                    const unsigned sl = half + (unsigned)q * tl.rec_f;
-                    const unsigned nb_prev = nbv_a + ((unsigned)((s - 1) & 1) * B + t) * sz;
-                    const T ri = lds<T>(sl + vf1);
-                    T acc = ri;
-                    if (z > 0) acc = acc - tile_coef_s(tl, sl, 0, t) * ycur;
-                    if (y > 0) {
-                        const T v = ly > 0 ? lds<T>(nb_prev - kTileX * sz)
-                                           : tile_cell(ctl, tmo, sm, ycell + (size_t)s * B,
-                                                       (s & 1) ? yp1 : yp0, 27);
-                        acc = acc - tile_coef_s(tl, sl, 1, t) * v;
-                    }
-                    if (x > 0) {
-                        const T v = lx > 0 ? lds<T>(nb_prev - sz)
-                                           : tile_cell(ctl, tmo, sm, xcell + (size_t)s * B,
-                                                       (s & 1) ? xp1 : xp0, 27);
-                        acc = acc - tile_coef_s(tl, sl, 2, t) * v;
-                    }
-                    const T d = lds<T>(sl + vf0);
-                    const T yv = acc * d;
-                    sts(nbv_a + ((unsigned)(s & 1) * B + t) * sz, yv);
-                    ycur = yv;
-                    const size_t idx = base + (size_t)s * B + t;
-                    Cell<T>::store(tl.wt + idx, yv);
-                    // the middle step of CG.f90:144-146, for the backward sweep
-                    const T mid = tl.recip ? yv * lds<T>(sl + vf2) : yv / (d + tiny_v<T>());
-                    unsigned char* rb = recb + (size_t)s * tl.rec_b;
-                    *reinterpret_cast<T*>(rb + vf1) = mid;
-                    *reinterpret_cast<T*>(rb + vf2) = ri;
-                    tl.zt[idx] = Cell<T>::sentinel();
-                }
-                __syncthreads();
-                if (s + 2 < S) prefetch(s + 2);
-            }
-            if (*sm.fail) {
-                tile_drain(tmo, sm, pend, phase);
-                ok = false;
-                break;
-            }
-            // this half consumed: refill it with the steps after the other half
-            const int first = s0 + 2 * H;
-            if (t == 0 && first < S) {
-                fence_proxy_async_smem();  // the half's reads before its refill
-                tile_issue(sm.ring + (size_t)hb * H * tl.rec_f, sm.bar + hb,
-                           recf + (size_t)first * tl.rec_f, tl.rec_f, min(H, S - first));
-                pend |= 1u << hb;
-            }
-        }
-    }
-    __syncthreads();
-    if (t == 0) *sm.phase = (int)phase;
-    __syncthreads();
-    return ok;
-}
-
-template <typename T, typename Epi>
-__device__ bool tile_backward(Grid& g, const Mat<T>& m, T* __restrict__ zout, Epi epi) {
-    const Tiles<T> tl = m.tile;  // a copy: the per-step fields stay in registers
-    DevCtl* const ctl = g.ctl;
-    const long long tmo = g.timeout_cyc;
-    const TileSmem sm = tile_smem(tl);
-    const int B = blockDim.x, t = threadIdx.x, lx = t % kTileX, ly = t / kTileX;
-    const int S = tl.steps, ntiles = tl.ntx * tl.nty, H = tl.half;
-    const size_t plane = (size_t)S * B;
-    const unsigned ring_a = smem_u32(sm.ring);
-    const unsigned nbv_a = ring_a + 2 * H * sm.slot;
-    const unsigned sz = (unsigned)sizeof(T);
-    const unsigned vf0 = tile_vfield(tl, 0) + t * sz, vf1 = tile_vfield(tl, 1) + t * sz,
-                   vf2 = tile_vfield(tl, 2) + t * sz;
-    __syncthreads();
-    unsigned phase = (unsigned)*sm.phase, pend = 0;
-    if (t == 0) fence_proxy_async_global();  // the records written before the barrier
-    bool ok = true;
-    // this block's tiles (g.bid, g.bid + nblocks, ...) in decreasing order
-    const int mine = g.bid < ntiles ? (ntiles - 1 - g.bid) / g.nblocks + 1 : 0;
-    for (int q = mine - 1; q >= 0 && ok; --q) {
-        const int k = g.bid + q * g.nblocks;
-        const int x = (k % tl.ntx) * kTileX + lx, y = (k / tl.ntx) * tl.ty + ly;
-        const bool inb = x < tl.nx && y < tl.ny;
-        const size_t base = (size_t)k * plane;
-        const unsigned char* recb = tl.bwd + (size_t)k * S * tl.rec_b;
-        // edge cells of the right (x+1) and upper (y+1) tiles at step s
-        // (used only where that tile exists: x < nx-1 resp. y < ny-1)
-        const long long sb = (long long)base, sp = (long long)plane;
-        const T* xcell = tl.zt + (sb + sp + ly * kTileX - (long long)(kTileX - 1) * B);
-        const T* ycell = tl.zt + (sb + tl.ntx * sp + lx - (long long)(tl.ty - 1) * B);
-        // half h holds the steps of indices j in [h H, h H + H), j = S-1-s;
-        // they are the records S-1-j, in decreasing order, so the copy
-        // starts at the lowest step of the range and slot u holds step
-        // S-1-j at position (H-1-(j mod H)) from the half's start
-        auto issue = [&](int h, int j0) {
-            const int cnt = min(H, S - j0);
-            const int slo = S - 1 - (j0 + cnt - 1);  // lowest step of the range
-            tile_issue(sm.ring + (size_t)(h * H + H - cnt) * tl.rec_b, sm.bar + h,
-                       recb + (size_t)slo * tl.rec_b, tl.rec_b, cnt);
-            pend |= 1u << h;
-        };
-        if (t == 0) {
-            fence_proxy_async_smem();
-            for (int h = 0; h < 2 && h * H < S; ++h) issue(h, h * H);
-        }
-        T xp0 = T(0), xp1 = T(0), yp0 = T(0), yp1 = T(0);
-        auto prefetch = [&](int j) {
-            const int s = S - 1 - j, z = s - lx - ly;
-            if (inb && z >= 0 && z < tl.nz) {
-                T xv = T(0), yv = T(0);
-                if (lx == kTileX - 1 && x < tl.nx - 1)
-                    xv = Cell<T>::value(Cell<T>::load(xcell + (size_t)s * B));
-                if (ly == tl.ty - 1 && y < tl.ny - 1)
-                    yv = Cell<T>::value(Cell<T>::load(ycell + (size_t)s * B));
-                if (j & 1) { xp1 = xv; yp1 = yv; } else { xp0 = xv; yp0 = yv; }
-            }
-        };
-        prefetch(0);
-        if (S > 1) prefetch(1);
-        T zcur = T(0);
-        int hb = 0;
-        for (int j0 = 0; j0 < S; j0 += H, hb ^= 1) {
-            tile_wait(ctl, tmo, sm, hb, (phase >> hb) & 1u, 28);
-            phase ^= 1u << hb;
-            pend &= ~(1u << hb);
-            const int cnt = min(H, S - j0);
-            // step S-1-(j0+q) sits at slot H-1-q of the half
-            const unsigned half = ring_a + (unsigned)(hb * H + H - 1) * tl.rec_b;
-            for (int q = 0; q < cnt; ++q) {
-                const int j = j0 + q;
-                const int s = S - 1 - j;
-                const int z = s - lx - ly;
-                if (inb && z >= 0 && z < tl.nz) {
-                    const unsigned sl = half - (unsigned)q * tl.rec_b;
-                    const unsigned nb_prev = nbv_a + ((unsigned)((j - 1) & 1) * B + t) * sz;
-                    const T d = lds<T>(sl + vf0);
-                    T acc = lds<T>(sl + vf1);  // mid
-                    const T ri = lds<T>(sl + vf2);
-                    if (x < tl.nx - 1) {
-                        const T v = lx < kTileX - 1
-                                        ? lds<T>(nb_prev + sz)
-                                        : tile_cell(ctl, tmo, sm, xcell + (size_t)s * B,
-                                                    (j & 1) ? xp1 : xp0, 29);
-                        acc = acc - tile_coef_s(tl, sl, 0, t) * v;
-                    }
-                    if (y < tl.ny - 1) {
-                        const T v = ly < tl.ty - 1
-                                        ? lds<T>(nb_prev + kTileX * sz)
-                                        : tile_cell(ctl, tmo, sm, ycell + (size_t)s * B,
-                                                    (j & 1) ? yp1 : yp0, 29);
-                        acc = acc - tile_coef_s(tl, sl, 1, t) * v;
-                    }
-                    if (z < tl.nz - 1) acc = acc - tile_coef_s(tl, sl, 2, t) * zcur;
-                    const T zi = acc * d;
-                    sts(nbv_a + ((unsigned)(j & 1) * B + t) * sz, zi);
-                    zcur = zi;
-                    const size_t idx = base + (size_t)s * B + t;
-                    Cell<T>::store(tl.zt + idx, zi);
-                    tl.wt[idx] = Cell<T>::sentinel();
-                    const int row = x + tl.nx * (y + tl.ny * z);
-                    zout[row] = zi;
-                    epi(row, zi, ri);
-                }
-                __syncthreads();
-                if (j + 2 < S) prefetch(j + 2);
-            }
-            if (*sm.fail) {
-                tile_drain(tmo, sm, pend, phase);
-                ok = false;
-                break;
-            }
-            const int jn = j0 + 2 * H;
-            if (t == 0 && jn < S) {
-                fence_proxy_async_smem();
-                issue(hb, jn);
-            }
-        }
-    }
-    __syncthreads();
-    if (t == 0) *sm.phase = (int)phase;
-    __syncthreads();
-    return ok;
-}
-
 // z = IC(0) apply of rhs by the tiled sweeps; epi(row, z_row, rhs_row) per row.
 template <typename T, typename Epi>
-__device__ bool ic_tiled_apply(Grid& g, const Mat<T>& m, const T* rhs, T* z, Epi epi) {
-    const bool ok = tile_forward(g, m, rhs);
-    if (!grid_sync(g, 25) || !ok) return false;
-    return tile_backward(g, m, z, epi);
+__device__ __forceinline__ bool ic_tiled_apply(Grid& g, const Mat<T>& m, const T* rhs, T* z, Epi epi) {
+    ++g.epoch;
+    if constexpr (sizeof(T) == 4) {
+        if (m.tile.lu_bf16)
+            return tile_sweep<0, unsigned short>(g, m, rhs, z, epi) &&
+                   tile_sweep<1, unsigned short>(g, m, rhs, z, epi);
+    }
+    return tile_sweep<0, T>(g, m, rhs, z, epi) && tile_sweep<1, T>(g, m, rhs, z, epi);
 }
 
 // The IC(0) apply the solve was configured for: `sweeps` Jacobi sweeps per

@@ -531,6 +531,13 @@ int autotune_on(tflows_topology* tp, SolveRequest& rq, const double* d_b, const 
     return TFLOWS_OK;
 }
 
+// One block size for all systems of a batched launch that names none.
+void default_batch_block(std::vector<BatchSpec>& specs) {
+    int block = 0;
+    for (auto& sp : specs) block = std::max(block, default_block(*sp.t, sp.rq));
+    for (auto& sp : specs) sp.rq.block = block;
+}
+
 void record(const SolveReport& rep, tflows_result* res) {
     tflows_result r{};
     r.status = rep.status;
@@ -585,6 +592,7 @@ int solve_on(tflows_topology* tp, const SolveRequest& rq0, const double* d_val, 
         TuneChoice ch;
         if (int st = autotune_on(tp, rq, d_b, d_x, s, ch); st != TFLOWS_OK) return st;
     }
+    rq.block = default_block(tp->t, rq);
     trace_mark("launch shape");
     // The kernels work on padded, 16-byte aligned workspace vectors: x and b
     // are staged into workspace slots 11 and 12 unless they already are them.
@@ -1044,6 +1052,7 @@ int tflows_solve_batched_device(int count, tflows_topology* const* topos, const 
         if (e != cudaSuccess) return cuda_fail(e, "batch staging");
         specs[k] = BatchSpec{&tp->t, ws, rq, X, R, &reps[k]};
     }
+    default_batch_block(specs);
     double sec = 0.0;
     int worst = run_batch(specs, s, &sec);
     std::string msg;
@@ -1122,6 +1131,7 @@ int tflows_plan_create(tflows_plan** out, int count, tflows_topology* const* top
                                    ws->vec64 + 12 * ws->vec_cap, &plan->reps[k]};
         plan->topos.push_back(tp);
     }
+    default_batch_block(plan->specs);
     cudaError_t e = cudaStreamCreateWithFlags(&plan->cap, cudaStreamNonBlocking);
     if (e != cudaSuccess) return cuda_fail(e, "plan stream");
     if (o.autotune && o.block_size == 0 && o.grid_blocks == 0) {
@@ -1301,6 +1311,7 @@ int tflows_ic_apply_device(tflows_topology* topo, const tflows_options* opt, con
         return fail(TFLOWS_BAD_INPUT, "IC(0) needs a triangular-ordered pattern");
     SolveRequest rq = make_request(o, TFLOWS_METHOD_CG, 2, 0, 0.0);
     if (std::string msg; !shape_ok(rq, msg)) return fail(TFLOWS_BAD_INPUT, msg);
+    rq.block = default_block(topo->t, rq);
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e = build_levels(topo->t);
     if (e == cudaSuccess) e = ensure_workspace(topo->ws, topo->t);
