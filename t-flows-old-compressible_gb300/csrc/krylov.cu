@@ -413,12 +413,15 @@ bool tiles_env_on() {
 
 size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
-// FP64 CG forms its search direction inside the product only on systems
-// whose vectors stay in L2 (measured: config 1, 32^3, 18.0 -> 16.7 us per
-// iteration; on 128^3 and 256^3 it was 20-30 % slower, the second gathered
-// vector and the per-neighbour z + beta p on the FP64 pipe costing more than
-// the update pass it saves).
-bool fuse_dir_fp64(const DeviceTopology& t) { return t.n <= (1 << 19); }
+// FP64 CG forms its search direction inside the product only on small
+// systems, where the grid barrier it saves (about 2 us) is worth more than
+// the FP64 operations it adds, one (reference arithmetic: two) per entry.
+// Measured, us per iteration inside the product / as a pass of its own, in
+// reference arithmetic: 16.6 / 17.4 at 32^3, 23.3 / 21.8 at 48^3; with
+// multiply-adds 16.0 / 16.3 at 48^3, 25.3 / 23.9 at 64^3.
+bool fuse_dir_fp64(const DeviceTopology& t, const SolveRequest& rq) {
+    return t.n <= (rq.precision == 0 ? 50 : 120) * 1000;
+}
 
 // Patches per tile: as many as the block has warps for, up to four, whose
 // shared memory fits an SM twice (one apply at 128^3, FP32: 190 us with four,
@@ -447,6 +450,11 @@ TileGeom tile_geom(const DeviceTopology& t, const SolveRequest& rq) {
     return g;
 }
 
+int tile_count(const DeviceTopology& t, const SolveRequest& rq) {
+    const TileGeom g = tile_geom(t, rq);
+    return g.ntx * g.nty;
+}
+
 // Coefficient and value bytes of a request's records.
 void tile_elem(const SolveRequest& rq, unsigned& ls, unsigned& sv) {
     if (rq.precision == 1) {
@@ -473,8 +481,24 @@ bool tiled_ic(const DeviceTopology& t, const SolveRequest& rq) {
     return rq.block == 0 || rq.block >= 32 * kWarpsPerPatch;
 }
 
-int default_block(const DeviceTopology& t, const SolveRequest& rq) {
-    return rq.block > 0 ? rq.block : (tiled_ic(t, rq) ? kMaxBlock : 0);
+void default_shape(const DeviceTopology& t, SolveRequest& rq) {
+    if (rq.block > 0) return;
+    const bool tiled = tiled_ic(t, rq);
+    if (tiled) rq.block = kMaxBlock;
+    if (rq.grid > 0 || rq.rows_per_warp > 0) return;
+    if (tiled) {
+        if (t.n <= 600 * 1000 && tile_count(t, rq) <= sms()) rq.grid = sms();
+    } else if (rq.precision == 1 && rq.prec != 2) {
+        // one row per thread while one block per SM holds them
+        if (t.n > kBlock * sms()) rq.block = kMaxBlock;
+        rq.grid = std::min(blocks_for(t.nslices, block_of(rq)), (t.n <= 600 * 1000 ? 1 : 2) * sms());
+    } else if (t.n <= 400 * 1000 || (rq.prec == 2 && rq.ic_sweeps == 0)) {
+        rq.grid = std::min(blocks_for(t.nslices), sms());
+    } else if (t.n <= (rq.precision == 0 ? 3000 : 1200) * 1000) {
+        rq.grid = std::min(blocks_for(t.nslices), 2 * sms());
+    } else {
+        rq.block = kMaxBlock;
+    }
 }
 
 unsigned tile_smem_for(const DeviceTopology& t, const SolveRequest& rq) {
@@ -562,7 +586,7 @@ cudaError_t prepare_fp64(const DeviceTopology& t, Workspace& ws, const SolveRequ
     P.mode = 0;
     P.stall = rq.inject_stall;
     P.cfg.ic_sweeps = rq.prec == 2 ? std::max(rq.ic_sweeps, 0) : 0;
-    P.cfg.fuse_dir = fuse_dir_fp64(t) ? 1 : 0;
+    P.cfg.fuse_dir = fuse_dir_fp64(t, rq) ? 1 : 0;
     cudaError_t e = cudaMemsetAsync(ws.ctl, 0, sizeof(DevCtl), s);
     if (rq.prec == 2) {
         const long long nvec = (long long)t.nslices * kWarp;
@@ -661,7 +685,7 @@ double solve_bytes(const DeviceTopology& t, const SolveRequest& rq, const DevSta
     // separate update pass: one vector fewer)
     const double per_it = cgs ? 2 * spmv64 + 8.0 * t.n * 22 + 2 * ic
                               : spmv64 + 8.0 * t.n * ((rq.prec == 1 ? 12 : 10) -
-                                                      (fuse_dir_fp64(t) ? 1 : 0)) + ic;
+                                                      (fuse_dir_fp64(t, rq) ? 1 : 0)) + ic;
     return per_it * it + spmv64 + 8.0 * t.n * 4;
 }
 

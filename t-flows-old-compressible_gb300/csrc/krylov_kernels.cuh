@@ -1344,6 +1344,28 @@ __device__ __forceinline__ bool ic_precond(Grid& g, const Mat<T>& m, Vecs<T>& v,
 template <typename T>
 __device__ __forceinline__ bool finite_val(T v) { return isfinite(v); }
 
+// The end of an iteration: two totals, and the third (finite entries of x and
+// r) only once the residual has turned non-finite.
+template <typename T>
+__device__ __forceinline__ bool reduce_watched(Grid& g, int slot, const T (&a)[3], bool all, int where,
+                                               double (&t)[3]) {
+    if (all) {
+        publish_t<3>(g, slot, a);
+        if (!grid_sync(g, where)) return false;
+        totals<3>(g, slot, t);
+    } else {
+        const T b[2] = {a[0], a[1]};
+        publish_t<2>(g, slot, b);
+        if (!grid_sync(g, where)) return false;
+        double u[2];
+        totals<2>(g, slot, u);
+        t[0] = u[0];
+        t[1] = u[1];
+        t[2] = 0.0;
+    }
+    return true;
+}
+
 // ---- the reference prologue: Prec1, ||b||, Resid, IniRes -------------------
 // Returns false when the launch aborted or an early exit was taken (out
 // records which).  On return true, `err` holds ||r0|| and, for prec 1 / 0,
@@ -1520,10 +1542,8 @@ __device__ void cg_solve(Grid& g, const Mat<T>& m, Vecs<T>& v, const SolveCfg& c
             st4(v.r + i, rr);
             if (prec == 1) st4(v.z + i, zz);
         }
-        publish_t<3>(g, SLOT_D, a3);
-        if (!grid_sync(g, 44)) { out.exit_kind = EXIT_ABORT; return; }
         double t3[3];
-        totals<3>(g, SLOT_D, t3);
+        if (!reduce_watched(g, SLOT_D, a3, nonfinite, 44, t3)) { out.exit_kind = EXIT_ABORT; return; }
         err = sqrt(t3[0]);
         out.fin_res = err;
         if (err < tol) {
@@ -1669,10 +1689,8 @@ __device__ void cgs_solve(Grid& g, const Mat<T>& m, Vecs<T>& v, const SolveCfg& 
                 }
             }
         }
-        publish_t<3>(g, SLOT_C, a3);
-        if (!grid_sync(g, 58)) { out.exit_kind = EXIT_ABORT; return; }
         double t3[3];
-        totals<3>(g, SLOT_C, t3);
+        if (!reduce_watched(g, SLOT_C, a3, nonfinite, 58, t3)) { out.exit_kind = EXIT_ABORT; return; }
         err = sqrt(t3[0]);
         out.fin_res = err;
         if (err < tol) {

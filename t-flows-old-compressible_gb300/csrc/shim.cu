@@ -534,7 +534,11 @@ int autotune_on(tflows_topology* tp, SolveRequest& rq, const double* d_b, const 
 // One block size for all systems of a batched launch that names none.
 void default_batch_block(std::vector<BatchSpec>& specs) {
     int block = 0;
-    for (auto& sp : specs) block = std::max(block, default_block(*sp.t, sp.rq));
+    for (auto& sp : specs) {
+        SolveRequest rq = sp.rq;
+        default_shape(*sp.t, rq);
+        block = std::max(block, tiled_ic(*sp.t, rq) ? rq.block : sp.rq.block);
+    }
     for (auto& sp : specs) sp.rq.block = block;
 }
 
@@ -592,7 +596,7 @@ int solve_on(tflows_topology* tp, const SolveRequest& rq0, const double* d_val, 
         TuneChoice ch;
         if (int st = autotune_on(tp, rq, d_b, d_x, s, ch); st != TFLOWS_OK) return st;
     }
-    rq.block = default_block(tp->t, rq);
+    default_shape(tp->t, rq);
     trace_mark("launch shape");
     // The kernels work on padded, 16-byte aligned workspace vectors: x and b
     // are staged into workspace slots 11 and 12 unless they already are them.
@@ -1311,7 +1315,7 @@ int tflows_ic_apply_device(tflows_topology* topo, const tflows_options* opt, con
         return fail(TFLOWS_BAD_INPUT, "IC(0) needs a triangular-ordered pattern");
     SolveRequest rq = make_request(o, TFLOWS_METHOD_CG, 2, 0, 0.0);
     if (std::string msg; !shape_ok(rq, msg)) return fail(TFLOWS_BAD_INPUT, msg);
-    rq.block = default_block(topo->t, rq);
+    default_shape(topo->t, rq);
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e = build_levels(topo->t);
     if (e == cudaSuccess) e = ensure_workspace(topo->ws, topo->t);
