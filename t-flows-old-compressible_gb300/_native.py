@@ -1,6 +1,6 @@
 """Build and load libtflows_krylov.so (the CUDA sm_103a kernels + C-ABI shim).
 
-The library is compiled in-tree with nvcc (one -gencode for sm_103a, both
+The library is compiled in-tree with nvcc (one -gencode for sm_103a, all
 translation units in parallel) and loaded with ctypes.  There is no CPU
 fallback: a missing or unloadable library raises.
 """
@@ -18,9 +18,10 @@ CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 BUILD = os.path.join(HERE, "_build")
 LIB_PATH = os.path.join(HERE, "libtflows_krylov.so")
-SOURCES = ("krylov.cu", "krylov_fma.cu", "shim.cu", "noalloc.cu", "tune.cu", "assembly.cu",
-           "momentum.cu", "halo.cu", "meshio.cpp")
-HEADERS = ("device_common.cuh", "krylov_kernels.cuh", "solver_entry.cuh", "internal.h",
+SOURCES = ("krylov.cu", "krylov_fma.cu", "krylov_mixed.cu", "shim.cu", "noalloc.cu", "tune.cu",
+           "assembly.cu", "momentum.cu", "halo.cu", "meshio.cpp")
+CONTRACTED = ("krylov_fma.cu", "krylov_mixed.cu")  # units built with fused multiply-adds
+HEADERS = ("device_common.cuh", "fp64_div.cuh", "krylov_kernels.cuh", "solver_entry.cuh", "internal.h",
            "assembly_internal.h")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
@@ -65,7 +66,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
             extra = os.environ.get("TFLOWS_NVCC_EXTRA", "").split()
             # the contracted build fuses multiply-adds; everything else keeps
             # the reference's separately rounded products and sums
-            fmad = ["--fmad=true"] if src == "krylov_fma.cu" else ["--fmad=false"]
+            fmad = ["--fmad=" + ("true" if src in CONTRACTED else "false")]
             cmd = [cc, *ARCH, *NVCC_FLAGS, *fmad, *extra, "-I", INCLUDE, "-c",
                    os.path.join(CSRC, src), "-o", obj]
             r = subprocess.run(cmd, capture_output=True, text=True)

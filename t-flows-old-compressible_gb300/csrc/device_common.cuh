@@ -10,6 +10,8 @@
 // * deterministic block and grid reductions (fixed summation tree)
 #pragma once
 
+#include "fp64_div.cuh"
+
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -280,10 +282,13 @@ __device__ __forceinline__ void publish(Grid& g, int slot, const double (&v)[K])
 }
 
 // After a grid_sync: every block computes the same K totals in the same
-// order (deterministic), one warp per value, broadcast through shared memory.
-template <int K>
-__device__ __forceinline__ void totals(Grid& g, int slot, double (&res)[K]) {
-    __shared__ double s_tot[K];
+// order (deterministic), one warp per value, broadcast through shared memory
+// together with what one thread derives from each: ext[k] = post(k, total).
+// (A division or a square root by every thread would hold the FP64 pipe for
+// some 160 cycles per warp, 2.6 us on an SM full of them.)
+template <int K, typename Post>
+__device__ __forceinline__ void totals(Grid& g, int slot, double (&res)[K], double (&ext)[K], Post post) {
+    __shared__ double s_tot[K], s_ext[K];
     const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int k = warp; k < K; k += nw) {
         const long long* src =
@@ -308,14 +313,59 @@ __device__ __forceinline__ void totals(Grid& g, int slot, double (&res)[K]) {
             s += w[0];
         }
         s = warp_sum(s);
-        if (g.lane == 0) s_tot[k] = s;
+        if (g.lane == 0) {
+            s_tot[k] = s;
+            s_ext[k] = post(k, s);
+        }
     }
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < K; ++k) res[k] = s_tot[k];
+    for (int k = 0; k < K; ++k) {
+        res[k] = s_tot[k];
+        ext[k] = s_ext[k];
+    }
     // no closing block barrier: the next write of s_tot comes after the
     // next grid_sync, whose opening __syncthreads every thread reaches after
     // reading these totals
+}
+template <int K>
+__device__ __forceinline__ void totals(Grid& g, int slot, double (&res)[K]) {
+    double ext[K];
+    totals<K>(g, slot, res, ext, [](int, double) { return 0.0; });
+}
+
+// sqrt(t) < tol as a comparison of t: the least t whose (rounded, monotonic)
+// square root is not below tol.  Set by one thread; lives in shared memory.
+struct NormTest {
+    double tol, least;
+    bool direct;  // tol^2 is not a comfortable number: compare square roots
+    __device__ void set(double tol_) {  // by one thread
+        tol = tol_;
+        direct = !(tol <= 0.0) && !(tol > 1e-140 && tol < 1e140);
+        double t = 0.0;  // tol <= 0: no norm is below it
+        if (tol > 0.0 && !direct) {
+            t = tol * tol;
+            while (sqrt(t) >= tol) t = __longlong_as_double(__double_as_longlong(t) - 1);
+            while (sqrt(t) < tol) t = __longlong_as_double(__double_as_longlong(t) + 1);
+        }
+        least = t;
+    }
+    // t: a sum of squares (not negative, or not a number)
+    __device__ bool below(double t) const { return direct ? sqrt(t) < tol : t < least; }
+};
+
+// A solver's scalars, one copy per block in shared memory.  Only the threads
+// that form totals (lane 0 of a summing warp) read and write them between
+// barriers; what every thread needs comes with the totals.
+struct Scalars {
+    double rho, rho_old;  // (r, z) of the current iteration and of the one before
+    double beta;
+    double rr;            // ||r||^2 at the end of the last iteration
+    NormTest conv, refine;
+};
+__device__ __forceinline__ Scalars& scalars() {
+    __shared__ Scalars s;
+    return s;
 }
 
 }  // namespace tflows

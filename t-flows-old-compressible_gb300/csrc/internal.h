@@ -19,6 +19,7 @@ struct DeviceTopology {
     int nslices = 0;
     long long sell_len = 0;
     int max_len = 0;
+    int width = 0;             // entries per row of every slice (0: slices differ)
     bool ic_ok = false;        // lower part = slots before the diagonal, ascending
     bool levels_built = false;
     bool tsym = false;         // every entry has its transpose (valid once tpos exists)
@@ -208,13 +209,14 @@ int halo_solve(int method, int n, int nb, int nonz, const double* A, const int* 
 int halo_resid(int n, int nb, int nonz, const double* A, const int* Acol, const int* Arow,
                const double* Ab, const double* x, double* r1, cudaStream_t s, std::string& msg);
 
-// The persistent kernels, built twice: krylov.cu with the reference's
-// arithmetic (separate rounded products and sums, dividing diagonal) and
-// krylov_fma.cu with fused multiply-adds (TFLOWS_FP64_FMA and mixed solves).
+// The persistent kernels: krylov.cu has the reference's arithmetic (separate
+// rounded products and sums, dividing diagonal), krylov_fma.cu and
+// krylov_mixed.cu fused multiply-adds (TFLOWS_FP64_FMA; the mixed solves).
 enum class KernelId { Cg, Cgs, BicgTrue, Prec1, IcApply, MixedRestart, MixedReliable, MixedCgs,
                       BatchFp64, BatchMixed };
 const void* ref_kernel(KernelId id);
 const void* fma_kernel(KernelId id);
+const void* mixed_kernel(KernelId id);
 
 // tune.cu: launch-shape autotuner.
 struct TuneChoice {

@@ -181,20 +181,17 @@ int sweep_gate_on() {
     return v;
 }
 
-// Column patterns feed the FP64 products and the standalone product; the
-// FP32 inner solves keep explicit columns (measured at 256^3: the mixed CG
-// 2 % slower with patterns -- its persistent kernel is latency-bound at 50 %
-// occupancy and the table lookup lengthens each slice's dependency chain
-// more than the saved index bytes shorten it).
 template <typename T>
-Mat<T> make_mat(const DeviceTopology& t, const T* sval, bool patterns = sizeof(T) == 8) {
+Mat<T> make_mat(const DeviceTopology& t, const T* sval) {
     Mat<T> m;
     m.n = t.n;
     m.nslices = t.nslices;
     m.soff = t.soff;
+    m.width = t.width;
+    m.narrow = t.max_len <= 8;
     m.scol = t.scol;
-    m.spat = patterns ? t.spat : nullptr;
-    m.poff = patterns ? t.poff : nullptr;
+    m.spat = t.spat;
+    m.poff = t.poff;
     m.sval = sval;
     m.meta = t.meta;
     m.perm_f = t.perm_f;
@@ -646,11 +643,11 @@ cudaError_t prepare_mixed(const DeviceTopology& t, Workspace& ws, const SolveReq
 // Algorithmic bytes of a finished solve (values + indices of each product,
 // each row's x gathered once, plus the vector passes of the schedule).
 double solve_bytes(const DeviceTopology& t, const SolveRequest& rq, const DevState& st) {
-    const double sl = 8.0 * (t.nslices + 1);
-    // column indices of one product: a pattern id per row (FP64 products of
-    // a topology with patterns), or 4 bytes per entry
-    const double idx64 = t.spat ? (double)t.n : 4.0 * t.nnz;
-    const double spmv64 = (double)t.nnz * 8.0 + idx64 + sl + 16.0 * t.n;
+    const double sl = t.width ? 0.0 : 8.0 * (t.nslices + 1);
+    // column indices of one product: a pattern id per row (a topology with
+    // patterns), or 4 bytes per entry
+    const double idx = t.spat ? (double)t.n : 4.0 * t.nnz;
+    const double spmv64 = (double)t.nnz * 8.0 + idx + sl + 16.0 * t.n;
     const bool cgs = rq.method == 2;
     // One IC(0) apply: the off-diagonal factor entries (value + index) once,
     // the row metadata, D and the right-hand side read and the result written
@@ -666,16 +663,13 @@ double solve_bytes(const DeviceTopology& t, const SolveRequest& rq, const DevSta
         return offd * (sv + 4.0) + 2.0 * t.n * (4.0 + 3.0 * sx);
     };
     if (rq.precision == 1) {
-        const double spmv32 = (double)t.nnz * 8.0 + sl + 8.0 * t.n;
+        const double spmv32 = (double)t.nnz * 4.0 + idx + sl + 8.0 * t.n;
         const double ic = rq.prec == 2 ? ic_bytes(rq.ic_bf16 ? 2.0 : 4.0, 4.0) : 0.0;
-        // restarted CG forms its search direction inside the product (z and
-        // p read once, p and q written once), so the product's own vector
-        // read and write are part of the 4·N·12 (resp. 10) vector bytes; the
-        // reliable-update loop keeps its separate direction pass
-        const double cg_fused = !rq.refine_restart ? 8.0 * t.n : 0.0;
+        // CG forms its search direction inside the product (z and p read once,
+        // p and q written once), so the product's own vector read and write
+        // are part of the 4·N·12 (resp. 10) vector bytes
         const double inner_it = cgs ? 2 * spmv32 + 4.0 * t.n * 22 + 2 * ic
-                                    : spmv32 - 8.0 * t.n + cg_fused +
-                                          4.0 * t.n * (rq.prec == 1 ? 12 : 10) + ic;
+                                    : spmv32 - 8.0 * t.n + 4.0 * t.n * (rq.prec == 1 ? 12 : 10) + ic;
         return inner_it * st.inner_iters + (spmv64 + 8.0 * t.n * 4) * (st.refinements + 1);
     }
     const int it = std::max(0, std::min(st.iterations, rq.maxiter));
@@ -752,16 +746,16 @@ namespace {
 // contracted build for TFLOWS_FP64_FMA and for the mixed solves.
 const void* solver_kernel(const SolveRequest& rq) {
     if (rq.precision == 1)
-        return fma_kernel(rq.method == 2 ? KernelId::MixedCgs
-                                         : (rq.refine_restart ? KernelId::MixedRestart
-                                                              : KernelId::MixedReliable));
+        return mixed_kernel(rq.method == 2 ? KernelId::MixedCgs
+                                           : (rq.refine_restart ? KernelId::MixedRestart
+                                                                : KernelId::MixedReliable));
     const KernelId id = rq.method == 2 ? KernelId::Cgs
                         : rq.method == 3 ? KernelId::BicgTrue : KernelId::Cg;
     return rq.precision == 2 ? fma_kernel(id) : ref_kernel(id);
 }
 
 const void* batch_kernel_for(int precision) {
-    return precision == 1 ? fma_kernel(KernelId::BatchMixed)
+    return precision == 1 ? mixed_kernel(KernelId::BatchMixed)
            : precision == 2 ? fma_kernel(KernelId::BatchFp64) : ref_kernel(KernelId::BatchFp64);
 }
 
@@ -1037,7 +1031,7 @@ cudaError_t run_spmv(const DeviceTopology& t, Workspace& ws, const double* x, do
     cudaEventRecord(ws.ev0, s);
     for (int k = 0; k < std::max(1, repeat); ++k) {
         if (fp32) {
-            spmv_kernel<float, float><<<nb, kBlock, 0, s>>>(make_mat<float>(t, ws.sval32, true), x32,
+            spmv_kernel<float, float><<<nb, kBlock, 0, s>>>(make_mat<float>(t, ws.sval32), x32,
                                                             y32);
         } else {
             spmv_kernel<double, double><<<nb, kBlock, 0, s>>>(make_mat<double>(t, ws.sval64), x, y);

@@ -110,6 +110,8 @@ struct Mat {
     int n;
     int nslices;
     const long long* __restrict__ soff;  // nslices + 1 slice offsets (elements)
+    int width;                           // entries per row of every slice (0: they differ)
+    int narrow;                          // 1: no row has more than 8 entries
     const int* __restrict__ scol;        // SELL column indices, -1 = padding
     // Column patterns (null when the topology has none): row i's entry t is
     // at column i + poff[8 * spat[i] + t], absent where that offset is
@@ -194,14 +196,14 @@ __device__ __forceinline__ V4<float> ld4(const float* p) {
 __device__ __forceinline__ void st4(float* p, const V4<float>& v) {
     *reinterpret_cast<float4*>(p) = make_float4(v.a[0], v.a[1], v.a[2], v.a[3]);
 }
+// Doubles as one 32-byte access: two of 16 bytes write every sector twice to
+// L2 (a warp's 16-byte stores at a 32-byte stride fill half of each).
 __device__ __forceinline__ V4<double> ld4(const double* p) {
-    const double2 u = reinterpret_cast<const double2*>(p)[0];
-    const double2 w = reinterpret_cast<const double2*>(p)[1];
-    return {{u.x, u.y, w.x, w.y}};
+    const double4_32a v = *reinterpret_cast<const double4_32a*>(p);
+    return {{v.x, v.y, v.z, v.w}};
 }
 __device__ __forceinline__ void st4(double* p, const V4<double>& v) {
-    reinterpret_cast<double2*>(p)[0] = make_double2(v.a[0], v.a[1]);
-    reinterpret_cast<double2*>(p)[1] = make_double2(v.a[2], v.a[3]);
+    *reinterpret_cast<double4_32a*>(p) = make_double4_32a(v.a[0], v.a[1], v.a[2], v.a[3]);
 }
 
 // Dot-product partials accumulate per thread in the working precision (FP64
@@ -224,9 +226,12 @@ constexpr bool kRecipDiag64 = true;
 __device__ __forceinline__ double jacobi(double r, double dinv) { return r * dinv; }
 #else
 constexpr bool kRecipDiag64 = false;
-__device__ __forceinline__ double jacobi(double r, double d) { return r / d; }
+__device__ __forceinline__ double jacobi(double r, double d) { return div_rn(r, d); }
 #endif
 __device__ __forceinline__ float jacobi(float r, float dinv) { return r * dinv; }
+
+__device__ __forceinline__ double divide(double a, double b) { return div_rn(a, b); }
+__device__ __forceinline__ float divide(float a, float b) { return a / b; }
 
 // Offset marking an absent entry of a column pattern: patterns are built
 // only for fewer than 2^30 rows, so i + kNoCol is negative for every row.
@@ -341,87 +346,187 @@ __device__ __forceinline__ double fused_dir(double z, double beta, double p, boo
     return first ? z : z + beta * p;
 }
 
-// The FP64 product with the next search direction formed in the gather
-// (column patterns where the topology has them, plain left-to-right sums as
-// the reference's product): the same direction and the same q as the
-// separate update pass followed by the product, bit for bit, with one vector
-// pass and one grid barrier less per iteration.
-__device__ __forceinline__ double sell_row_dir(const Mat<double>& m, int s, int lane,
-                                               const double* __restrict__ z,
-                                               const double* __restrict__ p, double beta,
-                                               bool first) {
-    const long long b0 = m.soff[s];
-    const int w = (int)((m.soff[s + 1] - b0) >> 5);
-    const int* cp = m.scol + b0 + lane;
-    const double* vp = m.sval + b0 + lane;
-    double acc = 0.0;
-    if (w <= 8) {
-        int c[8];
-        double v[8], zz[8], pp[8];
-        sell_cols8(m, s, lane, w, b0, c);
+// ---- the phases of an iteration ------------------------------------------------
+// They are inlined: as functions of their own they cost 30 us per iteration
+// at 4.1 M rows (registers saved around each call go through L2, and their
+// pointers lose the global address space).  The solver around them therefore
+// keeps its scalars in shared memory (Scalars), so that a loop has nearly the
+// whole register budget of 64.
+
+// q = A p over this warp's slices; returns the thread's sum of w_i q_i.  With
+// DIR the search direction is formed in the gather (p_i = z_i + beta p_i, or
+// z_i when `first`), stored to pn, and takes the place of w: the same
+// direction and the same q as a separate update pass followed by the
+// product, bit for bit, with one vector pass and one grid barrier less.
+// Bound by DRAM (FP32, and FP64 sums with fused multiply-adds on large
+// systems) or by the FP64 pipe's 2 lanes per clock and SM (separate products
+// and sums).  Slices of at most 8 entries per row: every load of a row is in
+// flight before its first use, with the pattern of the next row, so that
+// nothing waits twice; the values are streamed past L1, whose lines the
+// gathers of neighbouring warps share.  Of a CG iteration on 161 x 150 x 170
+// cells (512 x 304 threads) against an explicit column per entry, an offset
+// per slice and values through L1: FP64 322 -> 255 us (with the scalar
+// divisions off the FP64 pipe), fused multiply-adds 144 -> 139, FP32 105 ->
+// 85.  Values staged through shared memory by asynchronous copies took
+// 262, 162 and 93: what they hold is taken from L1.
+template <typename T, bool DIR, bool COLUMNS>
+__device__ __forceinline__ T product_narrow(const Mat<T>& m, int wg, int nw, const T* __restrict__ z,
+                                            const T* __restrict__ p, T* __restrict__ pn, T* __restrict__ q,
+                                            const T* __restrict__ w, T beta, bool first) {
+    const int lane = threadIdx.x & 31, n = m.n, nslices = m.nslices;
+    T sum = T(0);
+    unsigned id = !COLUMNS && wg < nslices ? m.spat[wg * kWarp + lane] : 0;
+    for (int s = wg; s < nslices; s += nw) {
+        const int i = s * kWarp + lane;
+        long long b0 = (long long)s * (kWarp * m.width);
+        int ww = m.width;
+        if (!ww) {
+            b0 = m.soff[s];
+            ww = (int)((m.soff[s + 1] - b0) >> 5);
+        }
+        T v[8];
 #pragma unroll
-        for (int t = 0; t < 8; ++t) v[t] = t < w ? vp[32 * t] : 0.0;
+        for (int t = 0; t < 8; ++t) v[t] = t < ww ? __ldcs(m.sval + b0 + 32 * t + lane) : T(0);
+        int c[8];
+        if (COLUMNS) {
+#pragma unroll
+            for (int t = 0; t < 8; ++t) c[t] = t < ww ? __ldcs(m.scol + b0 + 32 * t + lane) : -1;
+        } else {
+            const int4* const po = reinterpret_cast<const int4*>(m.poff) + 2 * id;
+            const int4 a = __ldg(po), b = __ldg(po + 1);
+            id = s + nw < nslices ? m.spat[(s + nw) * kWarp + lane] : 0;
+            c[0] = i + a.x; c[1] = i + a.y; c[2] = i + a.z; c[3] = i + a.w;
+            c[4] = i + b.x; c[5] = i + b.y; c[6] = i + b.z; c[7] = i + b.w;
+        }
+        T xi = T(0);  // the row's own direction (FP32 and DIR)
+        if ((DIR || sizeof(T) == 4) && i < n)
+            xi = DIR ? fused_dir(z[i], beta, first ? T(0) : p[i], first) : p[i];
+        T x[8], acc = T(0);
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
-            zz[t] = c[t] >= 0 ? z[c[t]] : 0.0;
-            pp[t] = c[t] >= 0 && !first ? p[c[t]] : 0.0;
+            const T pt = c[t] >= 0 && !(DIR && first) ? p[c[t]] : T(0);
+            x[t] = DIR ? (c[t] >= 0 ? fused_dir(z[c[t]], beta, pt, first) : T(0)) : pt;
         }
 #pragma unroll
         for (int t = 0; t < 8; ++t)
-            if (c[t] >= 0) acc = acc + v[t] * fused_dir(zz[t], beta, pp[t], first);
-        return acc;
+            if (c[t] >= 0) {
+                if constexpr (sizeof(T) == 4) acc = acc + diff_term(v[t], x[t], xi, c[t] == i);
+                else acc = acc + v[t] * x[t];
+            }
+        if (i < n) {
+            q[i] = acc;
+            if (DIR) pn[i] = xi;
+            sum += (DIR ? xi : w[i]) * acc;
+        }
     }
-    for (int t = 0; t < w; ++t) {
-        const int c = cp[32 * t];
-        if (c >= 0) acc = acc + vp[32 * t] * fused_dir(z[c], beta, first ? 0.0 : p[c], first);
-    }
-    return acc;
+    return sum;
 }
 
-
-__device__ __forceinline__ float sell_row_dir(const Mat<float>& m, int s, int lane,
-                                              const float* __restrict__ z,
-                                              const float* __restrict__ p, float beta, bool first) {
-    const long long b0 = m.soff[s];
-    const int w = (int)((m.soff[s + 1] - b0) >> 5);
-    const int* cp = m.scol + b0 + lane;
-    const float* vp = m.sval + b0 + lane;
-    float acc = 0.f;
-    if (w <= 8) {
-        // the FP32 inner solves read explicit columns (their matrices carry no
-        // patterns), so this loop has no pattern branch
-        int c[8];
-        float v[8], zz[8], pp[8];
-#pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            c[t] = t < w ? cp[32 * t] : -1;
-            v[t] = t < w ? vp[32 * t] : 0.f;
-        }
-#pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            zz[t] = c[t] >= 0 ? z[c[t]] : 0.f;
-            pp[t] = c[t] >= 0 && !first ? p[c[t]] : 0.f;
-        }
-        // difference form (see sell_row): the row's own direction first
+// The same for rows of any length.
+template <typename T, bool DIR>
+__device__ __noinline__ T product_wide(const Mat<T>& m, int wg, int nw, const T* z, const T* p, T* pn, T* q,
+                                       const T* w, T beta, bool first) {
+    const int lane = threadIdx.x & 31;
+    T sum = T(0);
+    for (int s = wg; s < m.nslices; s += nw) {
         const int i = s * kWarp + lane;
-        float di = 0.f;
-#pragma unroll
-        for (int t = 0; t < 8; ++t)
-            if (c[t] == i) di = fused_dir(zz[t], beta, pp[t], first);
-#pragma unroll
-        for (int t = 0; t < 8; ++t)
-            if (c[t] >= 0) acc = acc + diff_term(v[t], fused_dir(zz[t], beta, pp[t], first), di, c[t] == i);
-        return acc;
+        const long long b0 = m.soff[s];
+        const int ww = (int)((m.soff[s + 1] - b0) >> 5);
+        T xi = T(0), acc = T(0);
+        if ((DIR || sizeof(T) == 4) && i < m.n)
+            xi = DIR ? fused_dir(z[i], beta, first ? T(0) : p[i], first) : p[i];
+        for (int t = 0; t < ww; ++t) {
+            const int c = m.scol[b0 + 32 * t + lane];
+            if (c < 0) continue;
+            const T v = m.sval[b0 + 32 * t + lane];
+            const T x = DIR ? fused_dir(z[c], beta, first ? T(0) : p[c], first) : p[c];
+            if constexpr (sizeof(T) == 4) acc = acc + diff_term(v, x, xi, c == i);
+            else acc = acc + v * x;
+        }
+        if (i < m.n) {
+            q[i] = acc;
+            if (DIR) pn[i] = xi;
+            sum += (DIR ? xi : w[i]) * acc;
+        }
     }
-    const int i = s * kWarp + lane;
-    const float di = i < m.n ? fused_dir(z[i], beta, first ? 0.f : p[i], first) : 0.f;
-    for (int t = 0; t < w; ++t) {
-        const int c = cp[32 * t];
-        if (c >= 0)
-            acc = acc + diff_term(vp[32 * t], fused_dir(z[c], beta, first ? 0.f : p[c], first), di,
-                                  c == i);
+    return sum;
+}
+
+template <typename T, bool DIR>
+__device__ __forceinline__ T product_phase(const Mat<T>& m, int wg, int nw, const T* z, const T* p, T* pn,
+                                           T* q, const T* w, T beta, bool first) {
+    if (!m.narrow) return product_wide<T, DIR>(m, wg, nw, z, p, pn, q, w, beta, first);
+    if (m.spat) return product_narrow<T, DIR, false>(m, wg, nw, z, p, pn, q, w, beta, first);
+    return product_narrow<T, DIR, true>(m, wg, nw, z, p, pn, q, w, beta, first);
+}
+
+// p = z + beta p, or z when `first` (CG.f90:178-187).
+template <typename T>
+__device__ __forceinline__ void direction_phase(int tid, int nt, int n, const T* __restrict__ z,
+                                             T* __restrict__ p, T beta, bool first) {
+    if (first) {
+        for (int i = 4 * tid; i < n; i += 4 * nt) st4(p + i, ld4(z + i));
+        return;
     }
-    return acc;
+    for (int i = 4 * tid; i < n; i += 4 * nt) {
+        const V4<T> zz = ld4(z + i);
+        V4<T> pp = ld4(p + i);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) pp.a[u] = zz.a[u] + beta * pp.a[u];
+        st4(p + i, pp);
+    }
+}
+
+// x += alfa p, r -= alfa q (CG.f90:226-253), z = M^-1 r with the diagonal;
+// the thread's sums of r r, r z and (with `count`) the entries of x and r
+// that are numbers.
+template <typename T>
+struct Sums3 {
+    T a[3];
+};
+template <bool COUNT, typename T>
+__device__ __forceinline__ Sums3<T> update_loop(int tid, int nt, int n, T* __restrict__ x, T* __restrict__ r,
+                                                const T* __restrict__ p, const T* __restrict__ q,
+                                                const T* __restrict__ D, T* __restrict__ z, T alfa,
+                                                bool diag) {
+    Sums3<T> out;
+    T rr_ = T(0), rz_ = T(0), cnt = T(0);
+    for (int i = 4 * tid; i < n; i += 4 * nt) {
+        V4<T> xx = ld4(x + i), rr = ld4(r + i);
+        const V4<T> pp = ld4(p + i), qq = ld4(q + i);
+        V4<T> dd, zz;
+        if (diag) dd = ld4(D + i);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            xx.a[u] = xx.a[u] + alfa * pp.a[u];
+            rr.a[u] = rr.a[u] - alfa * qq.a[u];
+            if (diag) zz.a[u] = jacobi(rr.a[u], dd.a[u]);
+            if (i + u < n) {
+                rr_ += rr.a[u] * rr.a[u];
+                if (diag) rz_ += rr.a[u] * zz.a[u];
+                if (COUNT)
+                    cnt += (xx.a[u] == xx.a[u] ? T(1) : T(0)) + (rr.a[u] == rr.a[u] ? T(1) : T(0));
+            }
+        }
+        st4(x + i, xx);
+        st4(r + i, rr);
+        if (diag) st4(z + i, zz);
+    }
+    out.a[0] = rr_;
+    out.a[1] = rz_;
+    out.a[2] = cnt;
+    return out;
+}
+template <typename T>
+__device__ __noinline__ Sums3<T> update_count(int tid, int nt, int n, T* x, T* r, const T* p, const T* q,
+                                              const T* D, T* z, T alfa, bool diag) {
+    return update_loop<true>(tid, nt, n, x, r, p, q, D, z, alfa, diag);
+}
+template <typename T>
+__device__ __forceinline__ Sums3<T> update_phase(int tid, int nt, int n, T* x, T* r, const T* p, const T* q,
+                                                 const T* D, T* z, T alfa, bool diag, bool count) {
+    if (count) return update_count(tid, nt, n, x, r, p, q, D, z, alfa, diag);
+    return update_loop<false>(tid, nt, n, x, r, p, q, D, z, alfa, diag);
 }
 
 // r_i <- r_i - a_i1 x_1 - a_i2 x_2 - ... (Process/Resid.f90:28-33 order;
@@ -558,7 +663,7 @@ __device__ __forceinline__ bool sweep_chunk(const Grid& g, const Mat<T>& m, int 
                     ++cursor;
                 }
                 if (cursor == t1) {
-                    publish_row(KIND == 2 ? T(1) / acc : acc * dmul);
+                    publish_row(KIND == 2 ? divide(T(1), acc) : acc * dmul);
                     done = true;
                 }
             } else {
@@ -577,7 +682,7 @@ __device__ __forceinline__ bool sweep_chunk(const Grid& g, const Mat<T>& m, int 
 #pragma unroll
                     for (int u = 0; u < kSweepMax; ++u)
                         if (u < n) acc = KIND == 2 ? acc - v[u] * a[u] * a[u] : acc - a[u] * v[u];
-                    publish_row(KIND == 2 ? T(1) / acc : acc * dmul);
+                    publish_row(KIND == 2 ? divide(T(1), acc) : acc * dmul);
                     done = true;
                 }
             }
@@ -603,7 +708,7 @@ __device__ __forceinline__ bool sweep_chunk(const Grid& g, const Mat<T>& m, int 
 // prec 1: D_i = a_ii; prec 2: D_i = 1 / (a_ii - sum_{k<i} D_k a_ik a_ik);
 // otherwise D_i = 1 (Process/Prec1.f90:45-67).  IC ends with a grid barrier.
 template <typename T>
-__device__ bool prec1_phase(Grid& g, const Mat<T>& m, T* D, int prec) {
+__device__ __noinline__ bool prec1_phase(Grid& g, const Mat<T>& m, T* D, int prec) {
     if (prec == 2) {
         TF_FOR_ROWS(g, m, i) { D[i] = Cell<T>::sentinel(); }
         if (!grid_sync(g, 10)) return false;
@@ -627,21 +732,40 @@ __device__ bool prec1_phase(Grid& g, const Mat<T>& m, T* D, int prec) {
     }
     // with a reciprocal diagonal (contracted FP64 build) D holds 1 / a_ii
     TF_FOR_ROWS(g, m, i) {
-        D[i] = (prec == 1) ? (sizeof(T) == 8 && kRecipDiag64 ? T(1) / diag_value(m, i)
+        D[i] = (prec == 1) ? (sizeof(T) == 8 && kRecipDiag64 ? divide(T(1), diag_value(m, i))
                                                             : diag_value(m, i))
                            : T(1);
     }
     return true;  // made visible by the caller's next barrier
 }
 
+// What an IC apply does with each row of its result besides storing it:
+// kRowNone nothing, kRowDot sums rhs_row z_row, kRowAxpy x_row += alfa z_row.
+enum : int { kRowNone = 0, kRowDot = 1, kRowAxpy = 2 };
+template <int OP, typename T>
+struct RowOp {
+    T alfa, *x;
+    T dot;
+    __device__ __forceinline__ void operator()(int row, T z, T rhs) {
+        if (OP == kRowDot) dot += rhs * z;
+        if (OP == kRowAxpy) x[row] = x[row] + alfa * z;
+    }
+};
+template <typename T>
+struct Applied {
+    bool ok;
+    T dot;
+};
+
 // ---- IC(0) apply -------------------------------------------------------------
 // z = [(D~+U)^-1 D~ (D~+L)^-1] rhs with D~ = 1/D, computed as the reference
 // does: forward w_i = D_i (rhs_i - sum_{k<i} a_ik w_k); middle
 // w_i / (D_i + TINY); backward z_i = D_i (mid_i - sum_{k>i} a_ik z_k).
 // `w` cells must hold the sentinel on entry and hold it again on exit.
-// The backward phase calls `epi(row, z_row, rhs_row)` for fused per-row work.
+// The backward phase runs `epi` (RowOp) per row.
 template <typename T, typename Epi>
-__device__ bool ic_apply(Grid& g, const Mat<T>& m, const T* D, const T* rhs, T* w, T* z, Epi epi) {
+__device__ __noinline__ Applied<T> ic_apply(Grid& g, const Mat<T>& m, const T* D, const T* rhs, T* w, T* z,
+                                            Epi epi) {
     bool ok = true;
     const int nwf = sweep_warps(g, m.wide_f, m.sweep_mult);
     for (int ch = g.wg; g.wg < nwf && ch < m.nchunk_f && ok; ch += nwf) {
@@ -659,7 +783,7 @@ __device__ bool ic_apply(Grid& g, const Mat<T>& m, const T* D, const T* rhs, T* 
         ok = sweep_chunk<0>(g, m, row, 0, dslot, base, r0, d, w, 20,
                             [&](T val) { Cell<T>::store(w + row, val); });
     }
-    if (!grid_sync(g, 21) || !ok) return false;
+    if (!grid_sync(g, 21) || !ok) return {false, T(0)};
     const int nwb = sweep_warps(g, m.wide_b, m.sweep_mult);
     for (int ch = g.wg; g.wg < nwb && ch < m.nchunk_b && ok; ch += nwb) {
         const int row = m.perm_b[ch * kWarp + g.lane];
@@ -672,7 +796,7 @@ __device__ bool ic_apply(Grid& g, const Mat<T>& m, const T* D, const T* rhs, T* 
             dslot = meta >> 16;
             base = m.soff[row >> 5] + (row & 31);
             d = D[row];
-            mid = w[row] / (d + tiny_v<T>());
+            mid = divide(w[row], d + tiny_v<T>());
         }
         ok = sweep_chunk<1>(g, m, row, dslot + 1, row >= 0 ? len : dslot + 1, base, mid, d, z, 22,
                             [&](T zi) {
@@ -681,7 +805,7 @@ __device__ bool ic_apply(Grid& g, const Mat<T>& m, const T* D, const T* rhs, T* 
                                 epi(row, zi, rhs[row]);
                             });
     }
-    return ok;
+    return {ok, epi.dot};
 }
 
 // ---- IC(0) apply by Jacobi sweeps (FP32 inner solves, ic_sweeps = k > 0) ----
@@ -734,9 +858,9 @@ __device__ __forceinline__ void tri_jacobi(const Grid& g, const Mat<T>& m, const
 
 // k forward sweeps ping-pong between w and s (the last one stores the middle
 // vector), k backward sweeps between z and the other buffer, the last one
-// into z with `epi(row, z_row, rhs_row)` fused.  No barrier after the last sweep.
+// into z with `epi` (RowOp) fused.  No barrier after the last sweep.
 template <typename T, typename Epi>
-__device__ bool ic_jacobi_apply(Grid& g, const Mat<T>& m, const T* D, const T* rhs, T* w, T* sb,
+__device__ __noinline__ Applied<T> ic_jacobi_apply(Grid& g, const Mat<T>& m, const T* D, const T* rhs, T* w, T* sb,
                                 T* z, int k, Epi epi) {
     T* fb[2] = {w, sb};
     for (int sw = 1; sw <= k; ++sw) {
@@ -746,7 +870,7 @@ __device__ bool ic_jacobi_apply(Grid& g, const Mat<T>& m, const T* D, const T* r
             tri_jacobi<true>(g, m, D, rhs, y, o, [](int, T v) { return v; });
         else
             tri_jacobi<true>(g, m, D, rhs, y, o, [&](int i, T v) { return v / (D[i] + tiny_v<T>()); });
-        if (!grid_sync(g, 23)) return false;
+        if (!grid_sync(g, 23)) return {false, T(0)};
     }
     const T* mid = fb[k & 1];
     T* bb[2] = {z, fb[(k + 1) & 1]};
@@ -755,7 +879,7 @@ __device__ bool ic_jacobi_apply(Grid& g, const Mat<T>& m, const T* D, const T* r
         T* o = bb[(k - sw) & 1];
         if (sw < k) {
             tri_jacobi<false>(g, m, D, mid, y, o, [](int, T v) { return v; });
-            if (!grid_sync(g, 24)) return false;
+            if (!grid_sync(g, 24)) return {false, T(0)};
         } else {
             tri_jacobi<false>(g, m, D, mid, y, o, [&](int i, T v) {
                 epi(i, v, rhs[i]);
@@ -763,7 +887,7 @@ __device__ bool ic_jacobi_apply(Grid& g, const Mat<T>& m, const T* D, const T* r
             });
         }
     }
-    return true;
+    return {true, epi.dot};
 }
 
 // ---- tiled IC(0) sweeps (box-numbered patterns) --------------------------------
@@ -906,11 +1030,18 @@ __device__ __forceinline__ bool patch_cell(const Tiles<T>& tl, int dir, int x0, 
     return in;
 }
 
+// Tiles that block `bid` of a group of `nblocks` takes.
+template <typename T>
+__device__ __forceinline__ int tiles_of(const Tiles<T>& tl, int bid, int nblocks) {
+    const int n = tl.ntx * tl.nty;
+    return bid < n ? (n - 1 - bid) / nblocks + 1 : 0;
+}
+
 // Once per solve, before the first apply (a grid barrier must follow): the
 // pivots into both record kinds, epoch 0 into every edge word, the block's
 // progress counters cleared.
 template <typename T>
-__device__ void tiles_init(Grid& g, const Mat<T>& m, const T* __restrict__ D) {
+__device__ __noinline__ void tiles_init(Grid& g, const Mat<T>& m, const T* __restrict__ D) {
     const Tiles<T>& tl = m.tile;
     extern __shared__ __align__(128) unsigned char tf_smem[];
     const unsigned cb = tl.lu_bf16 ? 2u : (unsigned)sizeof(T);
@@ -982,11 +1113,11 @@ __device__ __forceinline__ bool tile_wait(DevCtl* ctl, long long limit, int wher
 
 // One sweep over this block's tiles, forward (BWD = 0) or backward.  Forward
 // reads rhs and writes tl.mid; backward reads tl.mid and rhs and writes zout,
-// with epi(row, z_row, rhs_row) per row.  False: a wait gave up (the launch
-// is aborted).
+// with epi (RowOp) per row.  Not ok: a wait gave up (the launch is aborted).
 template <int BWD, typename L, typename T, typename Epi>
-__device__ __forceinline__ bool tile_sweep(Grid& g, const Mat<T>& m, const T* __restrict__ rhs,
-                                           T* __restrict__ zout, Epi epi) {
+__device__ __forceinline__ Applied<T> tile_sweep(DevCtl* ctl, long long limit, int bid, int nblocks,
+                                              unsigned epoch, int first, const Mat<T>& m,
+                                              const T* __restrict__ rhs, T* __restrict__ zout, Epi epi) {
     extern __shared__ __align__(128) unsigned char tf_smem[];
     const Tiles<T>& tl = m.tile;
     constexpr unsigned kRec = tile_rec_bytes(sizeof(L), sizeof(T));
@@ -1000,14 +1131,12 @@ __device__ __forceinline__ bool tile_sweep(Grid& g, const Mat<T>& m, const T* __
     // this many behind the one filled.
     constexpr int kDrainLag = (kRing - kSkew) / kTileK - 1;
     constexpr int kNever = -(1 << 20);  // an offset that any progress meets
-    const int lane = g.lane, sw = tl.sw, px = sw > 1 ? 2 : 1, swy = sw / px;
+    const int lane = threadIdx.x & 31, sw = tl.sw, px = sw > 1 ? 2 : 1, swy = sw / px;
     // roles: 0 sweeps, 1 stages, 2 drains, 3 fetches edges
     const int wid = threadIdx.x >> 5, role = wid / sw, w = wid % sw;
-    const int ntiles = tl.ntx * tl.nty, chunks = tl.chunks, nz = tl.nz;
-    const int mine = g.bid < ntiles ? (ntiles - 1 - g.bid) / g.nblocks + 1 : 0;
-    const int first = g.chunk0;
-    g.chunk0 += mine * chunks;
-    if (role >= kWarpsPerPatch) return true;
+    const int chunks = tl.chunks, nz = tl.nz;
+    const int mine = tiles_of(tl, bid, nblocks);
+    if (role >= kWarpsPerPatch) return {true, T(0)};
     const unsigned prog = smem_u32(tf_smem) + 4 * w;  // chunks swept, staged, drained, fetched
     const unsigned staged = prog + 4 * kMaxSweepWarps, drained = staged + 4 * kMaxSweepWarps,
                    fetched = drained + 4 * kMaxSweepWarps;
@@ -1018,7 +1147,7 @@ __device__ __forceinline__ bool tile_sweep(Grid& g, const Mat<T>& m, const T* __
     T* const own = ring + (my + 1) * kRowS + mx + 1;  // this lane's cell in slot 0
     for (int q = 0; q < mine; ++q) {
         const int base = first + q * chunks;
-        const int k = g.bid + (BWD ? mine - 1 - q : q) * g.nblocks;
+        const int k = bid + (BWD ? mine - 1 - q : q) * nblocks;
         const int tx = k % tl.ntx, ty = k / tl.ntx, wx = w % px, wy = w / px;
         const int x0 = (px * tx + wx) * kPatchX, y0 = (swy * ty + wy) * kPatchY;
         if (x0 >= tl.nx || y0 >= tl.ny) {  // no such patch: nothing to hand over
@@ -1062,9 +1191,9 @@ __device__ __forceinline__ bool tile_sweep(Grid& g, const Mat<T>& m, const T* __
             T prev = T(0);
             for (int c = 0; c < chunks; ++c) {
                 const int target = base + min(c + off, chunks);
-                if (!tile_wait(g.ctl, g.timeout_cyc, BWD ? 28 : 26,
+                if (!tile_wait(ctl, limit, BWD ? 28 : 26,
                                [&] { return progress_load(watch) - target >= 0; }))
-                    return false;
+                    return {false, T(0)};
                 const unsigned char* const rc = s_rec + st * kChunkRec;
                 const T* const mc = s_mid + st * (kTileK * 32);
                 T* const cur = own + pos * kSlot;
@@ -1137,8 +1266,8 @@ __device__ __forceinline__ bool tile_sweep(Grid& g, const Mat<T>& m, const T* __
             // chunks stay in flight behind the one handed over.
             constexpr int kFlight = kStages - 2;
             if (BWD && q == 0) {  // it starts from what the forward sweep drained
-                if (!tile_wait(g.ctl, g.timeout_cyc, 29, [&] { return progress_load(drained) - base >= 0; }))
-                    return false;
+                if (!tile_wait(ctl, limit, 29, [&] { return progress_load(drained) - base >= 0; }))
+                    return {false, T(0)};
             }
             // lane 0: the stage is free; the others: the ring slots are
             // drained (the reference's middle step also reads the pivots)
@@ -1151,10 +1280,10 @@ __device__ __forceinline__ bool tile_sweep(Grid& g, const Mat<T>& m, const T* __
             for (int i = 0; i < chunks + kFlight; ++i) {
                 if (i < chunks) {
                     const int target = base + i + off;
-                    if (!tile_wait(g.ctl, g.timeout_cyc, BWD ? 29 : 27,
+                    if (!tile_wait(ctl, limit, BWD ? 29 : 27,
                                    [&] { return progress_load(watch) - target >= 0; })) {
                         cp_async_wait<0>();
-                        return false;
+                        return {false, T(0)};
                     }
                     const unsigned d = s_rec_a + st * kChunkRec;
 #pragma unroll
@@ -1201,7 +1330,6 @@ __device__ __forceinline__ bool tile_sweep(Grid& g, const Mat<T>& m, const T* __
                 progress_store(fetched, base + chunks, lane);
                 continue;
             }
-            const unsigned epoch = g.epoch;
             const bool want_x = up_x == 2 && row_in, want_y = up_y == 2 && x < tl.nx;
             const unsigned char* const in_x =
                 tl.edge[BWD] + ((size_t)((k - kDn) * sw + w + (px - 1) * kDn) * words + lane) * kEdge;
@@ -1222,7 +1350,7 @@ __device__ __forceinline__ bool tile_sweep(Grid& g, const Mat<T>& m, const T* __
                 // (the slots' last readers: the chunk before 32 steps ago)
                 const int room = base + c - (kRing / kTileK - 1);
                 bool again = false;
-                if (!tile_wait(g.ctl, g.timeout_cyc, BWD ? 29 : 27, [&] {
+                if (!tile_wait(ctl, limit, BWD ? 29 : 27, [&] {
                         const bool nx_ = hx && !ex.ready(epoch), ny_ = hy && !ey.ready(epoch);
                         ex.load(cx, again && nx_);
                         ey.load(cy, again && ny_);
@@ -1243,11 +1371,10 @@ __device__ __forceinline__ bool tile_sweep(Grid& g, const Mat<T>& m, const T* __
             fetch(0, ax, ay);
             fetch(1, bx, by);
             for (int c = 0; c < chunks; ++c)
-                if (!(c & 1 ? edges_in(c, bx, by) : edges_in(c, ax, ay))) return false;
+                if (!(c & 1 ? edges_in(c, bx, by) : edges_in(c, ax, ay))) return {false, T(0)};
             continue;
         }
         // ---- draining
-        const unsigned epoch = g.epoch;
         unsigned char* const out_x = tl.edge[BWD] + ((size_t)pt * words + lane) * kEdge;
         unsigned char* const out_y = out_x + (size_t)ywords * kEdge;
         const bool far_x = dn_x == 2 && row_in, far_y = dn_y == 2 && x < tl.nx, publish_far = dn_x == 2 || dn_y == 2;
@@ -1266,9 +1393,9 @@ __device__ __forceinline__ bool tile_sweep(Grid& g, const Mat<T>& m, const T* __
                 }
             }
             const int target = base + c + 1;
-            if (!tile_wait(g.ctl, g.timeout_cyc, BWD ? 29 : 27,
+            if (!tile_wait(ctl, limit, BWD ? 29 : 27,
                            [&] { return progress_load(prog) - target >= 0; }))
-                return false;
+                return {false, T(0)};
             if (publish_far) {
                 const int tx_ = c * kTileK + xq - (kPatchX - 1), ty_ = c * kTileK + my - (kPatchY - 1);  // the reader's steps
                 EdgeWord<T>::store(out_x + (c * kTileK - (kPatchX - 1)) * (int)(kPatchY * kEdge),
@@ -1288,8 +1415,8 @@ __device__ __forceinline__ bool tile_sweep(Grid& g, const Mat<T>& m, const T* __
                 for (int u = 0; u < kTileK; ++u) {
                     T v = vp[u * kSlot];
                     if constexpr (sizeof(T) == 8 && !kRecipDiag64)
-                        v = v / (*reinterpret_cast<const T*>(rc + u * kRec + TileRec<L, T>::at(3, lane)) +
-                                 tiny_v<T>());
+                        v = div_rn(v, *reinterpret_cast<const T*>(rc + u * kRec + TileRec<L, T>::at(3, lane)) +
+                                          tiny_v<T>());
                     mp[u * 32] = v;
                 }
             } else {
@@ -1314,65 +1441,102 @@ __device__ __forceinline__ bool tile_sweep(Grid& g, const Mat<T>& m, const T* __
             st = st + 1 == kStages ? 0 : st + 1;
         }
     }
-    return true;
+    return {true, epi.dot};
 }
 
-// z = IC(0) apply of rhs by the tiled sweeps; epi(row, z_row, rhs_row) per row.
-template <typename T, typename Epi>
-__device__ __forceinline__ bool ic_tiled_apply(Grid& g, const Mat<T>& m, const T* rhs, T* z, Epi epi) {
+// z = IC(0) apply of rhs by the tiled sweeps, epi (RowOp) per row.
+template <typename L, typename T, typename Epi>
+__device__ __forceinline__ Applied<T> ic_tiled_apply(Grid& g, const Mat<T>& m, const T* rhs, T* z, Epi epi) {
+    const int chunks = tiles_of(m.tile, g.bid, g.nblocks) * m.tile.chunks, first = g.chunk0;
     ++g.epoch;
-    if constexpr (sizeof(T) == 4) {
-        if (m.tile.lu_bf16)
-            return tile_sweep<0, unsigned short>(g, m, rhs, z, epi) &&
-                   tile_sweep<1, unsigned short>(g, m, rhs, z, epi);
-    }
-    return tile_sweep<0, T>(g, m, rhs, z, epi) && tile_sweep<1, T>(g, m, rhs, z, epi);
+    g.chunk0 = first + 2 * chunks;
+    // (all warps of the block go on to the backward sweep: its waits end by
+    // the abort flag if the forward sweep of another warp gave up)
+    const RowOp<kRowNone, T> none{T(0), nullptr, T(0)};
+    const bool ok =
+        tile_sweep<0, L, T>(g.ctl, g.timeout_cyc, g.bid, g.nblocks, g.epoch, first, m, rhs, z, none).ok;
+    Applied<T> a =
+        tile_sweep<1, L, T>(g.ctl, g.timeout_cyc, g.bid, g.nblocks, g.epoch, first + chunks, m, rhs, z, epi);
+    a.ok = a.ok && ok;
+    return a;
 }
 
 // The IC(0) apply the solve was configured for: `sweeps` Jacobi sweeps per
 // triangle (FP32 inner solves and contracted FP64 solves), else the exact
 // apply -- tiled sweeps on a box-numbered pattern, level-ordered sync-free
-// sweeps otherwise.  epi(row, z_row, rhs_row) runs once per row.
-template <typename T, typename Epi>
+// sweeps otherwise.  OP, alfa, x: what is done with each row (RowOp); the
+// thread's sum of kRowDot in `dot`.
+template <int OP, typename T>
 __device__ __forceinline__ bool ic_precond(Grid& g, const Mat<T>& m, Vecs<T>& v, int sweeps,
-                                           const T* rhs, T* z, Epi epi) {
-    if (sweeps > 0) return ic_jacobi_apply(g, m, v.D, rhs, v.w, v.s, z, sweeps, epi);
-    if (m.tile.on) return ic_tiled_apply(g, m, rhs, z, epi);
-    return ic_apply(g, m, v.D, rhs, v.w, z, epi);
+                                           const T* rhs, T* z, T& dot, T alfa = T(0), T* x = nullptr) {
+    const RowOp<OP, T> epi{alfa, x, T(0)};
+    Applied<T> a;
+    if (sweeps > 0) {
+        a = ic_jacobi_apply(g, m, v.D, rhs, v.w, v.s, z, sweeps, epi);
+    } else if (m.tile.on) {
+        if constexpr (sizeof(T) == 4)
+            a = m.tile.lu_bf16 ? ic_tiled_apply<unsigned short>(g, m, rhs, z, epi)
+                               : ic_tiled_apply<T>(g, m, rhs, z, epi);
+        else
+            a = ic_tiled_apply<T>(g, m, rhs, z, epi);
+    } else {
+        a = ic_apply(g, m, v.D, rhs, v.w, z, epi);
+    }
+    dot = a.dot;
+    return a.ok;
 }
 
 template <typename T>
 __device__ __forceinline__ bool finite_val(T v) { return isfinite(v); }
 
-// The end of an iteration: two totals, and the third (finite entries of x and
-// r) only once the residual has turned non-finite.
+// The end of an iteration: the totals of r r and of the second sum, and of the
+// third (finite entries of x and r) only once the residual has turned
+// non-finite.  beta, the ratio of the next rho (total `num`) and the current
+// one, which it replaces, is formed by the summing thread (`next_rho`).
+struct IterEnd {
+    double rr;       // ||r||^2
+    double beta;
+    bool converged;
+    bool all_nan;    // (with `all`) no entry of x and r is a number
+};
 template <typename T>
-__device__ __forceinline__ bool reduce_watched(Grid& g, int slot, const T (&a)[3], bool all, int where,
-                                               double (&t)[3]) {
+__device__ __forceinline__ bool reduce_end(Grid& g, int slot, const T (&a)[3], bool all, int where, int num,
+                                           bool next_rho, IterEnd& e) {
+    e.all_nan = false;
     if (all) {
-        publish_t<3>(g, slot, a);
+        const T c[1] = {a[2]};
+        publish_t<1>(g, slot + 2, c);
         if (!grid_sync(g, where)) return false;
-        totals<3>(g, slot, t);
-    } else {
-        const T b[2] = {a[0], a[1]};
-        publish_t<2>(g, slot, b);
-        if (!grid_sync(g, where)) return false;
-        double u[2];
-        totals<2>(g, slot, u);
-        t[0] = u[0];
-        t[1] = u[1];
-        t[2] = 0.0;
+        double t[1];
+        totals<1>(g, slot + 2, t);
+        e.all_nan = t[0] == 0.0;
     }
+    const T b[2] = {a[0], a[1]};
+    publish_t<2>(g, slot, b);
+    if (!grid_sync(g, where)) return false;
+    double u[2], x[2];
+    totals<2>(g, slot, u, x, [&](int k, double s) {
+        double r = 0.0;
+        if (k == num && next_rho) {
+            r = div_rn(s, scalars().rho);
+            scalars().rho = s;
+        }
+        if (k == 0) scalars().rr = s;
+        return r;
+    });
+    e.rr = u[0];
+    e.beta = x[num];
+    e.converged = scalars().conv.below(u[0]);
     return true;
 }
 
 // ---- the reference prologue: Prec1, ||b||, Resid, IniRes -------------------
 // Returns false when the launch aborted or an early exit was taken (out
-// records which).  On return true, `err` holds ||r0|| and, for prec 1 / 0,
-// rho0 = (r0, M^-1 r0) is in `rho0` (z written for prec 1).
+// records which).  On return true, the block's scalars hold the tolerance and,
+// for prec 1 / 0, rho = (r0, M^-1 r0) (z written for prec 1).
 template <typename T>
-__device__ bool prologue(Grid& g, const Mat<T>& m, Vecs<T>& v, const SolveCfg& cfg, SolveOut& out,
-                         double& tol, double& err, double& rho0, bool store_z) {
+__device__ __noinline__ bool prologue(Grid& g, const Mat<T>& m, Vecs<T>& v, const SolveCfg& cfg, SolveOut& out,
+                         bool store_z) {
     if (cfg.do_prec1 && !prec1_phase(g, m, v.D, cfg.prec)) {
         out.exit_kind = EXIT_ABORT;
         return false;
@@ -1389,9 +1553,10 @@ __device__ bool prologue(Grid& g, const Mat<T>& m, Vecs<T>& v, const SolveCfg& c
     }
     publish_t<1>(g, SLOT_A, acc);
     if (!grid_sync(g, 30)) { out.exit_kind = EXIT_ABORT; return false; }
-    double tot[1];
-    totals<1>(g, SLOT_A, tot);
-    const double bnrm2 = sqrt(tot[0]);
+    double tot[1], nrm[1];
+    totals<1>(g, SLOT_A, tot, nrm, [](int, double s) { return sqrt(s); });
+    const double bnrm2 = nrm[0];
+    double tol = cfg.tol;
     out.bnrm2 = bnrm2;
     if (cfg.tol_is_relative) tol = tol * bnrm2;
     if (bnrm2 < tol || (cfg.tol_is_relative && bnrm2 == 0.0)) {
@@ -1418,162 +1583,112 @@ __device__ bool prologue(Grid& g, const Mat<T>& m, Vecs<T>& v, const SolveCfg& c
     }
     publish_t<2>(g, SLOT_B, a2);
     if (!grid_sync(g, 31)) { out.exit_kind = EXIT_ABORT; return false; }
-    double t2[2];
-    totals<2>(g, SLOT_B, t2);
-    err = sqrt(t2[0]);
+    double t2[2], e2[2];
+    totals<2>(g, SLOT_B, t2, e2, [](int k, double s) { return k == 0 ? sqrt(s) : 0.0; });
+    const double err = e2[0];
     out.ini_res = err;
     out.fin_res = err;
-    rho0 = cfg.prec == 1 ? t2[1] : t2[0];
     if (err < tol) {
         out.exit_kind = EXIT_INIRES;
         out.iterations = 0;
         return false;
     }
+    if (threadIdx.x == 0) {
+        scalars().conv.set(tol);
+        scalars().rho = cfg.prec == 1 ? t2[1] : t2[0];
+    }
+    __syncthreads();
     return true;
 }
 
 // ---- CG (Process/CG.f90:113-259; also BiCG, whose iterates are CG's) --------
 template <typename T>
 __device__ void cg_solve(Grid& g, const Mat<T>& m, Vecs<T>& v, const SolveCfg& cfg, SolveOut& out) {
-    double tol = cfg.tol, err = 0.0, rho_next = 0.0;
-    if (!prologue(g, m, v, cfg, out, tol, err, rho_next, true)) return;
+    if (!prologue(g, m, v, cfg, out, true)) return;
     const int prec = (cfg.prec == 1 || cfg.prec == 2) ? cfg.prec : 0;
     const T* z = prec == 0 ? v.r : v.z;
-    double rho = 0.0, rhoold = 0.0;
     bool nonfinite = false;
     int iter = 1;
-    // search direction; the FP32 inner solves alternate between p and t
+    T beta = T(0);
+    IterEnd e;
+    // search direction; formed inside the product it alternates between p and t
     T* pcur = v.p;
     T* pnext = v.t;
     for (; iter <= cfg.maxiter; ++iter) {
         if (prec == 2) {
-            T a[1] = {T(0)};
-            const bool ok = ic_precond(g, m, v, cfg.ic_sweeps, v.r, v.z, [&](int, T zi, T ri) {
-                a[0] += ri * zi;
-            });
+            T a[1];
+            const bool ok = ic_precond<kRowDot>(g, m, v, cfg.ic_sweeps, v.r, v.z, a[0]);
             publish_t<1>(g, SLOT_A, a);
             if (!grid_sync(g, 41) || !ok) { out.exit_kind = EXIT_ABORT; return; }
-            double t[1];
-            totals<1>(g, SLOT_A, t);
-            rho = t[0];
-        } else {
-            rho = rho_next;
+            double t[1], x[1];
+            totals<1>(g, SLOT_A, t, x, [&](int, double s) {
+                const double b = iter == 1 ? 0.0 : div_rn(s, scalars().rho);
+                scalars().rho = s;
+                return b;
+            });
+            beta = T(x[0]);
         }
         // The new search direction formed inside the product, into the other
         // p buffer (no separate update pass, one barrier less per
         // iteration): always in the FP32 inner solves; in FP64 where the
-        // host asked for it (systems whose vectors stay in L2 -- on larger
-        // ones gathering z and p and forming z + beta p per neighbour on the
-        // FP64 pipe costs more than the pass it saves).
-        const bool fused = sizeof(T) == 4 || cfg.fuse_dir;
-        if (fused) {
-            const T beta = iter == 1 ? T(0) : T(rho / rhoold);
-            const bool first = iter == 1;
-            const T* pold = pcur;
-            T* pnew = pnext;
-            T a1[1] = {T(0)};
-            for (int s = g.wg; s < m.nslices; s += g.nw) {
-                const int i = s * kWarp + g.lane;
-                const T qi = sell_row_dir(m, s, g.lane, z, pold, beta, first);
-                if (i < m.n) {
-                    const T pi = fused_dir(z[i], beta, first ? T(0) : pold[i], first);
-                    pnew[i] = pi;
-                    v.q[i] = qi;
-                    a1[0] += pi * qi;
-                }
-            }
+        // host asked for it (small systems -- on larger ones gathering z and
+        // p and forming z + beta p per neighbour on the FP64 pipe costs more
+        // than the pass it saves).
+        T a1[1];
+        if (sizeof(T) == 4 || cfg.fuse_dir) {
+            T* const pnew = pnext;
+            a1[0] = product_phase<T, true>(m, g.wg, g.nw, z, pcur, pnew, v.q, nullptr, beta, iter == 1);
+            pnext = pcur;
             pcur = pnew;
-            pnext = const_cast<T*>(pold);
-            publish_t<1>(g, SLOT_C, a1);
-            if (!grid_sync(g, 43)) { out.exit_kind = EXIT_ABORT; return; }
-        }
-        if (!fused) {
-        // p = z + beta p  (CG.f90:178-187)
-        if (iter == 1) {
-            TF_FOR4(g, m, i) { st4(v.p + i, ld4(z + i)); }
         } else {
-            const T beta = T(rho / rhoold);
-            TF_FOR4(g, m, i) {
-                const V4<T> zz = ld4(z + i);
-                V4<T> pp = ld4(v.p + i);
-#pragma unroll
-                for (int u = 0; u < 4; ++u) pp.a[u] = zz.a[u] + beta * pp.a[u];
-                st4(v.p + i, pp);
-            }
-        }
-        if (!grid_sync(g, 42)) { out.exit_kind = EXIT_ABORT; return; }
-        // q = A p; (p, q)  (CG.f90:193-218)
-        T a1[1] = {T(0)};
-        for (int s = g.wg; s < m.nslices; s += g.nw) {
-            const int i = s * kWarp + g.lane;
-            const T qi = sell_row(m, s, g.lane, v.p);
-            if (i < m.n) {
-                v.q[i] = qi;
-                a1[0] += v.p[i] * qi;
-            }
+            direction_phase(g.tid, g.nt, m.n, z, v.p, beta, iter == 1);
+            if (!grid_sync(g, 42)) { out.exit_kind = EXIT_ABORT; return; }
+            // q = A p; (p, q)  (CG.f90:193-218)
+            a1[0] = product_phase<T, false>(m, g.wg, g.nw, nullptr, v.p, nullptr, v.q, v.p, T(0), false);
         }
         publish_t<1>(g, SLOT_C, a1);
         if (!grid_sync(g, 43)) { out.exit_kind = EXIT_ABORT; return; }
-        }
-        double t1[1];
-        totals<1>(g, SLOT_C, t1);
-        const double alfa_d = rho / t1[0];
-        const T alfa = T(alfa_d);
+        double t1[1], x1[1];
+        totals<1>(g, SLOT_C, t1, x1, [&](int, double s) { return div_rn(scalars().rho, s); });
+        const T alfa = T(x1[0]);
         // x += alfa p; r -= alfa q; ||r||; next z and rho  (CG.f90:226-253)
-        T a3[3] = {T(0), T(0), T(0)};
-        TF_FOR4(g, m, i) {
-            V4<T> xx = ld4(v.x + i), rr = ld4(v.r + i);
-            const V4<T> pp = ld4(pcur + i), qq = ld4(v.q + i);
-            V4<T> dd, zz;
-            if (prec == 1) dd = ld4(v.D + i);
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                xx.a[u] = xx.a[u] + alfa * pp.a[u];
-                rr.a[u] = rr.a[u] - alfa * qq.a[u];
-                if (prec == 1) zz.a[u] = jacobi(rr.a[u], dd.a[u]);
-                if (i + u < m.n) {
-                    a3[0] += rr.a[u] * rr.a[u];
-                    if (prec == 1) a3[1] += rr.a[u] * zz.a[u];
-                    if (nonfinite)
-                        a3[2] += (xx.a[u] == xx.a[u] ? T(1) : T(0)) + (rr.a[u] == rr.a[u] ? T(1) : T(0));
-                }
-            }
-            st4(v.x + i, xx);
-            st4(v.r + i, rr);
-            if (prec == 1) st4(v.z + i, zz);
-        }
-        double t3[3];
-        if (!reduce_watched(g, SLOT_D, a3, nonfinite, 44, t3)) { out.exit_kind = EXIT_ABORT; return; }
-        err = sqrt(t3[0]);
-        out.fin_res = err;
-        if (err < tol) {
-            out.exit_kind = EXIT_CONVERGED;
-            out.iterations = iter;
+        const Sums3<T> a3 =
+            update_phase(g.tid, g.nt, m.n, v.x, v.r, pcur, v.q, v.D, v.z, alfa, prec == 1, nonfinite);
+        if (!reduce_end(g, SLOT_D, a3.a, nonfinite, 44, prec == 1 ? 1 : 0, prec != 2, e)) {
+            out.exit_kind = EXIT_ABORT;
             return;
         }
-        rho_next = prec == 1 ? t3[1] : t3[0];
-        if (!finite_val(err)) {
+        beta = T(e.beta);
+        if (e.converged) {
+            out.exit_kind = EXIT_CONVERGED;
+            out.iterations = iter;
+            out.fin_res = sqrt(e.rr);
+            return;
+        }
+        if (!finite_val(e.rr)) {
             // From here on the reference keeps iterating on non-finite
             // values; once every x and r entry is NaN nothing changes any
             // more, so the remaining iterations can be skipped.
-            if (nonfinite && t3[2] == 0.0) {
+            if (e.all_nan) {
                 out.exit_kind = EXIT_NONFINITE;
                 out.iterations = cfg.maxiter + 1;
+                out.fin_res = sqrt(e.rr);
                 return;
             }
             nonfinite = true;
         }
-        rhoold = rho;
     }
     out.exit_kind = EXIT_MAXITER;
     out.iterations = iter;
+    if (iter > 1) out.fin_res = sqrt(scalars().rr);
 }
 
 // ---- CGS (Process/CGS.f90:112-333) -------------------------------------------
 template <typename T>
 __device__ void cgs_solve(Grid& g, const Mat<T>& m, Vecs<T>& v, const SolveCfg& cfg, SolveOut& out) {
-    double tol = cfg.tol, err = 0.0, dummy = 0.0;
-    if (!prologue(g, m, v, cfg, out, tol, err, dummy, false)) return;
+    if (!prologue(g, m, v, cfg, out, false)) return;
+    T beta = T(0);
+    IterEnd e;
     const int prec = (cfg.prec == 1 || cfg.prec == 2) ? cfg.prec : 0;
     // r2 = r1 (CGS.f90:84-86); rho = (r1, r2) for the first iteration.
     T a0[1] = {T(0)};
@@ -1586,14 +1701,12 @@ __device__ void cgs_solve(Grid& g, const Mat<T>& m, Vecs<T>& v, const SolveCfg& 
     }
     publish_t<1>(g, SLOT_A, a0);
     if (!grid_sync(g, 50)) { out.exit_kind = EXIT_ABORT; return; }
-    double t0[1];
-    totals<1>(g, SLOT_A, t0);
-    double rho = t0[0], rhoold = 0.0;
+    double t0[1], x0[1];
+    totals<1>(g, SLOT_A, t0, x0, [](int, double s) { return scalars().rho = s; });
     bool nonfinite = false;
     int iter = 1;
     for (; iter <= cfg.maxiter; ++iter) {
         // u1 = r1 + beta q1; u2 = u1 + beta (q1 + beta u2); p2 = M^-1 u2
-        const T beta = T(iter == 1 ? 0.0 : rho / rhoold);
         TF_FOR4(g, m, i) {
             const V4<T> rr = ld4(v.r + i);
             V4<T> u1, u2, p2;
@@ -1622,24 +1735,17 @@ __device__ void cgs_solve(Grid& g, const Mat<T>& m, Vecs<T>& v, const SolveCfg& 
         }
         if (!grid_sync(g, 51)) { out.exit_kind = EXIT_ABORT; return; }
         if (prec == 2) {
-            const bool ok = ic_precond(g, m, v, cfg.ic_sweeps, v.u2, v.p2, [](int, T, T) {});
+            T none;
+            const bool ok = ic_precond<kRowNone>(g, m, v, cfg.ic_sweeps, v.u2, v.p2, none);
             if (!grid_sync(g, 53) || !ok) { out.exit_kind = EXIT_ABORT; return; }
         }
         // v2 = A p2; alfa = rho / (r2, v2)
-        T a1[1] = {T(0)};
-        for (int s = g.wg; s < m.nslices; s += g.nw) {
-            const int i = s * kWarp + g.lane;
-            const T vi = sell_row(m, s, g.lane, v.p2);
-            if (i < m.n) {
-                v.v2[i] = vi;
-                a1[0] += v.r2[i] * vi;
-            }
-        }
+        const T a1[1] = {product_phase<T, false>(m, g.wg, g.nw, nullptr, v.p2, nullptr, v.v2, v.r2, T(0), false)};
         publish_t<1>(g, SLOT_B, a1);
         if (!grid_sync(g, 54)) { out.exit_kind = EXIT_ABORT; return; }
-        double t1[1];
-        totals<1>(g, SLOT_B, t1);
-        const T alfa = T(rho / t1[0]);
+        double t1[1], x1[1];
+        totals<1>(g, SLOT_B, t1, x1, [&](int, double s) { return div_rn(scalars().rho, s); });
+        const T alfa = T(x1[0]);
         // q1 = u1 - alfa v2; p1 = M^-1 (u1 + q1); x += alfa p1
         TF_FOR4(g, m, i) {
             const V4<T> u1 = ld4(v.u1 + i), v2 = ld4(v.v2 + i);
@@ -1667,10 +1773,8 @@ __device__ void cgs_solve(Grid& g, const Mat<T>& m, Vecs<T>& v, const SolveCfg& 
         }
         if (!grid_sync(g, 55)) { out.exit_kind = EXIT_ABORT; return; }
         if (prec == 2) {
-            T* xx = v.x;
-            const bool ok = ic_precond(g, m, v, cfg.ic_sweeps, v.t, v.p, [&](int row, T p1, T) {
-                xx[row] = xx[row] + alfa * p1;
-            });
+            T none;
+            const bool ok = ic_precond<kRowAxpy>(g, m, v, cfg.ic_sweeps, v.t, v.p, none, alfa, v.x);
             if (!grid_sync(g, 57) || !ok) { out.exit_kind = EXIT_ABORT; return; }
         }
         // q2 = A p1; r1 -= alfa q2; ||r1||; next rho = (r1, r2)
@@ -1689,28 +1793,30 @@ __device__ void cgs_solve(Grid& g, const Mat<T>& m, Vecs<T>& v, const SolveCfg& 
                 }
             }
         }
-        double t3[3];
-        if (!reduce_watched(g, SLOT_C, a3, nonfinite, 58, t3)) { out.exit_kind = EXIT_ABORT; return; }
-        err = sqrt(t3[0]);
-        out.fin_res = err;
-        if (err < tol) {
-            out.exit_kind = EXIT_CONVERGED;
-            out.iterations = iter;
+        if (!reduce_end(g, SLOT_C, a3, nonfinite, 58, 1, true, e)) {
+            out.exit_kind = EXIT_ABORT;
             return;
         }
-        if (!finite_val(err)) {
-            if (nonfinite && t3[2] == 0.0) {
+        beta = T(e.beta);
+        if (e.converged) {
+            out.exit_kind = EXIT_CONVERGED;
+            out.iterations = iter;
+            out.fin_res = sqrt(e.rr);
+            return;
+        }
+        if (!finite_val(e.rr)) {
+            if (e.all_nan) {
                 out.exit_kind = EXIT_NONFINITE;
                 out.iterations = cfg.maxiter + 1;
+                out.fin_res = sqrt(e.rr);
                 return;
             }
             nonfinite = true;
         }
-        rhoold = rho;
-        rho = t3[1];
     }
     out.exit_kind = EXIT_MAXITER;
     out.iterations = iter;
+    if (iter > 1) out.fin_res = sqrt(scalars().rr);
 }
 
 // ---- BiCG with the transposed shadow sequence (extension) ---------------------
@@ -1721,8 +1827,9 @@ __device__ void cgs_solve(Grid& g, const Mat<T>& m, Vecs<T>& v, const SolveCfg& 
 template <typename T>
 __device__ void bicg_true_solve(Grid& g, const Mat<T>& m, const Mat<T>& mT, Vecs<T>& v,
                                 const SolveCfg& cfg, SolveOut& out) {
-    double tol = cfg.tol, err = 0.0, dummy = 0.0;
-    if (!prologue(g, m, v, cfg, out, tol, err, dummy, false)) return;
+    if (!prologue(g, m, v, cfg, out, false)) return;
+    T beta = T(0);
+    IterEnd e;
     const bool diag = cfg.prec == 1;
     T* z2 = v.u1;
     T* q2 = v.v2;
@@ -1745,12 +1852,10 @@ __device__ void bicg_true_solve(Grid& g, const Mat<T>& m, const Mat<T>& mT, Vecs
     }
     publish_t<1>(g, SLOT_A, a0);
     if (!grid_sync(g, 60)) { out.exit_kind = EXIT_ABORT; return; }
-    double t0[1];
-    totals<1>(g, SLOT_A, t0);
-    double rho = t0[0], rhoold = 0.0;
+    double t0[1], x0[1];
+    totals<1>(g, SLOT_A, t0, x0, [](int, double s) { return scalars().rho = s; });
     int iter = 1;
     for (; iter <= cfg.maxiter; ++iter) {
-        const T beta = T(iter == 1 ? 0.0 : rho / rhoold);
         TF_FOR4(g, m, i) {
             const V4<T> z = ld4(v.z + i), zz = ld4(z2 + i);
             V4<T> p = z, pp = zz;
@@ -1780,10 +1885,10 @@ __device__ void bicg_true_solve(Grid& g, const Mat<T>& m, const Mat<T>& mT, Vecs
         }
         publish_t<1>(g, SLOT_B, a1);
         if (!grid_sync(g, 62)) { out.exit_kind = EXIT_ABORT; return; }
-        double t1[1];
-        totals<1>(g, SLOT_B, t1);
-        const T alfa = T(rho / t1[0]);
-        T a3[2] = {T(0), T(0)};
+        double t1[1], x1[1];
+        totals<1>(g, SLOT_B, t1, x1, [&](int, double s) { return div_rn(scalars().rho, s); });
+        const T alfa = T(x1[0]);
+        T a3[3] = {T(0), T(0), T(0)};
         TF_FOR4(g, m, i) {
             V4<T> x = ld4(v.x + i), r = ld4(v.r + i), rr = ld4(v.r2 + i);
             const V4<T> p = ld4(v.p + i), q = ld4(v.q + i), qq = ld4(q2 + i);
@@ -1807,27 +1912,24 @@ __device__ void bicg_true_solve(Grid& g, const Mat<T>& m, const Mat<T>& mT, Vecs
             st4(v.z + i, z);
             st4(z2 + i, zz);
         }
-        publish_t<2>(g, SLOT_C, a3);
-        if (!grid_sync(g, 63)) { out.exit_kind = EXIT_ABORT; return; }
-        double t3[2];
-        totals<2>(g, SLOT_C, t3);
-        err = sqrt(t3[0]);
-        out.fin_res = err;
-        if (err < tol) {
+        if (!reduce_end(g, SLOT_C, a3, false, 63, 1, true, e)) { out.exit_kind = EXIT_ABORT; return; }
+        beta = T(e.beta);
+        if (e.converged) {
             out.exit_kind = EXIT_CONVERGED;
             out.iterations = iter;
+            out.fin_res = sqrt(e.rr);
             return;
         }
-        if (!finite_val(err)) {
+        if (!finite_val(e.rr)) {
             out.exit_kind = EXIT_NONFINITE;
             out.iterations = cfg.maxiter + 1;
+            out.fin_res = sqrt(e.rr);
             return;
         }
-        rhoold = rho;
-        rho = t3[1];
     }
     out.exit_kind = EXIT_MAXITER;
     out.iterations = iter;
+    if (iter > 1) out.fin_res = sqrt(scalars().rr);
 }
 
 // ---- mixed precision: FP32 inner Krylov inside FP64 iterative refinement ---------
@@ -1877,9 +1979,9 @@ __device__ __forceinline__ bool mixed_residual(Grid& g, const Mat<double>& m64, 
     }
     publish<1>(g, SLOT_D + 3, a);
     if (!grid_sync(g, 70)) return false;
-    double t[1];
-    totals<1>(g, SLOT_D + 3, t);
-    err = sqrt(t[0]);
+    double t[1], e[1];
+    totals<1>(g, SLOT_D + 3, t, e, [](int, double s) { return sqrt(s); });
+    err = e[0];
     return true;
 }
 
@@ -1898,7 +2000,7 @@ static __device__ void mixed_solve(Grid& g, const Mat<double>& m64, const Mat<fl
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             // FP32 solves hold 1/D for the diagonal preconditioner
-            df.a[u] = c.prec == 1 ? (float)(kRecipDiag64 ? d.a[u] : 1.0 / d.a[u])
+            df.a[u] = c.prec == 1 ? (float)(kRecipDiag64 ? d.a[u] : div_rn(1.0, d.a[u]))
                                   : (float)d.a[u];
             wf.a[u] = Cell<float>::sentinel();
             if (i + u < m64.n) acc[0] += bb.a[u] * bb.a[u];
@@ -1910,9 +2012,9 @@ static __device__ void mixed_solve(Grid& g, const Mat<double>& m64, const Mat<fl
     if (!grid_sync(g, 71)) return;
     // (the residual pass below ends with a barrier before the first apply)
     if (c.prec == 2 && m32.tile.on) tiles_init(g, m32, v32.D);
-    double tot[1];
-    totals<1>(g, SLOT_A, tot);
-    const double bnrm2 = sqrt(tot[0]);
+    double tot[1], nrm[1];
+    totals<1>(g, SLOT_A, tot, nrm, [](int, double s) { return sqrt(s); });
+    const double bnrm2 = nrm[0];
     out.bnrm2 = bnrm2;
     double tol = c.tol_is_relative ? c.tol * bnrm2 : c.tol;
     if (bnrm2 < tol || (c.tol_is_relative && bnrm2 == 0.0)) {
@@ -2028,7 +2130,7 @@ static __device__ void mixed_cg_reliable(Grid& g, const Mat<double>& m64, const 
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             // FP32 solves hold 1/D for the diagonal preconditioner
-            df.a[u] = c.prec == 1 ? (float)(kRecipDiag64 ? d.a[u] : 1.0 / d.a[u])
+            df.a[u] = c.prec == 1 ? (float)(kRecipDiag64 ? d.a[u] : div_rn(1.0, d.a[u]))
                                   : (float)d.a[u];
             wf.a[u] = Cell<float>::sentinel();
             if (i + u < m64.n) acc[0] += bb.a[u] * bb.a[u];
@@ -2039,9 +2141,9 @@ static __device__ void mixed_cg_reliable(Grid& g, const Mat<double>& m64, const 
     publish<1>(g, SLOT_A, acc);
     if (!grid_sync(g, 81)) return;
     if (c.prec == 2 && m32.tile.on) tiles_init(g, m32, v.D);
-    double tot[1];
-    totals<1>(g, SLOT_A, tot);
-    const double bnrm2 = sqrt(tot[0]);
+    double tot[1], nrm[1];
+    totals<1>(g, SLOT_A, tot, nrm, [](int, double s) { return sqrt(s); });
+    const double bnrm2 = nrm[0];
     out.bnrm2 = bnrm2;
     const double tol = c.tol_is_relative ? c.tol * bnrm2 : c.tol;
     if (bnrm2 < tol || (c.tol_is_relative && bnrm2 == 0.0)) {
@@ -2080,26 +2182,30 @@ static __device__ void mixed_cg_reliable(Grid& g, const Mat<double>& m64, const 
         }
         publish<3>(g, SLOT_D, a);
         if (!grid_sync(g, 82)) return false;
-        double t[3];
-        totals<3>(g, SLOT_D, t);
-        err = sqrt(t[0]);
+        double t[3], e[3];
+        totals<3>(g, SLOT_D, t, e, [](int k, double s) { return k == 1 ? 0.0 : sqrt(s); });
+        err = e[0];
         rz = t[1];
-        if (drift) *drift = sqrt(t[2]);
+        if (drift) *drift = e[2];
         return true;
     };
-    auto ic = [&](double& rz) -> bool {
-        float a[1] = {0.f};
-        const bool ok = ic_precond(g, m32, v, c.ic_sweeps, v.r, v.z, [&](int, float zi, float ri) {
-            a[0] += ri * zi;
-        });
+    // rho = (r, M^-1 r), beta its ratio to the rho before
+    auto ic = [&](float& beta) -> bool {
+        float a[1];
+        const bool ok = ic_precond<kRowDot>(g, m32, v, c.ic_sweeps, v.r, v.z, a[0]);
         publish_t<1>(g, SLOT_A, a);
         if (!grid_sync(g, 83) || !ok) return false;
-        double t[1];
-        totals<1>(g, SLOT_A, t);
-        rz = t[0];
+        double t[1], e[1];
+        totals<1>(g, SLOT_A, t, e, [&](int, double s) {
+            const double b = div_rn(s, scalars().rho);
+            scalars().rho = s;
+            return b;
+        });
+        beta = (float)e[0];
         return true;
     };
     double err, rz;
+    const double delta = c.inner_rtol > 0.0 && c.inner_rtol < 1.0 ? c.inner_rtol : 0.1;
     if (!refresh(c.x_is_zero != 0, err, rz, nullptr)) return;
     out.ini_res = err;
     out.fin_res = err;
@@ -2108,77 +2214,60 @@ static __device__ void mixed_cg_reliable(Grid& g, const Mat<double>& m64, const 
         out.iterations = 0;
         return;
     }
-    if (prec == 2 && !ic(rz)) return;
+    float beta = 0.0f;
+    if (threadIdx.x == 0) {
+        scalars().rho = rz;
+        scalars().conv.set(tol);
+        scalars().refine.set(delta * err);
+    }
+    __syncthreads();
+    if (prec == 2 && !ic(beta)) return;
     // best FP64 iterate so far (returned if the iteration later diverges)
     auto keep_best = [&]() {
         TF_FOR4(g, m64, i) { st4(xbest + i, ld4(x64 + i)); }
     };
     keep_best();
-    double rho = rz, maxr = err, prev = err, best = err;
+    double prev = err, best = err;
     int nref = 0, stall = 0, it = 1;
     bool diverged = false, fresh = false;
-    const double delta = c.inner_rtol > 0.0 && c.inner_rtol < 1.0 ? c.inner_rtol : 0.1;
-    float beta = 0.0f;
+    float *pcur = v.p, *pnext = v.t;
     for (; it <= c.maxiter; ++it) {
-        if (it == 1 || fresh) {
-            TF_FOR4(g, m32, i) { st4(v.p + i, ld4(z + i)); }
-            fresh = false;
-        } else {
-            TF_FOR4(g, m32, i) {
-                const V4<float> zz = ld4(z + i);
-                V4<float> pp = ld4(v.p + i);
-#pragma unroll
-                for (int u = 0; u < 4; ++u) pp.a[u] = zz.a[u] + beta * pp.a[u];
-                st4(v.p + i, pp);
-            }
-        }
-        if (!grid_sync(g, 84)) return;
-        float a1[1] = {0.f};
-        for (int s = g.wg; s < m32.nslices; s += g.nw) {
-            const int i = s * kWarp + g.lane;
-            const float qi = sell_row(m32, s, g.lane, v.p);
-            if (i < m32.n) {
-                v.q[i] = qi;
-                a1[0] += v.p[i] * qi;
-            }
-        }
+        // the direction formed inside the product, into the other buffer
+        const float a1[1] = {product_phase<float, true>(m32, g.wg, g.nw, z, pcur, pnext, v.q, nullptr, beta,
+                                                        it == 1 || fresh)};
+        fresh = false;
+        float* const pold = pcur;
+        pcur = pnext;
+        pnext = pold;
         publish_t<1>(g, SLOT_C, a1);
         if (!grid_sync(g, 85)) return;
-        double t1[1];
-        totals<1>(g, SLOT_C, t1);
-        const float alfa = (float)(rho / t1[0]);
-        float a3[2] = {0.f, 0.f};
-        TF_FOR4(g, m32, i) {
-            V4<float> xx = ld4(v.x + i), rr = ld4(v.r + i), zz;
-            const V4<float> pp = ld4(v.p + i), qq = ld4(v.q + i);
-            V4<float> dd;
-            if (prec == 1) dd = ld4(v.D + i);
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                xx.a[u] = xx.a[u] + alfa * pp.a[u];
-                rr.a[u] = rr.a[u] - alfa * qq.a[u];
-                if (prec == 1) zz.a[u] = jacobi(rr.a[u], dd.a[u]);
-                if (i + u < m32.n) {
-                    a3[0] += rr.a[u] * rr.a[u];
-                    if (prec == 1) a3[1] += rr.a[u] * zz.a[u];
-                }
-            }
-            st4(v.x + i, xx);
-            st4(v.r + i, rr);
-            if (prec == 1) st4(v.z + i, zz);
-        }
+        double t1[1], e1[1];
+        totals<1>(g, SLOT_C, t1, e1, [&](int, double s) { return div_rn(scalars().rho, s); });
+        const float alfa = (float)e1[0];
+        const Sums3<float> u3 =
+            update_phase(g.tid, g.nt, m32.n, v.x, v.r, pcur, v.q, v.D, v.z, alfa, prec == 1, false);
+        const float a3[2] = {u3.a[0], u3.a[1]};
         publish_t<2>(g, SLOT_B, a3);
         if (!grid_sync(g, 86)) return;
-        double t3[2];
-        totals<2>(g, SLOT_B, t3);
-        const double rnorm = sqrt(t3[0]);
+        double t3[2], e3[2];
+        totals<2>(g, SLOT_B, t3, e3, [&](int k, double s) {  // next beta; whether to refine
+            if (k == 0 && prec != 0) return scalars().refine.below(s) || scalars().conv.below(s) ? 1.0 : 0.0;
+            if (prec == 2 || k != (prec == 1 ? 1 : 0)) return 0.0;
+            const double b = div_rn(s, scalars().rho);
+            scalars().rho_old = scalars().rho;
+            scalars().rho = s;
+            return b;
+        });
         out.iterations = it;
-        rz = prec == 1 ? t3[1] : t3[0];
-        if (!isfinite(rnorm)) {
+        if (!isfinite(t3[0])) {
             out.exit_kind = EXIT_NONFINITE;
             return;
         }
-        if (rnorm < delta * maxr || rnorm < tol) {
+        beta = (float)e3[prec == 1 ? 1 : 0];
+        const bool refine = prec != 0 ? e3[0] != 0.0
+                                      : scalars().refine.below(t3[0]) || scalars().conv.below(t3[0]);
+        if (refine) {
+            const double rnorm = sqrt(t3[0]);
             // refinement: x += xl in FP64, true residual, FP64 test
             TF_FOR4(g, m64, i) {
                 V4<double> xd = ld4(x64 + i);
@@ -2215,11 +2304,19 @@ static __device__ void mixed_cg_reliable(Grid& g, const Mat<double>& m64, const 
             stall = err > 0.999 * prev ? stall + 1 : 0;
             if (stall >= 4) break;
             prev = err;
-            maxr = err;
+            // the next rho is that of the refreshed residual; beta its ratio
+            // to the rho of the direction kept
+            if (threadIdx.x == 0) {
+                scalars().refine.set(delta * err);
+                if (prec != 2) {
+                    scalars().beta = div_rn(rz, scalars().rho_old);
+                    scalars().rho = rz;
+                }
+            }
+            __syncthreads();
+            if (prec != 2) beta = (float)scalars().beta;
         }
-        if (prec == 2 && !ic(rz)) return;
-        beta = (float)(rz / rho);
-        rho = rz;
+        if (prec == 2 && !ic(beta)) return;
     }
     // out of iterations: fold the pending correction into x, and fall back
     // to the best iterate if this one is worse

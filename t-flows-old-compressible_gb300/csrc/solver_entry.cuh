@@ -1,12 +1,12 @@
 // Kernel entry points of the persistent solvers and their parameter blocks.
 //
-// Included by two translation units that compile the same solver code with
+// Included by translation units that compile the same solver code with
 // different arithmetic: krylov.cu (namespace tflows::ref) with --fmad=false,
 // where every a*b+c is a rounded product followed by a rounded sum and the
-// diagonal preconditioner divides, as the reference does; krylov_fma.cu
-// (namespace tflows::fma) with contraction into fused multiply-adds and a
-// reciprocal diagonal, for the TFLOWS_FP64_FMA solves and the mixed-precision
-// solves.  The parameter blocks are shared types; the kernels of each unit
+// diagonal preconditioner divides, as the reference does; krylov_fma.cu and
+// krylov_mixed.cu (namespace tflows::fma) with contraction
+// into fused multiply-adds and a reciprocal diagonal, for the TFLOWS_FP64_FMA
+// solves and the mixed-precision solves.  The parameter blocks are shared types; the kernels of each unit
 // live in its own namespace so that the two builds never merge.
 #pragma once
 
@@ -72,7 +72,7 @@ struct BatchItem {
 
 namespace TFLOWS_KNS {
 
-__device__ int status_of(const SolveOut& o, const DevCtl* ctl) {
+static __device__ int status_of(const SolveOut& o, const DevCtl* ctl) {
     if (ctl->status != 0) return ctl->status;
     switch (o.exit_kind) {
         case EXIT_MAXITER: return isfinite(o.fin_res) ? ST_NOT_CONVERGED : ST_NONFINITE;
@@ -104,7 +104,8 @@ __global__ void __launch_bounds__(kMaxBlock, kMinBlocksAtMax) krylov_kernel(KPar
             tiles_init(g, P.m, P.v.D);
             ok = grid_sync(g, 14);
         }
-        if (ok) ok = ic_precond(g, P.m, P.v, P.cfg.ic_sweeps, P.v.r, P.v.z, [](int, T, T) {});
+        T none;
+        if (ok) ok = ic_precond<kRowNone>(g, P.m, P.v, P.cfg.ic_sweeps, P.v.r, P.v.z, none);
         out.exit_kind = ok ? EXIT_CONVERGED : EXIT_ABORT;
     } else if (METHOD == 2) {
         cgs_solve(g, P.m, P.v, P.cfg, out);
