@@ -21,7 +21,7 @@ LIB_PATH = os.path.join(HERE, "libtflows_krylov.so")
 SOURCES = ("krylov.cu", "krylov_fma.cu", "krylov_mixed.cu", "shim.cu", "noalloc.cu", "tune.cu",
            "assembly.cu", "momentum.cu", "halo.cu", "meshio.cpp")
 CONTRACTED = ("krylov_fma.cu", "krylov_mixed.cu")  # units built with fused multiply-adds
-HEADERS = ("device_common.cuh", "fp64_div.cuh", "krylov_kernels.cuh", "solver_entry.cuh", "internal.h",
+HEADERS = ("device_common.cuh", "fp64_div.cuh", "fp64_int.cuh", "krylov_kernels.cuh", "solver_entry.cuh", "internal.h",
            "assembly_internal.h")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]

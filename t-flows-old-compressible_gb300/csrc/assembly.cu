@@ -16,6 +16,7 @@
 // left-to-right sum, so b differs from the reference by the rounding of that
 // one scalar.
 #include "assembly_internal.h"
+#include "fp64_int.cuh"
 #include "internal.h"
 #include "tflows_krylov.h"
 
@@ -26,8 +27,14 @@
 
 namespace {
 
+using tflows::div_rn;
+using tflows::half;
+using tflows::mul_rn;
+using tflows::twice;
+
 // What a face adds to its cells (set by the face pass, read by the cell pass).
-enum : unsigned char { kDiag1 = 1, kB1 = 2, kCell2 = 4 };
+// (A face's c2, where it is a cell, takes both.)
+enum : unsigned char { kDiag1 = 1, kB1 = 2 };
 
 struct FaceGeom {
     const double* sx;
@@ -43,7 +50,6 @@ struct FaceGeom {
 
 struct CellFields {  // all over cells -NbC..NC, element c at [c + NbC]
     const double* vol;
-    const double* vdiva;  // volume / Asave of this call
     const double* asave;
     const double* rho_n;
     const double* rho_o;
@@ -59,9 +65,7 @@ struct CellFields {  // all over cells -NbC..NC, element c at [c + NbC]
 };
 
 // Quantities the face loop recomputes per face although they depend on the
-// mesh only (SMDPN, 1 - f) or on one cell only (volume / Asave) are formed
-// once, with the same operations, so the face pass is bit-identical to the
-// reference's and does a third of its FP64 work (the divides dominate).
+// mesh only (SMDPN, 1 - f) are formed once, with the same operations.
 __global__ void __launch_bounds__(kAsmBlock) geom_kernel(int NS, const double* __restrict__ sx,
                                                          const double* __restrict__ sy,
                                                          const double* __restrict__ sz,
@@ -78,23 +82,14 @@ __global__ void __launch_bounds__(kAsmBlock) geom_kernel(int NS, const double* _
     }
 }
 
-__global__ void __launch_bounds__(kAsmBlock) vdiva_kernel(int n, const double* __restrict__ vol,
-                                                          const double* __restrict__ asave,
-                                                          double* __restrict__ q) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        q[i] = vol[i] / asave[i];
-}
-
 // One thread per face: CalcPS.f90:71-164 for face s = i + 1.
 __global__ void __launch_bounds__(kAsmBlock) face_kernel(int NS, int NbC, const int* __restrict__ c1s,
                                                          const int* __restrict__ c2s,
-                                                         const int* __restrict__ pos1,
-                                                         const int* __restrict__ pos2, FaceGeom g,
-                                                         CellFields F, double* __restrict__ abou,
+                                                         FaceGeom g, CellFields F,
+                                                         double* __restrict__ abou,
                                                          double* __restrict__ flux,
-                                                         double* __restrict__ slot_a,
-                                                         double* __restrict__ slot_f,
-                                                         unsigned char* __restrict__ slot_k) {
+                                                         double2* __restrict__ rec,
+                                                         unsigned char* __restrict__ kind) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NS; i += gridDim.x * blockDim.x) {
         const int c1 = c1s[i] + NbC, c2 = c2s[i];
         const int k2 = c2 + NbC;
@@ -104,19 +99,20 @@ __global__ void __launch_bounds__(kAsmBlock) face_kernel(int NS, int NbC, const 
         const int t2 = c2 < 0 ? F.type[k2] : 0;
         if (c2 > 0 || (c2 < 0 && t2 == kBuffer)) {
             const double S = g.smdpn[i];
-            const double Urs = f * F.rho_n[c1] * F.u[c1] + omf * F.rho_n[k2] * F.u[k2];
-            const double Vrs = f * F.rho_n[c1] * F.v[c1] + omf * F.rho_n[k2] * F.v[k2];
-            const double Wrs = f * F.rho_n[c1] * F.w[c1] + omf * F.rho_n[k2] * F.w[k2];
-            A12 = 0.5 * S * (F.vdiva[c1] + F.vdiva[k2]);
+            const double r1 = f * F.rho_n[c1], r2 = omf * F.rho_n[k2];
+            const double Urs = mul_rn(r1, F.u[c1]) + mul_rn(r2, F.u[k2]);
+            const double Vrs = mul_rn(r1, F.v[c1]) + mul_rn(r2, F.v[k2]);
+            const double Wrs = mul_rn(r1, F.w[c1]) + mul_rn(r2, F.w[k2]);
+            A12 = half(S) * (div_rn(F.vol[c1], F.asave[c1]) + div_rn(F.vol[k2], F.asave[k2]));
             if (c2 > 0) {
-                kd = kDiag1 | kB1 | kCell2;  // the cell pass sets Aval(SidAij(:, s)) = -A12
+                kd = kDiag1 | kB1;  // the cell pass sets Aval(SidAij(:, s)) = -A12
             } else {
                 abou[k2] = -A12;
                 kd = kDiag1 | kB1;
             }
-            const double dPxi = .5 * (F.px[c1] + F.px[k2]) * g.dx[i];
-            const double dPyi = .5 * (F.py[c1] + F.py[k2]) * g.dy[i];
-            const double dPzi = .5 * (F.pz[c1] + F.pz[k2]) * g.dz[i];
+            const double dPxi = mul_rn(half(F.px[c1] + F.px[k2]), g.dx[i]);
+            const double dPyi = mul_rn(half(F.py[c1] + F.py[k2]), g.dy[i]);
+            const double dPzi = mul_rn(half(F.pz[c1] + F.pz[k2]), g.dz[i]);
             fl = (Urs * g.sx[i] + Vrs * g.sy[i] + Wrs * g.sz[i]) + A12 * (F.p[c1] - F.p[k2]) +
                  A12 * (dPxi + dPyi + dPzi);
         } else if (t2 == kInflow || t2 == kOutflow || t2 == kConvect) {
@@ -139,121 +135,132 @@ __global__ void __launch_bounds__(kAsmBlock) face_kernel(int NS, int NbC, const 
             kd = kB1 | kDiag1;
         }  // every other type (walls, symmetry): Flux(s) = 0, nothing added
         flux[i] = fl;
-        // the face's entries in its cells' contribution lists
-        const int p1 = pos1[i];
-        slot_a[p1] = A12;
-        slot_f[p1] = fl;
-        slot_k[p1] = kd & (kDiag1 | kB1);
-        if (c2 > 0) {
-            const int p2 = pos2[i];
-            slot_a[p2] = A12;
-            slot_f[p2] = fl;
-            slot_k[p2] = kCell2;
-        }
+        rec[i] = make_double2(A12, fl);
+        kind[i] = kd;
     }
 }
 
 // One thread per cell c = i + 1: its faces' contributions in face order,
 // Nmat times (CalcPS.f90:69-167), errmax (171-174), then the source
-// (186-193) and this cell's terms of the two sums of the mean.  The face
-// pass left each contribution in the cell's own list (entries cf_ptr[i] ..
-// cf_ptr[i+1]-1, faces in increasing order), so the reads are contiguous.
-// The cell also sets its row's off-diagonal entries Aval(SidAij) = -A12 in
-// face order, so where two faces join the same cells (one entry) the later
-// face's value stays, as in the reference.
+// (186-193) and this cell's terms of the two sums of the mean.  The cell also
+// sets its row's off-diagonal entries Aval(SidAij) = -A12 in face order, so
+// where two faces join the same cells (one entry) the later face's value
+// stays, as in the reference.  `single`: every entry of Aval is set here, no
+// zeros were stored before.  The last block to finish adds the blocks'
+// partial sums (in block order, whichever block it is) and leaves the mean
+// and errmax: one pass over them instead of one by every block of the next
+// kernel.
+__device__ __forceinline__ double block_sum(double v, double* smem) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __syncthreads();
+    if (lane == 0) smem[warp] = v;
+    __syncthreads();
+    v = lane < kAsmBlock / 32 ? smem[lane] : 0.0;
+    for (int o = kAsmBlock / 64; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    return v;  // valid in lane 0 of every warp
+}
+
+constexpr int kFaces = 6;  // of a hexahedron
+
 __global__ void __launch_bounds__(kAsmBlock) cell_kernel(
     int NC, int NbC, int Nmat, double dt, const int* __restrict__ cf_ptr,
     const int* __restrict__ slot_face, const int* __restrict__ sid1,
-    const int* __restrict__ sid2, const int* __restrict__ adia, const double* __restrict__ slot_a,
-    const double* __restrict__ slot_f, const unsigned char* __restrict__ slot_k, CellFields F,
-    double* __restrict__ aval, double* __restrict__ b, double* __restrict__ part_sum,
-    double* __restrict__ part_vol, unsigned long long* __restrict__ errmax_bits) {
-    __shared__ double s_sum[kAsmBlock / 32], s_vol[kAsmBlock / 32];
+    const int* __restrict__ sid2, const int* __restrict__ adia, const double2* __restrict__ rec,
+    const unsigned char* __restrict__ kind, bool single, CellFields F, double* __restrict__ aval,
+    double* __restrict__ b, AsmPartial* __restrict__ part, unsigned* __restrict__ done,
+    double* __restrict__ sums, volatile unsigned long long* errmax_bits) {
+    __shared__ double s_sum[kAsmBlock / 32];
+    __shared__ unsigned long long s_max;
+    __shared__ bool s_last;
     double my_sum = 0.0, my_vol = 0.0;
     unsigned long long my_max = 0ull;
-    for (int base = blockIdx.x * blockDim.x; base < NC; base += gridDim.x * blockDim.x) {
-        const int i = base + threadIdx.x;
-        if (i < NC) {
-            const int e0 = cf_ptr[i], e1 = cf_ptr[i + 1];
-            double d = 0.0, bb = 0.0;
-            bool diag = false;
-            for (int m = 0; m < Nmat; ++m)
-                for (int e = e0; e < e1; ++e) {
-                    const unsigned char kd = slot_k[e];
-                    if (kd & kCell2) {  // this cell is the face's c2
-                        d = d + slot_a[e];
-                        bb = bb + slot_f[e];
-                        diag = true;
-                    } else {
-                        if (kd & kDiag1) {
-                            d = d + slot_a[e];
-                            diag = true;
-                        }
-                        if (kd & kB1) bb = bb - slot_f[e];
+    if (threadIdx.x == 0) s_max = 0ull;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NC; i += gridDim.x * blockDim.x) {
+        const int e0 = cf_ptr[i], e1 = cf_ptr[i + 1];
+        double d = 0.0, bb = 0.0;
+        bool diag = false;
+        for (int m = 0; m < Nmat; ++m)
+            for (int e = e0; e < e1; e += kFaces) {
+                // the loads of kFaces faces in flight together, then their
+                // terms in order
+                int sf[kFaces];
+                double2 r[kFaces];
+                unsigned kd[kFaces];
+#pragma unroll
+                for (int u = 0; u < kFaces; ++u) sf[u] = slot_face[min(e + u, e1 - 1)];
+#pragma unroll
+                for (int u = 0; u < kFaces; ++u) {
+                    const int s = sf[u] >= 0 ? sf[u] : ~sf[u];
+                    r[u] = rec[s];
+                    kd[u] = sf[u] >= 0 ? kind[s] : kDiag1 | kB1;
+                    if (m == 0 && e + u < e1) {
+                        const int o = sf[u] >= 0 ? sid1[s] : sid2[s];
+                        if (o >= 0) aval[o] = -r[u].x;
                     }
                 }
-            if (diag) aval[adia[i]] = d;
-            for (int e = e0; e < e1; ++e) {
-                const int sf = slot_face[e];
-                const int o = sf >= 0 ? sid1[sf] : sid2[~sf];
-                if (o >= 0) aval[o] = -slot_a[e];
+#pragma unroll
+                for (int u = 0; u < kFaces; ++u) {
+                    if (e + u >= e1) break;
+                    if (kd[u] & kDiag1) {
+                        d = d + r[u].x;
+                        diag = true;
+                    }
+                    if (kd[u] & kB1) bb = bb + tflows::signed_by(r[u].y, sf[u] >= 0);
+                }
             }
-            my_max = max(my_max, (unsigned long long)__double_as_longlong(fabs(bb)));
-            const int c = i + 1 + NbC;
-            for (int m = 0; m < Nmat; ++m) {
-                bb = bb - F.vol[c] / dt * (1.5 * F.rho_n[c] - 2.0 * F.rho_o[c] + 0.5 * F.rho_oo[c]);
-                my_sum = my_sum + bb * F.vol[c];
-                my_vol = my_vol + F.vol[c];
-            }
-            b[i] = bb;
+        if (diag || single) aval[adia[i]] = d;
+        my_max = max(my_max, (unsigned long long)__double_as_longlong(fabs(bb)));
+        const int c = i + 1 + NbC;
+        const double vol = F.vol[c], q = div_rn(vol, dt);
+        const double w = 1.5 * F.rho_n[c] - twice(F.rho_o[c]) + half(F.rho_oo[c]);
+        for (int m = 0; m < Nmat; ++m) {
+            bb = bb - q * w;
+            my_sum = my_sum + bb * vol;
+            my_vol = my_vol + vol;
         }
+        b[i] = bb;
     }
     // block partial sums in a fixed order (deterministic)
-    for (int o = 16; o > 0; o >>= 1) {
-        my_sum += __shfl_down_sync(0xffffffffu, my_sum, o);
-        my_vol += __shfl_down_sync(0xffffffffu, my_vol, o);
-        my_max = max(my_max, __shfl_down_sync(0xffffffffu, my_max, o));
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) {
-        s_sum[warp] = my_sum;
-        s_vol[warp] = my_vol;
-        atomicMax(errmax_bits, my_max);
-    }
+    for (int o = 16; o > 0; o >>= 1) my_max = max(my_max, __shfl_down_sync(0xffffffffu, my_max, o));
+    my_sum = block_sum(my_sum, s_sum);
+    my_vol = block_sum(my_vol, s_sum);
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_max, my_max);
     __syncthreads();
     if (threadIdx.x == 0) {
-        double a = 0.0, v = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-            a += s_sum[w];
-            v += s_vol[w];
-        }
-        part_sum[blockIdx.x] = a;
-        part_vol[blockIdx.x] = v;
+        part[blockIdx.x] = {my_sum, my_vol, s_max};
+        __threadfence();
+        s_last = atomicAdd(done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    double a = 0.0, v = 0.0;
+    unsigned long long hi = 0ull;
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += kAsmBlock) {
+        a += __ldcg(&part[k].sum);
+        v += __ldcg(&part[k].vol);
+        hi = max(hi, __ldcg(&part[k].errmax));
+    }
+    a = block_sum(a, s_sum);
+    v = block_sum(v, s_sum);
+    if (threadIdx.x == 0) s_max = 0ull;
+    __syncthreads();
+    atomicMax(&s_max, hi);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        sums[0] = a;
+        sums[1] = v;
+        sums[2] = a / v;
+        *errmax_bits = s_max;
+        *done = 0u;  // for the next launch
     }
 }
 
-// b(c) = b(c) - bc_sum / vol (CalcPS.f90:199-202); every thread sums the
-// block partials in the same order.
-__global__ void __launch_bounds__(kAsmBlock) mean_kernel(int NC, int nparts,
-                                                         const double* __restrict__ part_sum,
-                                                         const double* __restrict__ part_vol,
-                                                         double* __restrict__ b,
-                                                         double* __restrict__ sums) {
-    __shared__ double s_shift;
-    if (threadIdx.x == 0) {
-        double a = 0.0, v = 0.0;
-        for (int k = 0; k < nparts; ++k) {
-            a += part_sum[k];
-            v += part_vol[k];
-        }
-        s_shift = a / v;
-        if (blockIdx.x == 0) {
-            sums[0] = a;
-            sums[1] = v;
-        }
-    }
-    __syncthreads();
-    const double shift = s_shift;
+// b(c) = b(c) - bc_sum / vol (CalcPS.f90:199-202).
+__global__ void __launch_bounds__(kAsmBlock) mean_kernel(int NC, const double* __restrict__ sums,
+                                                         double* __restrict__ b) {
+    const double shift = sums[2];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NC; i += gridDim.x * blockDim.x)
         b[i] = b[i] - shift;
 }
@@ -276,12 +283,13 @@ void tflows_assembly_destroy(tflows_assembly* a) {
     if (!a) return;
     cudaSetDevice(a->device);
     for (void* p : {(void*)a->c1, (void*)a->c2, (void*)a->sid1, (void*)a->sid2, (void*)a->adia,
-                    (void*)a->type, (void*)a->cf_ptr, (void*)a->pos1, (void*)a->pos2,
-                    (void*)a->geom, (void*)a->vol, (void*)a->slot_a, (void*)a->slot_f,
-                    (void*)a->slot_k, (void*)a->parts, (void*)a->errmax, (void*)a->vdiva,
-                    (void*)a->slot_face, (void*)a->bnd_ptr, (void*)a->bnd_face,
-                    a->mom_rec, (void*)a->mom_cells, (void*)a->mom_err})
+                    (void*)a->type, (void*)a->cf_ptr,
+                    (void*)a->geom, (void*)a->vol, (void*)a->rec, (void*)a->kind,
+                    (void*)a->parts, (void*)a->done, (void*)a->sums,
+                    (void*)a->slot_face, (void*)a->slot_cell, (void*)a->bnd_ptr, (void*)a->bnd_face,
+                    a->mom_rec, (void*)a->mom_cells})
         if (p) cudaFree(p);
+    if (a->note) cudaFreeHost(a->note);
     if (a->ev0) cudaEventDestroy(a->ev0);
     if (a->ev1) cudaEventDestroy(a->ev1);
     delete a;
@@ -319,19 +327,27 @@ int tflows_assembly_create(tflows_assembly** out, int NC, int NbC, int NS, int N
         adia[c] = Adia[c] - 1;
         if (adia[c] < 0 || adia[c] >= NONZ) return asm_fail(TFLOWS_BAD_INPUT, "Adia out of range");
     }
-    // each cell's faces in increasing face order: the entry of face s in the
-    // list of its c1 (pos1) and of its c2 (pos2, interior faces)
+    std::vector<int> owners(NONZ, 0);
+    for (int c = 0; c < NC; ++c) ++owners[adia[c]];
+    for (int s = 0; s < NS; ++s)
+        if (c2[s] > 0) {
+            ++owners[s1[s]];
+            ++owners[s2[s]];
+        }
+    const bool single = std::all_of(owners.begin(), owners.end(), [](int k) { return k == 1; });
+    // each cell's faces in increasing face order
     std::vector<int> ptr(NC + 1, 0);
     for (int c = 1; c <= NC; ++c) ptr[c] = ptr[c - 1] + deg[c];
-    std::vector<int> pos1(std::max(NS, 1)), pos2(std::max(NS, 1), -1);
     std::vector<int> fill(ptr.begin(), ptr.end() - 1);
-    std::vector<int> slot_face(std::max(ptr[NC], 1));
+    std::vector<int> slot_face(std::max(ptr[NC], 1)), slot_cell(std::max(ptr[NC], 1));
     for (int s = 0; s < NS; ++s) {
-        pos1[s] = fill[c1[s] - 1]++;
-        slot_face[pos1[s]] = s;
+        const int e1 = fill[c1[s] - 1]++;
+        slot_face[e1] = s;
+        slot_cell[e1] = c2[s] > 0 || TypeBC[c2[s] + NbC] == kBuffer ? c2[s] + NbC : -1;
         if (c2[s] > 0) {
-            pos2[s] = fill[c2[s] - 1]++;
-            slot_face[pos2[s]] = ~s;
+            const int e2 = fill[c2[s] - 1]++;
+            slot_face[e2] = ~s;
+            slot_cell[e2] = c1[s] + NbC;
         }
     }
     // each boundary cell's faces in increasing order
@@ -345,7 +361,6 @@ int tflows_assembly_create(tflows_assembly** out, int NC, int NbC, int NS, int N
         for (int s = 0; s < NS; ++s)
             if (c2[s] < 0) bface[bf[c2[s] + NbC]++] = s;
     }
-    const size_t nslot = std::max(ptr[NC], 1);
     if (device >= 0 && cudaSetDevice(device) != cudaSuccess)
         return asm_fail(TFLOWS_NO_DEVICE, "cudaSetDevice failed");
     auto* a = new tflows_assembly();
@@ -354,6 +369,7 @@ int tflows_assembly_create(tflows_assembly** out, int NC, int NbC, int NS, int N
     a->NbC = NbC;
     a->NS = NS;
     a->NONZ = NONZ;
+    a->single = single;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, a->device);
     a->nblocks = std::max(1, std::min((NC + kAsmBlock - 1) / kAsmBlock, 8 * std::max(sms, 1)));
@@ -367,9 +383,8 @@ int tflows_assembly_create(tflows_assembly** out, int NC, int NbC, int NS, int N
     if (e == cudaSuccess) e = upload(&a->adia, adia.data(), NC);
     if (e == cudaSuccess) e = upload(&a->type, TypeBC, (size_t)NbC + NC + 1);
     if (e == cudaSuccess) e = upload(&a->cf_ptr, ptr.data(), ptr.size());
-    if (e == cudaSuccess) e = upload(&a->pos1, pos1.data(), pos1.size());
-    if (e == cudaSuccess) e = upload(&a->pos2, pos2.data(), pos2.size());
     if (e == cudaSuccess) e = upload(&a->slot_face, slot_face.data(), slot_face.size());
+    if (e == cudaSuccess) e = upload(&a->slot_cell, slot_cell.data(), slot_cell.size());
     if (e == cudaSuccess) e = upload(&a->bnd_ptr, bptr.data(), bptr.size());
     if (e == cudaSuccess) e = upload(&a->bnd_face, bface.data(), bface.size());
     if (e == cudaSuccess) e = upload(&a->geom, geom.data(), geom.size());
@@ -383,12 +398,14 @@ int tflows_assembly_create(tflows_assembly** out, int NC, int NbC, int NS, int N
         e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaDeviceSynchronize();
     }
-    if (e == cudaSuccess) e = cudaMalloc(&a->vdiva, sizeof(double) * ((size_t)NbC + NC + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&a->slot_a, sizeof(double) * nslot);
-    if (e == cudaSuccess) e = cudaMalloc(&a->slot_f, sizeof(double) * nslot);
-    if (e == cudaSuccess) e = cudaMalloc(&a->slot_k, nslot);
-    if (e == cudaSuccess) e = cudaMalloc(&a->parts, sizeof(double) * (2 * a->nblocks + 2));
-    if (e == cudaSuccess) e = cudaMalloc(&a->errmax, sizeof(unsigned long long));
+    if (e == cudaSuccess) e = cudaMalloc(&a->rec, sizeof(double2) * std::max(NS, 1));
+    if (e == cudaSuccess) e = cudaMalloc(&a->kind, std::max(NS, 1));
+    if (e == cudaSuccess) e = cudaMalloc(&a->parts, sizeof(AsmPartial) * a->nblocks);
+    if (e == cudaSuccess) e = cudaMalloc(&a->sums, sizeof(double) * 3);
+    if (e == cudaSuccess) e = cudaMalloc(&a->done, sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMemset(a->done, 0, sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaHostAlloc(&a->note, sizeof(AsmNote), cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer((void**)&a->d_note, a->note, 0);
     if (e == cudaSuccess) e = cudaEventCreate(&a->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&a->ev1);
     if (e != cudaSuccess) {
@@ -416,45 +433,37 @@ int tflows_calcps_assemble_device(tflows_assembly* a, int Nmat, double dt,
     FaceGeom g{a->geom,          a->geom + ns,     a->geom + 2 * ns,
                a->geom + 3 * ns, a->geom + 4 * ns, a->geom + 5 * ns,
                a->geom + 6 * ns, a->geom + 7 * ns, a->geom + 8 * ns};
-    CellFields F{a->vol, a->vdiva, in->asave, in->rho_n, in->rho_o, in->rho_oo, in->u, in->v,
+    CellFields F{a->vol, in->asave, in->rho_n, in->rho_o, in->rho_oo, in->u, in->v,
                  in->w, in->p, in->px, in->py, in->pz, a->type};
     cudaEventRecord(a->ev0, s);
-    cudaError_t e = cudaMemsetAsync(aval, 0, sizeof(double) * a->NONZ, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(a->errmax, 0, sizeof(unsigned long long), s);
-    const int ncell = a->NbC + a->NC + 1;
-    if (e == cudaSuccess) {
-        vdiva_kernel<<<std::max(1, std::min((ncell + kAsmBlock - 1) / kAsmBlock, 65535)), kAsmBlock,
-                       0, s>>>(ncell, a->vol, in->asave, a->vdiva);
-        e = cudaGetLastError();
-    }
+    cudaError_t e = cudaSuccess;
+    if (!a->single) e = cudaMemsetAsync(aval, 0, sizeof(double) * a->NONZ, s);
     const int fb = std::max(1, std::min((a->NS + kAsmBlock - 1) / kAsmBlock, 65535));
     if (e == cudaSuccess && a->NS > 0) {
-        face_kernel<<<fb, kAsmBlock, 0, s>>>(a->NS, a->NbC, a->c1, a->c2, a->pos1, a->pos2, g,
-                                             F, abou, flux, a->slot_a, a->slot_f, a->slot_k);
+        face_kernel<<<fb, kAsmBlock, 0, s>>>(a->NS, a->NbC, a->c1, a->c2, g, F, abou, flux, a->rec,
+                                             a->kind);
         e = cudaGetLastError();
     }
-    double* ps = a->parts;
-    double* pv = a->parts + a->nblocks;
-    double* tot = a->parts + 2 * a->nblocks;
     if (e == cudaSuccess) {
         cell_kernel<<<a->nblocks, kAsmBlock, 0, s>>>(a->NC, a->NbC, Nmat, dt, a->cf_ptr,
                                                      a->slot_face, a->sid1, a->sid2, a->adia,
-                                                     a->slot_a, a->slot_f, a->slot_k, F, aval, b,
-                                                     ps, pv, a->errmax);
+                                                     a->rec, a->kind, a->single, F, aval, b,
+                                                     a->parts, a->done, a->sums,
+                                                     &a->d_note->errmax_bits);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
-        mean_kernel<<<a->nblocks, kAsmBlock, 0, s>>>(a->NC, a->nblocks, ps, pv, b, tot);
+        mean_kernel<<<a->nblocks, kAsmBlock, 0, s>>>(a->NC, a->sums, b);
         e = cudaGetLastError();
     }
     cudaEventRecord(a->ev1, s);
-    unsigned long long bits = 0;
-    if (e == cudaSuccess && errmax)
-        e = cudaMemcpyAsync(&bits, a->errmax, sizeof(bits), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess && (errmax || seconds)) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess)
         return asm_fail(TFLOWS_CUDA_ERROR, std::string("assembly: ") + cudaGetErrorString(e));
-    if (errmax) std::memcpy(errmax, &bits, sizeof(double));
+    if (errmax) {
+        const unsigned long long bits = a->note->errmax_bits;
+        std::memcpy(errmax, &bits, sizeof(double));
+    }
     if (seconds) {
         float ms = 0.f;
         cudaEventElapsedTime(&ms, a->ev0, a->ev1);

@@ -9,7 +9,7 @@
 // estimate, Knuth, TAOCP vol. 2, 4.3.1).  The last remainder makes the
 // quotient exact before it is rounded, so the result is IEEE
 // round-to-nearest-even, bit for bit.  Operands or results that are not
-// normal numbers go to the built-in division.
+// normal numbers (but for 0 / normal) go to the built-in division.
 #pragma once
 
 #include <cstdint>
@@ -69,9 +69,13 @@ TF_HD uint64_t div_significands(uint64_t ma, uint64_t mb, int32_t y) {
 #undef TF_MULHI
 }
 
+// (An opaque move on the device: the compiler turns tests of a number's bits
+// back into FP64 comparisons where it can see where they came from.)
 TF_HD uint64_t div_bits(double v) {
 #if defined(__CUDA_ARCH__)
-    return (uint64_t)__double_as_longlong(v);
+    uint64_t b;
+    asm("mov.b64 %0, %1;" : "=l"(b) : "d"(v));
+    return b;
 #else
     uint64_t b;
     __builtin_memcpy(&b, &v, 8);
@@ -112,7 +116,10 @@ TF_HD double div_rn(double a, double b) {
     const int ea = (int)(ba >> 52) & 0x7ff, eb = (int)(bb >> 52) & 0x7ff;
     const int e = ea - eb + 1023;  // exponent of a quotient >= 1
     // both normal; the quotient normal before and after rounding
-    if ((unsigned)(ea - 1) >= 2046u || (unsigned)(eb - 1) >= 2046u || (unsigned)(e - 2) >= 2044u) return a / b;
+    if ((unsigned)(ea - 1) >= 2046u || (unsigned)(eb - 1) >= 2046u || (unsigned)(e - 2) >= 2044u) {
+        if ((ba << 1) == 0 && (unsigned)(eb - 1) < 2046u) return div_value((ba ^ bb) & 0x8000000000000000ull);
+        return a / b;
+    }
     const uint64_t kOne = 1ull << 52, kFrac = kOne - 1;
     const uint64_t ma = (ba & kFrac) | kOne, mb = (bb & kFrac) | kOne;
     // 2^31 / x for the divisor's leading bits x in [1, 2), in (2^30, 2^31)

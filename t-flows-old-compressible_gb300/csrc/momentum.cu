@@ -22,6 +22,7 @@
 // Every sum sees the reference's operands in the reference's order (built
 // with --fmad=false), so Aval, b, Abou and Asave are bit-identical to it.
 #include "assembly_internal.h"
+#include "fp64_int.cuh"
 #include "internal.h"
 #include "tflows_krylov.h"
 
@@ -30,14 +31,22 @@
 
 namespace {
 
+using tflows::above_zero;
+using tflows::below_zero;
+using tflows::div_rn;
+using tflows::half;
+using tflows::less;
+using tflows::mul_rn;
+using tflows::signed_by;
+using tflows::twice;
+using tflows::zero_minus;
+using tflows::zero_plus;
+
 // Process/IniPar.f90:22-49
 enum : int {
     kCN = 2, kFI = 3, kLIN = 4, kPAR = 5, kYES = 10, kNO = 11, kCDS = 20, kQUICK = 21,
     kLUDS = 22, kMINMOD = 23, kSMART = 24, kAVL_SMART = 25, kSUPERBEE = 26, kGAMMA = 27
 };
-
-// input errors the kernels find (bits of *mom_err)
-enum : int { kErrBlend = 1, kErrMaterial = 2 };
 
 // what the cell pass does with a face (MomRec::flags)
 enum : int {
@@ -51,15 +60,28 @@ enum : int {
     kOtherB = 4        //   anything else: no matrix term
 };
 
-struct __align__(16) MomRec {
+// What a face adds to its two cells; its flags are a byte beside it, so that
+// a record is two whole sectors.
+struct __align__(64) MomRec {
     double t;         // Flux_u * rhoUiS
     double u;         // Flux_u * rhoUi(upwind cell)
     double fex, fim;  // exact and implicit diffusive flux of the cross terms
-    double a12, a21, d12, d21;
+    double fa;        // Flux_u where the face blends, else 0 (see convect)
+    double d12, d21;
     double bv;        // b(c1) term of a boundary face
-    int flags;
-    int pad;
 };
+
+// The two convective coefficients of a face from MomRec::fa:
+// A12 = 0 - MIN(fa, 0) and A21 = 0 + MAX(fa, 0) (NewUVW.f90:352-357).
+struct Convect {
+    double a12, a21;
+};
+__device__ __forceinline__ double pick(bool first, double x, double y) {
+    return tflows::div_value(first ? tflows::div_bits(x) : tflows::div_bits(y));
+}
+__device__ __forceinline__ Convect convect(double fa) {
+    return {above_zero(fa) ? 0.0 : zero_minus(fa), below_zero(fa) ? 0.0 : zero_plus(fa)};
+}
 
 struct MomCells {  // over cells -NbC..NC, element c at [c + NbC]
     const int* material;
@@ -88,12 +110,13 @@ struct MomScalars {
 // MIN / MAX: the first argument unless a later one is strictly smaller /
 // larger, as the statement-by-statement execution of the reference's text
 // gives (Fortran leaves equal signed zeros and NaN to the compiler).
-__device__ __forceinline__ double min2(double a, double b) { return b < a ? b : a; }
-__device__ __forceinline__ double max2(double a, double b) { return b > a ? b : a; }
+__device__ __forceinline__ double min2(double a, double b) { return less(b, a) ? b : a; }
+__device__ __forceinline__ double max2(double a, double b) { return less(a, b) ? b : a; }
+__device__ __forceinline__ double at_least_zero(double x) { return above_zero(x) ? x : 0.0; }  // max2(0, x)
 
-__device__ __forceinline__ int material_code(const int* tab, int nmat, int m, int* err) {
+__device__ __forceinline__ int material_code(const int* tab, int nmat, int m, AsmNote* err) {
     if (m < 1 || m > nmat) {
-        atomicOr(err, kErrMaterial);
+        err->material = 1;
         return kNO;
     }
     return tab[m - 1];
@@ -104,31 +127,30 @@ __device__ __forceinline__ int material_code(const int* tab, int nmat, int m, in
 __device__ bool conv_scheme(double& phis, int i, int c1, int c2, int NbC, const MomFaces& F,
                             const MomCells& K, const double* __restrict__ phi,
                             const double* __restrict__ pmax, const double* __restrict__ pmin,
-                            int blenda) {
-    double fj, sign;
+                            int blenda, double di, double dj, double dk) {
+    double fj;
     int C, D;
     const double fl = F.flux[i];
-    if (fl > 0.0) {
-        fj = 1.0 - F.f[i];
+    const bool ahead = above_zero(fl);
+    if (ahead) {
+        fj = F.omf[i];
         C = c1;
         D = c2;
-        sign = +1.0;
     } else {
         fj = F.f[i];
         C = c2;
         D = c1;
-        sign = -1.0;
     }
     const int kc = C + NbC, kd = D + NbC;
-    const double grad = K.duidi[kc] * F.di[i] + K.duidj[kc] * F.dj[i] + K.duidk[kc] * F.dk[i];
+    const double grad = K.duidi[kc] * di + K.duidj[kc] * dj + K.duidk[kc] * dk;
     const double phiC = phi[kc], phiD = phi[kd];
     if (blenda == kGAMMA) {
         // the value ConvScheme forms before its GAMMA block is overwritten
         // in every branch of it (:111-133)
         const double Beta = 0.1;
-        const double den = 2.0 * grad;
-        const double PhiUstar = fl > 0.0 ? 1.0 - (phiD - phiC) / den : 1.0 + (phiD - phiC) / den;
-        const double GammaC = PhiUstar / Beta;
+        const double den = twice(grad);
+        const double PhiUstar = 1.0 + signed_by(div_rn(phiD - phiC, den), ahead);
+        const double GammaC = div_rn(PhiUstar, Beta);
         if (PhiUstar < Beta && PhiUstar > 0.0)
             phis = (1.0 - GammaC * (1.0 - F.f[i])) * phiC + GammaC * (1.0 - F.f[i]) * phiD;
         else if (PhiUstar < 1.0 && PhiUstar >= Beta)
@@ -138,18 +160,18 @@ __device__ bool conv_scheme(double& phis, int i, int c1, int c2, int NbC, const 
         return true;
     }
     if (blenda == kYES) return true;
-    const double PhiUstar = fl > 0.0 ? phiD - 2.0 * grad : phiD + 2.0 * grad;
+    const double PhiUstar = phiD + signed_by(twice(grad), ahead);
     const double PhiU = max2(pmin[kc], min2(PhiUstar, pmax[kc]));
-    double rj = (phiC - PhiU) / (phiD - phiC + 1.0e-16);
-    const double gD = 0.5 * fj * (1.0 + fj);
-    const double gU = 0.5 * fj * (1.0 - fj);
+    double rj = blenda == kQUICK ? 0.0 : div_rn(phiC - PhiU, phiD - phiC + 1.0e-16);
+    const double gD = half(fj) * (1.0 + fj);
+    const double gU = half(fj) * (1.0 - fj);
     double Phij;
     switch (blenda) {
         case kCDS:
             Phij = fj;
             break;
         case kQUICK: {
-            rj = (phiC - PhiU) / (phiD - phiC + 1.0e-12);
+            rj = div_rn(phiC - PhiU, phiD - phiC + 1.0e-12);
             const double alfa = 0.0;
             Phij = (gD - alfa) + (gU + alfa) * rj;
             break;
@@ -160,34 +182,34 @@ __device__ bool conv_scheme(double& phis, int i, int c1, int c2, int NbC, const 
             break;
         }
         case kMINMOD:
-            Phij = fj * max2(0.0, min2(rj, 1.0));
+            Phij = fj * at_least_zero(min2(rj, 1.0));
             break;
         case kSMART: {
-            const double beta1 = 3.0, beta2 = 1.0;
-            Phij = max2(0.0, min2(min2((beta1 - 1.0) * rj, gD + gU * rj), beta2));
+            const double beta2 = 1.0;  // and BETA1 - 1 = 2
+            Phij = at_least_zero(min2(min2(twice(rj), gD + gU * rj), beta2));
             break;
         }
         case kAVL_SMART: {
             const double beta1 = 1.0 + fj * (2.0 + fj);
             const double beta2 = fj * (2.0 - fj);
-            Phij = max2(0.0, min2(min2((beta1 - 1.0) * rj, gD + gU * rj), beta2));
+            Phij = at_least_zero(min2(min2((beta1 - 1.0) * rj, gD + gU * rj), beta2));
             break;
         }
         case kSUPERBEE:
-            Phij = 0.5 * max2(max2(0.0, min2(2.0 * rj, 1.0)), min2(rj, 2.0));
+            Phij = half(max2(at_least_zero(min2(twice(rj), 1.0)), min2(rj, 2.0)));
             break;
         default:
             return false;
     }
-    phis = phiC + Phij * sign * (phi[c2 + NbC] - phi[c1 + NbC]);
+    phis = phiC + signed_by(Phij, !ahead) * (phi[c2 + NbC] - phi[c1 + NbC]);
     return true;
 }
 
 // rhoUi over all cells, and CalMinMax (CalMinMax.f90:20-36) when any
 // material blends.
 __global__ void __launch_bounds__(kAsmBlock) mom_bounds_kernel(
-    int NC, int NbC, const int* __restrict__ c1s, const int* __restrict__ c2s,
-    const int* __restrict__ cf_ptr, const int* __restrict__ slot_face,
+    int NC, int NbC, const int* __restrict__ c1s, const int* __restrict__ cf_ptr,
+    const int* __restrict__ slot_cell,
     const int* __restrict__ bnd_ptr, const int* __restrict__ bnd_face, MomCells K, MomMats Mt,
     double* __restrict__ rhoui, double* __restrict__ pmax, double* __restrict__ pmin) {
     bool blends = false;
@@ -199,16 +221,13 @@ __global__ void __launch_bounds__(kAsmBlock) mom_bounds_kernel(
         if (!blends) continue;
         double hi = own, lo = own;
         if (k > NbC) {  // interior cell: every face with an interior or BUFFER neighbour
-            for (int e = cf_ptr[k - NbC - 1]; e < cf_ptr[k - NbC]; ++e) {
-                const int sf = slot_face[e];
-                const int s = sf >= 0 ? sf : ~sf;
-                const int c2 = c2s[s];
-                if (c2 > 0 || K.type[c2 + NbC] == kBuffer) {
-                    const int o = (sf >= 0 ? c2 : c1s[s]) + NbC;
-                    const double v = K.rho_n[o] * K.ui_n[o];
-                    hi = max2(hi, v);
-                    lo = min2(lo, v);
-                }
+            const int e1 = cf_ptr[k - NbC];
+            for (int e = cf_ptr[k - NbC - 1]; e < e1; ++e) {
+                const int o = slot_cell[e];
+                if (o < 0) continue;
+                const double v = K.rho_n[o] * K.ui_n[o];
+                hi = max2(hi, v);
+                lo = min2(lo, v);
             }
         } else if (k < NbC && K.type[k] == kBuffer) {
             for (int e = bnd_ptr[k]; e < bnd_ptr[k + 1]; ++e) {
@@ -224,11 +243,11 @@ __global__ void __launch_bounds__(kAsmBlock) mom_bounds_kernel(
 }
 
 // One thread per face s = i + 1: NewUVW.f90:205-236 and 276-416.
-__global__ void __launch_bounds__(kAsmBlock) mom_face_kernel(
+__global__ void __launch_bounds__(kAsmBlock, 5) mom_face_kernel(
     int NS, int NbC, const int* __restrict__ c1s, const int* __restrict__ c2s, MomFaces F,
     MomCells K, MomMats Mt, MomScalars P, const double* __restrict__ rhoui,
     const double* __restrict__ pmax, const double* __restrict__ pmin, MomRec* __restrict__ rec,
-    int* __restrict__ err) {
+    unsigned char* __restrict__ kind, AsmNote* err) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NS; i += gridDim.x * blockDim.x) {
         const int c1 = c1s[i], c2 = c2s[i];
         const int k1 = c1 + NbC, k2 = c2 + NbC;
@@ -239,56 +258,56 @@ __global__ void __launch_bounds__(kAsmBlock) mom_face_kernel(
         const int bt2 = material_code(Mt.blend_tem, Mt.nmat, m2, err);
         MomRec r;
         int flags = 0;
+        const double di = F.di[i], dj = F.dj[i], dk = F.dk[i];
         // convection (:208-235)
-        double rhoUiS = F.f[i] * rhoui[k1] + F.omf[i] * rhoui[k2];
         const bool blend = bl1 != kNO || bl2 != kNO;
-        if (blend && !conv_scheme(rhoUiS, i, c1, c2, NbC, F, K, rhoui, pmax, pmin,
-                                  bl1 > bl2 ? bl1 : bl2))
-            atomicOr(err, kErrBlend);
+        const int code = bl1 > bl2 ? bl1 : bl2;
+        double rhoUiS = 0.0;  // overwritten by every scheme but YES, which keeps the central value
+        if (!blend || code == kYES) rhoUiS = F.f[i] * rhoui[k1] + F.omf[i] * rhoui[k2];
+        if (blend && !conv_scheme(rhoUiS, i, c1, c2, NbC, F, K, rhoui, pmax, pmin, code, di, dj, dk))
+            err->blend = 1;
         const double fu = F.flux_u[i];
         r.t = fu * rhoUiS;
         r.u = 0.0;
         if (bt1 != kNO || bt2 != kNO) {
             flags |= kUpwind;
-            r.u = fu < 0 ? fu * rhoui[k2] : fu * rhoui[k1];
+            r.u = fu * rhoui[below_zero(fu) ? k2 : k1];
         }
         // diffusion (:277-331)
-        const double ff = F.ff[i], omff = 1.0 - F.ff[i];
-        const double RhoS = ff * K.rho_n[k1] + omff * K.rho_n[k2];
-        const double VISeff = P.moin == 4 ? P.visc * RhoS : P.visc;
-        const double dUidiS = ff * K.duidi[k1] + omff * K.duidi[k2];
-        const double dUidjS = ff * K.duidj[k1] + omff * K.duidj[k2];
-        const double dUidkS = ff * K.duidk[k1] + omff * K.duidk[k2];
-        const double dUjdiS = ff * K.dujdi[k1] + omff * K.dujdi[k2];
-        const double dUkdiS = ff * K.dukdi[k1] + omff * K.dukdi[k2];
-        const double dUjdjS = ff * K.dujdj[k1] + omff * K.dujdj[k2];
-        const double dUkdkS = ff * K.dukdk[k1] + omff * K.dukdk[k2];
-        r.fex = VISeff * (4.0 / 3.0 * dUidiS * F.si[i] + (dUidjS + dUjdiS) * F.sj[i] +
-                          (dUidkS + dUkdiS) * F.sk[i] - 2.0 / 3.0 * (dUjdjS + dUkdkS) * F.si[i]);
-        const double A0 = VISeff * F.scoef[i];
-        r.fim = A0 * (dUidiS * F.di[i] + dUidjS * F.dj[i] + dUidkS * F.dk[i]);
+        const double ff = F.ff[i], omff = 1.0 - ff;
+        double VISeff = P.visc;
+        if (P.moin == 4) VISeff = P.visc * (ff * K.rho_n[k1] + omff * K.rho_n[k2]);
+        const auto at_face = [&](const double* __restrict__ v) {
+            return mul_rn(ff, v[k1]) + mul_rn(omff, v[k2]);
+        };
+        const double dUidiS = at_face(K.duidi), dUidjS = at_face(K.duidj), dUidkS = at_face(K.duidk);
+        const double dUjdiS = at_face(K.dujdi), dUkdiS = at_face(K.dukdi);
+        const double dUjdjS = at_face(K.dujdj), dUkdkS = at_face(K.dukdk);
+        const double si = F.si[i];
+        r.fex = VISeff * (4.0 / 3.0 * dUidiS * si + (dUidjS + dUjdiS) * F.sj[i] +
+                          (dUidkS + dUkdiS) * F.sk[i] - 2.0 / 3.0 * (dUjdjS + dUkdkS) * si);
+        const double A0 = mul_rn(VISeff, F.scoef[i]);
+        r.fim = mul_rn(A0, mul_rn(dUidiS, di) + mul_rn(dUidjS, dj) + mul_rn(dUidkS, dk));
         // matrix coefficients (:347-414)
-        double A12 = 0.0, A21 = 0.0, D12 = 0.0, D21 = 0.0;
+        r.fa = 0.0;
+        r.d12 = r.d21 = 0.0;
         r.bv = 0.0;
         if (P.diffus == kCN || P.diffus == kFI) {
             flags |= kMatrix;
             if (P.diffus == kFI) {
-                D12 = D12 + A0 / K.rho_n[k2];
-                D21 = D21 + A0 / K.rho_n[k1];
+                r.d12 = zero_plus(div_rn(A0, K.rho_n[k2]));
+                r.d21 = zero_plus(div_rn(A0, K.rho_n[k1]));
             }
-            if (blend) {
-                A12 = A12 - min2(fu, 0.0);
-                A21 = A21 + max2(fu, 0.0);
-            }
+            if (blend) r.fa = fu;
             int cls = kInterior;
             if (c2 < 0) {
                 const int t = K.type[k2];
                 if (t == kWall || t == kConvect || t == kInflow || t == kWallfl) {
                     cls = kWallLike;
-                    r.bv = (A12 + D12) * rhoui[k2];
+                    r.bv = (convect(r.fa).a12 + r.d12) * rhoui[k2];
                 } else if (t == kOutflow) {
                     cls = kOutflowB;
-                    r.bv = (A12)*rhoui[k2];
+                    r.bv = convect(r.fa).a12 * rhoui[k2];
                 } else if (t == kBuffer) {
                     cls = kBufferB;
                 } else {
@@ -297,34 +316,30 @@ __global__ void __launch_bounds__(kAsmBlock) mom_face_kernel(
             }
             flags |= cls << kShift;
         }
-        r.a12 = A12;
-        r.a21 = A21;
-        r.d12 = D12;
-        r.d21 = D21;
-        r.flags = flags;
-        r.pad = 0;
         rec[i] = r;
+        kind[i] = (unsigned char)flags;
     }
 }
 
 // One thread per cell: interior cell c = k - NbC takes its faces' records in
 // increasing face order (NewUVW.f90:205-499); boundary cell k < NbC sets
 // Abou from its last BUFFER face (:405), 0 otherwise (:146).
-__global__ void __launch_bounds__(kAsmBlock) mom_cell_kernel(
+__global__ void __launch_bounds__(kAsmBlock, 8) mom_cell_kernel(
     int NC, int NbC, const int* __restrict__ cf_ptr, const int* __restrict__ slot_face,
     const int* __restrict__ bnd_ptr, const int* __restrict__ bnd_face,
     const int* __restrict__ sid1, const int* __restrict__ sid2, const int* __restrict__ adia,
-    const MomRec* __restrict__ rec, MomCells K, MomMats Mt, MomScalars P,
+    const MomRec* __restrict__ rec, const unsigned char* __restrict__ kind, bool single, MomCells K,
+    MomMats Mt, MomScalars P,
     const double* __restrict__ rhoui, double* __restrict__ aval, double* __restrict__ b,
-    double* __restrict__ abou, double* __restrict__ asave, int* __restrict__ err) {
+    double* __restrict__ abou, double* __restrict__ asave, AsmNote* err) {
     const int ncell = NbC + NC + 1;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < ncell; k += gridDim.x * blockDim.x) {
         if (k < NbC) {
             double ab = 0.0;
             if (K.type[k] == kBuffer)
                 for (int e = bnd_ptr[k]; e < bnd_ptr[k + 1]; ++e) {
-                    const MomRec& r = rec[bnd_face[e]];
-                    if (r.flags & kMatrix) ab = -r.a12 - r.d12;
+                    const int s = bnd_face[e];
+                    if (kind[s] & kMatrix) ab = -convect(rec[s].fa).a12 - rec[s].d12;
                 }
             abou[k] = ab;
             continue;
@@ -332,79 +347,67 @@ __global__ void __launch_bounds__(kAsmBlock) mom_cell_kernel(
         if (k == NbC) continue;  // there is no cell 0
         const int i = k - NbC - 1;
         const int e0 = cf_ptr[i], e1 = cf_ptr[i + 1];
-        // convection and upwind sums (:205-236)
-        double C = 0.0, X = 0.0;
+        // convection C and upwind X sums (:205-236), cross diffusion Y, Aval
+        // (:276-416).  The boundary faces' terms of b come after urfc (C - X).
+        double C = 0.0, X = 0.0, Y = 0.0, d = 0.0;
+        bool edge = false;
         for (int e = e0; e < e1; ++e) {
             const int sf = slot_face[e];
-            const MomRec& r = rec[sf >= 0 ? sf : ~sf];
-            if (sf >= 0) {
-                C = C - r.t;
-                if (r.flags & kUpwind) X = X - r.u;
-            } else {
-                C = C + r.t;
-                if (r.flags & kUpwind) X = X + r.u;
+            const int s = sf >= 0 ? sf : ~sf;
+            const int flags = kind[s];
+            const MomRec r = rec[s];
+            const Convect a = convect(r.fa);
+            const bool first = sf >= 0;
+            C = C + signed_by(r.t, first);
+            if (flags & kUpwind) X = X + signed_by(r.u, first);
+            Y = (Y + signed_by(r.fex, !first)) + signed_by(r.fim, first);
+            if (!(flags & kMatrix)) continue;
+            const int cls = (flags >> kShift) & 7;
+            if (cls != kOtherB) {
+                d = d + pick(first, a.a21, a.a12);
+                if (cls != kOutflowB) d = d + pick(first, r.d21, r.d12);
             }
+            if (cls == kInterior) {
+                const int o = first ? sid1[s] : sid2[s];
+                const double own = pick(first, a.a12, a.a21);
+                aval[o] = (single ? zero_minus(own) : aval[o] - own) - pick(first, r.d12, r.d21);
+            }
+            edge |= cls == kWallLike || cls == kOutflowB;
         }
         double bb = 0.0;
         if (P.convec == kFI) {
             const int m = K.material[k];
             double urfc = 0.0;
             if (m < 1 || m > Mt.nmat)
-                atomicOr(err, kErrMaterial);
+                err->material = 1;
             else
                 urfc = Mt.urfc[m - 1];
-            bb = bb + urfc * (C - X);
+            bb = bb + mul_rn(urfc, C - X);
         }
-        // cross diffusion, Aval and boundary b terms (:276-416)
-        X = 0.0;
-        double d = 0.0;
-        for (int e = e0; e < e1; ++e) {
-            const int sf = slot_face[e];
-            const int s = sf >= 0 ? sf : ~sf;
-            const MomRec& r = rec[s];
-            if (sf >= 0) {
-                X = X + r.fex - r.fim;
-                if (r.flags & kMatrix) {
-                    const int cls = (r.flags >> kShift) & 7;
-                    if (cls == kInterior) {
-                        d = d + r.a21 + r.d21;
-                        const int o = sid1[s];
-                        aval[o] = aval[o] - r.a12 - r.d12;
-                    } else if (cls == kWallLike) {
-                        d = d + r.a21 + r.d21;
-                        bb = bb + r.bv;
-                    } else if (cls == kOutflowB) {
-                        d = d + r.a21;
-                        bb = bb + r.bv;
-                    } else if (cls == kBufferB) {
-                        d = d + r.a21 + r.d21;
-                    }
-                }
-            } else {
-                X = X - r.fex + r.fim;
-                if (r.flags & kMatrix) {
-                    d = d + r.a12 + r.d12;
-                    const int o = sid2[s];
-                    aval[o] = aval[o] - r.a21 - r.d21;
-                }
+        if (edge)
+            for (int e = e0; e < e1; ++e) {
+                const int s = slot_face[e];
+                if (s < 0 || !(kind[s] & kMatrix)) continue;
+                const int cls = (kind[s] >> kShift) & 7;
+                if (cls == kWallLike || cls == kOutflowB) bb = bb + rec[s].bv;
             }
-        }
-        if (P.cross == kFI) bb = bb + X;
+        if (P.cross == kFI) bb = bb + Y;
         // inertial terms (:451-460)
         const double vol = K.vol[k];
         if (P.inert == kLIN) {
-            d = d + vol / P.dt;
-            bb = bb + vol / P.dt * K.rho_o[k] * K.ui_o[k] + K.source[k] * vol;
+            const double a = div_rn(vol, P.dt);
+            d = d + a;
+            bb = bb + mul_rn(mul_rn(a, K.rho_o[k]), K.ui_o[k]) + mul_rn(K.source[k], vol);
         } else if (P.inert == kPAR) {
-            d = d + 1.5 * vol / P.dt;
-            bb = bb + 2.0 * vol / P.dt * K.rho_o[k] * K.ui_o[k] -
-                 0.5 * vol / P.dt * K.rho_oo[k] * K.ui_oo[k] + K.source[k] * vol;
+            d = d + div_rn(1.5 * vol, P.dt);
+            bb = bb + div_rn(twice(vol), P.dt) * K.rho_o[k] * K.ui_o[k] -
+                 div_rn(half(vol), P.dt) * K.rho_oo[k] * K.ui_oo[k] + K.source[k] * vol;
         }
-        bb = bb - K.pi[k] * vol;  // :488
+        bb = bb - mul_rn(K.pi[k], vol);  // :488
         // under-relaxation (:497-499)
         if (P.var == 1 && asave) asave[i] = d;
-        bb = bb + d * (1.0 - P.urf) * rhoui[k] / P.urf;
-        aval[adia[i]] = d / P.urf;
+        bb = bb + div_rn(mul_rn(mul_rn(d, 1.0 - P.urf), rhoui[k]), P.urf);
+        aval[adia[i]] = div_rn(d, P.urf);
         b[i] = bb;
     }
 }
@@ -434,11 +437,10 @@ extern "C" int tflows_newuvw_assemble_device(tflows_assembly* a, const tflows_ne
     const int ncell = a->NbC + a->NC + 1;
     cudaError_t e = cudaSuccess;
     if (!a->mom_rec) {
-        e = cudaMalloc(&a->mom_rec, sizeof(MomRec) * (size_t)std::max(a->NS, 1));
+        e = cudaMalloc(&a->mom_rec, (sizeof(MomRec) + 1) * (size_t)std::max(a->NS, 1));
         if (e == cudaSuccess) e = cudaMalloc(&a->mom_cells, sizeof(double) * 3 * (size_t)ncell);
-        if (e == cudaSuccess) e = cudaMalloc(&a->mom_err, sizeof(int));
         if (e != cudaSuccess) {
-            for (void** q : {&a->mom_rec, (void**)&a->mom_cells, (void**)&a->mom_err})
+            for (void** q : {&a->mom_rec, (void**)&a->mom_cells})
                 if (*q) {
                     cudaFree(*q);
                     *q = nullptr;
@@ -467,37 +469,38 @@ extern "C" int tflows_newuvw_assemble_device(tflows_assembly* a, const tflows_ne
     double* pmax = a->mom_cells + ncell;
     double* pmin = a->mom_cells + 2 * (size_t)ncell;
     auto* rec = (MomRec*)a->mom_rec;
+    auto* kind = (unsigned char*)(rec + std::max(a->NS, 1));
     const int cb = std::max(1, std::min((ncell + kAsmBlock - 1) / kAsmBlock, 65535));
     const int fb = std::max(1, std::min((a->NS + kAsmBlock - 1) / kAsmBlock, 65535));
     cudaEventRecord(a->ev0, s);
-    e = cudaMemsetAsync(aval, 0, sizeof(double) * a->NONZ, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(a->mom_err, 0, sizeof(int), s);
+    // every entry of Aval is set by one face or one diagonal: nothing to add to
+    const bool single = a->single && (p->diffus == kCN || p->diffus == kFI);
+    if (!single) e = cudaMemsetAsync(aval, 0, sizeof(double) * a->NONZ, s);
+    a->note->blend = a->note->material = 0;
     if (e == cudaSuccess) {
-        mom_bounds_kernel<<<cb, kAsmBlock, 0, s>>>(a->NC, a->NbC, a->c1, a->c2, a->cf_ptr,
-                                                   a->slot_face, a->bnd_ptr, a->bnd_face, K, Mt,
+        mom_bounds_kernel<<<cb, kAsmBlock, 0, s>>>(a->NC, a->NbC, a->c1, a->cf_ptr,
+                                                   a->slot_cell, a->bnd_ptr, a->bnd_face, K, Mt,
                                                    ru, pmax, pmin);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess && a->NS > 0) {
         mom_face_kernel<<<fb, kAsmBlock, 0, s>>>(a->NS, a->NbC, a->c1, a->c2, F, K, Mt, P, ru,
-                                                 pmax, pmin, rec, a->mom_err);
+                                                 pmax, pmin, rec, kind, a->d_note);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
         mom_cell_kernel<<<cb, kAsmBlock, 0, s>>>(a->NC, a->NbC, a->cf_ptr, a->slot_face,
                                                  a->bnd_ptr, a->bnd_face, a->sid1, a->sid2,
-                                                 a->adia, rec, K, Mt, P, ru, aval, b, abou,
-                                                 asave, a->mom_err);
+                                                 a->adia, rec, kind, single, K, Mt, P, ru, aval, b, abou,
+                                                 asave, a->d_note);
         e = cudaGetLastError();
     }
     cudaEventRecord(a->ev1, s);
-    int bad = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, a->mom_err, sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess)
         return mom_fail(TFLOWS_CUDA_ERROR, std::string("momentum assembly: ") + cudaGetErrorString(e));
-    if (bad & kErrMaterial) return mom_fail(TFLOWS_BAD_INPUT, "material index outside 1..nmat");
-    if (bad & kErrBlend)
+    if (a->note->material) return mom_fail(TFLOWS_BAD_INPUT, "material index outside 1..nmat");
+    if (a->note->blend)
         return mom_fail(TFLOWS_BAD_INPUT,
                         "a face joins a material blending with YES and one with NO: ConvScheme "
                         "has no value for that code");
