@@ -411,11 +411,12 @@ bool tiles_env_on() {
 size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
 // FP64 CG forms its search direction inside the product only on small
-// systems, where the grid barrier it saves (about 2 us) is worth more than
+// systems, where the grid barrier it saves (about 1.2 us) is worth more than
 // the FP64 operations it adds, one (reference arithmetic: two) per entry.
-// Measured, us per iteration inside the product / as a pass of its own, in
-// reference arithmetic: 16.6 / 17.4 at 32^3, 23.3 / 21.8 at 48^3; with
-// multiply-adds 16.0 / 16.3 at 48^3, 25.3 / 23.9 at 64^3.
+// Measured, us per iteration inside the product / as a pass of its own: in
+// reference arithmetic 13.1 / 13.9 at 24^3, 13.4 / 14.3 at 32^3, 16.3 / 15.8 at
+// 40^3; with multiply-adds 10.1 / 11.3 at 24^3, 13.4 / 13.6 at 48^3, 21.0 /
+// 19.2 at 64^3.
 bool fuse_dir_fp64(const DeviceTopology& t, const SolveRequest& rq) {
     return t.n <= (rq.precision == 0 ? 50 : 120) * 1000;
 }

@@ -27,6 +27,7 @@
 #pragma once
 
 #include "device_common.cuh"
+#include "fp64_int.cuh"
 
 #include <type_traits>
 
@@ -222,10 +223,12 @@ __device__ __forceinline__ void publish_t(Grid& g, int slot, const T (&v)[K]) {
 // reference's correctly rounded division; the contracted build
 // (TFLOWS_FP64_RECIP_DIAG) and the FP32 inner solves hold 1/D and multiply.
 #ifdef TFLOWS_FP64_RECIP_DIAG
+constexpr bool kIntProducts = false;
 constexpr bool kRecipDiag64 = true;
 __device__ __forceinline__ double jacobi(double r, double dinv) { return r * dinv; }
 #else
 constexpr bool kRecipDiag64 = false;
+constexpr bool kIntProducts = true;
 __device__ __forceinline__ double jacobi(double r, double d) { return div_rn(r, d); }
 #endif
 __device__ __forceinline__ float jacobi(float r, float dinv) { return r * dinv; }
@@ -331,6 +334,14 @@ __device__ __forceinline__ T sell_row(const Mat<T>& m, int s, int lane, const X*
     return acc;
 }
 
+// a * b of a reference-arithmetic product: on the integer pipe in the build
+// whose sums are separate (fp64_int.cuh), which the FP64 pipe bounds.
+template <typename T>
+__device__ __forceinline__ T prod(T a, T b) {
+    if constexpr (sizeof(T) == 8 && kIntProducts) return mul_rn(a, b);
+    else return a * b;
+}
+
 // q_i = sum_j a_ij (z_j + beta p_j): the product with the next search
 // direction formed inside the gather (FP32 inner solves), so the update
 // p = z + beta p needs no pass of its own and no grid barrier.  `first`:
@@ -346,6 +357,14 @@ __device__ __forceinline__ double fused_dir(double z, double beta, double p, boo
     return first ? z : z + beta * p;
 }
 
+// Entries of a row loaded ahead of their use; a hexahedron's row has as many.
+// (The FP64 pipe also does what a predicate turns off, so an eighth entry
+// that no row has would cost as much as the others.)
+// FP32 rows of more than eight entries have a function of their own: the loop
+// over the rest costs the others registers (85 -> 105 us per iteration).
+template <typename T>
+constexpr int kRowAhead = sizeof(T) == 8 ? 7 : 8;
+
 // ---- the phases of an iteration ------------------------------------------------
 // They are inlined: as functions of their own they cost 30 us per iteration
 // at 4.1 M rows (registers saved around each call go through L2, and their
@@ -360,19 +379,20 @@ __device__ __forceinline__ double fused_dir(double z, double beta, double p, boo
 // product, bit for bit, with one vector pass and one grid barrier less.
 // Bound by DRAM (FP32, and FP64 sums with fused multiply-adds on large
 // systems) or by the FP64 pipe's 2 lanes per clock and SM (separate products
-// and sums).  Slices of at most 8 entries per row: every load of a row is in
-// flight before its first use, with the pattern of the next row, so that
-// nothing waits twice; the values are streamed past L1, whose lines the
-// gathers of neighbouring warps share.  Of a CG iteration on 161 x 150 x 170
-// cells (512 x 304 threads) against an explicit column per entry, an offset
-// per slice and values through L1: FP64 322 -> 255 us (with the scalar
-// divisions off the FP64 pipe), fused multiply-adds 144 -> 139, FP32 105 ->
-// 85.  Values staged through shared memory by asynchronous copies took
-// 262, 162 and 93: what they hold is taken from L1.
+// and sums, of which the products go to the integer pipe).  The loads of a
+// row's first entries are in flight before their first use, with the pattern
+// of the next row, so that nothing waits twice; the values are streamed past
+// L1, whose lines the gathers of neighbouring warps share.  Of a CG iteration
+// on 161 x 150 x 170 cells (512 x 304 threads) against an explicit column per
+// entry, an offset per slice, values through L1 and every FP64 operation on
+// its pipe: FP64 322 -> 176 us (238 with the products on the FP64 pipe), fused
+// multiply-adds 144 -> 132, FP32 105 -> 85.  Values staged through shared
+// memory by asynchronous copies cost 7 % to 15 %: what they hold is taken from L1.
 template <typename T, bool DIR, bool COLUMNS>
-__device__ __forceinline__ T product_narrow(const Mat<T>& m, int wg, int nw, const T* __restrict__ z,
+__device__ __forceinline__ T product_rows(const Mat<T>& m, int wg, int nw, const T* __restrict__ z,
                                             const T* __restrict__ p, T* __restrict__ pn, T* __restrict__ q,
                                             const T* __restrict__ w, T beta, bool first) {
+    constexpr int kAhead = kRowAhead<T>;
     const int lane = threadIdx.x & 31, n = m.n, nslices = m.nslices;
     T sum = T(0);
     unsigned id = !COLUMNS && wg < nslices ? m.spat[wg * kWarp + lane] : 0;
@@ -384,35 +404,48 @@ __device__ __forceinline__ T product_narrow(const Mat<T>& m, int wg, int nw, con
             b0 = m.soff[s];
             ww = (int)((m.soff[s + 1] - b0) >> 5);
         }
-        T v[8];
+        T v[kAhead];
 #pragma unroll
-        for (int t = 0; t < 8; ++t) v[t] = t < ww ? __ldcs(m.sval + b0 + 32 * t + lane) : T(0);
-        int c[8];
+        for (int t = 0; t < kAhead; ++t) v[t] = t < ww ? __ldcs(m.sval + b0 + 32 * t + lane) : T(0);
+        int c[kAhead];
+        const unsigned pat = id;
         if (COLUMNS) {
 #pragma unroll
-            for (int t = 0; t < 8; ++t) c[t] = t < ww ? __ldcs(m.scol + b0 + 32 * t + lane) : -1;
+            for (int t = 0; t < kAhead; ++t) c[t] = t < ww ? __ldcs(m.scol + b0 + 32 * t + lane) : -1;
         } else {
-            const int4* const po = reinterpret_cast<const int4*>(m.poff) + 2 * id;
+            const int4* const po = reinterpret_cast<const int4*>(m.poff) + 2 * pat;
             const int4 a = __ldg(po), b = __ldg(po + 1);
             id = s + nw < nslices ? m.spat[(s + nw) * kWarp + lane] : 0;
             c[0] = i + a.x; c[1] = i + a.y; c[2] = i + a.z; c[3] = i + a.w;
-            c[4] = i + b.x; c[5] = i + b.y; c[6] = i + b.z; c[7] = i + b.w;
+            c[4] = i + b.x; c[5] = i + b.y; c[6] = i + b.z;
+            if (kAhead == 8) c[kAhead - 1] = i + b.w;
         }
         T xi = T(0);  // the row's own direction (FP32 and DIR)
         if ((DIR || sizeof(T) == 4) && i < n)
             xi = DIR ? fused_dir(z[i], beta, first ? T(0) : p[i], first) : p[i];
-        T x[8], acc = T(0);
+        T x[kAhead], acc = T(0);
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
+        for (int t = 0; t < kAhead; ++t) {
             const T pt = c[t] >= 0 && !(DIR && first) ? p[c[t]] : T(0);
             x[t] = DIR ? (c[t] >= 0 ? fused_dir(z[c[t]], beta, pt, first) : T(0)) : pt;
         }
 #pragma unroll
-        for (int t = 0; t < 8; ++t)
+        for (int t = 0; t < kAhead; ++t)
             if (c[t] >= 0) {
                 if constexpr (sizeof(T) == 4) acc = acc + diff_term(v[t], x[t], xi, c[t] == i);
-                else acc = acc + v[t] * x[t];
+                else acc = acc + (DIR ? v[t] * x[t] : prod(v[t], x[t]));
             }
+        if constexpr (kAhead < 8) {
+#pragma unroll 1
+            for (int t = kAhead; t < ww; ++t) {
+                const int j = COLUMNS ? m.scol[b0 + 32 * t + lane] : i + m.poff[8 * pat + t];
+                if (j < 0) continue;
+                T xt = first && DIR ? T(0) : p[j];
+                if (DIR) xt = fused_dir(z[j], beta, xt, first);
+                const T vt = m.sval[b0 + 32 * t + lane];
+                acc = acc + (DIR ? vt * xt : prod(vt, xt));
+            }
+        }
         if (i < n) {
             q[i] = acc;
             if (DIR) pn[i] = xi;
@@ -422,26 +455,23 @@ __device__ __forceinline__ T product_narrow(const Mat<T>& m, int wg, int nw, con
     return sum;
 }
 
-// The same for rows of any length.
-template <typename T, bool DIR>
-__device__ __noinline__ T product_wide(const Mat<T>& m, int wg, int nw, const T* z, const T* p, T* pn, T* q,
-                                       const T* w, T beta, bool first) {
+// The same for FP32 rows of more than eight entries.
+template <bool DIR>
+__device__ __noinline__ float product_wide(const Mat<float>& m, int wg, int nw, const float* z, const float* p,
+                                           float* pn, float* q, const float* w, float beta, bool first) {
     const int lane = threadIdx.x & 31;
-    T sum = T(0);
+    float sum = 0.f;
     for (int s = wg; s < m.nslices; s += nw) {
         const int i = s * kWarp + lane;
         const long long b0 = m.soff[s];
         const int ww = (int)((m.soff[s + 1] - b0) >> 5);
-        T xi = T(0), acc = T(0);
-        if ((DIR || sizeof(T) == 4) && i < m.n)
-            xi = DIR ? fused_dir(z[i], beta, first ? T(0) : p[i], first) : p[i];
+        float xi = 0.f, acc = 0.f;
+        if (i < m.n) xi = DIR ? fused_dir(z[i], beta, first ? 0.f : p[i], first) : p[i];
         for (int t = 0; t < ww; ++t) {
             const int c = m.scol[b0 + 32 * t + lane];
             if (c < 0) continue;
-            const T v = m.sval[b0 + 32 * t + lane];
-            const T x = DIR ? fused_dir(z[c], beta, first ? T(0) : p[c], first) : p[c];
-            if constexpr (sizeof(T) == 4) acc = acc + diff_term(v, x, xi, c == i);
-            else acc = acc + v * x;
+            const float x = DIR ? fused_dir(z[c], beta, first ? 0.f : p[c], first) : p[c];
+            acc = acc + diff_term(m.sval[b0 + 32 * t + lane], x, xi, c == i);
         }
         if (i < m.n) {
             q[i] = acc;
@@ -455,9 +485,11 @@ __device__ __noinline__ T product_wide(const Mat<T>& m, int wg, int nw, const T*
 template <typename T, bool DIR>
 __device__ __forceinline__ T product_phase(const Mat<T>& m, int wg, int nw, const T* z, const T* p, T* pn,
                                            T* q, const T* w, T beta, bool first) {
-    if (!m.narrow) return product_wide<T, DIR>(m, wg, nw, z, p, pn, q, w, beta, first);
-    if (m.spat) return product_narrow<T, DIR, false>(m, wg, nw, z, p, pn, q, w, beta, first);
-    return product_narrow<T, DIR, true>(m, wg, nw, z, p, pn, q, w, beta, first);
+    if constexpr (sizeof(T) == 4) {
+        if (!m.narrow) return product_wide<DIR>(m, wg, nw, z, p, pn, q, w, beta, first);
+    }
+    if (m.spat) return product_rows<T, DIR, false>(m, wg, nw, z, p, pn, q, w, beta, first);
+    return product_rows<T, DIR, true>(m, wg, nw, z, p, pn, q, w, beta, first);
 }
 
 // p = z + beta p, or z when `first` (CG.f90:178-187).
@@ -472,7 +504,7 @@ __device__ __forceinline__ void direction_phase(int tid, int nt, int n, const T*
         const V4<T> zz = ld4(z + i);
         V4<T> pp = ld4(p + i);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) pp.a[u] = zz.a[u] + beta * pp.a[u];
+        for (int u = 0; u < 4; ++u) pp.a[u] = zz.a[u] + prod(beta, pp.a[u]);
         st4(p + i, pp);
     }
 }
@@ -498,8 +530,8 @@ __device__ __forceinline__ Sums3<T> update_loop(int tid, int nt, int n, T* __res
         if (diag) dd = ld4(D + i);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            xx.a[u] = xx.a[u] + alfa * pp.a[u];
-            rr.a[u] = rr.a[u] - alfa * qq.a[u];
+            xx.a[u] = xx.a[u] + prod(alfa, pp.a[u]);
+            rr.a[u] = rr.a[u] - prod(alfa, qq.a[u]);
             if (diag) zz.a[u] = jacobi(rr.a[u], dd.a[u]);
             if (i + u < n) {
                 rr_ += rr.a[u] * rr.a[u];
