@@ -44,6 +44,7 @@ struct DeviceTopology {
     // exactly its 7-point neighbours in ascending order (what TopolM builds
     // for a structured block); enables the tiled IC sweeps
     int box_nx = 0, box_ny = 0, box_nz = 0;
+    int* box_row = nullptr;  // a box in another numbering: the row of each cell
     // host copies (0-based) for lazy derived data
     std::vector<int> h_rowptr, h_col, h_diag;
 };

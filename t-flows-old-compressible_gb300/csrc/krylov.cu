@@ -77,7 +77,8 @@ __global__ void permute_kernel(int n, const int* __restrict__ rowptr, const int*
 // absent neighbours and idle lanes hold 0.
 template <typename L, typename T>
 __global__ void tile_permute_kernel(Tiles<T> tl, long long total, const long long* __restrict__ soff,
-                                    const int* __restrict__ meta, const L* __restrict__ sval) {
+                                    const int* __restrict__ scol, const int* __restrict__ meta,
+                                    const L* __restrict__ sval) {
     const int sp = tl.chunks * kTileK;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
          i += (long long)gridDim.x * blockDim.x) {
@@ -88,15 +89,41 @@ __global__ void tile_permute_kernel(Tiles<T> tl, long long total, const long lon
         patch_origin(tl, pt, x0, y0);
         for (int dir = 0; dir < 2; ++dir) {
             L a[3] = {L(0), L(0), L(0)};
+            unsigned ord = kBoxOrder;
             if (patch_cell(tl, dir, x0, y0, s, lane, x, y, z)) {
-                const int row = x + tl.nx * (y + tl.ny * z);
+                const int cell = x + tl.nx * (y + tl.ny * z), row = tl.row ? tl.row[cell] : cell;
                 const long long base = soff[row >> 5] + (row & 31);
                 int q = dir ? (meta[row] >> 16) + 1 : 0;  // upper entries follow the diagonal
                 const bool has[3] = {dir ? x < tl.nx - 1 : z > 0, dir ? y < tl.ny - 1 : y > 0,
                                      dir ? z < tl.nz - 1 : x > 0};
-                for (int f = 0; f < 3; ++f)
-                    if (has[f]) a[f] = sval[base + 32LL * q++];
+                if (!tl.row) {
+                    for (int f = 0; f < 3; ++f)
+                        if (has[f]) a[f] = sval[base + 32LL * q++];
+                } else {
+                    const int nxy = tl.nx * tl.ny;
+                    const int nb[3] = {dir ? cell + 1 : cell - nxy, dir ? cell + tl.nx : cell - tl.nx,
+                                       dir ? cell + nxy : cell - 1};
+                    // entries in the row's order, then the absent ones
+                    unsigned place = 0, seen = 0;
+                    ord = 0;
+                    for (int e = 0; e < has[0] + has[1] + has[2]; ++e, ++q)
+                        for (int f = 0; f < 3; ++f)
+                            if (has[f] && tl.row[nb[f]] == scol[base + 32LL * q]) {
+                                a[f] = sval[base + 32LL * q];
+                                ord |= (unsigned)f << (2 * place++);
+                                seen |= 1u << f;
+                            }
+                    bool rising = true;  // absent entries (0 times 0) may go anywhere
+                    for (unsigned e = 1; e < place; ++e)
+                        rising = rising && (ord >> (2 * e) & 3u) > (ord >> (2 * e - 2) & 3u);
+                    for (int f = 0; f < 3; ++f)
+                        if (!(seen >> f & 1u)) ord |= (unsigned)f << (2 * place++);
+                    if (rising) ord = kBoxOrder;
+                }
             }
+            if (tl.ord[dir])
+                reinterpret_cast<unsigned char*>(tl.ord[dir])[((ps / kTileK) * 32 + lane) * kTileK + s % kTileK] =
+                    (unsigned char)ord;
             unsigned char* r = tl.rec[dir] + ps * tile_rec_bytes(sizeof(L), sizeof(T));
             for (int f = 0; f < 3; ++f) *reinterpret_cast<L*>(r + TileRec<L, T>::at(f, lane)) = a[f];
         }
@@ -467,6 +494,7 @@ void tile_elem(const SolveRequest& rq, unsigned& ls, unsigned& sv) {
 // Forward and backward records, the middle values, the edge words of both.
 size_t tile_buffer_bytes(const DeviceTopology& t, const TileGeom& g, unsigned ls, unsigned sv) {
     return 2 * align256(g.lanes * (3 * ls + sv)) + align256(g.lanes * sv) +
+           (t.box_row && sv == 8 ? 2 * align256(g.lanes) : 0) +
            2 * align256(g.patches * tile_edge_words(g.chunks) * tile_edge_bytes(sv));
 }
 
@@ -555,8 +583,11 @@ cudaError_t fill_tiles(const DeviceTopology& t, Workspace& ws, const SolveReques
     tl.mid = reinterpret_cast<T*>(take(tg.lanes * sizeof(T)));
     for (int dir = 0; dir < 2; ++dir)
         tl.edge[dir] = take(tg.patches * tile_edge_words(tg.chunks) * tile_edge_bytes(sizeof(T)));
+    tl.row = t.box_row;
+    if (t.box_row && sizeof(T) == 8)
+        for (int dir = 0; dir < 2; ++dir) tl.ord[dir] = (unsigned*)take(tg.lanes);
     const int nb = (int)std::min<long long>(std::max<long long>(1, (long long)(tg.lanes / 256)), sms() * 16LL);
-    tile_permute_kernel<L, T><<<nb, 256, 0, s>>>(tl, (long long)tg.lanes, t.soff, t.meta, sval);
+    tile_permute_kernel<L, T><<<nb, 256, 0, s>>>(tl, (long long)tg.lanes, t.soff, t.scol, t.meta, sval);
     return cudaGetLastError();
 }
 

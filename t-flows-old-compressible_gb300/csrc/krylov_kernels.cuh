@@ -45,8 +45,11 @@ __device__ __forceinline__ T tiny_v() {
 // Reduction slots in the partials array (each slot = one value per block).
 enum : int { SLOT_A = 0, SLOT_B = 4, SLOT_C = 8, SLOT_D = 12, NUM_SLOTS = 16 };
 
-// Tiled IC(0) sweeps on a box-numbered pattern (row = x + nx (y + ny z),
-// 7-point stencil in TopolM order).  A warp owns a patch of 8 x 4 columns of
+// Tiled IC(0) sweeps on a box (7-point stencil): numbered row = x + nx (y +
+// ny z), or in any way that numbers a cell after its three neighbours before
+// it along x, y and z, as the blocks of a block-structured mesh do (the
+// sweeps' order of dependence is the same; `row` then leads from a cell to its
+// row, and `ord` keeps the order of each row's sum).  A warp owns a patch of 8 x 4 columns of
 // the box over all z, one column per lane, and walks the wavefront: at step s
 // lane (mx, my) solves the cell z = s - mx - my of its column.  A tile is the
 // patches of one block, at most two of them side by side in x.
@@ -81,7 +84,16 @@ struct Tiles {
     unsigned char* rec[2];   // forward / backward records, [patch][step]
     T* mid;                  // what the backward sweep starts from, [patch][step][lane]
     unsigned char* edge[2];  // forward / backward edge words, [patch][tile_edge_words]
+    // A box in another numbering: the row of cell x + nx (y + ny z) (null: the
+    // cell itself), and the order in which each row adds its three
+    // neighbours, [patch][chunk][lane], one byte per step (reference
+    // arithmetic; null: kBoxOrder)
+    const int* row;
+    unsigned* ord[2];
 };
+// Two bits per place: which of a record's entries is added first, second, third.
+constexpr unsigned kBoxOrder = 0 | 1 << 2 | 2 << 4;
+constexpr unsigned kBoxOrders = kBoxOrder * 0x01010101u;
 
 // Edge words of a patch: per step of the reading patch its four edge cells
 // along x, then the eight along y.
@@ -1090,7 +1102,8 @@ __device__ __noinline__ void tiles_init(Grid& g, const Mat<T>& m, const T* __res
             const bool in = patch_cell(tl, dir, x0, y0, s, lane, x, y, z);
             const unsigned at = cb == sizeof(T) ? TileRec<T, T>::at(3, lane)
                                                 : TileRec<unsigned short, float>::at(3, lane);
-            const T d = in ? D[x + tl.nx * (y + tl.ny * z)] : T(0);
+            const int cell = x + tl.nx * (y + tl.ny * z);
+            const T d = in ? D[tl.row ? tl.row[cell] : cell] : T(0);
             unsigned char* const r = tl.rec[dir] + ps * rec;
             *reinterpret_cast<T*>(r + at) = d;
             if constexpr (kScaledRec<T>)
@@ -1146,7 +1159,7 @@ __device__ __forceinline__ bool tile_wait(DevCtl* ctl, long long limit, int wher
 // One sweep over this block's tiles, forward (BWD = 0) or backward.  Forward
 // reads rhs and writes tl.mid; backward reads tl.mid and rhs and writes zout,
 // with epi (RowOp) per row.  Not ok: a wait gave up (the launch is aborted).
-template <int BWD, typename L, typename T, typename Epi>
+template <int BWD, bool MAP, typename L, typename T, typename Epi>
 __device__ __forceinline__ Applied<T> tile_sweep(DevCtl* ctl, long long limit, int bid, int nblocks,
                                               unsigned epoch, int first, const Mat<T>& m,
                                               const T* __restrict__ rhs, T* __restrict__ zout, Epi epi) {
@@ -1221,7 +1234,13 @@ __device__ __forceinline__ Applied<T> tile_sweep(DevCtl* ctl, long long limit, i
             T* const to_y = give_y ? own + px * kDn * (int)(kWarpB / sizeof(T)) - kPatchY * kRowS : own;
             const unsigned back_x = give_x ? kPatchX : 0, back_y = give_y ? kPatchY : 0;
             T prev = T(0);
+            constexpr bool kOrders = MAP && sizeof(T) == 8 && !kScaledRec<T>;
+            const unsigned* const ords =
+                kOrders ? tl.ord[BWD] + (size_t)(k * sw + w) * chunks * 32 + lane : nullptr;
+            unsigned ord_next = kOrders ? ords[0] : kBoxOrders;
             for (int c = 0; c < chunks; ++c) {
+                const unsigned ord = ord_next;
+                if (kOrders && c + 1 < chunks) ord_next = ords[(c + 1) * 32];
                 const int target = base + min(c + off, chunks);
                 if (!tile_wait(ctl, limit, BWD ? 28 : 26,
                                [&] { return progress_load(watch) - target >= 0; }))
@@ -1232,7 +1251,7 @@ __device__ __forceinline__ Applied<T> tile_sweep(DevCtl* ctl, long long limit, i
                 const T* const before = own + ((pos - 1) & (kRing - 1)) * kSlot;
                 T* const gx = to_x + ((pos - back_x) & (kRing - 1)) * kSlot;
                 T* const gy = to_y + ((pos - back_y) & (kRing - 1)) * kSlot;
-                auto steps = [&](auto all_inside) {
+                auto steps = [&](auto all_inside, auto box_order) {
                     TileRec<L, T> r[kTileK];
                     T f[kTileK];
 #pragma unroll
@@ -1258,9 +1277,19 @@ __device__ __forceinline__ Applied<T> tile_sweep(DevCtl* ctl, long long limit, i
                             v = f[u] - a * r[u].d;
                         } else {
                             T a = f[u];
-                            a = a - r[u].a[0] * (BWD ? vx : prev);
-                            a = a - r[u].a[1] * vy;
-                            a = a - r[u].a[2] * (BWD ? prev : vx);
+                            if (decltype(box_order)::value) {
+                                a = a - r[u].a[0] * (BWD ? vx : prev);
+                                a = a - r[u].a[1] * vy;
+                                a = a - r[u].a[2] * (BWD ? prev : vx);
+                            } else {
+                                const T t0 = r[u].a[0] * (BWD ? vx : prev), t1 = r[u].a[1] * vy,
+                                        t2 = r[u].a[2] * (BWD ? prev : vx);
+#pragma unroll
+                                for (int e = 0; e < 3; ++e) {
+                                    const unsigned which = ord >> (8 * u + 2 * e) & 3u;
+                                    a = a - (which == 0 ? t0 : which == 1 ? t1 : t2);
+                                }
+                            }
                             v = a * r[u].d;
                         }
                         if (!decltype(all_inside)::value)
@@ -1272,10 +1301,16 @@ __device__ __forceinline__ Applied<T> tile_sweep(DevCtl* ctl, long long limit, i
                         __syncwarp();
                     }
                 };
-                if (whole && c * kTileK >= kSkew && (c + 1) * kTileK <= nz)
-                    steps(std::true_type{});
+                bool ordered = true;
+                if constexpr (kOrders) {
+                    ordered = __all_sync(0xffffffffu, ord == kBoxOrders);
+                    if (!ordered) steps(std::false_type{}, std::false_type{});
+                }
+                if (!ordered) {
+                } else if (whole && c * kTileK >= kSkew && (c + 1) * kTileK <= nz)
+                    steps(std::true_type{}, std::true_type{});
                 else
-                    steps(std::false_type{});
+                    steps(std::false_type{}, std::true_type{});
                 progress_store(prog, base + c + 1, lane);
                 pos = (pos + kTileK) & (kRing - 1);
                 st = st + 1 == kStages ? 0 : st + 1;
@@ -1309,6 +1344,12 @@ __device__ __forceinline__ Applied<T> tile_sweep(DevCtl* ctl, long long limit, i
             const T* src = BWD ? mid + (nz + kSkew - 1) * 32 + (31 - lane) : rhs + row0;
             const unsigned s_rec_a = smem_u32(s_rec) + lane * 16, s_mid_a = smem_u32(s_mid),
                            own_a = smem_u32(own);
+            // (another numbering: the rows of the next chunk's slabs)
+            const int* const rows = MAP ? tl.row + row0 : nullptr;
+            int next[kTileK];
+            if (!BWD && MAP)
+#pragma unroll
+                for (int u = 0; u < kTileK; ++u) next[u] = (unsigned)u < nzl ? rows[u * nxy] : 0;
             for (int i = 0; i < chunks + kFlight; ++i) {
                 if (i < chunks) {
                     const int target = base + i + off;
@@ -1324,7 +1365,16 @@ __device__ __forceinline__ Applied<T> tile_sweep(DevCtl* ctl, long long limit, i
                         else cp_async16(d + o, rec_src + o, lane * 16 < kChunkRec - o);
                     }
                     rec_src += kChunkRec;
-                    if (!BWD) {
+                    if (!BWD && MAP) {
+#pragma unroll
+                        for (int u = 0; u < kTileK; ++u) {
+                            const int z = i * kTileK + u;
+                            cp_async<sizeof(T)>(
+                                own_a + ((pos + u + skew) & (kRing - 1)) * (unsigned)(kSlot * sizeof(T)),
+                                rhs + next[u], (unsigned)z < nzl);
+                            next[u] = (unsigned)(z + kTileK) < nzl ? rows[(z + kTileK) * nxy] : 0;
+                        }
+                    } else if (!BWD) {
 #pragma unroll
                         for (int u = 0; u < kTileK; ++u) {
                             cp_async<sizeof(T)>(
@@ -1410,11 +1460,26 @@ __device__ __forceinline__ Applied<T> tile_sweep(DevCtl* ctl, long long limit, i
         unsigned char* const out_x = tl.edge[BWD] + ((size_t)pt * words + lane) * kEdge;
         unsigned char* const out_y = out_x + (size_t)ywords * kEdge;
         const bool far_x = dn_x == 2 && row_in, far_y = dn_y == 2 && x < tl.nx, publish_far = dn_x == 2 || dn_y == 2;
+        // (another numbering: the rows of the next chunk's slabs)
+        int next[kTileK];
+        if (BWD && MAP)
+#pragma unroll
+            for (int u = 0; u < kTileK; ++u)
+                next[u] = (unsigned)(u - kSkew) < nzl ? tl.row[row0 + (u - kSkew) * zstep] : 0;
         for (int c = 0; c < chunks; ++c) {
             const int z0 = c * kTileK - kSkew;  // backward: first of the slabs whose last lane is done
             const bool inside = whole && z0 >= 0 && z0 + kTileK <= nz;
             T rpre[kTileK];  // their right-hand side
-            if (BWD) {
+            int rows[kTileK];
+            if (BWD && MAP) {
+#pragma unroll
+                for (int u = 0; u < kTileK; ++u) {
+                    rows[u] = next[u];
+                    rpre[u] = (unsigned)(z0 + u) < nzl ? rhs[rows[u]] : T(0);
+                    const int z = z0 + kTileK + u;
+                    next[u] = (unsigned)z < nzl ? tl.row[row0 + z * zstep] : 0;
+                }
+            } else if (BWD) {
                 if (inside) {
 #pragma unroll
                     for (int u = 0; u < kTileK; ++u) rpre[u] = rhs[row0 + (z0 + u) * zstep];
@@ -1452,19 +1517,22 @@ __device__ __forceinline__ Applied<T> tile_sweep(DevCtl* ctl, long long limit, i
                     mp[u * 32] = v;
                 }
             } else {
-                auto flush = [&](int u) {
+                auto flush = [&](int u, int row) {
                     const T v = own[((pos - kSkew + u + skew) & (kRing - 1)) * kSlot];
-                    const int row = row0 + (z0 + u) * zstep;
                     zout[row] = v;
                     epi(row, v, rpre[u]);
                 };
-                if (inside) {
+                if (MAP) {
 #pragma unroll
-                    for (int u = 0; u < kTileK; ++u) flush(u);
+                    for (int u = 0; u < kTileK; ++u)
+                        if ((unsigned)(z0 + u) < nzl) flush(u, rows[u]);
+                } else if (inside) {
+#pragma unroll
+                    for (int u = 0; u < kTileK; ++u) flush(u, row0 + (z0 + u) * zstep);
                 } else {
 #pragma unroll
                     for (int u = 0; u < kTileK; ++u)
-                        if ((unsigned)(z0 + u) < nzl) flush(u);
+                        if ((unsigned)(z0 + u) < nzl) flush(u, row0 + (z0 + u) * zstep);
                 }
             }
             __syncwarp();
@@ -1477,7 +1545,7 @@ __device__ __forceinline__ Applied<T> tile_sweep(DevCtl* ctl, long long limit, i
 }
 
 // z = IC(0) apply of rhs by the tiled sweeps, epi (RowOp) per row.
-template <typename L, typename T, typename Epi>
+template <bool MAP, typename L, typename T, typename Epi>
 __device__ __forceinline__ Applied<T> ic_tiled_apply(Grid& g, const Mat<T>& m, const T* rhs, T* z, Epi epi) {
     const int chunks = tiles_of(m.tile, g.bid, g.nblocks) * m.tile.chunks, first = g.chunk0;
     ++g.epoch;
@@ -1486,11 +1554,19 @@ __device__ __forceinline__ Applied<T> ic_tiled_apply(Grid& g, const Mat<T>& m, c
     // the abort flag if the forward sweep of another warp gave up)
     const RowOp<kRowNone, T> none{T(0), nullptr, T(0)};
     const bool ok =
-        tile_sweep<0, L, T>(g.ctl, g.timeout_cyc, g.bid, g.nblocks, g.epoch, first, m, rhs, z, none).ok;
+        tile_sweep<0, MAP, L, T>(g.ctl, g.timeout_cyc, g.bid, g.nblocks, g.epoch, first, m, rhs, z, none).ok;
     Applied<T> a =
-        tile_sweep<1, L, T>(g.ctl, g.timeout_cyc, g.bid, g.nblocks, g.epoch, first + chunks, m, rhs, z, epi);
+        tile_sweep<1, MAP, L, T>(g.ctl, g.timeout_cyc, g.bid, g.nblocks, g.epoch, first + chunks, m, rhs, z, epi);
     a.ok = a.ok && ok;
     return a;
+}
+
+// On a box in another numbering.  A function of its own: the rows' look-up and
+// the order of their sums would cost the box numbering 4 to 7 % of an apply
+// (reference arithmetic, 109 x 83 x 97 cells: 527 -> 566 us per iteration).
+template <typename L, typename T, typename Epi>
+__device__ __noinline__ Applied<T> ic_mapped_apply(Grid& g, const Mat<T>& m, const T* rhs, T* z, Epi epi) {
+    return ic_tiled_apply<true, L>(g, m, rhs, z, epi);
 }
 
 // The IC(0) apply the solve was configured for: `sweeps` Jacobi sweeps per
@@ -1506,11 +1582,16 @@ __device__ __forceinline__ bool ic_precond(Grid& g, const Mat<T>& m, Vecs<T>& v,
     if (sweeps > 0) {
         a = ic_jacobi_apply(g, m, v.D, rhs, v.w, v.s, z, sweeps, epi);
     } else if (m.tile.on) {
-        if constexpr (sizeof(T) == 4)
-            a = m.tile.lu_bf16 ? ic_tiled_apply<unsigned short>(g, m, rhs, z, epi)
-                               : ic_tiled_apply<T>(g, m, rhs, z, epi);
-        else
-            a = ic_tiled_apply<T>(g, m, rhs, z, epi);
+        if constexpr (sizeof(T) == 4) {
+            if (m.tile.row)
+                a = m.tile.lu_bf16 ? ic_mapped_apply<unsigned short>(g, m, rhs, z, epi)
+                                   : ic_mapped_apply<T>(g, m, rhs, z, epi);
+            else
+                a = m.tile.lu_bf16 ? ic_tiled_apply<false, unsigned short>(g, m, rhs, z, epi)
+                                   : ic_tiled_apply<false, T>(g, m, rhs, z, epi);
+        } else {
+            a = m.tile.row ? ic_mapped_apply<T>(g, m, rhs, z, epi) : ic_tiled_apply<false, T>(g, m, rhs, z, epi);
+        }
     } else {
         a = ic_apply(g, m, v.D, rhs, v.w, z, epi);
     }

@@ -140,8 +140,9 @@ cudaError_t upload(T** dst, const T* src, size_t count) {
 void free_topology_arrays(DeviceTopology& t) {
     for (void* p : {(void*)t.rowptr, (void*)t.col, (void*)t.soff, (void*)t.scol, (void*)t.meta,
                     (void*)t.perm_f, (void*)t.perm_b, (void*)t.tpos, (void*)t.spat,
-                    (void*)t.poff})
+                    (void*)t.poff, (void*)t.box_row})
         if (p) cudaFree(p);
+    t.box_row = nullptr;
     t.rowptr = t.col = t.scol = t.meta = t.perm_f = t.perm_b = t.tpos = nullptr;
     t.soff = nullptr;
     t.spat = nullptr;
@@ -236,9 +237,104 @@ void detect_box(DeviceTopology& t) {
     t.box_nz = (int)nz;
 }
 
+// The same box in another numbering: every cell after its three neighbours
+// before it along x, y and z (blocks numbered one after the other, for
+// instance).  The one row without earlier neighbours, the first, is a corner;
+// rows with one earlier neighbour lie on the three axes, which gives the
+// dimensions; every other cell is the one later neighbour that the cells
+// before it share.  `row` is filled with the row of each cell, and every row
+// is checked against its cell.  A mesh that is no box leaves at the axes.
+bool find_box(const DeviceTopology& t, int dim[3], std::vector<int>& row) {
+    const int n = t.n;
+    const int* const rp = t.h_rowptr.data();
+    const int* const col = t.h_col.data();
+    const int* const dia = t.h_diag.data();
+    auto before = [&](int r) { return dia[r] - rp[r]; };
+    if (n < 8 || before(0) != 0 || rp[1] - rp[0] != 4 || col[dia[0]] != 0) return false;
+    std::vector<int> axis[3];
+    for (int a = 0; a < 3; ++a) {
+        axis[a].push_back(0);
+        int r = col[dia[0] + 1 + a];
+        while (true) {
+            if (r < 0 || r >= n || before(r) != 1 || (int)axis[a].size() >= n) return false;
+            axis[a].push_back(r);
+            int next = -1;
+            for (int k = dia[r] + 1; k < rp[r + 1]; ++k) {
+                const int c = col[k];
+                if (c <= r || c >= n) return false;
+                if (before(c) == 1) {
+                    if (next >= 0) return false;
+                    next = c;
+                }
+            }
+            if (next < 0) break;
+            r = next;
+        }
+        dim[a] = (int)axis[a].size();
+    }
+    const long long nx = dim[0], ny = dim[1], nz = dim[2], nxy = nx * ny;
+    if (nx < 2 || ny < 2 || nz < 2 || nxy > n || nxy * nz != n) return false;
+    row.assign(n, -1);
+    for (long long z = 0; z < nz; ++z)
+        for (long long y = 0; y < ny; ++y)
+            for (long long x = 0; x < nx; ++x) {
+                const long long i = x + nx * (y + ny * z);
+                const bool on[3] = {x > 0, y > 0, z > 0};
+                const int prev[3] = {on[0] ? row[i - 1] : -1, on[1] ? row[i - nx] : -1,
+                                     on[2] ? row[i - nxy] : -1};
+                int r = -1;
+                if (on[0] + on[1] + on[2] < 2) {
+                    r = on[0] ? axis[0][x] : on[1] ? axis[1][y] : axis[2][z];
+                } else {
+                    const int from = on[0] ? prev[0] : prev[1];
+                    for (int k = dia[from] + 1; k < rp[from + 1]; ++k) {
+                        const int c = col[k];
+                        int hits = 0;
+                        for (int q = rp[c]; q < dia[c]; ++q)
+                            for (int a = 0; a < 3; ++a) hits += on[a] && col[q] == prev[a];
+                        if (before(c) == on[0] + on[1] + on[2] && hits == before(c)) r = c;
+                    }
+                }
+                if (r < 0) return false;
+                row[i] = r;
+            }
+    // Every row exactly once, with its cell's neighbours and no others, the
+    // earlier ones before the diagonal.
+    std::vector<char> used(n, 0);
+    for (long long i = 0; i < n; ++i) {
+        const int r = row[i];
+        if (used[r]) return false;
+        used[r] = 1;
+        const long long x = i % nx, y = (i / nx) % ny, z = i / nxy;
+        const bool has[6] = {x > 0, y > 0, z > 0, x < nx - 1, y < ny - 1, z < nz - 1};
+        const long long step[3] = {1, nx, nxy};
+        int lower = 0, upper = 0;
+        for (int f = 0; f < 6; ++f) {
+            if (!has[f]) continue;
+            const int c = row[f < 3 ? i - step[f] : i + step[f - 3]];
+            ++(f < 3 ? lower : upper);
+            const int* const b = f < 3 ? col + rp[r] : col + dia[r] + 1;
+            const int* const e = f < 3 ? col + dia[r] : col + rp[r + 1];
+            if ((f < 3) != (c < r) || std::find(b, e, c) == e) return false;
+        }
+        if (before(r) != lower || rp[r + 1] - dia[r] - 1 != upper) return false;
+    }
+    return true;
+}
+
 // SELL-32 layout: slice s holds rows 32s..32s+31, width = longest row.
 cudaError_t build_device(DeviceTopology& t) {
     detect_box(t);
+    if (t.box_nx == 0 && t.ic_ok) {
+        int dim[3];
+        std::vector<int> row;
+        if (find_box(t, dim, row)) {
+            if (cudaError_t e = upload(&t.box_row, row.data(), row.size()); e != cudaSuccess) return e;
+            t.box_nx = dim[0];
+            t.box_ny = dim[1];
+            t.box_nz = dim[2];
+        }
+    }
     const int n = t.n;
     t.nslices = (n + 31) / 32;
     std::vector<long long> soff((size_t)t.nslices + 1, 0);
