@@ -170,15 +170,16 @@ int planned_grid(const DeviceTopology& t, const SolveRequest& rq);
 bool tiled_ic(const DeviceTopology& t, const SolveRequest& rq);
 // The launch shape of a request that names none.  Every block adds to what a
 // reduction costs (arrivals, partial sums, and FP64 additions on a pipe of 2
-// lanes per clock and SM, which few warps already keep busy), so small
-// systems run in one 256-thread block per SM, middle ones in two, large ones
-// in two of 512 threads.  Measured, us per iteration of a diagonal CG in
-// reference arithmetic / with multiply-adds: 64^3 41.8 / 25.3 in 152 blocks,
-// 58.8 / 34.1 in 608; 96^3 84.6 / 47.6 in 304, 98.5 / 49.9 in 608;
-// 161x150x170 323 / 146 in 304 of 512, 331 / 145 in 608.  The mixed solves'
-// products are FP32 and want the threads: 18.2 at 64^3 and 31.3 at 96^3 in 152
-// blocks of 512 (19.5 and 42.5 of 256, 26.9 and 34.8 in 608 of 256), 107 at
-// 161x150x170 in 304 of 512 (110 in 608 of 256).  The tiled sweeps take 512 threads
+// lanes per clock and SM), so small systems run in one 256-thread block per
+// SM, middle ones in one of 512, large ones in two of 512.  Measured, us per
+// iteration of a diagonal CG in reference arithmetic / with multiply-adds, in
+// 152 blocks of 256, 304 of 256, 152 of 512, 304 of 512: 48^3 17.5 / 13.9,
+// 19.7 / 16.9, 19.7 / 16.2, 26.2 / 20.9; 64^3 27.1 / 19.7, 24.0 / 20.1,
+// 23.6 / 19.2, 29.5 / 23.6; 96^3 70.2 / 49.3, 52.0 / 39.8, 51.3 / 38.5,
+// 52.9 / 41.2; 128^3 163 / 119, 112 / 82, 110 / 82, 103 / 78.  The mixed
+// solves' products are FP32 and want the threads: 14.3 at 64^3 in 152 blocks of
+// 512 (16.8 of 256, 15.4 in 304 of 512), 24.7 at 96^3 and 44 at 128^3 in 304
+// of 512 (28.8 and 57 in 152).  The tiled sweeps take 512 threads
 // (four patches a block: one apply at 256^3, FP32, 529 us in two such blocks
 // per SM, 582 in four of 256), the level sweeps one block per SM (898 against
 // 1063 us per iteration at 140,000 rows, 1667 against 1828 at 720,000).

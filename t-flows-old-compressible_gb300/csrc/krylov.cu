@@ -518,12 +518,11 @@ void default_shape(const DeviceTopology& t, SolveRequest& rq) {
         // one row per thread while one block per SM holds them
         if (t.n > kBlock * sms()) rq.block = kMaxBlock;
         rq.grid = std::min(blocks_for(t.nslices, block_of(rq)), (t.n <= 600 * 1000 ? 1 : 2) * sms());
-    } else if (t.n <= 400 * 1000 || (rq.prec == 2 && rq.ic_sweeps == 0)) {
+    } else if (t.n <= 150 * 1000 || (rq.prec == 2 && rq.ic_sweeps == 0)) {
         rq.grid = std::min(blocks_for(t.nslices), sms());
-    } else if (t.n <= (rq.precision == 0 ? 3000 : 1200) * 1000) {
-        rq.grid = std::min(blocks_for(t.nslices), 2 * sms());
     } else {
         rq.block = kMaxBlock;
+        if (t.n <= 1200 * 1000) rq.grid = sms();
     }
 }
 
