@@ -97,10 +97,11 @@ typedef struct tflows_options {
                             representative cell until it is ready, 0 = every
                             lane polls every input, -1 = the default (on,
                             TFLOWS_SWEEP_GATE=0 turns it off)              */
-    int ic_tiled;        /* exact IC(0) on a box-numbered pattern (row =
-                            x + nx (y + ny z), 7-point TopolM rows): 1 =
-                            tiled sweeps (block-local wavefront steps, bulk
-                            copies into shared memory), 0 = level-ordered
+    int ic_tiled;        /* exact IC(0) on a 7-point box (row = x + nx (y +
+                            ny z), or any numbering that puts every cell
+                            after its three neighbours before it): 1 =
+                            tiled sweeps (wavefront steps in a warp per
+                            patch of columns), 0 = level-ordered
                             sweeps, -1 = the default (tiled, TFLOWS_IC_TILED=0
                             turns it off).  In reference arithmetic both give
                             the same apply bit for bit.  Other patterns always

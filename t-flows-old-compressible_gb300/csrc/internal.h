@@ -42,7 +42,8 @@ struct DeviceTopology {
     int* tpos = nullptr;       // transpose map (lazy)
     // box numbering (0 = not a box): row = x + nx (y + ny z), each row holding
     // exactly its 7-point neighbours in ascending order (what TopolM builds
-    // for a structured block); enables the tiled IC sweeps
+    // for a structured block), or another numbering (box_row); enables the
+    // tiled IC sweeps
     int box_nx = 0, box_ny = 0, box_nz = 0;
     int* box_row = nullptr;  // a box in another numbering: the row of each cell
     // host copies (0-based) for lazy derived data

@@ -425,7 +425,7 @@ int run_prec1(const DeviceTopology& t, Workspace& ws, int prec, double* D, doubl
 
 namespace {
 
-// Exact IC(0) on a box-numbered pattern runs the tiled sweeps, unless the
+// Exact IC(0) on a box runs the tiled sweeps, unless the
 // request asks for the level-ordered ones or TFLOWS_IC_TILED=0 does.
 bool tiles_env_on() {
     static const int v = [] {

@@ -934,7 +934,7 @@ __device__ __noinline__ Applied<T> ic_jacobi_apply(Grid& g, const Mat<T>& m, con
     return {true, epi.dot};
 }
 
-// ---- tiled IC(0) sweeps (box-numbered patterns) --------------------------------
+// ---- tiled IC(0) sweeps (boxes) ------------------------------------------------
 // Forward: row (x, y, z) needs (x, y, z-1), (x, y-1, z), (x-1, y, z), in the
 // stored order of its lower entries (columns ascending, CG.f90:135-142).  The
 // first is the lane's own last result, the other two lie in the step before
@@ -1571,7 +1571,7 @@ __device__ __noinline__ Applied<T> ic_mapped_apply(Grid& g, const Mat<T>& m, con
 
 // The IC(0) apply the solve was configured for: `sweeps` Jacobi sweeps per
 // triangle (FP32 inner solves and contracted FP64 solves), else the exact
-// apply -- tiled sweeps on a box-numbered pattern, level-ordered sync-free
+// apply -- tiled sweeps on a box, level-ordered sync-free
 // sweeps otherwise.  OP, alfa, x: what is done with each row (RowOp); the
 // thread's sum of kRowDot in `dot`.
 template <int OP, typename T>
