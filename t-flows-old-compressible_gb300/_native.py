@@ -18,9 +18,9 @@ CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 BUILD = os.path.join(HERE, "_build")
 LIB_PATH = os.path.join(HERE, "libtflows_krylov.so")
-SOURCES = ("krylov.cu", "krylov_fma.cu", "krylov_mixed.cu", "shim.cu", "noalloc.cu", "tune.cu",
+SOURCES = ("krylov.cu", "krylov_fma.cu", "krylov_mixed.cu", "krylov_mixed_batch.cu", "shim.cu", "noalloc.cu", "tune.cu",
            "assembly.cu", "momentum.cu", "halo.cu", "meshio.cpp")
-CONTRACTED = ("krylov_fma.cu", "krylov_mixed.cu")  # units built with fused multiply-adds
+CONTRACTED = ("krylov_fma.cu", "krylov_mixed.cu", "krylov_mixed_batch.cu")  # units built with fused multiply-adds
 HEADERS = ("device_common.cuh", "fp64_div.cuh", "fp64_int.cuh", "krylov_kernels.cuh", "solver_entry.cuh", "internal.h",
            "assembly_internal.h")
 

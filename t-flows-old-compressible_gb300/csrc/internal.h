@@ -220,6 +220,7 @@ enum class KernelId { Cg, Cgs, BicgTrue, Prec1, IcApply, MixedRestart, MixedReli
 const void* ref_kernel(KernelId id);
 const void* fma_kernel(KernelId id);
 const void* mixed_kernel(KernelId id);
+const void* mixed_batch_kernel(KernelId id);
 
 // tune.cu: launch-shape autotuner.
 struct TuneChoice {

@@ -13,9 +13,7 @@ const void* mixed_kernel(KernelId id) {
     switch (id) {
         case KernelId::MixedRestart: return (const void*)fma::mixed_kernel<0>;
         case KernelId::MixedReliable: return (const void*)fma::mixed_kernel<1>;
-        case KernelId::MixedCgs: return (const void*)fma::mixed_kernel<2>;
-        case KernelId::BatchMixed: return (const void*)fma::batch_kernel<1>;
-        default: return nullptr;
+        default: return mixed_batch_kernel(id);
     }
 }
 
