@@ -91,12 +91,20 @@ __device__ __forceinline__ void red_release_add_u64(unsigned long long* p, unsig
 }
 
 // Raise an abort: first status wins; everyone polling `abort` leaves, and so
-// does every barrier, whose counter the bit lifts past any target.
+// does every barrier, whose counter the bit lifts past any target.  The bit
+// comes first: a warp that has left a wait for the flag (read with acquire) is
+// then met by a barrier that fails for its whole block.
 constexpr unsigned long long kBarAbort = 1ull << 62;
 __device__ __forceinline__ void raise_abort(DevCtl* c, int status, int where) {
     if (atomicCAS(&c->status, 0, status) == 0) c->where = where;
-    atomicExch(&c->abort, 1);
     atomicOr(&c->bar, kBarAbort);
+    __threadfence();
+    atomicExch(&c->abort, 1);
+}
+__device__ __forceinline__ bool aborted(const DevCtl* c) {
+    int v;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(&c->abort) : "memory");
+    return v != 0;
 }
 
 // ---- asynchronous copies global -> shared (per thread, in commit groups) ----------

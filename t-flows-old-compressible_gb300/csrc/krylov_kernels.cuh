@@ -738,7 +738,7 @@ __device__ __forceinline__ bool sweep_chunk(const Grid& g, const Mat<T>& m, int 
         if (m.sweep_sleep > 0 && spins > 4u)
             __nanosleep(min((unsigned)m.sweep_sleep, 8u << min(spins - 4u, 10u)));
         if ((spins & 63u) == 0u) {
-            bool quit = ld_relaxed_s32(&g.ctl->abort) != 0;
+            bool quit = aborted(g.ctl);
             if (!quit && clock64() - start > g.timeout_cyc) {
                 raise_abort(g.ctl, ST_TIMEOUT, where);
                 quit = true;
@@ -1178,7 +1178,7 @@ __device__ __forceinline__ bool tile_wait(DevCtl* ctl, long long limit, int wher
         unsigned spins = 0;
         do {
             if ((++spins & 63u) == 0u) {
-                bool quit = ld_relaxed_s32(&ctl->abort) != 0;
+                bool quit = aborted(ctl);
                 if (!quit && clock64() - t0 > limit) {
                     raise_abort(ctl, ST_TIMEOUT, where);
                     quit = true;
