@@ -192,7 +192,6 @@ struct Grid {
     int nt;   // threads in the group
     int bid;  // block index within the group
     unsigned epoch;  // tiled IC sweeps: number of the current apply
-    int chunk0;      // and this block's chunks of all sweeps so far
     int stall;      // test hook: block 0 skips its first barrier arrival
 };
 
@@ -214,7 +213,6 @@ __device__ __forceinline__ void grid_init_group(Grid& g, DevCtl* ctl, double* pa
     g.wg = g.tid >> 5;
     g.nw = g.nt >> 5;
     g.epoch = 0;
-    g.chunk0 = 0;
     g.stall = 0;
 }
 

@@ -1117,12 +1117,10 @@ __device__ __forceinline__ int tiles_of(const Tiles<T>& tl, int bid, int nblocks
 }
 
 // Once per solve, before the first apply (a grid barrier must follow): the
-// pivots into both record kinds, epoch 0 into every edge word, the block's
-// progress counters cleared.
+// pivots into both record kinds, epoch 0 into every edge word.
 template <typename T>
 __device__ __noinline__ void tiles_init(Grid& g, const Mat<T>& m, const T* __restrict__ D) {
     const Tiles<T>& tl = m.tile;
-    extern __shared__ __align__(128) unsigned char tf_smem[];
     const unsigned cb = tl.lu_bf16 ? 2u : (unsigned)sizeof(T);
     const unsigned rec = tile_rec_bytes(cb, sizeof(T));
     const int sp = tl.chunks * kTileK, patches = tl.ntx * tl.nty * tl.sw;
@@ -1149,13 +1147,10 @@ __device__ __noinline__ void tiles_init(Grid& g, const Mat<T>& m, const T* __res
     for (int dir = 0; dir < 2; ++dir)
         for (long long i = g.tid; i < words; i += g.nt)
             reinterpret_cast<unsigned long long*>(tl.edge[dir])[i] = 0ull;
-    if (threadIdx.x < kWarpsPerPatch * kMaxSweepWarps) reinterpret_cast<int*>(tf_smem)[threadIdx.x] = 0;
     g.epoch = 0;
-    g.chunk0 = 0;
-    __syncthreads();
 }
 
-// Progress counters in shared memory: chunks done, over all sweeps.
+// Progress counters in shared memory: chunks done in this apply.
 __device__ __forceinline__ int progress_load(unsigned a) {
     int v;
     asm volatile("ld.acquire.cta.shared.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
@@ -1582,16 +1577,21 @@ __device__ __forceinline__ Applied<T> tile_sweep(DevCtl* ctl, long long limit, i
 // z = IC(0) apply of rhs by the tiled sweeps, epi (RowOp) per row.
 template <bool MAP, typename L, typename T, typename Epi>
 __device__ __forceinline__ Applied<T> ic_tiled_apply(Grid& g, const Mat<T>& m, const T* rhs, T* z, Epi epi) {
-    const int chunks = tiles_of(m.tile, g.bid, g.nblocks) * m.tile.chunks, first = g.chunk0;
+    extern __shared__ __align__(128) unsigned char tf_smem[];
+    const int chunks = tiles_of(m.tile, g.bid, g.nblocks) * m.tile.chunks;
     ++g.epoch;
-    g.chunk0 = first + 2 * chunks;
+    // The counters start at 0 in each apply, so that they stay within one
+    // apply's chunks however long the solve (a grid barrier separates the
+    // applies: no warp reads them any more).
+    if (threadIdx.x < kWarpsPerPatch * kMaxSweepWarps) reinterpret_cast<int*>(tf_smem)[threadIdx.x] = 0;
+    __syncthreads();
     // (all warps of the block go on to the backward sweep: its waits end by
     // the abort flag if the forward sweep of another warp gave up)
     const RowOp<kRowNone, T> none{T(0), nullptr, T(0)};
     const bool ok =
-        tile_sweep<0, MAP, L, T>(g.ctl, g.timeout_cyc, g.bid, g.nblocks, g.epoch, first, m, rhs, z, none).ok;
+        tile_sweep<0, MAP, L, T>(g.ctl, g.timeout_cyc, g.bid, g.nblocks, g.epoch, 0, m, rhs, z, none).ok;
     Applied<T> a =
-        tile_sweep<1, MAP, L, T>(g.ctl, g.timeout_cyc, g.bid, g.nblocks, g.epoch, first + chunks, m, rhs, z, epi);
+        tile_sweep<1, MAP, L, T>(g.ctl, g.timeout_cyc, g.bid, g.nblocks, g.epoch, chunks, m, rhs, z, epi);
     a.ok = a.ok && ok;
     return a;
 }
