@@ -452,9 +452,8 @@ bool fuse_dir_fp64(const DeviceTopology& t, const SolveRequest& rq) {
 // shared memory fits an SM twice (one apply at 128^3, FP32: 190 us with four,
 // 220 with two, 240 with one: every tile edge costs a hand-over through L2).
 int tile_patches(const SolveRequest& rq) {
-    const int block = rq.block > 0 ? rq.block : kMaxBlock;
     int sw = 1;
-    while (2 * sw <= kMaxSweepWarps && 2 * sw * kWarpsPerPatch * 32 <= block) sw *= 2;
+    while (2 * sw <= kMaxSweepWarps && 2 * sw * kWarpsPerPatch * 32 <= block_of(rq)) sw *= 2;
     return sw;
 }
 
@@ -504,7 +503,7 @@ bool tiled_ic(const DeviceTopology& t, const SolveRequest& rq) {
     if (rq.prec != 2 || rq.ic_sweeps > 0 || t.box_nx <= 0 || rq.ic_tiled == 0) return false;
     if (rq.ic_tiled < 0 && !tiles_env_on()) return false;
     // (a patch takes four warps; smaller blocks run the level sweeps)
-    return rq.block == 0 || rq.block >= 32 * kWarpsPerPatch;
+    return block_of(rq) >= 32 * kWarpsPerPatch;
 }
 
 void default_shape(const DeviceTopology& t, SolveRequest& rq) {
