@@ -99,6 +99,7 @@ struct SolveRequest {
     int autotune = 0;       // take block/rows_per_warp/sweep_mult from the tuner
     int ic_tiled = -1;      // exact IC on a box pattern: 1 tiled sweeps, 0 level
                             // sweeps, -1 tiled unless TFLOWS_IC_TILED=0
+    int patches = 0;        // most patches of a tile (0 = the block's warps decide)
 };
 
 struct SolveReport {
@@ -160,6 +161,13 @@ void batch_destroy(BatchLaunch* L);
 // Allocate the launch buffers for `count` systems up front (before a capture).
 cudaError_t batch_reserve(BatchLaunch* L, int count, int block = 0);
 int batch_enqueue(BatchLaunch* L, std::vector<BatchSpec>& specs, cudaStream_t s);
+// One block size for all systems of a batch that names none: 512 threads where
+// one of them runs tiled sweeps and every system still gets a block (two such
+// blocks fit an SM), else 256.  Then fit_batch.
+void default_batch_shape(std::vector<BatchSpec>& specs);
+// The largest tiles with which every system gets a block: in FP64 two patches
+// in a block of 256 threads leave three blocks per SM, one patch leaves four.
+void fit_batch(std::vector<BatchSpec>& specs);
 int batch_collect(BatchLaunch* L, std::vector<BatchSpec>& specs, cudaStream_t s, double seconds);
 cudaError_t run_resid(const DeviceTopology& t, Workspace& ws, const double* x, double* r,
                       cudaStream_t s);

@@ -452,8 +452,9 @@ bool fuse_dir_fp64(const DeviceTopology& t, const SolveRequest& rq) {
 // shared memory fits an SM twice (one apply at 128^3, FP32: 190 us with four,
 // 220 with two, 240 with one: every tile edge costs a hand-over through L2).
 int tile_patches(const SolveRequest& rq) {
+    const int most = rq.patches > 0 ? rq.patches : kMaxSweepWarps;
     int sw = 1;
-    while (2 * sw <= kMaxSweepWarps && 2 * sw * kWarpsPerPatch * 32 <= block_of(rq)) sw *= 2;
+    while (2 * sw <= most && 2 * sw * kWarpsPerPatch * 32 <= block_of(rq)) sw *= 2;
     return sw;
 }
 
@@ -894,6 +895,38 @@ void fail_all(std::vector<BatchSpec>& specs, int status, const std::string& msg)
 }
 
 }  // namespace
+
+namespace {
+
+// Blocks of the batch's shape that are resident together.
+int batch_room(const std::vector<BatchSpec>& specs) {
+    unsigned smem = 0;
+    for (auto& sp : specs) smem = std::max(smem, tile_smem_for(*sp.t, sp.rq));
+    return max_coresident(batch_kernel_for(specs[0].rq.precision), block_of(specs[0].rq), smem);
+}
+
+}  // namespace
+
+void fit_batch(std::vector<BatchSpec>& specs) {
+    for (int patches = kMaxSweepWarps; patches > 0; patches /= 2) {
+        for (auto& sp : specs) sp.rq.patches = patches;
+        if ((int)specs.size() <= batch_room(specs)) return;
+    }
+}
+
+void default_batch_shape(std::vector<BatchSpec>& specs) {
+    int block = 0;
+    for (auto& sp : specs) {
+        SolveRequest rq = sp.rq;
+        default_shape(*sp.t, rq);
+        block = std::max(block, tiled_ic(*sp.t, rq) ? rq.block : sp.rq.block);
+    }
+    const bool named = specs[0].rq.block > 0;
+    for (auto& sp : specs) sp.rq.block = block;
+    if (!named && (int)specs.size() > batch_room(specs))
+        for (auto& sp : specs) sp.rq.block = 0;
+    fit_batch(specs);
+}
 
 cudaError_t batch_reserve(BatchLaunch* L, int count, int block) {
     if (block <= 0) block = kBlock;

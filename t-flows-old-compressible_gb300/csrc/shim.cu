@@ -636,17 +636,6 @@ int autotune_on(tflows_topology* tp, SolveRequest& rq, const double* d_b, const 
     return TFLOWS_OK;
 }
 
-// One block size for all systems of a batched launch that names none.
-void default_batch_block(std::vector<BatchSpec>& specs) {
-    int block = 0;
-    for (auto& sp : specs) {
-        SolveRequest rq = sp.rq;
-        default_shape(*sp.t, rq);
-        block = std::max(block, tiled_ic(*sp.t, rq) ? rq.block : sp.rq.block);
-    }
-    for (auto& sp : specs) sp.rq.block = block;
-}
-
 void record(const SolveReport& rep, tflows_result* res) {
     tflows_result r{};
     r.status = rep.status;
@@ -1161,7 +1150,7 @@ int tflows_solve_batched_device(int count, tflows_topology* const* topos, const 
         if (e != cudaSuccess) return cuda_fail(e, "batch staging");
         specs[k] = BatchSpec{&tp->t, ws, rq, X, R, &reps[k]};
     }
-    default_batch_block(specs);
+    default_batch_shape(specs);
     double sec = 0.0;
     int worst = run_batch(specs, s, &sec);
     std::string msg;
@@ -1240,7 +1229,7 @@ int tflows_plan_create(tflows_plan** out, int count, tflows_topology* const* top
                                    ws->vec64 + 12 * ws->vec_cap, &plan->reps[k]};
         plan->topos.push_back(tp);
     }
-    default_batch_block(plan->specs);
+    default_batch_shape(plan->specs);
     cudaError_t e = cudaStreamCreateWithFlags(&plan->cap, cudaStreamNonBlocking);
     if (e != cudaSuccess) return cuda_fail(e, "plan stream");
     if (o.autotune && o.block_size == 0 && o.grid_blocks == 0) {

@@ -270,6 +270,7 @@ int tune_batch(std::vector<BatchSpec>& specs, const std::function<cudaError_t()>
             specs[k].rq.grid = 0;
             specs[k].weight = weights[k];
         }
+        fit_batch(specs);
         cudaError_t e = restage();
         if (e != cudaSuccess) {
             msg = std::string("batch tuning: ") + cudaGetErrorString(e);
@@ -318,6 +319,7 @@ int tune_batch(std::vector<BatchSpec>& specs, const std::function<cudaError_t()>
         specs[k].rq.grid = 0;
         specs[k].weight = best_w[k];
     }
+    fit_batch(specs);
     out.block = best_block;
     return TFLOWS_OK;
 }
