@@ -79,8 +79,9 @@ typedef struct tflows_options {
     int ic_bf16;         /* mixed + prec 2: IC off-diagonals stored in BF16 */
     double timeout_s;    /* limit for any single device-side wait           */
     int block_size;      /* threads per block (multiple of 32, 64..512),
-                            0 = 256 or the tuned value                      */
-    int grid_blocks;     /* persistent blocks, 0 = from rows_per_warp       */
+                            0 = by the system's size, or the tuned value    */
+    int grid_blocks;     /* persistent blocks, 0 = from rows_per_warp or,
+                            where that is 0 too, by the system's size       */
     int device;          /* CUDA device ordinal, -1 = current                */
     int inject_stall;    /* test hook: 1 = the first block withholds its
                             arrival at the first grid barrier, so every
@@ -90,7 +91,8 @@ typedef struct tflows_options {
                             candidates on the first solve of a new system
                             class (block_size and grid_blocks 0); batched
                             launches also balance their block groups       */
-    int rows_per_warp;   /* rows each warp owns, sets the grid (0 = 32)     */
+    int rows_per_warp;   /* rows each warp owns, sets the grid (0 = by the
+                            system's size; 32 where block_size is set)      */
     int sweep_warps;     /* IC sweeps: warps per chunk of the widest
                             wavefront level (0 = 4)                         */
     int sweep_gate;      /* IC sweeps: 1 = a waiting warp polls one
@@ -131,7 +133,7 @@ typedef struct tflows_tuning {
     int candidates;      /* launch shapes timed (0 when from the table)     */
     int from_table;      /* 1 = the table already held this class           */
     double us_per_iteration;         /* chosen shape                        */
-    double default_us_per_iteration; /* 256 threads, one slice per warp     */
+    double default_us_per_iteration; /* the shape of an untuned solve       */
     int sweep_gate;      /* IC sweeps: gated polling chosen (-1 = default)  */
 } tflows_tuning;
 
@@ -139,7 +141,7 @@ typedef struct tflows_tuning {
 typedef struct tflows_batch_tuning {
     int block_size;
     int runs;               /* full batched solves timed                    */
-    double default_seconds; /* N^(4/3) group split, 256 threads             */
+    double default_seconds; /* N^(4/3) group split, default block size      */
     double tuned_seconds;   /* chosen block size and group split            */
 } tflows_batch_tuning;
 

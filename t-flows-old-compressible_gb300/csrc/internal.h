@@ -232,7 +232,7 @@ const void* mixed_batch_kernel(KernelId id);
 
 // tune.cu: launch-shape autotuner.
 struct TuneChoice {
-    int block = 256;
+    int block = 256;  // 0: the shape of an untuned request (default_shape)
     int rows_per_warp = 0;
     int grid = 0;
     int sweep_mult = 0;

@@ -1369,7 +1369,8 @@ int tflows_autotune(tflows_topology* topo, int method, int prec, const tflows_op
     TuneChoice ch;
     const int st = autotune_on(topo, rq, b, nullptr, s, ch);
     if (st != TFLOWS_OK) return st;
-    out->block_size = ch.block;
+    default_shape(topo->t, rq);
+    out->block_size = rq.block > 0 ? rq.block : 256;
     out->rows_per_warp = ch.rows_per_warp;
     out->grid_blocks = planned_grid(topo->t, rq);
     out->sweep_warps = ch.sweep_mult;

@@ -9,7 +9,7 @@
 //     blocks pays less per grid barrier, a large one wants every SM;
 //   * for IC(0), the warps per chunk of the widest wavefront level that take
 //     part in the sync-free sweeps.
-// tune_solve times candidate shapes on the caller's own system (a capped
+// tune_solve times the shape of an untuned request and other candidates on the caller's own system (a capped
 // number of iterations from x0 = 0) and keeps the fastest per iteration in a
 // process-wide table keyed by device, method, preconditioner, precision
 // options and size class; the table can be kept in a text file.  tune_batch
@@ -78,8 +78,9 @@ const char* table_path() {
     return p && *p ? p : nullptr;
 }
 
-// One line per entry: the key fields, then block rows_per_warp sweep_mult
-// sweep_gate and the measured microseconds per iteration.
+// One line per entry: the key fields, then block (0: the shape of an untuned
+// request) rows_per_warp sweep_mult sweep_gate and the measured microseconds
+// per iteration.
 void load_file(Table& T) {
     T.loaded = true;
     const char* path = table_path();
@@ -122,6 +123,7 @@ int time_shape(const DeviceTopology& t, Workspace& ws, const SolveRequest& base,
     rq.block = block;
     rq.rows_per_warp = rpw;
     rq.grid = 0;
+    default_shape(t, rq);
     rq.sweep_mult = sweep_mult;
     rq.sweep_gate = sweep_gate;
     rq.tol = 1e-30;  // relative: never reached within the cap
@@ -176,37 +178,39 @@ void tune_apply(const TuneChoice& ch, SolveRequest& rq) {
 
 int tune_solve(const DeviceTopology& t, Workspace& ws, const SolveRequest& rq, const double* b,
                cudaStream_t s, TuneChoice& out, std::string& msg) {
-    static const int kBlocks[] = {256, 128, 512};
-    static const int kRows[] = {0, 128, 512, 2048};
+    // The shape of an untuned request (block 0) comes first, so that what is
+    // chosen is never slower than it by these timings.
+    std::vector<std::pair<int, int>> shapes = {{0, 0}};
+    for (int blk : {256, 128, 512})
+        for (int rpw : {0, 128, 512, 2048}) shapes.emplace_back(blk, rpw);
     TuneChoice best;
     best.us_per_iter = 1e300;
     int count = 0;
     std::vector<std::pair<int, int>> seen;  // (block, grid) already timed
-    for (int blk : kBlocks)
-        for (int rpw : kRows) {
-            // shapes that give the same grid (co-residency clamps large
-            // systems) are timed once
-            SolveRequest probe = rq;
-            probe.block = blk;
-            probe.rows_per_warp = rpw;
-            probe.grid = 0;
-            const int want = planned_grid(t, probe);
-            if (std::find(seen.begin(), seen.end(), std::make_pair(blk, want)) != seen.end())
-                continue;
-            seen.emplace_back(blk, want);
-            double us = 0.0;
-            int grid = 0;
-            const int st = time_shape(t, ws, rq, b, blk, rpw, 0, rq.sweep_gate, s, us, grid, msg);
-            if (st != TFLOWS_OK) return st;
-            ++count;
-            if (blk == 256 && rpw == 0) out.default_us_per_iter = us;
-            if (us < best.us_per_iter) {
-                best.block = blk;
-                best.rows_per_warp = rpw;
-                best.grid = grid;
-                best.us_per_iter = us;
-            }
+    for (auto [blk, rpw] : shapes) {
+        // shapes that give the same grid (co-residency clamps large
+        // systems) are timed once
+        SolveRequest probe = rq;
+        probe.block = blk;
+        probe.rows_per_warp = rpw;
+        probe.grid = 0;
+        default_shape(t, probe);
+        const auto shape = std::make_pair(probe.block > 0 ? probe.block : 256, planned_grid(t, probe));
+        if (std::find(seen.begin(), seen.end(), shape) != seen.end()) continue;
+        seen.push_back(shape);
+        double us = 0.0;
+        int grid = 0;
+        const int st = time_shape(t, ws, rq, b, blk, rpw, 0, rq.sweep_gate, s, us, grid, msg);
+        if (st != TFLOWS_OK) return st;
+        ++count;
+        if (blk == 0) out.default_us_per_iter = us;
+        if (us < best.us_per_iter) {
+            best.block = blk;
+            best.rows_per_warp = rpw;
+            best.grid = grid;
+            best.us_per_iter = us;
         }
+    }
     if (rq.prec == 2 && rq.ic_sweeps == 0 && !tiled_ic(t, rq)) {
         for (int sm : {2, 8}) {
             double us = 0.0;
@@ -263,7 +267,8 @@ int tune_batch(std::vector<BatchSpec>& specs, const std::function<cudaError_t()>
     out.default_seconds = 0.0;
     out.tuned_seconds = 1e300;
     out.runs = 0;
-    int best_block = 256;
+    const int default_block = specs[0].rq.block > 0 ? specs[0].rq.block : 256;
+    int best_block = default_block;
     auto run = [&](int block, const std::vector<double>& weights, double& sec) -> int {
         for (int k = 0; k < count; ++k) {
             specs[k].rq.block = block;
@@ -285,12 +290,12 @@ int tune_batch(std::vector<BatchSpec>& specs, const std::function<cudaError_t()>
         }
         return TFLOWS_OK;
     };
-    // 256 threads: the N^(4/3) split, then two rebalancing passes that give
+    // The default block size: the N^(4/3) split, then two rebalancing passes that give
     // each system blocks in proportion to its measured work (its own solve
     // time times the blocks it had).
     for (int pass = 0; pass < 3; ++pass) {
         double sec = 0.0;
-        const int st = run(256, w, sec);
+        const int st = run(default_block, w, sec);
         if (st != TFLOWS_OK) return st;
         if (pass == 0) out.default_seconds = sec;
         if (sec < out.tuned_seconds) {
@@ -305,7 +310,8 @@ int tune_batch(std::vector<BatchSpec>& specs, const std::function<cudaError_t()>
         }
         if (tot <= 0.0) break;
     }
-    for (int block : {512, 128}) {
+    for (int block : {512, 256, 128}) {
+        if (block == default_block) continue;
         double sec = 0.0;
         const int st = run(block, best_w, sec);
         if (st != TFLOWS_OK) return st;
