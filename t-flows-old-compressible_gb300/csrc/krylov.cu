@@ -682,15 +682,19 @@ double solve_bytes(const DeviceTopology& t, const SolveRequest& rq, const DevSta
     const bool cgs = rq.method == 2;
     // One IC(0) apply: the off-diagonal factor entries (value + index) once,
     // the row metadata, D and the right-hand side read and the result written
-    // per triangle.  Jacobi sweeps: each sweep reads one triangle's entries.
+    // per triangle.  Jacobi sweeps: each sweep reads one triangle's entries and
+    // their columns (patterns where there are any).
     const double offd = (double)std::max(0, t.nnz - t.n);
     // The tiled sweeps read no indices: the factor entries once, and per row
-    // D twice, the right-hand side once, w written and read, z written.
+    // D twice, the right-hand side once, w written and read, z written.  A box
+    // in another numbering: also its row once per triangle and, in reference
+    // arithmetic, a byte for the order of its sum.
     const bool tiled = tiled_ic(t, rq);
+    const double rows = t.box_row ? 2.0 * t.n * (rq.precision == 0 ? 5.0 : 4.0) : 0.0;
     auto ic_bytes = [&](double sv, double sx) {
         if (rq.ic_sweeps > 0)
-            return rq.ic_sweeps * (offd * (sv + 4.0) + 2.0 * t.n * (4.0 + 3.0 * sx));
-        if (tiled) return offd * sv + 6.0 * t.n * sx;
+            return rq.ic_sweeps * (offd * sv + (t.spat ? 2.0 * t.n : 4.0 * offd) + 2.0 * t.n * (4.0 + 3.0 * sx));
+        if (tiled) return offd * sv + 6.0 * t.n * sx + rows;
         return offd * (sv + 4.0) + 2.0 * t.n * (4.0 + 3.0 * sx);
     };
     if (rq.precision == 1) {
