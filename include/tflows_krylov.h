@@ -106,8 +106,9 @@ typedef struct tflows_options {
                             patch of columns), 0 = level-ordered
                             sweeps, -1 = the default (tiled, TFLOWS_IC_TILED=0
                             turns it off).  In reference arithmetic both give
-                            the same apply bit for bit.  Other patterns always
-                            use the level sweeps                            */
+                            the same apply bit for bit.  Other patterns, and
+                            blocks of fewer than 128 threads, always use the
+                            level sweeps                                    */
 } tflows_options;
 
 typedef struct tflows_result {
@@ -260,6 +261,11 @@ const int *tflows_topology_transpose_map(tflows_topology *topo);
  * the topology was created).  Either way the products see the same columns
  * in the same order. */
 int tflows_topology_patterns(tflows_topology *topo);
+/* The box on which exact IC(0) solves of this topology run the tiled sweeps:
+ * 1 (row = x + nx (y + ny z)) or 2 (another numbering, see `ic_tiled`) with
+ * nx, ny, nz in dims (may be NULL), or 0.  Another numbering is looked for in
+ * the topology's first exact IC(0) call that takes tiled sweeps. */
+int tflows_topology_box(tflows_topology *topo, int *dims);
 
 /* Solve A x = b with device arrays in the topology's stored order: val
  * (nnz FP64), b (n), x (n, in/out: initial guess and solution), r_out (n,

@@ -307,6 +307,14 @@ class Topology:
         """Distinct column patterns the products read (0: explicit columns)."""
         return int(lib().tflows_topology_patterns(self._h))
 
+    @property
+    def box(self):
+        """(nx, ny, nz) of the box on which exact IC(0) solves run the tiled
+        sweeps, or None.  Numberings other than x + nx (y + ny z) are looked
+        for in the first exact IC(0) call."""
+        d = (ctypes.c_int * 3)()
+        return tuple(d) if lib().tflows_topology_box(self._h, d) else None
+
     def transpose_map(self):
         """Device pointer of the transposed-entry map (int32, nnz)."""
         p = lib().tflows_topology_transpose_map(self._h)

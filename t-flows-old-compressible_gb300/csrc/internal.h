@@ -46,6 +46,7 @@ struct DeviceTopology {
     // tiled IC sweeps
     int box_nx = 0, box_ny = 0, box_nz = 0;
     int* box_row = nullptr;  // a box in another numbering: the row of each cell
+    bool box_sought = false; // such a numbering has been looked for
     // host copies (0-based) for lazy derived data
     std::vector<int> h_rowptr, h_col, h_diag;
 };
@@ -177,6 +178,8 @@ int planned_grid(const DeviceTopology& t, const SolveRequest& rq);
 // a launch needs for them, and their step records (allocated here, so call
 // before a stream capture).
 bool tiled_ic(const DeviceTopology& t, const SolveRequest& rq);
+// The part of that which the request decides, but for its block size.
+bool tiles_wanted(const SolveRequest& rq);
 // The launch shape of a request that names none.  Every block adds to what a
 // reduction costs (arrivals, partial sums, and FP64 additions on a pipe of 2
 // lanes per clock and SM), so small systems run in one 256-thread block per

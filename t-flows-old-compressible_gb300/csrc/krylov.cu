@@ -500,11 +500,14 @@ size_t tile_buffer_bytes(const DeviceTopology& t, const TileGeom& g, unsigned ls
 
 }  // namespace
 
+bool tiles_wanted(const SolveRequest& rq) {
+    if (rq.prec != 2 || rq.ic_sweeps > 0 || rq.ic_tiled == 0) return false;
+    return rq.ic_tiled > 0 || tiles_env_on();
+}
+
 bool tiled_ic(const DeviceTopology& t, const SolveRequest& rq) {
-    if (rq.prec != 2 || rq.ic_sweeps > 0 || t.box_nx <= 0 || rq.ic_tiled == 0) return false;
-    if (rq.ic_tiled < 0 && !tiles_env_on()) return false;
     // (a patch takes four warps; smaller blocks run the level sweeps)
-    return block_of(rq) >= 32 * kWarpsPerPatch;
+    return t.box_nx > 0 && tiles_wanted(rq) && block_of(rq) >= 32 * kWarpsPerPatch;
 }
 
 void default_shape(const DeviceTopology& t, SolveRequest& rq) {

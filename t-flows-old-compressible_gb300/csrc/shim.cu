@@ -325,16 +325,6 @@ bool find_box(const DeviceTopology& t, int dim[3], std::vector<int>& row) {
 // SELL-32 layout: slice s holds rows 32s..32s+31, width = longest row.
 cudaError_t build_device(DeviceTopology& t) {
     detect_box(t);
-    if (t.box_nx == 0 && t.ic_ok) {
-        int dim[3];
-        std::vector<int> row;
-        if (find_box(t, dim, row)) {
-            if (cudaError_t e = upload(&t.box_row, row.data(), row.size()); e != cudaSuccess) return e;
-            t.box_nx = dim[0];
-            t.box_ny = dim[1];
-            t.box_nz = dim[2];
-        }
-    }
     const int n = t.n;
     t.nslices = (n + 31) / 32;
     std::vector<long long> soff((size_t)t.nslices + 1, 0);
@@ -415,6 +405,25 @@ cudaError_t build_levels(DeviceTopology& t) {
     e = make_perm(false, &t.perm_b, &t.nchunk_b, &t.nlev_b, &t.wide_b);
     if (e != cudaSuccess) return e;
     t.levels_built = true;
+    return cudaSuccess;
+}
+
+// What an IC(0) request needs of its topology, built on the first one: the
+// levels and, unless it asks for other sweeps than the tiled ones, the box in
+// another numbering (a few passes over the rows, 0.1 s for 2 million; other
+// solves never read it).
+cudaError_t build_ic(DeviceTopology& t, const SolveRequest& rq) {
+    if (cudaError_t e = build_levels(t); e != cudaSuccess) return e;
+    if (t.box_sought || t.box_nx > 0 || !t.ic_ok || !tiles_wanted(rq)) return cudaSuccess;
+    int dim[3];
+    std::vector<int> row;
+    if (find_box(t, dim, row)) {
+        if (cudaError_t e = upload(&t.box_row, row.data(), row.size()); e != cudaSuccess) return e;
+        t.box_nx = dim[0];
+        t.box_ny = dim[1];
+        t.box_nz = dim[2];
+    }
+    t.box_sought = true;
     return cudaSuccess;
 }
 
@@ -673,7 +682,7 @@ int solve_on(tflows_topology* tp, const SolveRequest& rq0, const double* d_val, 
             return fail(TFLOWS_BAD_INPUT,
                         "IC(0) needs each row's entries before Adia to have smaller column "
                         "indices and those after it larger ones");
-        cudaError_t e = build_levels(tp->t);
+        cudaError_t e = build_ic(tp->t, rq);
         if (e != cudaSuccess) return cuda_fail(e, "level sets");
     }
     cudaError_t e = ensure_workspace(tp->ws, tp->t);
@@ -1063,6 +1072,19 @@ void tflows_topology_destroy(tflows_topology* topo) {
 
 int tflows_topology_patterns(tflows_topology* topo) { return topo ? topo->t.npat : 0; }
 
+int tflows_topology_box(tflows_topology* topo, int* dims) {
+    if (!topo) return 0;
+    std::lock_guard<std::mutex> lk(topo->mu);
+    const DeviceTopology& t = topo->t;
+    if (t.box_nx == 0) return 0;
+    if (dims) {
+        dims[0] = t.box_nx;
+        dims[1] = t.box_ny;
+        dims[2] = t.box_nz;
+    }
+    return t.box_row ? 2 : 1;
+}
+
 const int* tflows_topology_transpose_map(tflows_topology* topo) {
     if (!topo) return nullptr;
     std::lock_guard<std::mutex> lk(topo->mu);
@@ -1134,7 +1156,7 @@ int tflows_solve_batched_device(int count, tflows_topology* const* topos, const 
             return fail(TFLOWS_UNSUPPORTED, "true BiCG is not available in batched solves");
         if (rq.prec == 2) {
             if (!tp->t.ic_ok) return fail(TFLOWS_BAD_INPUT, "IC(0) needs a triangular-ordered pattern");
-            cudaError_t e = build_levels(tp->t);
+            cudaError_t e = build_ic(tp->t, rq);
             if (e != cudaSuccess) return cuda_fail(e, "level sets");
         }
         cudaError_t e = ensure_workspace(*ws, tp->t);
@@ -1218,7 +1240,7 @@ int tflows_plan_create(tflows_plan** out, int count, tflows_topology* const* top
             return fail(TFLOWS_UNSUPPORTED, "true BiCG is not available in batched solves");
         if (rq.prec == 2) {
             if (!tp->t.ic_ok) return fail(TFLOWS_BAD_INPUT, "IC(0) needs a triangular-ordered pattern");
-            if (cudaError_t e = build_levels(tp->t); e != cudaSuccess) return cuda_fail(e, "level sets");
+            if (cudaError_t e = build_ic(tp->t, rq); e != cudaSuccess) return cuda_fail(e, "level sets");
         }
         plan->ws.emplace_back(new Workspace());
         cudaError_t ew = ensure_workspace(*plan->ws.back(), tp->t);
@@ -1357,7 +1379,7 @@ int tflows_autotune(tflows_topology* topo, int method, int prec, const tflows_op
         return fail(TFLOWS_UNSUPPORTED, "the tuner covers CG, BiCG and CGS");
     if (rq.prec == 2) {
         if (!topo->t.ic_ok) return fail(TFLOWS_BAD_INPUT, "IC(0) needs a triangular-ordered pattern");
-        if (cudaError_t e = build_levels(topo->t); e != cudaSuccess) return cuda_fail(e, "level sets");
+        if (cudaError_t e = build_ic(topo->t, rq); e != cudaSuccess) return cuda_fail(e, "level sets");
     }
     cudaStream_t s = (cudaStream_t)stream;
     cudaError_t e = ensure_workspace(topo->ws, topo->t);
@@ -1410,9 +1432,9 @@ int tflows_ic_apply_device(tflows_topology* topo, const tflows_options* opt, con
         return fail(TFLOWS_BAD_INPUT, "IC(0) needs a triangular-ordered pattern");
     SolveRequest rq = make_request(o, TFLOWS_METHOD_CG, 2, 0, 0.0);
     if (std::string msg; !shape_ok(rq, msg)) return fail(TFLOWS_BAD_INPUT, msg);
-    default_shape(topo->t, rq);
     cudaStream_t s = (cudaStream_t)stream;
-    cudaError_t e = build_levels(topo->t);
+    cudaError_t e = build_ic(topo->t, rq);
+    default_shape(topo->t, rq);
     if (e == cudaSuccess) e = ensure_workspace(topo->ws, topo->t);
     if (e == cudaSuccess) e = permute_values(topo->t, topo->ws, val, true, false, s);
     if (e != cudaSuccess) return cuda_fail(e, "ic apply");
