@@ -124,7 +124,7 @@ struct Mat {
     int nslices;
     const long long* __restrict__ soff;  // nslices + 1 slice offsets (elements)
     int width;                           // entries per row of every slice (0: they differ)
-    int narrow;                          // 1: no row has more than 8 entries
+    int narrow;                          // 1: products by product_rows (FP32: no row has more than 8 entries)
     const int* __restrict__ scol;        // SELL column indices, -1 = padding
     // Column patterns (null when the topology has none): row i's entry t is
     // at column i + poff[8 * spat[i] + t], absent where that offset is
@@ -371,9 +371,8 @@ __device__ __forceinline__ double fused_dir(double z, double beta, double p, boo
 
 // Entries of a row loaded ahead of their use.  FP64: a hexahedron's row has
 // seven (the FP64 pipe also does what a predicate turns off, so an eighth
-// that no row has would cost as much as the others).  FP32 rows of more than
-// eight entries have a function of their own: a loop over the rest costs the
-// others registers (85 -> 105 us per iteration, 4.1 M rows).
+// that no row has would cost as much as the others).  Longer rows:
+// product_columns.
 template <typename T>
 constexpr int kRowAhead = sizeof(T) == 8 ? 7 : 8;
 
@@ -467,25 +466,56 @@ __device__ __forceinline__ T product_rows(const Mat<T>& m, int wg, int nw, const
     return sum;
 }
 
-// The same for FP32 rows of more than eight entries.
-template <bool DIR>
-__device__ __noinline__ float product_wide(const Mat<float>& m, int wg, int nw, const float* z, const float* p,
-                                           float* pn, float* q, const float* w, float beta, bool first) {
-    const int lane = threadIdx.x & 31;
-    float sum = 0.f;
-    for (int s = wg; s < m.nslices; s += nw) {
+// The same for longer rows (explicit columns), eight entries loaded ahead of
+// their use.  A function of its own: a loop over the rest of a row costs the
+// hexahedra above registers (FP32: 85 -> 105 us per iteration, 4.1 M rows).  A
+// CG iteration on 128^3 rows of 15 entries against one entry at a time, and
+// against the form above in FP64: FP32 269 -> 92 us, multiply-adds 191 -> 124,
+// reference arithmetic 228 -> 152; 64^3: 40 -> 24, 32.1 -> 29.3, 41.8 -> 35.1.
+template <typename T, bool DIR>
+__device__ __noinline__ T product_columns(const Mat<T>& m, int wg, int nw, const T* __restrict__ z,
+                                          const T* __restrict__ p, T* __restrict__ pn, T* __restrict__ q,
+                                          const T* __restrict__ w, T beta, bool first) {
+    constexpr int kAhead = 8;
+    const int lane = threadIdx.x & 31, n = m.n, nslices = m.nslices, width = m.width;
+    const long long* __restrict__ const soff = m.soff;
+    const int* __restrict__ const cols = m.scol;
+    const T* __restrict__ const vals = m.sval;
+    __builtin_assume(__isGlobal(p) && __isGlobal(q) && __isGlobal(cols) && __isGlobal(vals));
+    if (DIR) __builtin_assume(__isGlobal(z) && __isGlobal(pn));
+    else __builtin_assume(__isGlobal(w));
+    T sum = T(0);
+    for (int s = wg; s < nslices; s += nw) {
         const int i = s * kWarp + lane;
-        const long long b0 = m.soff[s];
-        const int ww = (int)((m.soff[s + 1] - b0) >> 5);
-        float xi = 0.f, acc = 0.f;
-        if (i < m.n) xi = DIR ? fused_dir(z[i], beta, first ? 0.f : p[i], first) : p[i];
-        for (int t = 0; t < ww; ++t) {
-            const int c = m.scol[b0 + 32 * t + lane];
-            if (c < 0) continue;
-            const float x = DIR ? fused_dir(z[c], beta, first ? 0.f : p[c], first) : p[c];
-            acc = acc + diff_term(m.sval[b0 + 32 * t + lane], x, xi, c == i);
+        const long long b0 = width ? (long long)s * (kWarp * width) : soff[s];
+        const int ww = width ? width : (int)((soff[s + 1] - b0) >> 5);
+        const int* const cp = cols + b0 + lane;
+        const T* const vp = vals + b0 + lane;
+        T xi = T(0), acc = T(0);  // xi: the row's own direction (FP32 and DIR)
+        if ((DIR || sizeof(T) == 4) && i < n)
+            xi = DIR ? fused_dir(z[i], beta, first ? T(0) : p[i], first) : p[i];
+#pragma unroll 1
+        for (int t0 = 0; t0 < ww; t0 += kAhead) {
+            int c[kAhead];
+            T v[kAhead], x[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                c[u] = t0 + u < ww ? __ldcs(cp + 32 * (t0 + u)) : -1;
+                v[u] = t0 + u < ww ? __ldcs(vp + 32 * (t0 + u)) : T(0);
+            }
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) {
+                const T pt = c[u] >= 0 && !(DIR && first) ? p[c[u]] : T(0);
+                x[u] = DIR ? (c[u] >= 0 ? fused_dir(z[c[u]], beta, pt, first) : T(0)) : pt;
+            }
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
+                if (c[u] >= 0) {
+                    if constexpr (sizeof(T) == 4) acc = acc + diff_term(v[u], x[u], xi, c[u] == i);
+                    else acc = acc + (DIR ? v[u] * x[u] : prod(v[u], x[u]));
+                }
         }
-        if (i < m.n) {
+        if (i < n) {
             q[i] = acc;
             if (DIR) pn[i] = xi;
             sum += (DIR ? xi : w[i]) * acc;
@@ -497,9 +527,7 @@ __device__ __noinline__ float product_wide(const Mat<float>& m, int wg, int nw, 
 template <typename T, bool DIR>
 __device__ __forceinline__ T product_phase(const Mat<T>& m, int wg, int nw, const T* z, const T* p, T* pn,
                                            T* q, const T* w, T beta, bool first) {
-    if constexpr (sizeof(T) == 4) {
-        if (!m.narrow) return product_wide<DIR>(m, wg, nw, z, p, pn, q, w, beta, first);
-    }
+    if (!m.narrow) return product_columns<T, DIR>(m, wg, nw, z, p, pn, q, w, beta, first);
     if (m.spat) return product_rows<T, DIR, false>(m, wg, nw, z, p, pn, q, w, beta, first);
     return product_rows<T, DIR, true>(m, wg, nw, z, p, pn, q, w, beta, first);
 }
