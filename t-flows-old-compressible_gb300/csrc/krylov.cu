@@ -451,6 +451,14 @@ bool fuse_dir_fp64(const DeviceTopology& t, const SolveRequest& rq) {
     return t.n <= (rq.precision == 0 ? 50 : 120) * 1000;
 }
 
+// The mixed reliable-update CG forms it there too, but for large systems with
+// explicit columns, whose two gathers per entry (z and p) miss the caches.
+// Measured, us per iteration inside / as a pass of its own: natural numbering
+// 14.6 / 15.7 at 197,000 rows, 29.0 / 26.8 at 547,000, 52.0 / 47.7 at 1.6
+// million; random numbering 25.4 / 26.5 at 262,000, 51.9 / 39.6 at 729,000,
+// 127 / 87 at 2.1 million.
+bool fuse_dir_mixed(const DeviceTopology& t) { return t.spat || t.n <= 500 * 1000; }
+
 // Patches per tile: as many as the block has warps for, up to four, whose
 // shared memory fits an SM twice (one apply at 128^3, FP32: 190 us with four,
 // 220 with two, 240 with one: every tile edge costs a hand-over through L2).
@@ -661,6 +669,7 @@ cudaError_t prepare_mixed(const DeviceTopology& t, Workspace& ws, const SolveReq
     P.cfg.tol_is_relative = rq.tol_relative;
     P.cfg.x_is_zero = rq.x_is_zero;
     P.cfg.ic_sweeps = rq.prec == 2 ? std::max(rq.ic_sweeps, 0) : 0;
+    P.cfg.fuse_dir = fuse_dir_mixed(t) ? 1 : 0;
     if (rq.prec == 2 && rq.ic_bf16) {
         if (!ws.sval16) return cudaErrorInvalidValue;  // filled by permute_values
         P.m32.lu16 = ws.sval16;
@@ -707,10 +716,12 @@ double solve_bytes(const DeviceTopology& t, const SolveRequest& rq, const DevSta
         const double spmv32 = (double)t.nnz * 4.0 + idx + sl + 8.0 * t.n;
         const double ic = rq.prec == 2 ? ic_bytes(rq.ic_bf16 ? 2.0 : 4.0, 4.0) : 0.0;
         // CG forms its search direction inside the product (z and p read once,
-        // p and q written once), so the product's own vector read and write
-        // are part of the 4·N·12 (resp. 10) vector bytes
+        // p and q written once) but for some reliable-update solves; the
+        // product's own vector read and write are then part of the 4·N·12
+        // (resp. 10) vector bytes
+        const bool fused = rq.refine_restart || fuse_dir_mixed(t);
         const double inner_it = cgs ? 2 * spmv32 + 4.0 * t.n * 22 + 2 * ic
-                                    : spmv32 - 8.0 * t.n + 4.0 * t.n * (rq.prec == 1 ? 12 : 10) + ic;
+                                    : spmv32 - (fused ? 8.0 * t.n : 0.0) + 4.0 * t.n * (rq.prec == 1 ? 12 : 10) + ic;
         return inner_it * st.inner_iters + (spmv64 + 8.0 * t.n * 4) * (st.refinements + 1);
     }
     const int it = std::max(0, std::min(st.iterations, rq.maxiter));

@@ -2126,6 +2126,7 @@ struct MixedCfg {
     int tol_is_relative;
     int x_is_zero;
     int ic_sweeps;       // prec 2: 0 exact sweeps, k > 0 Jacobi sweeps
+    int fuse_dir;        // reliable updates: form the search direction inside the product
 };
 
 struct MixedOut {
@@ -2284,6 +2285,16 @@ static __device__ void mixed_solve(Grid& g, const Mat<double>& m64, const Mat<fl
 // latter, above which a reliable update also restarts the search direction.
 constexpr double kReliableDrift = 0.3;
 
+// The search direction in a pass of its own, then the product with explicit
+// columns (a function of its own: registers).
+static __device__ __noinline__ bool product_apart(Grid& g, const Mat<float>& m, const float* z, float* p,
+                                                  float* q, float beta, bool first, float& sum) {
+    direction_phase(g.tid, g.nt, m.n, z, p, beta, first);
+    if (!grid_sync(g, 84)) return false;
+    sum = product_columns<float, false>(m, g.wg, g.nw, nullptr, p, nullptr, q, p, 0.0f, false);
+    return true;
+}
+
 // One FP32 preconditioned CG iteration stream (FP32 values and vectors, FP64
 // reductions).  Whenever its recursive residual has dropped by `inner_rtol`
 // since the last refinement (or below the tolerance), the FP32 correction is
@@ -2408,13 +2419,18 @@ static __device__ void mixed_cg_reliable(Grid& g, const Mat<double>& m64, const 
     bool diverged = false, fresh = false;
     float *pcur = v.p, *pnext = v.t;
     for (; it <= c.maxiter; ++it) {
-        // the direction formed inside the product, into the other buffer
-        const float a1[1] = {product_phase<float, true>(m32, g.wg, g.nw, z, pcur, pnext, v.q, nullptr, beta,
-                                                        it == 1 || fresh)};
+        const bool along = it == 1 || fresh;  // p = z
+        float a1[1];
+        if (c.fuse_dir) {
+            // the direction formed inside the product, into the other buffer
+            a1[0] = product_phase<float, true>(m32, g.wg, g.nw, z, pcur, pnext, v.q, nullptr, beta, along);
+            float* const pold = pcur;
+            pcur = pnext;
+            pnext = pold;
+        } else if (!product_apart(g, m32, z, pcur, v.q, beta, along, a1[0])) {
+            return;
+        }
         fresh = false;
-        float* const pold = pcur;
-        pcur = pnext;
-        pnext = pold;
         publish_t<1>(g, SLOT_C, a1);
         if (!grid_sync(g, 85)) return;
         double t1[1], e1[1];
