@@ -18,9 +18,13 @@ CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 BUILD = os.path.join(HERE, "_build")
 LIB_PATH = os.path.join(HERE, "libtflows_krylov.so")
-SOURCES = ("krylov.cu", "krylov_fma.cu", "krylov_mixed.cu", "krylov_mixed_batch.cu", "shim.cu", "noalloc.cu", "tune.cu",
-           "assembly.cu", "momentum.cu", "halo.cu", "meshio.cpp")
-CONTRACTED = ("krylov_fma.cu", "krylov_mixed.cu", "krylov_mixed_batch.cu")  # units built with fused multiply-adds
+SOURCES = ("krylov.cu", "krylov_fma.cu", "krylov_mixed.cu", "krylov_diag.cu", "krylov_diag_fma.cu", "krylov_level.cu",
+           "krylov_level_fma.cu", "krylov_mapped.cu", "krylov_mapped_fma.cu", "krylov_long.cu", "krylov_long_fma.cu",
+           "krylov_box_batch.cu", "krylov_box_batch_fma.cu", "krylov_batch.cu", "krylov_batch_fma.cu",
+           "krylov_batch_mixed.cu", "shim.cu", "noalloc.cu", "tune.cu", "assembly.cu", "momentum.cu", "halo.cu",
+           "meshio.cpp")
+# units built with fused multiply-adds
+CONTRACTED = tuple(s for s in SOURCES if s.endswith(("_fma.cu", "_mixed.cu")))
 HEADERS = ("device_common.cuh", "fp64_div.cuh", "fp64_int.cuh", "krylov_kernels.cuh", "solver_entry.cuh", "internal.h",
            "assembly_internal.h")
 

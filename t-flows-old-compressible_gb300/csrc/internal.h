@@ -178,7 +178,9 @@ int planned_grid(const DeviceTopology& t, const SolveRequest& rq);
 // a launch needs for them, and their step records (allocated here, so call
 // before a stream capture).
 bool tiled_ic(const DeviceTopology& t, const SolveRequest& rq);
-// The part of that which the request decides, but for its block size.
+// Exact IC(0) by level-ordered sweeps.
+bool level_ic(const DeviceTopology& t, const SolveRequest& rq);
+// The part of tiled_ic that the request decides, but for its block size.
 bool tiles_wanted(const SolveRequest& rq);
 // The launch shape of a request that names none.  Every block adds to what a
 // reduction costs (arrivals, partial sums, and FP64 additions on a pipe of 2
@@ -225,12 +227,26 @@ int halo_resid(int n, int nb, int nonz, const double* A, const int* Acol, const 
 
 // The persistent kernels: krylov.cu has the reference's arithmetic (separate
 // rounded products and sums, dividing diagonal), krylov_fma.cu and
-// krylov_mixed.cu fused multiply-adds (TFLOWS_FP64_FMA; the mixed solves).
-enum class KernelId { Cg, Cgs, BicgTrue, Prec1, IcApply, MixedRestart, MixedReliable, MixedCgs,
-                      BatchFp64, BatchMixed };
+// krylov_mixed.cu fused multiply-adds (TFLOWS_FP64_FMA; the mixed solves); the
+// _diag, _level, _mapped, _long and _batch units have the same solvers for what their
+// names say (krylov_kernels.cuh).  Null where a unit has no such kernel.
+enum class KernelId { Cg, CgFused, CgNone, CgNoneFused, Cgs, BicgTrue, Prec1, IcApply, MixedRestart, MixedReliable, MixedCgs,
+                      BatchFp64, BatchMixed, BatchReliable };
 const void* ref_kernel(KernelId id);
 const void* fma_kernel(KernelId id);
 const void* mixed_kernel(KernelId id);
+const void* ref_diag_kernel(KernelId id);
+const void* fma_diag_kernel(KernelId id);
+const void* ref_level_kernel(KernelId id);
+const void* fma_level_kernel(KernelId id);
+const void* ref_mapped_kernel(KernelId id);
+const void* fma_mapped_kernel(KernelId id);
+const void* ref_long_kernel(KernelId id);
+const void* fma_long_kernel(KernelId id);
+const void* ref_box_batch_kernel(KernelId id);
+const void* fma_box_batch_kernel(KernelId id);
+const void* ref_batch_kernel(KernelId id);
+const void* fma_batch_kernel(KernelId id);
 const void* mixed_batch_kernel(KernelId id);
 
 // tune.cu: launch-shape autotuner.

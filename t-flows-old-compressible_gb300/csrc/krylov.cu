@@ -208,6 +208,12 @@ int sweep_gate_on() {
     return v;
 }
 
+// FP64 rows for which the products load eight entries ahead in as many trips
+// as it takes, and not seven and then the rest one by one: the latter costs
+// less up to four more (a mean of 9.5 entries per slice, 524,288 rows,
+// multiply-adds: 35.6 against 40.4 us per iteration).
+bool long_fp64(const DeviceTopology& t) { return t.sell_len > 11LL * kWarp * t.nslices; }
+
 template <typename T>
 Mat<T> make_mat(const DeviceTopology& t, const T* sval) {
     Mat<T> m;
@@ -215,10 +221,7 @@ Mat<T> make_mat(const DeviceTopology& t, const T* sval) {
     m.nslices = t.nslices;
     m.soff = t.soff;
     m.width = t.width;
-    // FP64: up to four entries beyond the seven loaded ahead cost less one by
-    // one than in a second trip of eight (a mean of 9.5 entries per slice,
-    // 524,288 rows, multiply-adds: 35.6 against 40.4 us per iteration)
-    m.narrow = sizeof(T) == 8 ? t.sell_len <= 11LL * kWarp * t.nslices : t.max_len <= 8;
+    m.narrow = sizeof(T) == 8 ? !long_fp64(t) : t.max_len <= 8;
     m.scol = t.scol;
     m.spat = t.spat;
     m.poff = t.poff;
@@ -521,6 +524,10 @@ bool tiled_ic(const DeviceTopology& t, const SolveRequest& rq) {
     return t.box_nx > 0 && tiles_wanted(rq) && block_of(rq) >= 32 * kWarpsPerPatch;
 }
 
+bool level_ic(const DeviceTopology& t, const SolveRequest& rq) {
+    return rq.prec == 2 && rq.ic_sweeps == 0 && !tiled_ic(t, rq);
+}
+
 void default_shape(const DeviceTopology& t, SolveRequest& rq) {
     if (rq.block > 0) return;
     const bool tiled = tiled_ic(t, rq);
@@ -669,7 +676,7 @@ cudaError_t prepare_mixed(const DeviceTopology& t, Workspace& ws, const SolveReq
     P.cfg.tol_is_relative = rq.tol_relative;
     P.cfg.x_is_zero = rq.x_is_zero;
     P.cfg.ic_sweeps = rq.prec == 2 ? std::max(rq.ic_sweeps, 0) : 0;
-    P.cfg.fuse_dir = fuse_dir_mixed(t) ? 1 : 0;
+    P.cfg.fuse_dir = fuse_dir_mixed(t) || tiled_ic(t, rq) ? 1 : 0;
     if (rq.prec == 2 && rq.ic_bf16) {
         if (!ws.sval16) return cudaErrorInvalidValue;  // filled by permute_values
         P.m32.lu16 = ws.sval16;
@@ -719,7 +726,7 @@ double solve_bytes(const DeviceTopology& t, const SolveRequest& rq, const DevSta
         // p and q written once) but for some reliable-update solves; the
         // product's own vector read and write are then part of the 4·N·12
         // (resp. 10) vector bytes
-        const bool fused = rq.refine_restart || fuse_dir_mixed(t);
+        const bool fused = rq.refine_restart || fuse_dir_mixed(t) || tiled;
         const double inner_it = cgs ? 2 * spmv32 + 4.0 * t.n * 22 + 2 * ic
                                     : spmv32 - (fused ? 8.0 * t.n : 0.0) + 4.0 * t.n * (rq.prec == 1 ? 12 : 10) + ic;
         return inner_it * st.inner_iters + (spmv64 + 8.0 * t.n * 4) * (st.refinements + 1);
@@ -783,8 +790,8 @@ int launch_and_report(K kern, P& params, const DeviceTopology& t, Workspace& ws,
 const void* ref_kernel(KernelId id) {
     switch (id) {
         case KernelId::Cg: return (const void*)ref::krylov_kernel<double, 0>;
+        case KernelId::CgFused: return (const void*)ref::krylov_kernel<double, 1>;
         case KernelId::Cgs: return (const void*)ref::krylov_kernel<double, 2>;
-        case KernelId::BicgTrue: return (const void*)ref::krylov_kernel<double, 3>;
         case KernelId::Prec1: return (const void*)ref::krylov_kernel<double, 9>;
         case KernelId::IcApply: return (const void*)ref::krylov_kernel<double, 8>;
         case KernelId::BatchFp64: return (const void*)ref::batch_kernel<0>;
@@ -794,27 +801,80 @@ const void* ref_kernel(KernelId id) {
 
 namespace {
 
-// The kernel a request runs: reference arithmetic for TFLOWS_FP64, the
-// contracted build for TFLOWS_FP64_FMA and for the mixed solves.
-const void* solver_kernel(const SolveRequest& rq) {
-    if (rq.precision == 1)
-        return mixed_kernel(rq.method == 2 ? KernelId::MixedCgs
-                                           : (rq.refine_restart ? KernelId::MixedRestart
-                                                                : KernelId::MixedReliable));
-    const KernelId id = rq.method == 2 ? KernelId::Cgs
-                        : rq.method == 3 ? KernelId::BicgTrue : KernelId::Cg;
-    return rq.precision == 2 ? fma_kernel(id) : ref_kernel(id);
+// Rows for the kernels of long ones: FP32 rows of more than eight entries and
+// the reliable-update solves whose direction is not formed in the product;
+// long_fp64.
+bool long_rows(const DeviceTopology& t, const SolveRequest& rq) {
+    if (rq.precision != 1) return long_fp64(t);
+    return t.max_len > 8 || (rq.method != 2 && !rq.refine_restart && !fuse_dir_mixed(t));
 }
 
-const void* batch_kernel_for(int precision) {
-    return precision == 1 ? mixed_kernel(KernelId::BatchMixed)
-           : precision == 2 ? fma_kernel(KernelId::BatchFp64) : ref_kernel(KernelId::BatchFp64);
+// The unit (krylov_kernels.cuh) whose kernels a request runs.
+enum class Unit { Boxes, Mapped, Level, Long, Diag, None };
+Unit unit_of(const DeviceTopology& t, const SolveRequest& rq) {
+    if (tiled_ic(t, rq)) return t.box_row ? Unit::Mapped : Unit::Boxes;
+    if (level_ic(t, rq)) return Unit::Level;
+    if (rq.method != 3 && long_rows(t, rq)) return Unit::Long;
+    return rq.prec == 2 ? Unit::Boxes : Unit::Diag;
+}
+
+// Its kernel: reference arithmetic for TFLOWS_FP64, the contracted build for
+// TFLOWS_FP64_FMA and for the mixed solves.
+const void* unit_kernel(Unit u, int precision, KernelId id) {
+    const bool ref = precision == 0;
+    switch (u) {
+        case Unit::Mapped: return ref ? ref_mapped_kernel(id) : fma_mapped_kernel(id);
+        case Unit::Level: return ref ? ref_level_kernel(id) : fma_level_kernel(id);
+        case Unit::Long: return ref ? ref_long_kernel(id) : fma_long_kernel(id);
+        case Unit::Diag: return ref ? ref_diag_kernel(id) : fma_diag_kernel(id);
+        case Unit::Boxes: return precision == 1 ? mixed_kernel(id) : ref ? ref_kernel(id) : fma_kernel(id);
+        default: return nullptr;
+    }
+}
+
+const void* kernel_of(const DeviceTopology& t, const SolveRequest& rq, KernelId id) {
+    const Unit u = unit_of(t, rq);
+    if (u == Unit::Diag && rq.prec != 1)
+        id = id == KernelId::Cg ? KernelId::CgNone : id == KernelId::CgFused ? KernelId::CgNoneFused : id;
+    return unit_kernel(u, rq.precision, id);
+}
+
+const void* solver_kernel(const DeviceTopology& t, const SolveRequest& rq) {
+    if (rq.precision == 1)
+        return kernel_of(t, rq, rq.method == 2 ? KernelId::MixedCgs
+                                : rq.refine_restart ? KernelId::MixedRestart : KernelId::MixedReliable);
+    return kernel_of(t, rq, rq.method == 2         ? KernelId::Cgs
+                            : rq.method == 3       ? KernelId::BicgTrue
+                            : fuse_dir_fp64(t, rq) ? KernelId::CgFused : KernelId::Cg);
+}
+
+// The kernels a batch may run, in the order of preference: of the unit that all
+// its systems share (where that has one), of boxes, of everything.
+const void* batch_kernel(int precision, bool reliable, Unit shared, bool boxes) {
+    const KernelId id = precision != 1 ? KernelId::BatchFp64 : reliable ? KernelId::BatchReliable : KernelId::BatchMixed;
+    const void* k = unit_kernel(shared, precision, id);
+    if (!k && boxes) k = precision == 0 ? ref_box_batch_kernel(id) : fma_box_batch_kernel(id);
+    if (k) return k;
+    return precision == 1   ? mixed_batch_kernel(KernelId::BatchMixed)
+           : precision == 2 ? fma_batch_kernel(id) : ref_batch_kernel(id);
+}
+
+const void* batch_kernel_for(const std::vector<BatchSpec>& specs) {
+    const Unit u = unit_of(*specs[0].t, specs[0].rq);
+    bool same = true, boxes = true, reliable = true;
+    for (auto& sp : specs) {
+        const Unit k = unit_of(*sp.t, sp.rq);
+        same = same && k == u;
+        boxes = boxes && (k == Unit::Boxes || k == Unit::Diag);
+        reliable = reliable && sp.rq.method != 2 && !sp.rq.refine_restart;
+    }
+    return batch_kernel(specs[0].rq.precision, reliable, same ? u : Unit::None, boxes);
 }
 
 }  // namespace
 
 int planned_grid(const DeviceTopology& t, const SolveRequest& rq) {
-    return choose_grid(t, rq, max_coresident(solver_kernel(rq), block_of(rq), tile_smem_for(t, rq)));
+    return choose_grid(t, rq, max_coresident(solver_kernel(t, rq), block_of(rq), tile_smem_for(t, rq)));
 }
 
 int run_ic_apply(const DeviceTopology& t, Workspace& ws, const SolveRequest& rq0, const double* r,
@@ -827,8 +887,7 @@ int run_ic_apply(const DeviceTopology& t, Workspace& ws, const SolveRequest& rq0
     KParams<double> P;
     cudaError_t e = cudaMemcpyAsync(R, r, sizeof(double) * t.n, cudaMemcpyDeviceToDevice, s);
     if (e == cudaSuccess) e = prepare_fp64(t, ws, rq, ws.vec64 + 11 * ws.vec_cap, R, s, P);
-    const void* kern = rq.precision == 2 ? fma_kernel(KernelId::IcApply) : ref_kernel(KernelId::IcApply);
-    const int st = launch_and_report(kern, P, t, ws, rq, s, rep, e);
+    const int st = launch_and_report(kernel_of(t, rq, KernelId::IcApply), P, t, ws, rq, s, rep, e);
     if (st == ST_CUDA_ERROR) return st;
     e = cudaMemcpyAsync(z, P.v.z, sizeof(double) * t.n, cudaMemcpyDeviceToDevice, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -845,11 +904,11 @@ int run_solve(const DeviceTopology& t, Workspace& ws, const SolveRequest& rq, do
     if (rq.precision == 1) {
         MixedParams P;
         cudaError_t e = prepare_mixed(t, ws, rq, x, r, s, P);
-        return launch_and_report(solver_kernel(rq), P, t, ws, rq, s, rep, e);
+        return launch_and_report(solver_kernel(t, rq), P, t, ws, rq, s, rep, e);
     }
     KParams<double> P;
     cudaError_t e = prepare_fp64(t, ws, rq, x, r, s, P);
-    return launch_and_report(solver_kernel(rq), P, t, ws, rq, s, rep, e);
+    return launch_and_report(solver_kernel(t, rq), P, t, ws, rq, s, rep, e);
 }
 
 // Persistent launch state of a batched solve: pinned host and device copies
@@ -923,7 +982,7 @@ namespace {
 int batch_room(const std::vector<BatchSpec>& specs) {
     unsigned smem = 0;
     for (auto& sp : specs) smem = std::max(smem, tile_smem_for(*sp.t, sp.rq));
-    return max_coresident(batch_kernel_for(specs[0].rq.precision), block_of(specs[0].rq), smem);
+    return max_coresident(batch_kernel_for(specs), block_of(specs[0].rq), smem);
 }
 
 }  // namespace
@@ -951,8 +1010,11 @@ void default_batch_shape(std::vector<BatchSpec>& specs) {
 
 cudaError_t batch_reserve(BatchLaunch* L, int count, int block) {
     if (block <= 0) block = kBlock;
-    int maxb = 1;
-    for (int p : {0, 1, 2}) maxb = std::max(maxb, max_coresident(batch_kernel_for(p), block));
+    // (a bound for every kernel: asking each for its occupancy would load it)
+    int dev = 0, threads = 2048;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&threads, cudaDevAttrMaxThreadsPerMultiProcessor, dev);
+    const int maxb = sms() * std::max(1, threads / block);
     return grow(*L, count, maxb);
 }
 
@@ -966,7 +1028,7 @@ int batch_enqueue(BatchLaunch* L, std::vector<BatchSpec>& specs, cudaStream_t s)
             fail_all(specs, ST_BAD_INPUT, "one precision per batched launch");
             return ST_BAD_INPUT;
         }
-    const void* kern = batch_kernel_for(precision);
+    const void* kern = batch_kernel_for(specs);
     const int block = block_of(specs[0].rq);
     unsigned smem = 0;
     for (auto& sp : specs) {

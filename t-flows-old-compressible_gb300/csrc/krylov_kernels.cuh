@@ -245,6 +245,52 @@ __device__ __forceinline__ double jacobi(double r, double d) { return div_rn(r, 
 #endif
 __device__ __forceinline__ float jacobi(float r, float dinv) { return r * dinv; }
 
+// What the unit's solvers are built for.  Code that a solve never runs costs
+// the rest of its kernel registers (64 a thread, spilled beyond): with the
+// products of long rows beside those of boxes a diagonal CG lost 2 to 5 %.
+// Apart, against one kernel for everything, us per iteration: 64^3 diagonal in
+// reference arithmetic 24.3 -> 23.0, multiply-adds 19.5 -> 18.5; 128^3 mixed
+// diagonal 52.8 -> 50.8, with IC(0) 331 -> 323; 100 x 87 x 75 cells numbered in
+// blocks, IC(0), reference arithmetic 576 -> 512, mixed 209 -> 198.
+// * TFLOWS_FOR_DIAG: the diagonal or no preconditioner, short rows;
+// * TFLOWS_FOR_LONG: those and Jacobi-sweep IC(0), long rows (product_columns);
+// * TFLOWS_FOR_LEVEL: exact IC(0) by level-ordered sweeps, any rows;
+// * TFLOWS_FOR_MAPPED: tiled IC(0) on boxes in other numberings;
+// * TFLOWS_FOR_BOX_BATCH: the diagonal, tiled IC(0) on boxes in their own
+//   numbering and Jacobi-sweep IC(0), short rows (batches of such systems);
+// * TFLOWS_FOR_ANY: everything (batches of any others);
+// * none of these: tiled IC(0) on boxes in their own numbering and Jacobi-sweep
+//   IC(0), short rows.
+#if defined(TFLOWS_FOR_DIAG)
+constexpr bool kDiagPrec = true, kJacobiIc = false, kTiledIc = false, kLevelIc = false;
+constexpr bool kShortRows = true, kLongRows = false;
+#elif defined(TFLOWS_FOR_LONG)
+constexpr bool kDiagPrec = true, kJacobiIc = true, kTiledIc = false, kLevelIc = false;
+constexpr bool kShortRows = false, kLongRows = true;
+#elif defined(TFLOWS_FOR_LEVEL)
+constexpr bool kDiagPrec = false, kJacobiIc = false, kTiledIc = false, kLevelIc = true;
+constexpr bool kShortRows = true, kLongRows = true;
+#elif defined(TFLOWS_FOR_MAPPED)
+constexpr bool kDiagPrec = false, kJacobiIc = false, kTiledIc = true, kLevelIc = false;
+constexpr bool kShortRows = true, kLongRows = false;
+#elif defined(TFLOWS_FOR_BOX_BATCH)
+constexpr bool kDiagPrec = true, kJacobiIc = true, kTiledIc = true, kLevelIc = false;
+constexpr bool kShortRows = true, kLongRows = false;
+#elif defined(TFLOWS_FOR_ANY)
+constexpr bool kDiagPrec = true, kJacobiIc = true, kTiledIc = true, kLevelIc = true;
+constexpr bool kShortRows = true, kLongRows = true;
+#else
+constexpr bool kDiagPrec = false, kJacobiIc = true, kTiledIc = true, kLevelIc = false;
+constexpr bool kShortRows = true, kLongRows = false;
+#endif
+// (batches keep the direction inside the product on any rows)
+constexpr bool kApart = kLongRows && !(kDiagPrec && kLevelIc);
+__device__ __forceinline__ int prec_of(int prec) {
+    if (!kDiagPrec) return 2;
+    if (!kJacobiIc && !kTiledIc && !kLevelIc) return prec == 1 ? 1 : 0;
+    return prec == 1 || prec == 2 ? prec : 0;
+}
+
 __device__ __forceinline__ double divide(double a, double b) { return div_rn(a, b); }
 __device__ __forceinline__ float divide(float a, float b) { return a / b; }
 
@@ -467,13 +513,11 @@ __device__ __forceinline__ T product_rows(const Mat<T>& m, int wg, int nw, const
 }
 
 // The same for longer rows (explicit columns), eight entries loaded ahead of
-// their use.  A function of its own: a loop over the rest of a row costs the
-// hexahedra above registers (FP32: 85 -> 105 us per iteration, 4.1 M rows).  A
-// CG iteration on 128^3 rows of 15 entries against one entry at a time, and
+// their use; not beside the loop above where registers count.  A CG iteration on 128^3 rows of 15 entries against one entry at a time, and
 // against the form above in FP64: FP32 269 -> 92 us, multiply-adds 191 -> 124,
 // reference arithmetic 228 -> 152; 64^3: 40 -> 24, 32.1 -> 29.3, 41.8 -> 35.1.
 template <typename T, bool DIR>
-__device__ __noinline__ T product_columns(const Mat<T>& m, int wg, int nw, const T* __restrict__ z,
+__device__ __forceinline__ T columns_loop(const Mat<T>& m, int wg, int nw, const T* __restrict__ z,
                                           const T* __restrict__ p, T* __restrict__ pn, T* __restrict__ q,
                                           const T* __restrict__ w, T beta, bool first) {
     constexpr int kAhead = 8;
@@ -525,11 +569,23 @@ __device__ __noinline__ T product_columns(const Mat<T>& m, int wg, int nw, const
 }
 
 template <typename T, bool DIR>
+__device__ __noinline__ T product_columns(const Mat<T>& m, int wg, int nw, const T* z, const T* p, T* pn, T* q,
+                                          const T* w, T beta, bool first) {
+    return columns_loop<T, DIR>(m, wg, nw, z, p, pn, q, w, beta, first);
+}
+
+template <typename T, bool DIR>
 __device__ __forceinline__ T product_phase(const Mat<T>& m, int wg, int nw, const T* z, const T* p, T* pn,
                                            T* q, const T* w, T beta, bool first) {
-    if (!m.narrow) return product_columns<T, DIR>(m, wg, nw, z, p, pn, q, w, beta, first);
-    if (m.spat) return product_rows<T, DIR, false>(m, wg, nw, z, p, pn, q, w, beta, first);
-    return product_rows<T, DIR, true>(m, wg, nw, z, p, pn, q, w, beta, first);
+    if constexpr (!kShortRows) {
+        return columns_loop<T, DIR>(m, wg, nw, z, p, pn, q, w, beta, first);
+    } else {
+        if constexpr (kLongRows) {
+            if (!m.narrow) return product_columns<T, DIR>(m, wg, nw, z, p, pn, q, w, beta, first);
+        }
+        if (m.spat) return product_rows<T, DIR, false>(m, wg, nw, z, p, pn, q, w, beta, first);
+        return product_rows<T, DIR, true>(m, wg, nw, z, p, pn, q, w, beta, first);
+    }
 }
 
 // p = z + beta p, or z when `first` (CG.f90:178-187).
@@ -836,8 +892,8 @@ struct Applied {
 // `w` cells must hold the sentinel on entry and hold it again on exit.
 // The backward phase runs `epi` (RowOp) per row.
 template <typename T, typename Epi>
-__device__ __noinline__ Applied<T> ic_apply(Grid& g, const Mat<T>& m, const T* D, const T* rhs, T* w, T* z,
-                                            Epi epi) {
+__device__ __forceinline__ Applied<T> level_apply(Grid& g, const Mat<T>& m, const T* D, const T* rhs, T* w, T* z,
+                                                  Epi epi) {
     bool ok = true;
     const int nwf = sweep_warps(g, m.wide_f, m.sweep_mult);
     for (int ch = g.wg; g.wg < nwf && ch < m.nchunk_f && ok; ch += nwf) {
@@ -880,6 +936,12 @@ __device__ __noinline__ Applied<T> ic_apply(Grid& g, const Mat<T>& m, const T* D
     return {ok, epi.dot};
 }
 
+template <typename T, typename Epi>
+__device__ __noinline__ Applied<T> ic_apply(Grid& g, const Mat<T>& m, const T* D, const T* rhs, T* w, T* z,
+                                            Epi epi) {
+    return level_apply(g, m, D, rhs, w, z, epi);
+}
+
 // ---- IC(0) apply by Jacobi sweeps (FP32 inner solves, ic_sweeps = k > 0) ----
 // Each triangular solve of the exact apply is replaced by k Jacobi sweeps
 //     y^s_i = D_i (f_i - sum_{t in the triangle of row i} a_it y^(s-1)_t),
@@ -896,13 +958,15 @@ __device__ __noinline__ Applied<T> ic_apply(Grid& g, const Mat<T>& m, const T* D
 // again after every store), in global space, with the next row's pattern and
 // length a trip ahead; a row of a box has three entries in a triangle, so four
 // are loaded together and a loop takes the rest (the FP64 pipe also does what
-// a predicate turns off).  Inlined: as a function of its own it cost FP32 2 to
+// a predicate turns off); LONG: four at a time, which costs a box 6 % (128^3
+// rows of 15 entries, one sweep per triangle, mixed: 481 -> 262 us with the
+// products of such rows).  Inlined: as a function of its own it cost FP32 2 to
 // 3 %.  A CG iteration with one / two sweeps per triangle, 161 x 150 x 170
 // cells, against eight entries and explicit columns in 608 blocks of 256:
 // FP32 269 -> 260 / 395 -> 389 us, multiply-adds 473 -> 361 / 670 -> 505.
 constexpr int kTriAhead = 4;
 
-template <bool FWD, typename T, typename Fin>
+template <bool FWD, bool LONG, typename T, typename Fin>
 __device__ __forceinline__ void tri_jacobi(const Grid& g, const Mat<T>& m, const T* __restrict__ D,
                                            const T* __restrict__ f, const T* __restrict__ y,
                                            T* __restrict__ out, Fin fin) {
@@ -941,23 +1005,28 @@ __device__ __forceinline__ void tri_jacobi(const Grid& g, const Mat<T>& m, const
         auto column = [&](int u) { return po ? i + po[t0 + u] : cols[base + 32LL * u]; };
         T acc = f[i];
         const T di = D[i];
-        int c[kTriAhead];
-        T a[kTriAhead], yv[kTriAhead];
-#pragma unroll
-        for (int u = 0; u < kTriAhead; ++u) {
-            c[u] = u < nt ? column(u) : 0;
-            a[u] = u < nt ? value(base + 32LL * u) : T(0);
-        }
-#pragma unroll
-        for (int u = 0; u < kTriAhead; ++u)
-            yv[u] = u < nt ? (y ? y[c[u]] : D[c[u]] * f[c[u]]) : T(0);
-#pragma unroll
-        for (int u = 0; u < kTriAhead; ++u)
-            if (u < nt) acc = acc - a[u] * yv[u];
 #pragma unroll 1
-        for (int u = kTriAhead; u < nt; ++u) {
-            const int j = column(u);
-            acc = acc - value(base + 32LL * u) * (y ? y[j] : D[j] * f[j]);
+        for (int u0 = 0; u0 < (LONG ? nt : 1); u0 += kTriAhead) {
+            int c[kTriAhead];
+            T a[kTriAhead], yv[kTriAhead];
+#pragma unroll
+            for (int u = 0; u < kTriAhead; ++u) {
+                c[u] = u0 + u < nt ? column(u0 + u) : 0;
+                a[u] = u0 + u < nt ? value(base + 32LL * (u0 + u)) : T(0);
+            }
+#pragma unroll
+            for (int u = 0; u < kTriAhead; ++u)
+                yv[u] = u0 + u < nt ? (y ? y[c[u]] : D[c[u]] * f[c[u]]) : T(0);
+#pragma unroll
+            for (int u = 0; u < kTriAhead; ++u)
+                if (u0 + u < nt) acc = acc - a[u] * yv[u];
+        }
+        if constexpr (!LONG) {
+#pragma unroll 1
+            for (int u = kTriAhead; u < nt; ++u) {
+                const int j = column(u);
+                acc = acc - value(base + 32LL * u) * (y ? y[j] : D[j] * f[j]);
+            }
         }
         out[i] = fin(i, acc * di);
     }
@@ -966,17 +1035,17 @@ __device__ __forceinline__ void tri_jacobi(const Grid& g, const Mat<T>& m, const
 // k forward sweeps ping-pong between w and s (the last one stores the middle
 // vector), k backward sweeps between z and the other buffer, the last one
 // into z with `epi` (RowOp) fused.  No barrier after the last sweep.
-template <typename T, typename Epi>
-__device__ __forceinline__ Applied<T> ic_jacobi_apply(Grid& g, const Mat<T>& m, const T* D, const T* rhs, T* w, T* sb,
+template <bool LONG, typename T, typename Epi>
+__device__ __forceinline__ Applied<T> jacobi_apply(Grid& g, const Mat<T>& m, const T* D, const T* rhs, T* w, T* sb,
                                 T* z, int k, Epi epi) {
     T* fb[2] = {w, sb};
     for (int sw = 1; sw <= k; ++sw) {
         const T* y = sw == 1 ? nullptr : fb[(sw - 1) & 1];
         T* o = fb[sw & 1];
         if (sw < k)
-            tri_jacobi<true>(g, m, D, rhs, y, o, [](int, T v) { return v; });
+            tri_jacobi<true, LONG>(g, m, D, rhs, y, o, [](int, T v) { return v; });
         else
-            tri_jacobi<true>(g, m, D, rhs, y, o, [&](int i, T v) { return v / (D[i] + tiny_v<T>()); });
+            tri_jacobi<true, LONG>(g, m, D, rhs, y, o, [&](int i, T v) { return v / (D[i] + tiny_v<T>()); });
         if (!grid_sync(g, 23)) return {false, T(0)};
     }
     const T* mid = fb[k & 1];
@@ -985,16 +1054,21 @@ __device__ __forceinline__ Applied<T> ic_jacobi_apply(Grid& g, const Mat<T>& m, 
         const T* y = sw == 1 ? nullptr : bb[(k - sw + 1) & 1];
         T* o = bb[(k - sw) & 1];
         if (sw < k) {
-            tri_jacobi<false>(g, m, D, mid, y, o, [](int, T v) { return v; });
+            tri_jacobi<false, LONG>(g, m, D, mid, y, o, [](int, T v) { return v; });
             if (!grid_sync(g, 24)) return {false, T(0)};
         } else {
-            tri_jacobi<false>(g, m, D, mid, y, o, [&](int i, T v) {
+            tri_jacobi<false, LONG>(g, m, D, mid, y, o, [&](int i, T v) {
                 epi(i, v, rhs[i]);
                 return v;
             });
         }
     }
     return {true, epi.dot};
+}
+template <typename T, typename Epi>
+__device__ __noinline__ Applied<T> long_jacobi_apply(Grid& g, const Mat<T>& m, const T* D, const T* rhs, T* w,
+                                                     T* sb, T* z, int k, Epi epi) {
+    return jacobi_apply<true>(g, m, D, rhs, w, sb, z, k, epi);
 }
 
 // ---- tiled IC(0) sweeps (boxes) ------------------------------------------------
@@ -1624,9 +1698,10 @@ __device__ __forceinline__ Applied<T> ic_tiled_apply(Grid& g, const Mat<T>& m, c
     return a;
 }
 
-// On a box in another numbering.  A function of its own: the rows' look-up and
-// the order of their sums would cost the box numbering 4 to 7 % of an apply
-// (reference arithmetic, 109 x 83 x 97 cells: 527 -> 566 us per iteration).
+// On a box in another numbering, beside the box's own: a function, as the rows'
+// look-up and the order of their sums would cost the box numbering 4 to 7 % of
+// an apply (reference arithmetic, 109 x 83 x 97 cells: 527 -> 566 us per
+// iteration).
 template <typename L, typename T, typename Epi>
 __device__ __noinline__ Applied<T> ic_mapped_apply(Grid& g, const Mat<T>& m, const T* rhs, T* z, Epi epi) {
     return ic_tiled_apply<true, L>(g, m, rhs, z, epi);
@@ -1641,22 +1716,33 @@ template <int OP, typename T>
 __device__ __forceinline__ bool ic_precond(Grid& g, const Mat<T>& m, Vecs<T>& v, int sweeps,
                                            const T* rhs, T* z, T& dot, T alfa = T(0), T* x = nullptr) {
     const RowOp<OP, T> epi{alfa, x, T(0)};
-    Applied<T> a;
-    if (sweeps > 0) {
-        a = ic_jacobi_apply(g, m, v.D, rhs, v.w, v.s, z, sweeps, epi);
-    } else if (m.tile.on) {
-        if constexpr (sizeof(T) == 4) {
-            if (m.tile.row)
-                a = m.tile.lu_bf16 ? ic_mapped_apply<unsigned short>(g, m, rhs, z, epi)
-                                   : ic_mapped_apply<T>(g, m, rhs, z, epi);
+    Applied<T> a{false, T(0)};
+    if (kJacobiIc && (sweeps > 0 || !(kTiledIc || kLevelIc))) {
+        if constexpr (!kShortRows) a = long_jacobi_apply(g, m, v.D, rhs, v.w, v.s, z, sweeps, epi);
+        else if constexpr (kJacobiIc) a = jacobi_apply<false>(g, m, v.D, rhs, v.w, v.s, z, sweeps, epi);
+    } else if (kTiledIc && (!kLevelIc || m.tile.on)) {
+        if constexpr (kTiledIc && !kJacobiIc) {  // TFLOWS_FOR_MAPPED
+            if constexpr (sizeof(T) == 4)
+                a = m.tile.lu_bf16 ? ic_tiled_apply<true, unsigned short>(g, m, rhs, z, epi)
+                                   : ic_tiled_apply<true, T>(g, m, rhs, z, epi);
             else
-                a = m.tile.lu_bf16 ? ic_tiled_apply<false, unsigned short>(g, m, rhs, z, epi)
-                                   : ic_tiled_apply<false, T>(g, m, rhs, z, epi);
-        } else {
-            a = m.tile.row ? ic_mapped_apply<T>(g, m, rhs, z, epi) : ic_tiled_apply<false, T>(g, m, rhs, z, epi);
+                a = ic_tiled_apply<true, T>(g, m, rhs, z, epi);
+        } else if constexpr (kTiledIc) {
+            const bool mapped = kLevelIc && m.tile.row;
+            if constexpr (sizeof(T) == 4) {
+                if (mapped)
+                    a = m.tile.lu_bf16 ? ic_mapped_apply<unsigned short>(g, m, rhs, z, epi)
+                                       : ic_mapped_apply<T>(g, m, rhs, z, epi);
+                else
+                    a = m.tile.lu_bf16 ? ic_tiled_apply<false, unsigned short>(g, m, rhs, z, epi)
+                                       : ic_tiled_apply<false, T>(g, m, rhs, z, epi);
+            } else {
+                a = mapped ? ic_mapped_apply<T>(g, m, rhs, z, epi) : ic_tiled_apply<false, T>(g, m, rhs, z, epi);
+            }
         }
-    } else {
-        a = ic_apply(g, m, v.D, rhs, v.w, z, epi);
+    } else if constexpr (kLevelIc) {
+        if constexpr (kDiagPrec || sizeof(T) == 8) a = ic_apply(g, m, v.D, rhs, v.w, z, epi);
+        else a = level_apply(g, m, v.D, rhs, v.w, z, epi);
     }
     dot = a.dot;
     return a.ok;
@@ -1719,7 +1805,7 @@ __device__ __noinline__ bool prologue(Grid& g, const Mat<T>& m, Vecs<T>& v, cons
     }
     // (IC pivots complete: prec1_phase ends with a barrier; the barrier
     // below orders the tiled layout before the first apply)
-    if (cfg.do_prec1 && cfg.prec == 2 && m.tile.on) tiles_init(g, m, v.D);
+    if (kTiledIc && cfg.do_prec1 && cfg.prec == 2 && m.tile.on) tiles_init(g, m, v.D);
     T acc[1] = {T(0)};
     TF_FOR4(g, m, i) {
         const V4<T> r = ld4(v.r + i);
@@ -1778,10 +1864,13 @@ __device__ __noinline__ bool prologue(Grid& g, const Mat<T>& m, Vecs<T>& v, cons
 }
 
 // ---- CG (Process/CG.f90:113-259; also BiCG, whose iterates are CG's) --------
-template <typename T>
+// FUSE: the search direction formed inside the product, 1 always, 0 never, -1
+// as cfg.fuse_dir says (two forms of the product in one kernel).  PREC: the
+// preconditioner where the kernel has but one, -1 as prec_of says.
+template <int FUSE, int PREC, typename T>
 __device__ void cg_solve(Grid& g, const Mat<T>& m, Vecs<T>& v, const SolveCfg& cfg, SolveOut& out) {
     if (!prologue(g, m, v, cfg, out, true)) return;
-    const int prec = (cfg.prec == 1 || cfg.prec == 2) ? cfg.prec : 0;
+    const int prec = PREC < 0 ? prec_of(cfg.prec) : PREC;
     const T* z = prec == 0 ? v.r : v.z;
     bool nonfinite = false;
     int iter = 1;
@@ -1811,7 +1900,7 @@ __device__ void cg_solve(Grid& g, const Mat<T>& m, Vecs<T>& v, const SolveCfg& c
         // p and forming z + beta p per neighbour on the FP64 pipe costs more
         // than the pass it saves).
         T a1[1];
-        if (sizeof(T) == 4 || cfg.fuse_dir) {
+        if (FUSE < 0 ? cfg.fuse_dir != 0 : FUSE != 0) {
             T* const pnew = pnext;
             a1[0] = product_phase<T, true>(m, g.wg, g.nw, z, pcur, pnew, v.q, nullptr, beta, iter == 1);
             pnext = pcur;
@@ -1865,7 +1954,7 @@ __device__ void cgs_solve(Grid& g, const Mat<T>& m, Vecs<T>& v, const SolveCfg& 
     if (!prologue(g, m, v, cfg, out, false)) return;
     T beta = T(0);
     IterEnd e;
-    const int prec = (cfg.prec == 1 || cfg.prec == 2) ? cfg.prec : 0;
+    const int prec = prec_of(cfg.prec);
     // r2 = r1 (CGS.f90:84-86); rho = (r1, r2) for the first iteration.
     T a0[1] = {T(0)};
     TF_FOR4(g, m, i) {
@@ -2162,7 +2251,8 @@ __device__ __forceinline__ bool mixed_residual(Grid& g, const Mat<double>& m64, 
     return true;
 }
 
-static __device__ void mixed_solve(Grid& g, const Mat<double>& m64, const Mat<float>& m32, double* x64,
+template <bool CGS>
+__device__ __forceinline__ void mixed_solve(Grid& g, const Mat<double>& m64, const Mat<float>& m32, double* x64,
                             double* r64, const double* b64, double* D64, Vecs<float>& v32,
                             const MixedCfg& c, MixedOut& out) {
     out.exit_kind = EXIT_ABORT;
@@ -2188,7 +2278,7 @@ static __device__ void mixed_solve(Grid& g, const Mat<double>& m64, const Mat<fl
     publish<1>(g, SLOT_A, acc);
     if (!grid_sync(g, 71)) return;
     // (the residual pass below ends with a barrier before the first apply)
-    if (c.prec == 2 && m32.tile.on) tiles_init(g, m32, v32.D);
+    if (kTiledIc && c.prec == 2 && m32.tile.on) tiles_init(g, m32, v32.D);
     double tot[1], nrm[1];
     totals<1>(g, SLOT_A, tot, nrm, [](int, double s) { return sqrt(s); });
     const double bnrm2 = nrm[0];
@@ -2226,8 +2316,8 @@ static __device__ void mixed_solve(Grid& g, const Mat<double>& m64, const Mat<fl
         oi.exit_kind = 0;
         oi.iterations = 0;
         oi.fin_res = 0.0;
-        if (c.method == 2) cgs_solve<float>(g, m32, v32, ci, oi);
-        else cg_solve<float>(g, m32, v32, ci, oi);
+        if constexpr (CGS) cgs_solve<float>(g, m32, v32, ci, oi);
+        else cg_solve<1, -1>(g, m32, v32, ci, oi);
         if (oi.exit_kind == EXIT_ABORT) return;
         total += oi.exit_kind == EXIT_MAXITER || oi.exit_kind == EXIT_NONFINITE ? ci.maxiter
                                                                                  : oi.iterations;
@@ -2291,7 +2381,7 @@ static __device__ __noinline__ bool product_apart(Grid& g, const Mat<float>& m, 
                                                   float* q, float beta, bool first, float& sum) {
     direction_phase(g.tid, g.nt, m.n, z, p, beta, first);
     if (!grid_sync(g, 84)) return false;
-    sum = product_columns<float, false>(m, g.wg, g.nw, nullptr, p, nullptr, q, p, 0.0f, false);
+    sum = columns_loop<float, false>(m, g.wg, g.nw, nullptr, p, nullptr, q, p, 0.0f, false);
     return true;
 }
 
@@ -2302,12 +2392,12 @@ static __device__ __noinline__ bool product_apart(Grid& g, const Mat<float>& m, 
 // values, the convergence test ||r|| < tol is made on it in FP64, and the
 // FP32 residual is replaced by it.  Unlike a restarted refinement the search
 // direction is kept, so the iteration count stays close to the FP64 solve's.
-static __device__ void mixed_cg_reliable(Grid& g, const Mat<double>& m64, const Mat<float>& m32,
+static __device__ __forceinline__ void mixed_cg_reliable(Grid& g, const Mat<double>& m64, const Mat<float>& m32,
                                   double* x64, double* r64, const double* b64, double* D64,
                                   double* xbest, Vecs<float>& v, const MixedCfg& c,
                                   MixedOut& out) {
     out.exit_kind = EXIT_ABORT;
-    const int prec = (c.prec == 1 || c.prec == 2) ? c.prec : 0;
+    const int prec = prec_of(c.prec);
     if (!prec1_phase(g, m64, D64, c.prec)) return;
     if (!grid_sync(g, 80)) return;
     double acc[1] = {0.0};
@@ -2327,7 +2417,7 @@ static __device__ void mixed_cg_reliable(Grid& g, const Mat<double>& m64, const 
     }
     publish<1>(g, SLOT_A, acc);
     if (!grid_sync(g, 81)) return;
-    if (c.prec == 2 && m32.tile.on) tiles_init(g, m32, v.D);
+    if (kTiledIc && c.prec == 2 && m32.tile.on) tiles_init(g, m32, v.D);
     double tot[1], nrm[1];
     totals<1>(g, SLOT_A, tot, nrm, [](int, double s) { return sqrt(s); });
     const double bnrm2 = nrm[0];
@@ -2421,7 +2511,7 @@ static __device__ void mixed_cg_reliable(Grid& g, const Mat<double>& m64, const 
     for (; it <= c.maxiter; ++it) {
         const bool along = it == 1 || fresh;  // p = z
         float a1[1];
-        if (c.fuse_dir) {
+        if (!kApart || c.fuse_dir) {
             // the direction formed inside the product, into the other buffer
             a1[0] = product_phase<float, true>(m32, g.wg, g.nw, z, pcur, pnext, v.q, nullptr, beta, along);
             float* const pold = pcur;

@@ -1,0 +1,23 @@
+// As krylov_long.cu, with fused multiply-adds and a reciprocal diagonal:
+// TFLOWS_FP64_FMA and the mixed solves.
+#define TFLOWS_KNS fma_long
+#define TFLOWS_FP64_RECIP_DIAG 1
+#define TFLOWS_FOR_LONG 1
+#include "internal.h"
+#include "solver_entry.cuh"
+
+namespace tflows {
+
+const void* fma_long_kernel(KernelId id) {
+    switch (id) {
+        case KernelId::Cg:
+        case KernelId::CgFused: return (const void*)fma_long::krylov_kernel<double, 4>;
+        case KernelId::Cgs: return (const void*)fma_long::krylov_kernel<double, 2>;
+        case KernelId::MixedRestart: return (const void*)fma_long::mixed_kernel<0>;
+        case KernelId::MixedReliable: return (const void*)fma_long::mixed_kernel<1>;
+        case KernelId::MixedCgs: return (const void*)fma_long::mixed_kernel<2>;
+        default: return nullptr;
+    }
+}
+
+}  // namespace tflows

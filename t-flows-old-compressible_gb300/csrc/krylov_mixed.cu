@@ -1,7 +1,6 @@
 // Kernels of the mixed-precision solves (FP32 inner iterations, FP64
-// refinement), compiled with fused multiply-adds (--fmad=true) and a
-// reciprocal diagonal; they make no bitwise claim.  A unit of its own, so that
-// it compiles beside krylov_fma.cu.
+// refinement) with tiled or Jacobi-sweep IC(0), compiled with fused multiply-adds (--fmad=true) and a
+// reciprocal diagonal; they make no bitwise claim.
 #define TFLOWS_KNS fma
 #define TFLOWS_FP64_RECIP_DIAG 1
 #include "internal.h"
@@ -13,7 +12,9 @@ const void* mixed_kernel(KernelId id) {
     switch (id) {
         case KernelId::MixedRestart: return (const void*)fma::mixed_kernel<0>;
         case KernelId::MixedReliable: return (const void*)fma::mixed_kernel<1>;
-        default: return mixed_batch_kernel(id);
+        case KernelId::MixedCgs: return (const void*)fma::mixed_kernel<2>;
+        case KernelId::BatchReliable: return (const void*)fma::batch_kernel<2>;
+        default: return nullptr;
     }
 }
 

@@ -1,13 +1,15 @@
 // Kernel entry points of the persistent solvers and their parameter blocks.
 //
 // Included by translation units that compile the same solver code with
-// different arithmetic: krylov.cu (namespace tflows::ref) with --fmad=false,
-// where every a*b+c is a rounded product followed by a rounded sum and the
-// diagonal preconditioner divides, as the reference does; krylov_fma.cu and
-// krylov_mixed.cu (namespace tflows::fma) with contraction
-// into fused multiply-adds and a reciprocal diagonal, for the TFLOWS_FP64_FMA
-// solves and the mixed-precision solves.  The parameter blocks are shared types; the kernels of each unit
-// live in its own namespace so that the two builds never merge.
+// different arithmetic and for different solves: krylov.cu (namespace
+// tflows::ref) with --fmad=false, where every a*b+c is a rounded product
+// followed by a rounded sum and the diagonal preconditioner divides, as the
+// reference does; krylov_fma.cu and krylov_mixed.cu (namespace tflows::fma)
+// with contraction into fused multiply-adds and a reciprocal diagonal, for the
+// TFLOWS_FP64_FMA solves and the mixed-precision solves; and the _diag, _level,
+// _mapped, _long and _batch units (krylov_kernels.cuh: TFLOWS_FOR_DIAG and the others).
+// The parameter blocks are shared types; the kernels of each unit live in its
+// own namespace so that the builds never merge.
 #pragma once
 
 #include "krylov_kernels.cuh"
@@ -82,7 +84,9 @@ static __device__ int status_of(const SolveOut& o, const DevCtl* ctl) {
     }
 }
 
-// METHOD: 0 CG (and BiCG), 2 CGS, 3 true BiCG, 9 Prec1 only, 8 the IC(0)
+// METHOD: 0 CG (and BiCG), 1 CG with the search direction formed inside the
+// product, 4 either (SolveCfg), 5 and 6 as 0 and 1 without a preconditioner
+// (TFLOWS_FOR_DIAG, where 0 and 1 are with the diagonal), 2 CGS, 3 true BiCG, 9 Prec1 only, 8 the IC(0)
 // pivots (Prec1 prec 2) and one apply z = M^-1 r (v.r in, v.z out).
 template <typename T, int METHOD>
 __global__ void __launch_bounds__(kMaxBlock, kMinBlocksAtMax) krylov_kernel(KParams<T> P) {
@@ -112,7 +116,8 @@ __global__ void __launch_bounds__(kMaxBlock, kMinBlocksAtMax) krylov_kernel(KPar
     } else if (METHOD == 3) {
         bicg_true_solve(g, P.m, P.mT, P.v, P.cfg, out);
     } else {
-        cg_solve(g, P.m, P.v, P.cfg, out);
+        constexpr int kPrec = METHOD == 5 || METHOD == 6 ? 0 : kDiagPrec && !kJacobiIc ? 1 : -1;
+        cg_solve<METHOD == 4 ? -1 : METHOD == 1 || METHOD == 6, kPrec>(g, P.m, P.v, P.cfg, out);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         DevState* s = P.state;
@@ -146,7 +151,7 @@ __global__ void __launch_bounds__(kMaxBlock, kMinBlocksAtMax) mixed_kernel(Mixed
         mixed_cg_reliable(g, P.m64, P.m32, P.x64, P.r64, P.b64, P.D64, P.xbest, P.v32, P.cfg,
                           out);
     else
-        mixed_solve(g, P.m64, P.m32, P.x64, P.r64, P.b64, P.D64, P.v32, P.cfg, out);
+        mixed_solve<KIND == 2>(g, P.m64, P.m32, P.x64, P.r64, P.b64, P.D64, P.v32, P.cfg, out);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         DevState* s = P.state;
         SolveOut o;
@@ -166,6 +171,8 @@ __global__ void __launch_bounds__(kMaxBlock, kMinBlocksAtMax) mixed_kernel(Mixed
 
 // ---- batched solves: one cooperative launch, one block group per system ------
 
+// MIXED: 0 FP64 systems, 1 mixed ones, 2 mixed ones that are all CG or BiCG
+// with reliable updates.
 template <int MIXED>
 __global__ void __launch_bounds__(kMaxBlock, kMinBlocksAtMax)
     batch_kernel(const BatchItem* __restrict__ items, const int* __restrict__ block_item) {
@@ -182,7 +189,7 @@ __global__ void __launch_bounds__(kMaxBlock, kMinBlocksAtMax)
         out.fin_res = 0.0;
         out.bnrm2 = 0.0;
         if (it.method == 2) cgs_solve(g, P.m, P.v, P.cfg, out);
-        else cg_solve(g, P.m, P.v, P.cfg, out);
+        else cg_solve<-1, -1>(g, P.m, P.v, P.cfg, out);
         if (g.bid == 0 && threadIdx.x == 0) {
             DevState* s = P.state;
             s->status = status_of(out, P.ctl);
@@ -207,11 +214,16 @@ __global__ void __launch_bounds__(kMaxBlock, kMinBlocksAtMax)
         out.fin_res = 0.0;
         out.bnrm2 = 0.0;
         // the refinement the system asked for, as in its single-system solve
-        if (it.method != 2 && !P.cfg.restart)
+        if (MIXED == 2)
             mixed_cg_reliable(g, P.m64, P.m32, P.x64, P.r64, P.b64, P.D64, P.xbest, P.v32, P.cfg,
                               out);
+        else if (it.method == 2)
+            mixed_solve<true>(g, P.m64, P.m32, P.x64, P.r64, P.b64, P.D64, P.v32, P.cfg, out);
+        else if (P.cfg.restart)
+            mixed_solve<false>(g, P.m64, P.m32, P.x64, P.r64, P.b64, P.D64, P.v32, P.cfg, out);
         else
-            mixed_solve(g, P.m64, P.m32, P.x64, P.r64, P.b64, P.D64, P.v32, P.cfg, out);
+            mixed_cg_reliable(g, P.m64, P.m32, P.x64, P.r64, P.b64, P.D64, P.xbest, P.v32, P.cfg,
+                              out);
         if (g.bid == 0 && threadIdx.x == 0) {
             DevState* s = P.state;
             SolveOut o;
