@@ -195,8 +195,7 @@ bool tiles_wanted(const SolveRequest& rq);
 // 512 (16.8 of 256, 15.4 in 304 of 512), 24.7 at 96^3 and 44 at 128^3 in 304
 // of 512 (28.8 and 57 in 152).  The tiled sweeps take 512 threads
 // (four patches a block: one apply at 256^3, FP32, 529 us in two such blocks
-// per SM, 582 in four of 256), the level sweeps one block per SM (898 against
-// 1063 us per iteration at 140,000 rows, 1667 against 1828 at 720,000).
+// per SM, 582 in four of 256); the level sweeps blocks of 256 (level_blocks).
 void default_shape(const DeviceTopology& t, SolveRequest& rq);
 unsigned tile_smem_for(const DeviceTopology& t, const SolveRequest& rq);
 cudaError_t ensure_tiles(const DeviceTopology& t, Workspace& ws, const SolveRequest& rq);

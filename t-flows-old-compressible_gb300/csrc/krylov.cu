@@ -528,6 +528,22 @@ bool level_ic(const DeviceTopology& t, const SolveRequest& rq) {
     return rq.prec == 2 && rq.ic_sweeps == 0 && !tiled_ic(t, rq);
 }
 
+// Blocks of 256 threads per SM for level-ordered IC(0).  A sweep hands over
+// from level to level, so narrow levels want few warps that poll; wide levels
+// and the vector passes between the sweeps want them all.  Measured, us per
+// iteration with 1 / 2 / 4 blocks per SM, by rows per level: L-shaped meshes,
+// 970: FP64 801 / 832 / 930, mixed 485 / 508 / 542; 4960: 2109 / 2148 / 2226,
+// 1312 / 1319 / 1348; 7730: 2793 / 2937 / 2910, 1844 / 1745 / 1774; 12,060
+// (42 million entries): 3938 / 3937 / 4012, 2868 / 2413 / 2435; 15 entries a
+// row, 3310 (31 million): 6067 / 5744 / 5933, 4716 / 4473 / 4428; random
+// numberings, 14,600: 176 / 171 / 190, 138 / 124 / 131; 38,400: 371 / 285 /
+// 266, 282 / 212 / 194; 110,000: 1077 / 685 / 594, 819 / 518 / 412.
+int level_blocks(const DeviceTopology& t, const SolveRequest& rq) {
+    const double rows = t.nlev_f > 0 ? 32.0 * t.nchunk_f / t.nlev_f : 0.0;  // per level
+    if (rows >= 20000) return 4;
+    return t.nnz > 25 * 1000 * 1000 || (rq.precision == 1 && rows >= 5000) ? 2 : 1;
+}
+
 void default_shape(const DeviceTopology& t, SolveRequest& rq) {
     if (rq.block > 0) return;
     const bool tiled = tiled_ic(t, rq);
@@ -539,7 +555,9 @@ void default_shape(const DeviceTopology& t, SolveRequest& rq) {
         // one row per thread while one block per SM holds them
         if (t.n > kBlock * sms()) rq.block = kMaxBlock;
         rq.grid = std::min(blocks_for(t.nslices, block_of(rq)), (t.n <= 600 * 1000 ? 1 : 2) * sms());
-    } else if (t.n <= 150 * 1000 || (rq.prec == 2 && rq.ic_sweeps == 0)) {
+    } else if (level_ic(t, rq)) {
+        rq.grid = std::min(blocks_for(t.nslices), level_blocks(t, rq) * sms());
+    } else if (t.n <= 150 * 1000) {
         rq.grid = std::min(blocks_for(t.nslices), sms());
     } else {
         rq.block = kMaxBlock;
