@@ -54,10 +54,8 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 // Control block shared by all blocks of one persistent launch.
 struct DevCtl {
     unsigned long long bar;  // monotonically increasing arrival counter; kBarAbort once aborted
-    int abort;               // set by whoever gives up; every wait checks it
     int status;              // first error status raised
     int where;
-    int pad;
 };
 
 // Wait limits are measured in SM clock cycles (clock64: monotonic and local
@@ -90,21 +88,17 @@ __device__ __forceinline__ void red_release_add_u64(unsigned long long* p, unsig
     asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// Raise an abort: first status wins; everyone polling `abort` leaves, and so
-// does every barrier, whose counter the bit lifts past any target.  The bit
-// comes first: a warp that has left a wait for the flag (read with acquire) is
-// then met by a barrier that fails for its whole block.
+// Raise an abort: first status wins.  One bit of the barrier's counter ends
+// every barrier, as it lifts the counter past any target, and every other wait,
+// which polls the same word: a warp that has left a wait for it is met by a
+// barrier that fails for its whole block.
 constexpr unsigned long long kBarAbort = 1ull << 62;
 __device__ __forceinline__ void raise_abort(DevCtl* c, int status, int where) {
     if (atomicCAS(&c->status, 0, status) == 0) c->where = where;
     atomicOr(&c->bar, kBarAbort);
-    __threadfence();
-    atomicExch(&c->abort, 1);
 }
 __device__ __forceinline__ bool aborted(const DevCtl* c) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(&c->abort) : "memory");
-    return v != 0;
+    return (unsigned long long)ld_relaxed_s64(reinterpret_cast<const long long*>(&c->bar)) >= kBarAbort;
 }
 
 // ---- asynchronous copies global -> shared (per thread, in commit groups) ----------
