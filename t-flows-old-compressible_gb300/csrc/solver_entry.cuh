@@ -188,8 +188,14 @@ __global__ void __launch_bounds__(kMaxBlock, kMinBlocksAtMax)
         out.ini_res = 0.0;
         out.fin_res = 0.0;
         out.bnrm2 = 0.0;
-        if (it.method == 2) cgs_solve(g, P.m, P.v, P.cfg, out);
-        else cg_solve<-1, -1>(g, P.m, P.v, P.cfg, out);
+        if (it.method == 2)
+            cgs_solve(g, P.m, P.v, P.cfg, out);
+        else if (kDiagPrec && !kJacobiIc && P.cfg.prec == 1 && P.cfg.fuse_dir)  // TFLOWS_FOR_DIAG
+            cg_solve<1, 1>(g, P.m, P.v, P.cfg, out);
+        else if (kDiagPrec && !kJacobiIc && P.cfg.prec == 1)
+            cg_solve<0, 1>(g, P.m, P.v, P.cfg, out);
+        else
+            cg_solve<-1, kDiagPrec && !kJacobiIc ? 0 : -1>(g, P.m, P.v, P.cfg, out);
         if (g.bid == 0 && threadIdx.x == 0) {
             DevState* s = P.state;
             s->status = status_of(out, P.ctl);
