@@ -1144,7 +1144,8 @@ def main():
                           else f"{args.ic_sweeps} Jacobi sweeps per triangle")
                        if prec == 2 else ""),
         "launch": ({"autotuned": True, **tuning} if tuning else
-                   {"autotuned": False, "block_size": 256}),
+                   {"autotuned": False, "block_size": last["block_size"],
+                    "grid_blocks": last["grid_blocks"]}),
         "iterations": last["inner_iterations"] if mixed else last["iterations"],
         "refinements": last["refinements"] if mixed else None,
         "fin_res": last["fin_res"], "tol": s.tol,

@@ -1,6 +1,6 @@
-// Kernels and launchers of libtflows_krylov.so.
-// Kernels of the reference-arithmetic build (--fmad=false) and the host
-// side of every solve, batched launch and plan.
+// Kernels and launchers of libtflows_krylov.so: the solvers in reference
+// arithmetic (--fmad=false) with tiled or Jacobi-sweep IC(0), the small kernels
+// around them, and the host side of every solve, batched launch and plan.
 #define TFLOWS_KNS ref
 #include "internal.h"
 #include "solver_entry.cuh"

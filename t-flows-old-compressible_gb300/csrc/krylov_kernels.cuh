@@ -714,8 +714,6 @@ __device__ __forceinline__ T diag_value(const Mat<T>& m, int i) {
 // which sit in chunks of lower index, so with all warps resident the sweep
 // cannot deadlock.
 constexpr int kSweepMax = 8;  // dependencies prefetched per row
-// Longest pause between polls of not-yet-ready cells, in ns (0: poll back to
-// back).
 // Warps taking part in a sweep: at most `per_chunk` (a tuning parameter,
 // default 4) per chunk of the widest level, so that a warp's next chunk is
 // only a few levels ahead of the front and its polls rarely spin long.
