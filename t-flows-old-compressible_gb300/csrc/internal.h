@@ -229,7 +229,7 @@ int halo_resid(int n, int nb, int nonz, const double* A, const int* Acol, const 
 // krylov_mixed.cu fused multiply-adds (TFLOWS_FP64_FMA; the mixed solves); the
 // _diag, _level, _mapped, _long and _batch units have the same solvers for what their
 // names say (krylov_kernels.cuh).  Null where a unit has no such kernel.
-enum class KernelId { Cg, CgFused, CgNone, CgNoneFused, Cgs, BicgTrue, Prec1, IcApply, MixedRestart, MixedReliable, MixedCgs,
+enum class KernelId { Cg, CgFused, CgNone, CgNoneFused, Cgs, BicgTrue, Prec1, IcApply, MixedRestart, MixedReliable, MixedApart, MixedCgs,
                       BatchFp64, BatchMixed, BatchReliable };
 const void* ref_kernel(KernelId id);
 const void* fma_kernel(KernelId id);

@@ -462,6 +462,12 @@ bool fuse_dir_fp64(const DeviceTopology& t, const SolveRequest& rq) {
 // 127 / 87 at 2.1 million.
 bool fuse_dir_mixed(const DeviceTopology& t) { return t.spat || t.n <= 500 * 1000; }
 
+// Without IC(0) the pass of its own is the better one on large systems whatever
+// their columns, with a kernel that has no other form: us per iteration of a
+// diagonal CG inside / as a pass, 128^3 50.8 / 47.1, 160^3 102 / 93, 200^3 191 /
+// 181, 240^3 327 / 310 (322 with both preconditioners in one kernel).
+bool apart_mixed(const DeviceTopology& t) { return t.n > 1500 * 1000; }
+
 // Patches per tile: as many as the block has warps for, up to four, whose
 // shared memory fits an SM twice (one apply at 128^3, FP32: 190 us with four,
 // 220 with two, 240 with one: every tile edge costs a hand-over through L2).
@@ -744,7 +750,7 @@ double solve_bytes(const DeviceTopology& t, const SolveRequest& rq, const DevSta
         // p and q written once) but for some reliable-update solves; the
         // product's own vector read and write are then part of the 4·N·12
         // (resp. 10) vector bytes
-        const bool fused = rq.refine_restart || fuse_dir_mixed(t) || tiled;
+        const bool fused = rq.refine_restart || tiled || (fuse_dir_mixed(t) && (rq.prec == 2 || !apart_mixed(t)));
         const double inner_it = cgs ? 2 * spmv32 + 4.0 * t.n * 22 + 2 * ic
                                     : spmv32 - (fused ? 8.0 * t.n : 0.0) + 4.0 * t.n * (rq.prec == 1 ? 12 : 10) + ic;
         return inner_it * st.inner_iters + (spmv64 + 8.0 * t.n * 4) * (st.refinements + 1);
@@ -854,6 +860,7 @@ const void* kernel_of(const DeviceTopology& t, const SolveRequest& rq, KernelId 
     const Unit u = unit_of(t, rq);
     if (u == Unit::Diag && rq.prec != 1)
         id = id == KernelId::Cg ? KernelId::CgNone : id == KernelId::CgFused ? KernelId::CgNoneFused : id;
+    if (u == Unit::Diag && id == KernelId::MixedReliable && apart_mixed(t)) id = KernelId::MixedApart;
     return unit_kernel(u, rq.precision, id);
 }
 

@@ -18,6 +18,7 @@ const void* fma_diag_kernel(KernelId id) {
         case KernelId::BicgTrue: return (const void*)fma_diag::krylov_kernel<double, 3>;
         case KernelId::MixedRestart: return (const void*)fma_diag::mixed_kernel<0>;
         case KernelId::MixedReliable: return (const void*)fma_diag::mixed_kernel<1>;
+        case KernelId::MixedApart: return (const void*)fma_diag::mixed_kernel<3>;
         case KernelId::MixedCgs: return (const void*)fma_diag::mixed_kernel<2>;
         case KernelId::BatchFp64: return (const void*)fma_diag::batch_kernel<0>;
         case KernelId::BatchReliable: return (const void*)fma_diag::batch_kernel<2>;

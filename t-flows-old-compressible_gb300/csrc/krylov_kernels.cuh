@@ -953,8 +953,9 @@ __device__ __noinline__ Applied<T> ic_apply(Grid& g, const Mat<T>& m, const T* D
 // are loaded together and a loop takes the rest (the FP64 pipe also does what
 // a predicate turns off); LONG: four at a time, which costs a box 6 % (128^3
 // rows of 15 entries, one sweep per triangle, mixed: 481 -> 262 us with the
-// products of such rows).  Inlined: as a function of its own it cost FP32 2 to
-// 3 %.  A CG iteration with one / two sweeps per triangle, 161 x 150 x 170
+// products of such rows).  FP32: a function of its own (inlined beside the tiled
+// sweeps, 240^3 cells took 809 us per iteration, so 750; two sweeps 1383 and
+// 1264).  A CG iteration with one / two sweeps per triangle, 161 x 150 x 170
 // cells, against eight entries and explicit columns in 608 blocks of 256:
 // FP32 269 -> 260 / 395 -> 389 us, multiply-adds 473 -> 361 / 670 -> 505.
 constexpr int kTriAhead = 4;
@@ -1058,10 +1059,10 @@ __device__ __forceinline__ Applied<T> jacobi_apply(Grid& g, const Mat<T>& m, con
     }
     return {true, epi.dot};
 }
-template <typename T, typename Epi>
-__device__ __noinline__ Applied<T> long_jacobi_apply(Grid& g, const Mat<T>& m, const T* D, const T* rhs, T* w,
-                                                     T* sb, T* z, int k, Epi epi) {
-    return jacobi_apply<true>(g, m, D, rhs, w, sb, z, k, epi);
+template <bool LONG, typename T, typename Epi>
+__device__ __noinline__ Applied<T> jacobi_function(Grid& g, const Mat<T>& m, const T* D, const T* rhs, T* w, T* sb,
+                                                   T* z, int k, Epi epi) {
+    return jacobi_apply<LONG>(g, m, D, rhs, w, sb, z, k, epi);
 }
 
 // ---- tiled IC(0) sweeps (boxes) ------------------------------------------------
@@ -1711,7 +1712,8 @@ __device__ __forceinline__ bool ic_precond(Grid& g, const Mat<T>& m, Vecs<T>& v,
     const RowOp<OP, T> epi{alfa, x, T(0)};
     Applied<T> a{false, T(0)};
     if (kJacobiIc && (sweeps > 0 || !(kTiledIc || kLevelIc))) {
-        if constexpr (!kShortRows) a = long_jacobi_apply(g, m, v.D, rhs, v.w, v.s, z, sweeps, epi);
+        if constexpr (!kShortRows) a = jacobi_function<true>(g, m, v.D, rhs, v.w, v.s, z, sweeps, epi);
+        else if constexpr (sizeof(T) == 4) a = jacobi_function<false>(g, m, v.D, rhs, v.w, v.s, z, sweeps, epi);
         else if constexpr (kJacobiIc) a = jacobi_apply<false>(g, m, v.D, rhs, v.w, v.s, z, sweeps, epi);
     } else if (kTiledIc && (!kLevelIc || m.tile.on)) {
         if constexpr (kTiledIc && !kJacobiIc) {  // TFLOWS_FOR_MAPPED
@@ -2384,7 +2386,8 @@ static __device__ __noinline__ bool product_apart(Grid& g, const Mat<float>& m, 
 // values, the convergence test ||r|| < tol is made on it in FP64, and the
 // FP32 residual is replaced by it.  Unlike a restarted refinement the search
 // direction is kept, so the iteration count stays close to the FP64 solve's.
-static __device__ __forceinline__ void mixed_cg_reliable(Grid& g, const Mat<double>& m64, const Mat<float>& m32,
+template <bool APART>
+__device__ __forceinline__ void mixed_cg_reliable(Grid& g, const Mat<double>& m64, const Mat<float>& m32,
                                   double* x64, double* r64, const double* b64, double* D64,
                                   double* xbest, Vecs<float>& v, const MixedCfg& c,
                                   MixedOut& out) {
@@ -2503,7 +2506,11 @@ static __device__ __forceinline__ void mixed_cg_reliable(Grid& g, const Mat<doub
     for (; it <= c.maxiter; ++it) {
         const bool along = it == 1 || fresh;  // p = z
         float a1[1];
-        if (!kApart || c.fuse_dir) {
+        if (APART) {
+            direction_phase(g.tid, g.nt, m32.n, z, pcur, beta, along);
+            if (!grid_sync(g, 84)) return;
+            a1[0] = product_phase<float, false>(m32, g.wg, g.nw, nullptr, pcur, nullptr, v.q, pcur, 0.0f, false);
+        } else if (!kApart || c.fuse_dir) {
             // the direction formed inside the product, into the other buffer
             a1[0] = product_phase<float, true>(m32, g.wg, g.nw, z, pcur, pnext, v.q, nullptr, beta, along);
             float* const pold = pcur;

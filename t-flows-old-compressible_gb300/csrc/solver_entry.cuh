@@ -134,7 +134,8 @@ __global__ void __launch_bounds__(kMaxBlock, kMinBlocksAtMax) krylov_kernel(KPar
 }
 
 
-// KIND: 0 restarted CG, 2 restarted CGS, 1 CG with reliable updates.
+// KIND: 0 restarted CG, 2 restarted CGS, 1 CG with reliable updates, 3 the
+// same with the search direction in a pass of its own (TFLOWS_FOR_DIAG).
 template <int KIND>
 __global__ void __launch_bounds__(kMaxBlock, kMinBlocksAtMax) mixed_kernel(MixedParams P) {
     Grid g;
@@ -147,8 +148,8 @@ __global__ void __launch_bounds__(kMaxBlock, kMinBlocksAtMax) mixed_kernel(Mixed
     out.ini_res = 0.0;
     out.fin_res = 0.0;
     out.bnrm2 = 0.0;
-    if (KIND == 1)
-        mixed_cg_reliable(g, P.m64, P.m32, P.x64, P.r64, P.b64, P.D64, P.xbest, P.v32, P.cfg,
+    if (KIND == 1 || KIND == 3)
+        mixed_cg_reliable<KIND == 3>(g, P.m64, P.m32, P.x64, P.r64, P.b64, P.D64, P.xbest, P.v32, P.cfg,
                           out);
     else
         mixed_solve<KIND == 2>(g, P.m64, P.m32, P.x64, P.r64, P.b64, P.D64, P.v32, P.cfg, out);
@@ -221,14 +222,14 @@ __global__ void __launch_bounds__(kMaxBlock, kMinBlocksAtMax)
         out.bnrm2 = 0.0;
         // the refinement the system asked for, as in its single-system solve
         if (MIXED == 2)
-            mixed_cg_reliable(g, P.m64, P.m32, P.x64, P.r64, P.b64, P.D64, P.xbest, P.v32, P.cfg,
+            mixed_cg_reliable<false>(g, P.m64, P.m32, P.x64, P.r64, P.b64, P.D64, P.xbest, P.v32, P.cfg,
                               out);
         else if (it.method == 2)
             mixed_solve<true>(g, P.m64, P.m32, P.x64, P.r64, P.b64, P.D64, P.v32, P.cfg, out);
         else if (P.cfg.restart)
             mixed_solve<false>(g, P.m64, P.m32, P.x64, P.r64, P.b64, P.D64, P.v32, P.cfg, out);
         else
-            mixed_cg_reliable(g, P.m64, P.m32, P.x64, P.r64, P.b64, P.D64, P.xbest, P.v32, P.cfg,
+            mixed_cg_reliable<false>(g, P.m64, P.m32, P.x64, P.r64, P.b64, P.D64, P.xbest, P.v32, P.cfg,
                               out);
         if (g.bid == 0 && threadIdx.x == 0) {
             DevState* s = P.state;
