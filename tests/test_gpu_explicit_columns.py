@@ -1,7 +1,9 @@
-"""Mixed solves on both sides of the size at which explicit columns take the
-search direction out of the product: each reaches its FP64 tolerance, in as
-many iterations as the same system with column patterns (to a quarter: the
-rounding of the reductions decides when a direction is restarted)."""
+"""Mixed solves on both sides of the sizes at which the search direction leaves
+the product (500,000 rows with explicit columns, 1.5 million with any): each
+reaches its FP64 tolerance, in as many iterations as the same system with column
+patterns (to a quarter: the rounding of the reductions decides when a direction
+is restarted)."""
+import functools
 import os
 
 import numpy as np
@@ -13,11 +15,17 @@ mesh = tflows.mesh
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("dims", [(80, 80, 78), (80, 80, 79)])  # 499,200 and 505,600 rows
+@functools.lru_cache(maxsize=1)
+def _pressure(dims):
+    return mesh.pressure_system(*dims, perturb=0.2, seed=3, variable_density=True)
+
+
+# 499,200, 505,600, 1,494,425 and 1,507,650 rows
+@pytest.mark.parametrize("dims", [(80, 80, 78), (80, 80, 79), (115, 115, 113), (115, 115, 114)])
 @pytest.mark.parametrize("prec,kw", [(0, {}), (1, {}), (1, {"refine_restart": 1}), (2, {"ic_sweeps": 1})])
 def test_mixed_solves(dims, prec, kw):
     import torch
-    s = mesh.pressure_system(*dims, perturb=0.2, seed=3, variable_density=True)
+    s = _pressure(dims)
     val, b = torch.from_numpy(s.A[:-1].copy()).cuda(), torch.from_numpy(s.b).cuda()
     tol = 1e-8 * float(np.linalg.norm(s.b))
     its = {}
